@@ -134,7 +134,8 @@ typedef struct tdc_start_stats {
     int path;             /* tdc_path used */
     int kernel_launches;  /* launches of this library's kernels inside start() */
     int stage_samples;    /* samples of a chirp row per pipeline stage of the FP32 kernels
-                             (the whole row, or one segment of a long row; 0 on FP64 paths) */
+                             (the whole row, or one segment of a long row; 0 on FP64 paths and where
+                             the FP32-bulk path focuses through range profiles, which stage no rows) */
     int stage_chirps;     /* chirp rows per pipeline stage (1 when rows are staged in segments) */
     int general_variant;  /* FP32 general kernel variant bits (1 per-sample positions, 2 per-sample
                              windows, 4 wide phase correction); 0 on the other paths */
@@ -144,7 +145,8 @@ typedef struct tdc_start_stats {
     int adjoint_stored;   /* the last adjoint read the kept per-chirp sums (1) or recomputed them (0) */
     int motion_segment;   /* smooth-motion path: samples per linearised segment; 0 on the other paths */
     int anchor_pixels;    /* FP32-bulk path with anchored ranges: consecutive pixels sharing one anchor
-                             (32); 0 when every pixel's range is formed in double-float */
+                             (32; 8, 4 or 2 through range profiles); 0 when every pixel's range is formed
+                             in double-float */
     int span_permille;    /* chirps the work units visit, per mille of tiles x chirps: below 1000 when a
                              finite Doppler band lets units skip chirps out of band for their whole tile */
 } tdc_start_stats;
@@ -188,7 +190,12 @@ int tdc_processor_set_plan_pixels(tdc_processor *proc, int64_t n_pix);
  * next focus. */
 int tdc_processor_set_motion_path(tdc_processor *proc, int enable);
 
-/* Anchored ranges in the FP32-bulk kernel on (1, default) or off (0). With an unbounded Doppler
+/* Large focuses on the FP32-bulk path (at least 5e8 correlations and 4 pixels a sample, an
+ * unbounded Doppler band) read each (pixel, chirp) sum from a table of the chirp's spectrum
+ * over the grid's ranges instead of adding up its samples (range profiles): the same sums to
+ * FP32 rounding, at a cost that does not grow with the row's length.
+ *
+ * Anchored ranges in the FP32-bulk kernel on (1, default) or off (0). With an unbounded Doppler
  * band, finite velocities, no kept per-chirp sums and rows of 3-16 chirps per pipeline stage
  * (about 128-700 samples), groups of 32 consecutive pixels share an anchor pixel whose
  * range and phase terms are formed in double-float once per chirp; each pixel adds its range
@@ -196,7 +203,8 @@ int tdc_processor_set_motion_path(tdc_processor *proc, int enable);
  * Taken only when no pixel lies farther than 5 cm from its anchor (grids whose rows are a
  * multiple of 32 pixels, or narrower than 5 cm, at up to 3 mm spacing), which keeps each
  * (pixel, chirp) phase within about 3e-5 rad of the per-pixel double-float range's at 77 GHz
- * (1e-5 rad on 1 mm grids). Off: every (pixel, chirp) range in double-float. Extension without
+ * (1e-5 rad on 1 mm grids). Through range profiles groups of 8, 4 or 2 consecutive pixels of a
+ * row share an anchor, the largest that stays within one range cell of it. Off: every (pixel, chirp) range in double-float. Extension without
  * a reference counterpart; takes effect at the next focus. */
 int tdc_processor_set_anchored_ranges(tdc_processor *proc, int enable);
 

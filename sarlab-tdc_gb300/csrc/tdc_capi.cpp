@@ -613,6 +613,36 @@ int prepare(tdc_processor *p, const StartOpts &o, int &launches)
     return TDC_OK;
 }
 
+// Reach of the anchored pixel groups of the resident grid (range profiles): flag[10..12] on the
+// device, as float bits.
+int enqueue_group_reach(tdc_processor *p, cudaStream_t st, int &launches)
+{
+    int *reach = p->flag.as<int>() + 10;
+    TDC_CK(cudaMemsetAsync(reach, 0, 12, st), "reset reach");
+    TDC_CK(launch_group_reach(p->grid_hi.as<float4>(), p->P, p->grid_run, reach, st), "reach kernel");
+    launches += 1;
+    return TDC_OK;
+}
+
+void set_group_reach(tdc_processor *p, const int *bits)
+{
+    for (int k = 0; k < 3; ++k) {
+        float f;
+        std::memcpy(&f, &bits[k], 4);
+        p->group_reach[k] = f;
+    }
+    p->reach_known = true;
+}
+
+int read_group_reach(tdc_processor *p, cudaStream_t st)
+{
+    int bits[3];
+    TDC_CK(cudaMemcpyAsync(bits, p->flag.as<int>() + 10, sizeof(bits), cudaMemcpyDeviceToHost, st), "read reach");
+    TDC_CK(cudaStreamSynchronize(st), "reach sync");
+    set_group_reach(p, bits);
+    return TDC_OK;
+}
+
 // Device grid from a host (FP32 or FP64) grid.
 int upload_grid(tdc_processor *p, int &launches)
 {
@@ -716,24 +746,33 @@ int upload_grid(tdc_processor *p, int &launches)
         p->grid_lo_valid = false;
     }
     launches += 1;
+    TDC_CK(p->flag.ensure(64), "alloc flag");
+    p->grid_run = detect_run(
+        P, [&](long long i, int k) { return p->grid64 ? p->grid64[3 * i + k] : (double)p->grid[3 * i + k]; });
+    // (small focuses do not ask for it: measured when a plan first does)
+    p->reach_known = p->has_raw && profile_pays((double)std::max(P, p->plan_pixels), p->C, p->S);
+    if (p->reach_known)
+        if (int rc = enqueue_group_reach(p, st, launches)) return rc;
     if (p->host_reads && P > 0) {
         // bounding box of the grid on the device (order-preserving integer keys of the floats)
         const int init[6] = {0x7fffffff, 0x7fffffff, 0x7fffffff, (int)0x80000000, (int)0x80000000,
                              (int)0x80000000};
-        int keys[6];
-        TDC_CK(p->flag.ensure(64), "alloc flag");
+        int keys[9];
         int *box = p->flag.as<int>() + 4;
         TDC_CK(cudaMemcpyAsync(box, init, sizeof(init), cudaMemcpyHostToDevice, st), "init bbox");
         TDC_CK(launch_grid_bbox(p->grid_hi.as<float4>(), P, box, st), "bbox kernel");
         TDC_CK(cudaMemcpyAsync(keys, box, sizeof(keys), cudaMemcpyDeviceToHost, st), "read bbox");
         TDC_CK(cudaStreamSynchronize(st), "grid sync");
         launches += 1;
+        set_group_reach(p, keys + 6);
         for (int k = 0; k < 6; ++k) {
             const int bits = keys[k] >= 0 ? keys[k] : keys[k] ^ 0x7fffffff;
             float f;
             std::memcpy(&f, &bits, 4);
             (k < 3 ? p->grid_min[k] : p->grid_max[k - 3]) = f;
         }
+    } else if (p->reach_known) {
+        return read_group_reach(p, st);
     }
     return TDC_OK;
 }
@@ -1118,6 +1157,88 @@ bool anchor_eligible(const tdc_processor *p, int cb)
     return 2.0 * M_PI * 8.0 * std::fabs(g1) * p->anchor_span <= 0.25;
 }
 
+// Range profiles (tdc_profile.cu). The table costs about S x (nodes the grid spans, at most 2 S)
+// complex MACs a chirp, so it needs pixels enough to share it (a direct focus costs S a pixel),
+// and a launch large enough for one more kernel. Whole focus, direct / profiles, 2 mm grids: at
+// 0.54 Gcorr 211 / 157 us (128^2 pixels x 128 chirps x 256 samples), 206 / 139 (256^2 x 128 x 64),
+// 429 / 373 (64^2 x 512 x 256); at 0.27 Gcorr 175 / 151 (128^2 x 128 x 128), 104 / 128 (64^2 x 256 x
+// 256); 64^2 pixels = 4 x 1024 samples, 1024 chirps: 885 / 413.
+#ifndef TDC_PROFILE_MIN_WORK
+#define TDC_PROFILE_MIN_WORK 5e8
+#endif
+bool profile_pays(double n_pix, double n_pri, double n_samples)
+{
+    return n_pix >= 4.0 * n_samples && n_pix * n_pri * n_samples >= TDC_PROFILE_MIN_WORK;
+}
+
+bool profile_table_fits(int n_cells, int n_samples, double table_ratio)
+{
+    return table_ratio <= 0.0 || n_cells * (kProfileCoefs * 8.0) <= table_ratio * (n_samples * 8.0);
+}
+
+// Cells for ranges spread over `diagonal` metres: the spread, half a cell either side, and the
+// two cells that profile_build_kernel's even first cell can start early.
+int profile_cells(double cells_per_m, double diagonal)
+{
+    return ((int)std::ceil(std::fabs(cells_per_m) * diagonal) + 7) / 2 * 2;
+}
+
+// Pixels sharing an anchor of a range-profile focus of the resident acquisition and grid, or 0
+// where the direct kernels run: finite band, kept per-chirp sums, non-finite inputs, small
+// focuses (profile_pays), a grid wider than the unambiguous range, ranges beyond what the cell
+// index resolves in FP32, or a table larger than half the free device memory.
+int profile_group(tdc_processor *p, ProfileBuild &b)
+{
+    if (p->keep_sums || !p->rec_finite || std::isfinite(p->opts.bw / 2.0f)) return 0;
+    const long long P = std::max(p->P, p->plan_pixels);
+    if (!profile_pays((double)P, p->C, p->S)) return 0;
+    const double g1 = 2.0 * p->F1 / kC0, gc = 2.0 * p->F0 / kC0 + g1 * (p->S / 2);
+    b.cells_per_m = 4.0 * p->S * g1;
+    double diag2 = 0.0;
+    for (int k = 0; k < 3; ++k) {
+        b.box_min[k] = p->grid_min[k];
+        b.box_max[k] = p->grid_max[k];
+        diag2 += (p->grid_max[k] - p->grid_min[k]) * (p->grid_max[k] - p->grid_min[k]);
+    }
+    const double rmax = max_range(p->ant_min, p->ant_max, p->grid_min, p->grid_max);
+    if (!(std::fabs(b.cells_per_m) * rmax < 2097152.0) || !(diag2 >= 0.0) || !(std::fabs(gc) > 0.0)) return 0;
+    b.n_cells = profile_cells(b.cells_per_m, std::sqrt(diag2));
+    if (b.n_cells > 4LL * p->S || !profile_table_fits(b.n_cells, p->S, p->table_ratio)) return 0;
+    b.C = p->C;
+    b.S = p->S;
+    b.s_pad = p->s_pad;
+    const size_t bytes = (size_t)p->C * b.n_cells * kProfileCoefs * 8;
+    if (bytes > p->cells.cap) {
+        size_t free_b = 0, total_b = 0;
+        if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || bytes > free_b / 2) return 0;
+    }
+    if (!p->reach_known) {
+        int launches = 0;
+        if (enqueue_group_reach(p, p->stream, launches) || read_group_reach(p, p->stream)) return 0;
+    }
+    if (!std::isfinite(p->group_reach[0])) return 0;
+    if (!p->anchor_enabled) return 1;
+    // |t| <= 1/2 (the anchor's place in its cell) + the group's reach
+    for (int k = 0; k < 3; ++k)
+        if (std::fabs(b.cells_per_m) * p->group_reach[k] <= kProfileReach - 0.52) return 8 >> k;
+    return 1;
+}
+
+int profile_build(tdc_processor *p, const FocusPlan &plan, cudaStream_t st, int &launches)
+{
+    const int S = p->S;
+    float2 *tw = p->twiddle.as<float2>();
+    float *factor = reinterpret_cast<float *>(tw + (size_t)S * kProfileNodes);
+    if (p->twiddle_S != S) {
+        TDC_CK(launch_profile_twiddle(tw, factor, S, st), "profile constants kernel");
+        p->twiddle_S = S;
+        ++launches;
+    }
+    TDC_CK(launch_profile_build(plan.build, st), "profile table kernel");
+    ++launches;
+    return TDC_OK;
+}
+
 int focus_plan(tdc_processor *p, FocusPlan &plan, double max_unit_work)
 {
     if (!p->prepared) return fail(TDC_ERR_STATE, "acquisition not prepared");
@@ -1154,7 +1275,11 @@ int focus_plan(tdc_processor *p, FocusPlan &plan, double max_unit_work)
     const bool motion_exact_ql = path == TDC_PATH_FP32_MOTION && !(2.0 * M_PI * 8.0 * motion_slope_bound(p) <= 0.8);
     int slots;
     bool anchored = false;
-    if (path == TDC_PATH_FP32_MOTION) {
+    ProfileBuild build{};
+    const int profile = path == TDC_PATH_FP32_BULK ? profile_group(p, build) : 0;
+    if (profile) {
+        slots = p->n_sm * kProfileCtasPerSm;
+    } else if (path == TDC_PATH_FP32_MOTION) {
         const int bps = focus_motion_blocks_per_sm(stage_bytes);
         if (bps <= 0) return fail(TDC_ERR_CUDA, "smooth-motion focus kernel does not fit on the device");
         slots = p->n_sm * bps;
@@ -1172,17 +1297,22 @@ int focus_plan(tdc_processor *p, FocusPlan &plan, double max_unit_work)
     }
 
     const int tile_cols = choose_tile_cols(p);
-    const long long n_tiles = tile_count(P, tile_cols, p->cols);
+    const int run = profile ? p->grid_run : 0;
+    const long long n_tiles = profile ? profile_tiles(P, run) : tile_count(P, tile_cols, p->cols);
     // (block tiles also depend on the grid's shape, not only on its pixel count)
     const int plan_cols = tile_cols ? p->cols : 0;
     // The chirp groups (each pixel's summation order) follow the grid the job is planned for:
     // its own, or a larger one whose row block this grid is (pixel sharding across GPUs).
-    const long long plan_tiles = p->plan_pixels > P ? tile_count(p->plan_pixels, tile_cols, p->cols) : n_tiles;
+    const long long plan_tiles = p->plan_pixels <= P ? n_tiles
+                                 : profile           ? profile_tiles(p->plan_pixels, run)
+                                                     : tile_count(p->plan_pixels, tile_cols, p->cols);
     if (path != p->plan_path || P != p->plan_P || C != p->plan_C || slots != p->plan_slots ||
         max_unit_work != p->plan_unit_cap || tile_cols != p->plan_tile_cols || plan_cols != p->plan_cols ||
-        plan_tiles != p->plan_tiles) {
-        int min_units = path == TDC_PATH_GENERAL ? kGeneralMinUnitsPerSlot : kFocusMinUnitsPerSlot;
-        if (path == TDC_PATH_FP32_BULK && max_unit_work <= 0) {
+        plan_tiles != p->plan_tiles || profile != p->plan_profile || run != p->plan_run) {
+        int min_units = profile                    ? kProfileMinUnitsPerSlot
+                        : path == TDC_PATH_GENERAL ? kGeneralMinUnitsPerSlot
+                                                   : kFocusMinUnitsPerSlot;
+        if (path == TDC_PATH_FP32_BULK && !profile && max_unit_work <= 0) {
             // Long launches end on their last units: units of about kUnitTargetCorr correlations
             // (up to 32 per CTA slot) shorten that tail; short launches keep fewer, larger units.
             // (Request-loop launches bound their units by max_unit_work instead: finer units there
@@ -1195,7 +1325,8 @@ int focus_plan(tdc_processor *p, FocusPlan &plan, double max_unit_work)
         p->plan_tiles = plan_tiles;
         if (max_unit_work > 0) {
             // bound the work of one unit (tile x chirp group): at most cap / (tile x S) chirps per group
-            const int cpg_cap = std::max(1, (int)(max_unit_work / ((double)kFocusTile * p->S)));
+            const double per_pair = profile ? kProfilePairCost : (double)p->S;
+            const int cpg_cap = std::max(1, (int)(max_unit_work / ((double)kFocusTile * per_pair)));
             if (p->plan_cpg > cpg_cap) {
                 p->plan_cpg = cpg_cap;
                 p->plan_groups = (C + cpg_cap - 1) / cpg_cap;
@@ -1206,19 +1337,33 @@ int focus_plan(tdc_processor *p, FocusPlan &plan, double max_unit_work)
         p->plan_cols = plan_cols;
         p->units_host.clear();
         p->units_host.reserve((size_t)(n_tiles * p->plan_groups));
-        for (long long t = 0; t < n_tiles; ++t)
-            for (int g = 0; g < p->plan_groups; ++g) p->units_host.push_back(FocusUnit{0, (int)t, g, 0});
+        // (range profiles: all tiles of a chirp group together, so that the group's cells stay in L2)
+        if (profile)
+            for (int g = 0; g < p->plan_groups; ++g)
+                for (long long t = 0; t < n_tiles; ++t) p->units_host.push_back(FocusUnit{0, (int)t, g, 0});
+        else
+            for (long long t = 0; t < n_tiles; ++t)
+                for (int g = 0; g < p->plan_groups; ++g) p->units_host.push_back(FocusUnit{0, (int)t, g, 0});
         // (only the whole-row FP32-bulk focus reads unit spans, and not when it keeps its
         // per-chirp sums: those would be left unwritten for the skipped chirps)
         p->span_permille = 1000;
-        if (path != TDC_PATH_FP64_PHASE && path != TDC_PATH_GENERAL_FP64)
+        if (!profile && path != TDC_PATH_FP64_PHASE && path != TDC_PATH_GENERAL_FP64)
             plan_unit_order_and_spans(p, tile_cols,
                                 path == TDC_PATH_FP32_BULK && !seg && !p->keep_sums && !p->offsets_applied);
         p->plan_path = path;
         p->plan_P = P;
         p->plan_C = C;
         p->plan_slots = slots;
+        p->plan_profile = profile;
+        p->plan_run = run;
         p->plan_uploaded = false;
+    }
+    if (profile) {
+        TDC_CK(p->cells.ensure((size_t)p->C * build.n_cells * kProfileCoefs * 8), "alloc range profiles");
+        TDC_CK(p->cell_base.ensure(sizeof(ProfileJob) + (size_t)p->C * 4), "alloc range profile bases");
+        const size_t tw_bytes = (size_t)p->S * (kProfileNodes * 8 + 4);
+        if (tw_bytes > p->twiddle.cap) p->twiddle_S = 0;
+        TDC_CK(p->twiddle.ensure(tw_bytes), "alloc profile constants");
     }
     const int n_units = (int)p->units_host.size();
     const ScratchLayout L = scratch_layout(P, n_units, p->plan_groups);
@@ -1234,6 +1379,7 @@ int focus_plan(tdc_processor *p, FocusPlan &plan, double max_unit_work)
     plan.stage_bytes = stage_bytes;
     plan.slots = slots;
     plan.anchored = anchored;
+    plan.profile = profile;
     plan.off_job = L.off_job;
     plan.off_units = L.off_units;
     plan.job = make_job(p, reinterpret_cast<float4 *>(scr + L.off_partial), cb, path);
@@ -1244,6 +1390,30 @@ int focus_plan(tdc_processor *p, FocusPlan &plan, double max_unit_work)
     plan.job.tile_cols = tile_cols;
     plan.job.grid_cols = p->cols;
     plan.job.n_tiles = (int)n_tiles;
+    if (profile) {
+        build.rows = p->xw.as<const float2>();
+        build.chirps = plan.job.chirps;
+        build.twiddle = p->twiddle.as<const float2>();
+        build.factor = reinterpret_cast<const float *>(build.twiddle + (size_t)p->S * kProfileNodes);
+        build.cells = p->cells.as<float4>();
+        build.job_out = p->cell_base.as<ProfileJob>();
+        build.cell_base = reinterpret_cast<int *>(build.job_out + 1);
+        ProfileJob &job = build.job;
+        const double g1 = 2.0 * p->F1 / kC0, gc = 2.0 * p->F0 / kC0 + g1 * (p->S / 2);
+        plan.job.tile_cols = 0;
+        plan.job.grid_cols = run;
+        plan.job.profile = build.job_out;
+        job.n_cells = build.n_cells;
+        job.cells = build.cells;
+        job.cell_base = build.cell_base;
+        split_dd(gc, job.gc_hi, job.gc_lo);
+        split_dd(build.cells_per_m, job.cells_hi, job.cells_lo);
+        job.cells_per_cycle = (float)(build.cells_per_m / gc);
+        job.inv_gc2x4 = (float)(4.0 / (gc * gc));
+        const double reach = profile == 8 ? p->group_reach[0] : profile == 4 ? p->group_reach[1] : p->group_reach[2];
+        job.r_safe = (float)(reach / 0.03);
+        plan.build = build;
+    }
     // narrow variants take the phase correction in radians
     if (path == TDC_PATH_GENERAL && !(variant & 4)) plan.job.gsam = p->gres.as<const float>() + 2 * (size_t)p->s_pad;
     return TDC_OK;
@@ -1270,6 +1440,7 @@ void processor_release_memory(tdc_processor *p)
     p->plan_path = -1;
     p->plan_uploaded = false;
     p->grid_lo_valid = false;
+    p->twiddle_S = 0;
 }
 
 size_t processor_device_bytes(tdc_processor *p)
@@ -1319,7 +1490,12 @@ int focus_resident(tdc_processor *p, float2 *image_dev, cudaStream_t st, int &la
     const FocusUnit *units_dev = reinterpret_cast<const FocusUnit *>(scr + L.off_units);
     int *counter = reinterpret_cast<int *>(scr);
     int *status = counter + 1;
-    if (path == TDC_PATH_FP32_BULK) {
+    if (plan.profile) {
+        if (int rc = profile_build(p, plan, st, launches)) return rc;
+        const int grid = std::min(n_units, p->n_sm * focus_profile_blocks_per_sm(plan.profile));
+        TDC_CK(launch_focus_profile(plan.profile, jobs_dev, units_dev, n_units, counter, grid, st),
+               "focus kernel (range profiles)");
+    } else if (path == TDC_PATH_FP32_BULK) {
         const int grid = std::min(n_units, slots);
         // the zero-window-skipping instances also map block tiles (which come with a finite band)
         const bool skip_zero = std::isfinite(job.half_bw) || job.tile_cols != 0;
@@ -1349,7 +1525,7 @@ int focus_resident(tdc_processor *p, float2 *image_dev, cudaStream_t st, int &la
     p->sums_epoch = store ? p->state_epoch : 0;
     p->stats.path = path;
     p->stats.correlations = (int64_t)P * C * p->S;
-    const bool staged = path == TDC_PATH_FP32_BULK || path == TDC_PATH_GENERAL || path == TDC_PATH_FP32_MOTION;
+    const bool staged = (path == TDC_PATH_FP32_BULK && !plan.profile) || path == TDC_PATH_GENERAL || path == TDC_PATH_FP32_MOTION;
     const int row = path == TDC_PATH_GENERAL ? job.seg_len : plan.seg ? kSegmentSamples : p->s_pad;
     p->stats.stage_samples = staged ? std::min(row, p->s_pad) : 0;
     p->stats.stage_chirps = staged ? (row < p->s_pad ? 1 : plan.cb) : 0;
@@ -1357,7 +1533,7 @@ int focus_resident(tdc_processor *p, float2 *image_dev, cudaStream_t st, int &la
     p->stats.tile_cols = job.tile_cols;
     p->stats.motion_segment = path == TDC_PATH_FP32_MOTION ? job.seg_len : 0;
     p->stats.span_permille = path == TDC_PATH_FP32_BULK && !plan.seg && !store ? p->span_permille : 1000;
-    p->stats.anchor_pixels = 0;
+    p->stats.anchor_pixels = plan.profile > 1 ? plan.profile : 0;
     if (path == TDC_PATH_FP32_BULK && !plan.seg && plan.anchored && !store && !std::isfinite(job.half_bw) &&
         job.tile_cols == 0)
         p->stats.anchor_pixels = 32;

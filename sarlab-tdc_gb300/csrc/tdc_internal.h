@@ -136,9 +136,24 @@ struct FocusJob {
                              // whole rows; FP32 general: s_pad for whole rows)
     int tile_cols;           // 0: a tile is kFocusTile consecutive pixels; else kFocusTile / tile_cols grid
                              // rows x tile_cols columns of the grid_cols-wide row-major grid
-    int grid_cols;           // columns of the focus grid (block tiles)
+    int grid_cols;           // columns of the focus grid (block tiles); length of its runs (range profiles)
     int pad_;
+    const struct ProfileJob *profile;  // range profiles (tdc_profile.cu), else null
 };
+
+// What a focus through range profiles needs beside its FocusJob (16-byte groups: the kernel
+// loads four words together).
+struct __align__(16) ProfileJob {
+    float gc_hi, gc_lo;        // g0 + g1 (S / 2) as a double-float pair: carrier phase [cycles / m]
+    float cells_hi, cells_lo;  // cells per metre of range, 4 S g1, as a double-float pair
+    float inv_gc2x4;           // 4 / gc^2
+    float cells_per_cycle;     // cells per cycle of carrier phase
+    float r_safe;              // ranges below take the exact range difference (reach of a group / 0.03)
+    int n_cells;               // cells per chirp
+    const float4 *cells;       // [C][n_cells][kProfileCoefs / 2]: pairs of complex polynomial coefficients
+    const int *cell_base;      // [C] absolute index of each chirp's first cell
+};
+static_assert(sizeof(ProfileJob) == 48, "ProfileJob layout");
 
 // Kernels copy a FocusJob into shared memory one int per thread (128 threads); the
 // no-allocation scratch reserves 256 bytes for it.
@@ -151,6 +166,47 @@ inline long long tile_count(long long P, int tile_cols, int grid_cols)
     const long long rows = (P + grid_cols - 1) / grid_cols;
     const int tile_rows = kFocusTile / tile_cols;
     return ((rows + tile_rows - 1) / tile_rows) * ((grid_cols + tile_cols - 1) / tile_cols);
+}
+
+// ---- range profiles (tdc_profile.cu) ----
+constexpr int kProfileThreads = 64;     // a tile's kFocusTile pixels, 8 consecutive pixels a thread
+constexpr int kProfilePixels = kFocusTile / kProfileThreads;
+constexpr int kProfileNodes = 64;       // nodes one CTA of the table's construction forms
+constexpr int kProfileCoefs = 8;        // complex coefficients per cell
+constexpr double kProfileReach = 1.5;   // |t| a cell's polynomial is made for [cells]
+// CTAs per SM the planner counts on (the focus kernel's launch bound), and units per CTA.
+#ifndef TDC_PROFILE_CTAS
+#define TDC_PROFILE_CTAS 8
+#endif
+constexpr int kProfileCtasPerSm = TDC_PROFILE_CTAS;
+#ifndef TDC_PROFILE_MIN_UNITS
+#define TDC_PROFILE_MIN_UNITS 3
+#endif
+constexpr int kProfileMinUnitsPerSlot = TDC_PROFILE_MIN_UNITS;
+
+// Inputs and outputs of profile_build_kernel.
+struct ProfileBuild {
+    const float2 *rows;      // [C][s_pad] windowed samples
+    const ChirpRec *chirps;  // [C]
+    const float2 *twiddle;   // [S][kProfileNodes], launch_profile_twiddle
+    const float *factor;     // [S]
+    float4 *cells;           // [C][n_cells][kProfileCoefs / 2]
+    int *cell_base;          // [C]
+    ProfileJob *job_out;     // receives `job`
+    ProfileJob job;
+    double box_min[3], box_max[3];  // bounding box of the grid
+    double cells_per_m;
+    int C, S, s_pad, n_cells;
+};
+
+// Tiles of a P-pixel grid whose runs are `run` pixels long: groups of kProfilePixels
+// consecutive pixels of a run, kProfileThreads groups a tile (in bands of kProfileBand runs).
+constexpr int kProfileBand = 8;
+inline long long profile_tiles(long long P, int run)
+{
+    const long long per = (run + kProfilePixels - 1) / kProfilePixels;
+    const long long groups = (P + run - 1) / run * per;
+    return (groups + kProfileThreads - 1) / kProfileThreads;
 }
 
 struct FocusUnit {
@@ -222,6 +278,18 @@ cudaError_t launch_focus_general(int variant, const FocusJob *jobs_dev, const Fo
                                  int *counter_dev, int *status_dev, int stage_bytes, int grid_ctas, cudaStream_t st);
 int focus_general_blocks_per_sm(int variant, int stage_bytes);
 int focus_general_smem_bytes(int stage_bytes);
+
+// Range profiles: the per-length constants (twiddle [S][kProfileNodes], factor [S]), the table
+// of the resident acquisition over the grid's ranges, and the focus that reads it, with
+// `group` (8, 4, 2 or 1) consecutive pixels sharing an anchor.
+cudaError_t launch_profile_twiddle(float2 *twiddle, float *factor, int S, cudaStream_t st);
+cudaError_t launch_profile_build(const ProfileBuild &b, cudaStream_t st);
+cudaError_t launch_focus_profile(int group, const FocusJob *jobs_dev, const FocusUnit *units_dev, int n_units,
+                                 int *counter_dev, int grid_ctas, cudaStream_t st);
+int focus_profile_blocks_per_sm(int group);
+// out[0..2] = max(out, largest distance of a pixel from the anchor of its group of 8 / 4 / 2
+// consecutive pixels of a run) as float bits (out starts at 0; a NaN compares above any distance).
+cudaError_t launch_group_reach(const float4 *hi, long long P, int run, int *out, cudaStream_t st);
 
 // Adjoint of the FP32-bulk focus w.r.t. per-chirp position offsets: per-(tile, chirp)
 // float4 partials, then an FP64 sum over tiles into grad[C][3]. stored: job.xw holds the

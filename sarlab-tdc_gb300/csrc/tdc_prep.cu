@@ -142,6 +142,39 @@ __global__ void grid_bbox_kernel(const float4 *__restrict__ hi, long long P, int
     }
 }
 
+// Reach of the anchored pixel groups of the range-profile focus: the largest distance from a
+// group's anchor (its middle pixel) to its other pixels, for groups of 8, 4 and 2 consecutive
+// pixels of a run; one thread per 8 pixels of a run.
+__global__ void group_reach_kernel(const float4 *__restrict__ hi, long long P, int run, int *__restrict__ out)
+{
+    const int per = (run + 7) / 8;
+    const long long n = (P / run) * per + (P % run + 7) / 8;
+    float reach[3] = {0.f, 0.f, 0.f};
+    for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x) {
+        const long long r = q / per;
+        const int col = (int)(q - r * per) * 8;
+        const long long p0 = r * run + col;
+        const int valid = (int)min((long long)min(8, run - col), P - p0);
+        for (int k = 0; k < 3; ++k) {
+            const int g = 8 >> k;
+            for (int s = 0; s < valid; s += g) {
+                const int m = min(g, valid - s);
+                const float4 a = hi[p0 + s + m / 2];
+                for (int i = 0; i < m; ++i) {
+                    const float4 v = hi[p0 + s + i];
+                    const float dx = v.x - a.x, dy = v.y - a.y, dz = v.z - a.z;
+                    const float d = sqrtf(dx * dx + dy * dy + dz * dz);
+                    reach[k] = d > reach[k] || d != d ? d : reach[k];
+                }
+            }
+        }
+    }
+    for (int k = 0; k < 3; ++k) {
+        const int v = __reduce_max_sync(0xffffffffu, __float_as_int(fabsf(reach[k])));
+        if ((threadIdx.x & 31) == 0 && v > 0) atomicMax(&out[k], v);
+    }
+}
+
 __global__ void grid_f32_kernel(const float *__restrict__ g, long long P, float4 *__restrict__ hi)
 {
     const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -248,6 +281,16 @@ cudaError_t launch_grid_bbox(const float4 *hi, long long P, int *out, cudaStream
     long long blocks = (P + 255) / 256;
     if (blocks > 152 * 8) blocks = 152 * 8;
     grid_bbox_kernel<<<(unsigned)blocks, 256, 0, st>>>(hi, P, out);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_group_reach(const float4 *hi, long long P, int run, int *out, cudaStream_t st)
+{
+    if (P <= 0 || run <= 0) return cudaSuccess;
+    long long blocks = (P / 8 + 255) / 256;
+    if (blocks > 152 * 8) blocks = 152 * 8;
+    if (blocks < 1) blocks = 1;
+    group_reach_kernel<<<(unsigned)blocks, 256, 0, st>>>(hi, P, run, out);
     return cudaGetLastError();
 }
 

@@ -189,6 +189,14 @@ struct tdc_processor {
     // takes them when this is within kAnchorMaxDistance, unless switched off.
     double anchor_span = 0.0;
     bool anchor_enabled = true;
+    // Range profiles (tdc_profile.cu): consecutive pixels without a jump (a grid row), the reach of
+    // the groups of 8 / 4 / 2 pixels sharing an anchor, the table and the per-length constants.
+    int grid_run = 1;
+    double group_reach[3] = {0, 0, 0};
+    bool reach_known = false;  // group_reach is the resident grid's
+    tdc::impl::DevBuf cells, cell_base, twiddle;
+    double table_ratio = 0.0;  // largest table taken, in bytes per byte of samples (0: no limit)
+    int twiddle_S = 0;  // samples the constants in `twiddle` are for (0: none)
     bool rec_finite = false;  // every chirp record's velocity and window centre is finite
     double vel_dir[3] = {0, 0, 0};                         // mean antenna velocity direction (0: at rest)
     tdc::impl::DevBuf grid_stage, grid_hi, grid_lo;
@@ -208,7 +216,7 @@ struct tdc_processor {
     std::vector<tdc::FocusUnit> units_host;
     long long plan_P = -1;
     int plan_C = -1, plan_groups = 0, plan_cpg = 0, plan_path = -1, plan_slots = 0, plan_tile_cols = -1,
-        plan_cols = -1;
+        plan_cols = -1, plan_profile = -1, plan_run = 0;
     double plan_unit_cap = 0.0;
     long long plan_tiles = -1;   // tiles the chirp groups were planned for
     long long plan_pixels = 0;   // plan the chirp groups for a grid of this many pixels (0: the grid's own)
@@ -231,7 +239,7 @@ struct tdc_processor {
     {
         return {&xw,      &chirps,     &skip,    &gs,      &pos_base, &wr,      &offsets,     &flag,     &gen_rec,
                 &traj,    &wins,       &wdot,    &gres,    &grid_stage, &grid_hi, &grid_lo, &scratch, &adj_scratch,
-                &chirp_sums, &xs_scaled, &motion_rec,
+                &chirp_sums, &xs_scaled, &motion_rec, &cells, &cell_base, &twiddle,
                 &image_dev};
     }
 };
@@ -248,6 +256,8 @@ struct FocusPlan {
     int stage_bytes = 0;  // bytes per pipeline stage
     int slots = 0;        // resident CTAs of the kernel on the device
     bool anchored = false;  // FP32-bulk kernel with anchored ranges
+    int profile = 0;      // FP32-bulk focus through range profiles: pixels sharing an anchor (8, 4, 2, 1); else 0
+    ProfileBuild build{};  // its table (profile > 0)
     size_t off_job = 0;   // job record and unit table offsets in the processor's scratch
     size_t off_units = 0;
     FocusJob job{};       // partial -> the processor's scratch
@@ -280,6 +290,42 @@ FocusJob make_job(const tdc_processor *p, float4 *partial, int cb, int path);
 // Plan units (p->units_host) and make sure the processor's scratch holds them and the partials.
 // max_unit_work > 0 bounds the correlations of one unit (the request loop's granularity).
 int focus_plan(tdc_processor *p, FocusPlan &plan, double max_unit_work = 0.0);
+// A (pixel, chirp) pair of a range-profile focus in correlations of the direct FP32-bulk kernel's
+// time (work budgets of the request loop).
+constexpr double kProfilePairCost = 14.0;
+// Range profiles: whether a focus of n_pix pixels x n_pri chirps x n_samples samples is large enough
+// for its table to pay, the run length of a point list, and the table cells a grid's bounding box
+// diagonal asks for.
+// (table_ratio: the largest table taken, in bytes per byte of samples; 0: no limit.)
+bool profile_table_fits(int n_cells, int n_samples, double table_ratio);
+bool profile_pays(double n_pix, double n_pri, double n_samples);
+int profile_cells(double cells_per_m, double diagonal);
+template <class Get>
+int detect_run(long long P, const Get &g)
+{
+    // the first step longer than 1.5 x the first one ends a run; short runs (under 4 pixels) and
+    // lists without a jump are one run
+    auto step2 = [&](long long p) {
+        double s = 0.0;
+        for (int k = 0; k < 3; ++k) {
+            const double d = g(p, k) - g(p - 1, k);
+            s += d * d;
+        }
+        return s;
+    };
+    const long long most = P < (1LL << 30) ? P : (1LL << 30);
+    if (P < 2) return 1;
+    const double first = step2(1);
+    long long run = most;
+    for (long long p = 2; p < most; ++p)
+        if (step2(p) > 2.25 * first) {
+            run = p;
+            break;
+        }
+    return (int)(run < 4 ? most : run);
+}
+// Enqueue the table of a planned range-profile focus on `st`, ahead of its launch.
+int profile_build(tdc_processor *p, const FocusPlan &plan, cudaStream_t st, int &launches);
 // Request-loop slots: recreate the processor's stream at `priority` (cudaDeviceGetStreamPriorityRange
 // order) and take its device buffers from the stream-ordered pool on that stream.
 int processor_use_slot_stream(tdc_processor *p, int priority);

@@ -1,0 +1,724 @@
+// tdc_profile.cu -- focus through range profiles: the FP32-bulk focus for grids of many pixels.
+//
+// With one range R per (pixel, chirp) and uniformly spaced samples, a pixel's sum over a
+// chirp's samples is the chirp's centred spectrum at beta = g1 R [cycles / sample],
+//
+//   sum_s x[s] exp(j 2 pi (g0 + g1 s) R) = exp(j 2 pi gc R) A(beta),
+//   A(beta) = sum_s x[s] exp(j 2 pi beta (s - sc)),  sc = S / 2,  gc = g0 + g1 sc,
+//
+// the same smooth function for every pixel. The direct kernels evaluate it from scratch, 4 S
+// FMAs a pixel; here profile_build_kernel tabulates it once per chirp over the ranges the grid
+// can take, and profile_focus_kernel reads one polynomial value per (pixel, chirp).
+//
+// The table ("cells"): A on cells of 1 / (4 S) cycles / sample (a quarter of the range
+// resolution), each a polynomial of degree 7 in t = 4 S beta - cell, good for |t| <= 1.5, so
+// that a group of neighbouring pixels reads one cell although their ranges differ. Built from
+// A at nodes 1 / (2 S) apart (a product of the chirps' rows with a fixed matrix of phasors)
+// by Kaiser-Bessel interpolation (9 nodes wide, the samples divided by the kernel's transform
+// beforehand) at 8 Chebyshev points of the cell. Error of the interpolation and of the
+// polynomial together: <= 2e-7 rms of a row's norm at |t| = 1.5, 1e-8 within the cell.
+//
+// Whole focus, direct kernels -> profiles (GB300, resident acquisition): 1024^2 pixels x 4096
+// chirps x 1024 samples 532 -> 7.4 ms; 1.05 M voxels x 16,384 x 256 587 -> 27.7 ms; 256^2 x 1024 x
+// 512 4.5 -> 0.24 ms; 256^2 x 64 x 12,345 6.5 -> 1.0 ms.
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+#include <cmath>
+
+#include "tdc_device.cuh"
+#include "tdc_internal.h"
+
+namespace tdc {
+
+namespace {
+
+// ---- table construction -----------------------------------------------------
+
+constexpr int kNodes = kProfileNodes;            // nodes one CTA forms
+constexpr int kTaps = 11;                        // nodes a cell reads: -5 .. +5 about its own
+constexpr int kOwn = kProfileNodes - kTaps + 1;  // nodes whose two cells the CTA writes
+constexpr int kBuildChirps = 16;
+constexpr int kBuildThreads = 256;
+constexpr int kBuildStep = 64;                   // samples per shared-memory tile
+constexpr double kKbWidth = 9.0;
+constexpr double kKbBeta = 2.3 * kKbWidth;
+
+// Real weights of a cell's polynomial coefficients: a_m = sum_j c[parity][m][j] V[node + j - 5].
+struct ProfileStencil {
+    float c[2][kProfileCoefs][kTaps];
+};
+
+double bessel_i0(double x)
+{
+    // sum_k (x^2 / 4)^k / (k!)^2
+    double term = 1.0, sum = 1.0;
+    for (int k = 1; k < 200 && term > 1e-18 * sum; ++k) {
+        term *= (x * x / 4.0) / ((double)k * k);
+        sum += term;
+    }
+    return sum;
+}
+
+ProfileStencil make_stencil()
+{
+    // f(x) = sum_j phi(x - j) V_j at the Chebyshev points t_i of the cell (x = t / 2 from the
+    // cell's centre, which lies on a node or half way to the next), then the polynomial through
+    // the 8 values: a = V^-1 f, V the Vandermonde matrix of the points (Gauss-Jordan in FP64).
+    constexpr int n = kProfileCoefs;
+    ProfileStencil st{};
+    double t[n], a[n][2 * n];
+    for (int i = 0; i < n; ++i) {
+        t[i] = kProfileReach * std::cos(M_PI * (i + 0.5) / n);
+        for (int m = 0; m < n; ++m) {
+            a[i][m] = std::pow(t[i], m);
+            a[i][n + m] = i == m ? 1.0 : 0.0;
+        }
+    }
+    for (int k = 0; k < n; ++k) {
+        int piv = k;
+        for (int i = k + 1; i < n; ++i)
+            if (std::fabs(a[i][k]) > std::fabs(a[piv][k])) piv = i;
+        for (int m = 0; m < 2 * n; ++m) std::swap(a[k][m], a[piv][m]);
+        const double d = a[k][k];
+        for (int m = 0; m < 2 * n; ++m) a[k][m] /= d;
+        for (int i = 0; i < n; ++i) {
+            if (i == k) continue;
+            const double f = a[i][k];
+            for (int m = 0; m < 2 * n; ++m) a[i][m] -= f * a[k][m];
+        }
+    }
+    // normalised so that the samples' factors (profile_twiddle_kernel) are about 1
+    const double norm = kKbBeta / std::sinh(kKbBeta) / kKbWidth;
+    for (int par = 0; par < 2; ++par)
+        for (int m = 0; m < n; ++m)
+            for (int j = 0; j < kTaps; ++j) {
+                double s = 0.0;
+                for (int i = 0; i < n; ++i) {
+                    const double z = (0.5 * par + 0.5 * t[i] - (j - 5)) * 2.0 / kKbWidth;
+                    if (std::fabs(z) < 1.0) s += a[m][n + i] * bessel_i0(kKbBeta * std::sqrt(1.0 - z * z)) * norm;
+                }
+                st.c[par][m][j] = (float)s;
+            }
+    return st;
+}
+
+// Per-length constants: phasors e^{j 2 pi n (s - sc) / (2 S)} for the nodes of one CTA
+// ([S][kNodes]) and the samples' factors 1 / phi^ (the Kaiser-Bessel kernel's transform at the
+// sample's frequency in node units).
+__global__ void profile_twiddle_kernel(float2 *__restrict__ tw, float *__restrict__ factor, int S)
+{
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= (long long)S * kNodes) return;
+    const int s = (int)(i / kNodes), n = (int)(i - (long long)s * kNodes);
+    const long long nn = 2LL * S, d = s - S / 2;
+    long long r = (n * d) % nn;
+    if (r < 0) r += nn;
+    double sn, cs;
+    sincospi(2.0 * (double)r / (double)nn, &sn, &cs);
+    tw[i] = make_float2((float)cs, (float)sn);
+    if (n == 0) {
+        const double q2 = 0.5 * kKbWidth * 2.0 * 3.14159265358979323846 * (double)d / (double)nn;
+        const double q = sqrt(kKbBeta * kKbBeta - q2 * q2);
+        factor[s] = (float)(q / sinh(q) * (sinh(kKbBeta) / kKbBeta));
+    }
+}
+
+// One CTA: 16 chirps x one block of kOwn nodes (2 kOwn cells). Blocks lie at multiples of kOwn
+// of the absolute node index, so a cell's value does not depend on where the table starts
+// (the row blocks of a sharded grid build the same cells bit for bit). The rows are shifted by
+// the block's first node while they are staged, then multiplied by the fixed phasor matrix
+// (2 nodes x 4 chirps per thread: 32 FFMA per 4 shared loads; the two halves of the warps take
+// the two halves of a tile's samples), summed 64 samples at a time so that FP32 rounding does
+// not grow with the row, and the cells' coefficients are formed from the nodes in shared memory.
+// Bound: FP32 FMA; C x S x (nodes the grid spans + up to one block) complex MACs, a few per cent
+// of the focus it serves.
+__global__ void __launch_bounds__(kBuildThreads)
+    profile_build_kernel(const ProfileBuild b, const __grid_constant__ ProfileStencil stencil)
+{
+    __shared__ __align__(16) float2 sx[kBuildStep][kBuildChirps];
+    __shared__ __align__(16) float2 sv[kBuildStep * kNodes];  // phasors of a tile; then the nodes' values
+    __shared__ int s_base[kBuildChirps];            // the chirp's first cell (absolute, even)
+    __shared__ int s_cell[kBuildChirps];            // the block's first cell within the chirp's table
+    __shared__ unsigned int s_shift[kBuildChirps];  // first node of the block modulo 2 S
+    static_assert(kBuildStep >= 2 * kBuildChirps, "node values reuse the phasor tile");
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int c0 = blockIdx.x * kBuildChirps;
+    const unsigned int nn = 2u * (unsigned)b.S;
+
+    if (blockIdx.x == 0 && blockIdx.y == 0 && tid == 0) *b.job_out = b.job;
+    if (tid < kBuildChirps) {
+        // first cell: the smallest cell coordinate of any point in the grid's bounding box
+        const int c = min(c0 + tid, b.C - 1);
+        const ChirpRec r = b.chirps[c];
+        const double p[3] = {(double)r.p_hi.x + r.p_lo.x, (double)r.p_hi.y + r.p_lo.y, (double)r.p_hi.z + r.p_lo.z};
+        double near2 = 0.0, far2 = 0.0;
+        for (int k = 0; k < 3; ++k) {
+            const double lo = b.box_min[k] - p[k], hi = p[k] - b.box_max[k];
+            const double n = fmax(0.0, fmax(lo, hi)), f = fmax(fabs(lo), fabs(hi));
+            near2 += n * n;
+            far2 += f * f;
+        }
+        const double u = fmin(b.cells_per_m * sqrt(near2), b.cells_per_m * sqrt(far2));
+        // (positions far outside what the table can index: any base will do, reads are clamped)
+        const int base = fabs(u) < 1e9 ? 2 * (int)floor(0.5 * u) - 2 : 0;
+        if (blockIdx.y == 0 && c0 + tid < b.C) b.cell_base[c0 + tid] = base;
+        const int node = base >> 1;
+        const int block = (node >= 0 ? node / kOwn : -((kOwn - 1 - node) / kOwn)) + (int)blockIdx.y;
+        s_cell[tid] = 2 * (block * kOwn - node);
+        long long n0 = ((long long)block * kOwn - kTaps / 2) % (long long)nn;
+        s_shift[tid] = (unsigned)(n0 < 0 ? n0 + nn : n0);
+    }
+    __syncthreads();
+    if (!__syncthreads_or(tid < kBuildChirps && s_cell[tid & (kBuildChirps - 1)] < b.n_cells)) return;
+
+    const int cq = 4 * (warp & 3), half = warp >> 2;
+    float2 acc[4][2], run[4][2];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int k = 0; k < 2; ++k) acc[i][k] = run[i][k] = make_float2(0.f, 0.f);
+
+    for (int s0 = 0, tile = 0; s0 < b.S; s0 += kBuildStep, ++tile) {
+        // rows: shifted by the block's first node, scaled, zero past the row's end
+#pragma unroll
+        for (int i = 0; i < kBuildStep * kBuildChirps / kBuildThreads; ++i) {
+            const int q = (warp >> 1) + 4 * i, si = (warp & 1) * 32 + lane;
+            const int s = s0 + si;
+            float2 v = make_float2(0.f, 0.f);
+            if (s < b.S && c0 + q < b.C) {
+                const float2 x = b.rows[(size_t)(c0 + q) * b.s_pad + s];
+                const float f = b.factor[s];
+                const int d = s - b.S / 2;
+                const unsigned int dm = d < 0 ? (unsigned)(d + (int)nn) : (unsigned)d;
+                // (nn < 2^16: the product fits 32 bits)
+                const unsigned int r = nn < 65536u ? (s_shift[q] * dm) % nn
+                                                   : (unsigned)(((unsigned long long)s_shift[q] * dm) % nn);
+                const int rc = r > nn / 2 ? (int)r - (int)nn : (int)r;
+                float sn, cs;
+                sincospif(2.0f * __fdiv_rn((float)rc, (float)nn), &sn, &cs);
+                v = make_float2(f * fmaf(x.x, cs, -x.y * sn), f * fmaf(x.x, sn, x.y * cs));
+            }
+            sx[si][q] = v;
+        }
+        // phasors: kBuildStep x kNodes, contiguous in memory (rows past the end meet zero samples)
+        {
+            const int ns = min(kBuildStep, b.S - s0);
+            const float4 *src = reinterpret_cast<const float4 *>(b.twiddle + (size_t)s0 * kNodes);
+            float4 *dst = reinterpret_cast<float4 *>(sv);
+#pragma unroll
+            for (int i = 0; i < kBuildStep * kNodes / 2 / kBuildThreads; ++i) {
+                const int e = tid + i * kBuildThreads;
+                dst[e] = e < ns * kNodes / 2 ? __ldg(&src[e]) : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+        }
+        __syncthreads();
+#pragma unroll 8
+        for (int si = 0; si < kBuildStep / 2; ++si) {
+            const int s = half * (kBuildStep / 2) + si;
+            const float4 xa = *reinterpret_cast<const float4 *>(&sx[s][cq]);
+            const float4 xb = *reinterpret_cast<const float4 *>(&sx[s][cq + 2]);
+            const float2 x[4] = {make_float2(xa.x, xa.y), make_float2(xa.z, xa.w), make_float2(xb.x, xb.y),
+                                 make_float2(xb.z, xb.w)};
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                const float2 z = sv[s * kNodes + lane + 32 * k];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    run[i][k].x = fmaf(x[i].x, z.x, run[i][k].x);
+                    run[i][k].x = fmaf(-x[i].y, z.y, run[i][k].x);
+                    run[i][k].y = fmaf(x[i].x, z.y, run[i][k].y);
+                    run[i][k].y = fmaf(x[i].y, z.x, run[i][k].y);
+                }
+            }
+        }
+        if ((tile & 1) || s0 + kBuildStep >= b.S) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int k = 0; k < 2; ++k) {
+                    acc[i][k].x += run[i][k].x;
+                    acc[i][k].y += run[i][k].y;
+                    run[i][k] = make_float2(0.f, 0.f);
+                }
+        }
+        __syncthreads();
+    }
+
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int k = 0; k < 2; ++k) sv[(half * kBuildChirps + cq + i) * kNodes + lane + 32 * k] = acc[i][k];
+    __syncthreads();
+    for (int i = tid; i < kBuildChirps * kNodes; i += kBuildThreads) {
+        const float2 a = sv[i], z = sv[kBuildChirps * kNodes + i];
+        sv[i] = make_float2(a.x + z.x, a.y + z.y);
+    }
+    __syncthreads();
+
+    for (int i = tid; i < kBuildChirps * kOwn; i += kBuildThreads) {
+        const int q = i / kOwn, j = i - q * kOwn;
+        const int c = c0 + q;
+        if (c >= b.C) break;
+        const int l = s_cell[q] + 2 * j;  // cell within the chirp's table
+        if (l < 0 || l >= b.n_cells) continue;
+        float2 v[kTaps];
+#pragma unroll
+        for (int k = 0; k < kTaps; ++k) v[k] = sv[q * kNodes + j + k];
+        float4 *__restrict__ out = b.cells + ((size_t)c * b.n_cells + l) * (kProfileCoefs / 2);
+#pragma unroll
+        for (int par = 0; par < 2; ++par)
+#pragma unroll
+            for (int m = 0; m < kProfileCoefs; m += 2) {
+                float2 a0 = make_float2(0.f, 0.f), a1 = a0;
+#pragma unroll
+                for (int k = 0; k < kTaps; ++k) {
+                    a0.x = fmaf(stencil.c[par][m][k], v[k].x, a0.x);
+                    a0.y = fmaf(stencil.c[par][m][k], v[k].y, a0.y);
+                    a1.x = fmaf(stencil.c[par][m + 1][k], v[k].x, a1.x);
+                    a1.y = fmaf(stencil.c[par][m + 1][k], v[k].y, a1.y);
+                }
+                out[par * (kProfileCoefs / 2) + m / 2] = make_float4(a0.x, a0.y, a1.x, a1.y);
+            }
+    }
+}
+
+// ---- focus ------------------------------------------------------------------
+
+constexpr int kThreads = kProfileThreads;
+static_assert(kThreads == 64, "records are staged by 64 threads");
+constexpr int kPT = kFocusTile / kProfileThreads;  // pixels per thread: consecutive pixels of a run
+#ifndef TDC_PROFILE_MINB
+#define TDC_PROFILE_MINB 8
+#endif
+constexpr int kFlush = 32;                         // chirps summed in plain FP32 between Kahan steps
+
+struct SharedSums {
+    float4 s[kPT][kThreads];       // (sum.re, sum.im, comp.re, comp.im)
+    float2 dz[kPT / 2][kThreads];  // z offsets and |d|^2 of the thread's pixel pairs
+    float2 dd[kPT / 2][kThreads];
+};
+
+// Chirp records of kFlush chirps at a time: position (high, low) and first cell.
+struct SharedChirps {
+    float4 p[kFlush][2];
+    int base[kFlush];
+};
+
+// Kahan step of pixel i's sums: + sum over chirps of (cos + j sin) h, given as sum h cos, sum h sin.
+__device__ __forceinline__ void stash(SharedSums &sums, int i, int tid, float2 hc, float2 hs)
+{
+    float4 s = sums.s[i][tid];
+    const float yr = (hc.x - hs.y) - s.z, yi = (hc.y + hs.x) - s.w;
+    const float tr = s.x + yr, ti = s.y + yi;
+    s.z = (tr - s.x) - yr;
+    s.w = (ti - s.y) - yi;
+    s.x = tr;
+    s.y = ti;
+    sums.s[i][tid] = s;
+}
+
+// First pixel of thread `tid` of tile t, and how many it has (consecutive ones, up to kPT; 0
+// past the grid's end). Threads take kPT consecutive pixels of a run (a grid row: consecutive
+// pixels without a jump), so no thread's pixels straddle the end of one. Groups are numbered
+// down the runs of a band of 8 runs, then along it: a warp covers a block of 8 runs x 32
+// pixels, whose ranges, and so the cells it reads, lie closer together than 256 pixels of one
+// run's do.
+__device__ __forceinline__ long long run_pixels(long long P, int run, int t, int tid, int &count)
+{
+    const int per_run = (run + kPT - 1) / kPT;
+    const long long runs = (P + run - 1) / run;
+    const long long q = (long long)t * kThreads + tid;
+    const long long band = q / ((long long)kProfileBand * per_run);
+    const int rem = (int)(q - band * kProfileBand * per_run);
+    const int height = (int)min((long long)kProfileBand, runs - band * kProfileBand);
+    count = 0;
+    if (height <= 0) return 0;
+    const int col = rem / height * kPT;
+    const long long p = (band * kProfileBand + rem % height) * run + col;
+    if (col < run && p < P) count = (int)min((long long)min(kPT, run - col), P - p);
+    return p;
+}
+
+// Pairs of FP32 values in one instruction (FFMA2 and its kin): the same FMA-pipe time as two
+// scalar ones, half the issue slots, which is what bounds the scalar form of this kernel.
+__device__ __forceinline__ float2 both(float v) { return make_float2(v, v); }
+
+// Asynchronous copy of 4 or 16 bytes into shared memory.
+template <int BYTES>
+__device__ __forceinline__ void copy_async(void *dst, const void *src)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(smem_u32(dst)), "l"(src), "n"(BYTES) : "memory");
+}
+
+__device__ __forceinline__ void copy_async_wait()
+{
+    asm volatile("cp.async.wait_all;" ::: "memory");
+}
+
+// Shared memory loaded where it is used: these values would otherwise sit in registers through the
+// whole loop.
+__device__ __forceinline__ float4 fresh(const float *p)
+{
+    float4 v;
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+                 : "r"(smem_u32(p)));
+    return v;
+}
+
+__device__ __forceinline__ float2 fresh2(const float2 *p)
+{
+    float2 v;
+    asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(smem_u32(p)));
+    return v;
+}
+
+// One (chirp, anchor pixel): e = antenna - anchor, R0, gc / (2 R0), the carrier phase 2 pi frac(gc R0),
+// and the anchor's cell and place in it.
+struct Anchor {
+    float ex, ey, ez, rh, h, turn, t0;
+    float2 a[kProfileCoefs];
+};
+
+// One chirp's contributions to two pixels with phase differences psi (cycles) from their
+// anchor: e^{j (turn + 2 pi psi)} A(t0 + psi cells_per_cycle), A the cell's polynomial with
+// coefficients a. Real and imaginary part of the value h advance together; the product with
+// the phasor is kept as h cos and h sin (c_i, s_i) and combined when the sums are flushed.
+__device__ __forceinline__ void add_pair(float2 psi, float turn, float t0, float cells_per_cycle,
+                                         const float2 (&a)[kProfileCoefs], float2 &c0, float2 &s0, float2 &c1,
+                                         float2 &s1)
+{
+    const float2 n = __fadd2_rn(__fadd2_rn(psi, both(12582912.0f)), both(-12582912.0f));  // nearest integer
+    const float2 x = __ffma2_rn(__fadd2_rn(psi, make_float2(-n.x, -n.y)), both(kTwoPiF), both(turn));
+    const float2 t = __ffma2_rn(psi, both(cells_per_cycle), both(t0));
+    float sn0, cs0, sn1, cs1;
+    __sincosf(x.x, &sn0, &cs0);
+    __sincosf(x.y, &sn1, &cs1);
+    const float2 ta = both(t.x), tb = both(t.y);
+    float2 h0 = a[kProfileCoefs - 1], h1 = h0;
+#pragma unroll
+    for (int m = kProfileCoefs - 2; m >= 0; --m) {
+        h0 = __ffma2_rn(h0, ta, a[m]);
+        h1 = __ffma2_rn(h1, tb, a[m]);
+    }
+    c0 = __ffma2_rn(h0, both(cs0), c0);
+    s0 = __ffma2_rn(h0, both(sn0), s0);
+    c1 = __ffma2_rn(h1, both(cs1), c1);
+    s1 = __ffma2_rn(h1, both(sn1), s1);
+}
+
+// Persistent CTAs of 64 threads over units (tile x chirp group) from an atomic counter, 8
+// pixels a thread. Per chirp, each G consecutive pixels share an anchor pixel: its range R0,
+// the carrier phase frac(gc R0) and the cell it reads (64 bytes, from L1 / L2: neighbouring
+// threads read the same few cells) are formed once in double-float. A pixel then takes its
+// phase difference from the anchor, psi = gc (R - R0) cycles, from
+//   Q = gc (R^2 - R0^2) / (2 R0) = d.e' + |d|^2 h     (d = pixel - anchor, 4 operations),
+//   psi = Q (1 + b1 Q + b2 Q^2 + b3 Q^3 + b4 Q^4)     (sqrt(1 + y) - 1, y = Q k2 small),
+// where y is small (relative error below 3e-8 for reach / R0 <= 0.03), or from the exact
+// quotient otherwise, and the cell's polynomial at t0 + psi x cells per cycle. About 36
+// operations a pixel and chirp plus 100 per anchor, whatever the row's length.
+//
+// Bound: the FMA pipe (72% busy, 61% of the issue slots, on 512^2 x 2048 x 1024). What brought it
+// there, 1024^2 x 4096 x 1024 each: scalar FMAs 9.6 ms; pairs of pixels in FFMA2 (half the issue
+// slots) 7.7; the next anchor formed beside this one's pixels 7.5; blocks of 8 runs x 32 pixels a
+// warp instead of 256 pixels of a run, and chirp records staged in shared memory 32 at a time,
+// 7.2-7.4 (the cells' wait for memory: 1.5 -> 0.4 cycles an instruction). 64-thread CTAs at 128
+// registers: 16 warps an SM; 12 or 18 warps are 2-6% slower.
+template <int G>
+__global__ void __launch_bounds__(kThreads, G == 1 ? 6 : TDC_PROFILE_MINB)
+    profile_focus_kernel(const FocusJob *__restrict__ jobs, const FocusUnit *__restrict__ units, int n_units,
+                         int *__restrict__ counter)
+{
+    constexpr int kSub = kPT / G;  // anchors per thread
+    __shared__ SharedSums sums;
+    __shared__ __align__(16) SharedChirps recs[2];
+    __shared__ int s_unit;
+    __shared__ FocusUnit un;
+    __shared__ FocusJob sJ;
+    __shared__ ProfileJob sP;
+    const int tid = threadIdx.x;
+
+    for (;;) {
+        __syncthreads();
+        if (tid == 0) {
+            s_unit = atomicAdd(counter, 1);
+            if (s_unit < n_units) un = units[s_unit];
+        }
+        __syncthreads();
+        if (s_unit >= n_units) break;
+        for (int i = tid; i < (int)(sizeof(FocusJob) / sizeof(int)); i += kThreads)
+            reinterpret_cast<int *>(&sJ)[i] = reinterpret_cast<const int *>(&jobs[un.job])[i];
+        if (tid < (int)(sizeof(ProfileJob) / 16))
+            reinterpret_cast<float4 *>(&sP)[tid] = reinterpret_cast<const float4 *>(jobs[un.job].profile)[tid];
+        __syncthreads();
+
+        const int c0 = un.group * sJ.chirps_per_group;
+        const int c1 = min(sJ.C, c0 + sJ.chirps_per_group);
+
+        // anchors (the middle pixel of each group) and the pixels' offsets from them, in pairs
+        float ax[kSub][6];
+        float2 dx[kPT / 2], dy[kPT / 2];
+        int count;
+        long long p0 = run_pixels(sJ.P, sJ.grid_cols, un.tile, tid, count);
+#pragma unroll
+        for (int g = 0; g < kSub; ++g) {
+            const int valid = min(max(count - g * G, 0), G);
+            float4 hi = make_float4(0.f, 0.f, 0.f, 0.f), lo = hi;
+            if (valid) {
+                const long long a = p0 + g * G + valid / 2;
+                hi = __ldg(&sJ.grid_hi[a]);
+                if (sJ.grid_lo) lo = __ldg(&sJ.grid_lo[a]);
+            }
+            ax[g][0] = hi.x;
+            ax[g][1] = hi.y;
+            ax[g][2] = hi.z;
+            ax[g][3] = lo.x;
+            ax[g][4] = lo.y;
+            ax[g][5] = lo.z;
+            if (G > 1) {
+                float ox[G], oy[G], oz[G];
+#pragma unroll
+                for (int i = 0; i < G; ++i) {
+                    const int s = g * G + i;
+                    ox[i] = oy[i] = oz[i] = 0.f;
+                    if (s < count) {
+                        const float4 h = __ldg(&sJ.grid_hi[p0 + s]);
+                        const float4 l = sJ.grid_lo ? __ldg(&sJ.grid_lo[p0 + s]) : make_float4(0.f, 0.f, 0.f, 0.f);
+                        ox[i] = (h.x - hi.x) + (l.x - lo.x);
+                        oy[i] = (h.y - hi.y) + (l.y - lo.y);
+                        oz[i] = (h.z - hi.z) + (l.z - lo.z);
+                    }
+                }
+#pragma unroll
+                for (int i = 0; i + 1 < G; i += 2) {
+                    const int q = (g * G + i) / 2;
+                    dx[q] = make_float2(ox[i], ox[i + 1]);
+                    dy[q] = make_float2(oy[i], oy[i + 1]);
+                    const float2 dz = make_float2(oz[i], oz[i + 1]);
+                    sums.dz[q][tid] = dz;
+                    sums.dd[q][tid] = __ffma2_rn(dx[q], dx[q], __ffma2_rn(dy[q], dy[q], __fmul2_rn(dz, dz)));
+                }
+            }
+        }
+        float2 hc[kPT], hs[kPT];  // (hs stays zero where a pixel is its own anchor)
+#pragma unroll
+        for (int i = 0; i < kPT; ++i) {
+            hc[i] = hs[i] = make_float2(0.f, 0.f);
+            sums.s[i][tid] = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+
+        const ChirpRec *__restrict__ chirps = sJ.chirps;
+        const int *__restrict__ cell_base = sP.cell_base;
+        const float4 *__restrict__ cells = sP.cells;
+        const bool skip_test = (sJ.flags & kFlagSkipTest) != 0;
+        unsigned int dropped = 0;  // pixels whose current chunk the skip test drops
+        int chunk_end = c0;
+
+        int b0 = c0, buf = 0;  // first chirp of the staged records, and their buffer
+        auto anchor_of = [&](int k, const float (&p)[6]) {
+            Anchor n;
+            const float4 ph = recs[buf].p[k][0], pl = recs[buf].p[k][1];
+            const int base = recs[buf].base[k];
+            const float4 g = fresh(&sP.gc_hi);  // gc and cells per metre, high and low parts
+            const int n_cells = __float_as_int(fresh(&sP.inv_gc2x4).w);
+            float exl, eyl, ezl, rl, rs, dh;
+            dd_sub(ph.x, pl.x, p[0], p[3], n.ex, exl);
+            dd_sub(ph.y, pl.y, p[1], p[4], n.ey, eyl);
+            dd_sub(ph.z, pl.z, p[2], p[5], n.ez, ezl);
+            dd_range(n.ex, exl, n.ey, eyl, n.ez, ezl, n.rh, rl, rs, dh);
+            // its cell, and its place in it
+            const float kf = rintf(g.z * n.rh);
+            n.t0 = fmaf(g.z, n.rh, -kf);
+            n.t0 = fmaf(g.z, rl, n.t0);
+            n.t0 = fmaf(g.w, n.rh, n.t0);
+            const int cell = min(max((int)kf - base, 0), n_cells - 1);
+            const float4 *__restrict__ pc = cells + ((size_t)(b0 + k) * n_cells + cell) * (kProfileCoefs / 2);
+#pragma unroll
+            for (int m = 0; m < kProfileCoefs / 2; ++m) {
+                const float4 v = __ldg(pc + m);
+                n.a[2 * m] = make_float2(v.x, v.y);
+                n.a[2 * m + 1] = make_float2(v.z, v.w);
+            }
+            n.turn = kTwoPiF * dd_frac_mul(g.x, g.y, n.rh, rl);
+            // gc / (2 R0), 1 / R0 to FP32 rounding (rsqrt is not)
+            n.h = 0.5f * g.x * fmaf(rs, fmaf(-rl, rs, fmaf(-n.rh, rs, 1.0f)), rs);
+            return n;
+        };
+        // the next block's records are copied while this one is worked on: thread tid copies half of
+        // record tid / 2
+        auto copy_ahead = [&](int first, int to) {
+            if (first + (tid >> 1) < c1)
+                copy_async<16>(&recs[to].p[tid >> 1][tid & 1], &chirps[first + (tid >> 1)].p_hi + (tid & 1));
+            if (tid < kFlush && first + tid < c1) copy_async<4>(&recs[to].base[tid], &cell_base[first + tid]);
+        };
+        copy_ahead(c0, 0);
+
+        while (b0 < c1) {
+            copy_async_wait();
+            __syncthreads();  // this block's records are in, every thread is done with the last one's
+            if (skip_test && b0 >= chunk_end) {
+                // unbounded band: a chunk is dropped only where the test's first point is NaN
+                const int k = b0 / sJ.chunk;
+                chunk_end = (k + 1) * sJ.chunk;
+                dropped = 0;
+                p0 = run_pixels(sJ.P, sJ.grid_cols, un.tile, tid, count);  // (cheaper than two registers)
+                const float4 pf = __ldg(&sJ.skip[(size_t)k * 9].pos_fdc);
+                const float4 v = __ldg(&sJ.skip[(size_t)k * 9].vel);
+#pragma unroll 1
+                for (int i = 0; i < count; ++i) {
+                    const float4 h = __ldg(&sJ.grid_hi[p0 + i]);
+                    const float ex = pf.x - h.x, ey = pf.y - h.y, ez = pf.z - h.z;
+                    const float rs = rsqrtf(ex * ex + ey * ey + ez * ez);
+                    const float val =
+                        fabsf(doppler_freq(sJ.two_over_lambda, v.x, v.y, v.z, ex, ey, ez, rs) - pf.w);
+                    if (!(val <= sJ.half_bw)) dropped |= 1u << i;
+                }
+            }
+            int n = min(kFlush, c1 - b0);
+            if (skip_test) n = min(n, chunk_end - b0);
+            copy_ahead(b0 + n, buf ^ 1);
+            Anchor next;
+            if (G > 2) next = anchor_of(0, ax[0]);
+            for (int k = 0; k < n; ++k) {
+#pragma unroll
+                for (int g = 0; g < kSub; ++g) {
+                    // (one or two pixels an anchor: the thread's other anchors cover the latency)
+                    const Anchor cur = G > 2 ? next : anchor_of(k, ax[g]);
+                    if constexpr (G == 1) {
+                        // (the antenna on the pixel: NaN Doppler, zero window)
+                        float sn, cs;
+                        __sincosf(cur.turn, &sn, &cs);
+                        if (!(cur.rh > 0.0f)) sn = cs = 0.0f;
+                        float2 h = cur.a[kProfileCoefs - 1];
+#pragma unroll
+                        for (int m = kProfileCoefs - 2; m >= 0; --m) h = __ffma2_rn(h, both(cur.t0), cur.a[m]);
+                        hc[g].x = fmaf(cs, h.x, fmaf(-sn, h.y, hc[g].x));
+                        hc[g].y = fmaf(cs, h.y, fmaf(sn, h.x, hc[g].y));
+                    } else {
+                        float2 psi[G / 2];
+                        unsigned int zero = 0;  // pixels the antenna stands on
+                        const float4 jc = fresh(&sP.inv_gc2x4);  // 4 / gc^2, cells per cycle, r_safe
+                        if (cur.rh >= jc.z) {
+                            const float h = cur.h, h2 = -2.0f * h;
+                            const float e2x = h2 * cur.ex, e2y = h2 * cur.ey, e2z = h2 * cur.ez;
+                            const float k2 = h * jc.x;
+                            const float b1 = -0.25f * k2, b2 = 0.125f * k2 * k2;
+                            const float b3 = -0.625f * b2 * k2, b4 = 0.4375f * b2 * k2 * k2;
+#pragma unroll
+                            for (int i = 0; i < G / 2; ++i) {
+                                const int s = g * (G / 2) + i;
+                                const float2 q =
+                                    __ffma2_rn(dx[s], both(e2x),
+                                               __ffma2_rn(dy[s], both(e2y),
+                                                          __ffma2_rn(fresh2(&sums.dz[s][tid]), both(e2z), __fmul2_rn(fresh2(&sums.dd[s][tid]), both(h)))));
+                                float2 f = __ffma2_rn(q, both(b4), both(b3));
+                                f = __ffma2_rn(q, f, both(b2));
+                                f = __ffma2_rn(q, f, both(b1));
+                                psi[i] = __ffma2_rn(__fmul2_rn(q, q), f, q);
+                            }
+                        } else {
+                            // R - R0 = d.(d - 2 e) / (R0 + R): no cancellation, any R0
+#pragma unroll
+                            for (int i = 0; i < G; ++i) {
+                                const int s = (g * G + i) / 2;
+                                const float x = i & 1 ? dx[s].y : dx[s].x, y = i & 1 ? dy[s].y : dy[s].x,
+                                            z = i & 1 ? sums.dz[s][tid].y : sums.dz[s][tid].x;
+                                const float vx = cur.ex - x, vy = cur.ey - y, vz = cur.ez - z;
+                                const float num = fmaf(x, fmaf(-2.0f, cur.ex, x),
+                                                       fmaf(y, fmaf(-2.0f, cur.ey, y), z * fmaf(-2.0f, cur.ez, z)));
+                                const float r2 = fmaf(vx, vx, fmaf(vy, vy, vz * vz));
+                                const float den = cur.rh + sqrtf(r2);
+                                const float v = den > 0.0f ? sP.gc_hi * (num / den) : 0.0f;
+                                if (i & 1) psi[i / 2].y = v;
+                                else psi[i / 2].x = v;
+                                // (the antenna on the pixel: NaN Doppler, zero window)
+                                if (!(r2 > 0.0f)) zero |= 1u << i;
+                            }
+                        }
+                        if (zero) {
+#pragma unroll
+                            for (int i = 0; i < G; ++i)
+                                if ((zero & ~(dropped >> (g * G))) >> i & 1u)
+                                    stash(sums, g * G + i, tid, hc[g * G + i], hs[g * G + i]);
+                        }
+                        // the next anchor's chain of dependent operations runs beside this one's pixels
+                        if (G > 2) next = anchor_of(g + 1 < kSub ? k : min(k + 1, n - 1), ax[g + 1 < kSub ? g + 1 : 0]);
+#pragma unroll
+                        for (int i = 0; i < G; i += 2) {
+                            const int s = g * G + i;
+                            add_pair(psi[i / 2], cur.turn, cur.t0, jc.y, cur.a, hc[s], hs[s], hc[s + 1],
+                                     hs[s + 1]);
+                        }
+                        if (zero) {
+#pragma unroll
+                            for (int i = 0; i < G; ++i)
+                                if (zero >> i & 1u) hc[g * G + i] = hs[g * G + i] = make_float2(0.f, 0.f);
+                        }
+                    }
+                }
+            }
+            // the plain sums of these chirps (of one skip-test chunk) into the Kahan sums
+#pragma unroll
+            for (int i = 0; i < kPT; ++i) {
+                if (!(dropped >> i & 1u)) stash(sums, i, tid, hc[i], hs[i]);
+                hc[i] = hs[i] = make_float2(0.f, 0.f);
+            }
+            b0 += n;
+            buf ^= 1;
+        }
+
+        p0 = run_pixels(sJ.P, sJ.grid_cols, un.tile, tid, count);
+        float4 *__restrict__ part = sJ.partial + (size_t)un.group * sJ.P;
+#pragma unroll
+        for (int i = 0; i < kPT; ++i)
+            if (i < count) part[p0 + i] = sums.s[i][tid];
+    }
+}
+
+}  // namespace
+
+cudaError_t launch_profile_twiddle(float2 *twiddle, float *factor, int S, cudaStream_t st)
+{
+    const long long n = (long long)S * kNodes;
+    profile_twiddle_kernel<<<(unsigned)((n + 127) / 128), 128, 0, st>>>(twiddle, factor, S);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_profile_build(const ProfileBuild &b, cudaStream_t st)
+{
+    static const ProfileStencil stencil = make_stencil();
+    // nodes of n_cells / 2 from an even cell on, wherever the first block starts
+    const int blocks = (b.n_cells / 2 + kOwn - 2) / kOwn + 1;
+    const dim3 grid((b.C + kBuildChirps - 1) / kBuildChirps, blocks);
+    profile_build_kernel<<<grid, kBuildThreads, 0, st>>>(b, stencil);
+    return cudaGetLastError();
+}
+
+using ProfileFn = void (*)(const FocusJob *, const FocusUnit *, int, int *);
+
+static ProfileFn profile_fn(int group)
+{
+    switch (group) {
+    case 8: return profile_focus_kernel<8>;
+    case 4: return profile_focus_kernel<4>;
+    case 2: return profile_focus_kernel<2>;
+    default: return profile_focus_kernel<1>;
+    }
+}
+
+cudaError_t launch_focus_profile(int group, const FocusJob *jobs_dev, const FocusUnit *units_dev, int n_units,
+                                 int *counter_dev, int grid_ctas, cudaStream_t st)
+{
+    profile_fn(group)<<<grid_ctas, kThreads, 0, st>>>(jobs_dev, units_dev, n_units, counter_dev);
+    return cudaGetLastError();
+}
+
+int focus_profile_blocks_per_sm(int group)
+{
+    int blocks = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, profile_fn(group), kThreads, 0) != cudaSuccess) return 0;
+    return blocks;
+}
+
+}  // namespace tdc

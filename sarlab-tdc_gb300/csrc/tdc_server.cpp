@@ -91,6 +91,10 @@ constexpr int kMaxBatchJobs = 64;
 // gave p50 8.1-8.2 s against 8.5-8.8 s with 1e12, 8.7 s with 2.5e11 and 10.3 s with 2e12, at
 // the same p99 and throughput.)
 constexpr double kServerUnitWork = 1.0e9;
+// Range-profile tables of at most this many bytes per byte of a job's samples: the loop admits
+// jobs by their device memory, and a table many times the samples (a grid metres wide under few
+// samples a chirp) would keep several other jobs out. Such a job keeps the direct kernels.
+constexpr double kServerTableRatio = 6.0;
 #ifndef TDC_SERVER_BATCH_WORK
 #define TDC_SERVER_BATCH_WORK 5.0e11
 #endif
@@ -111,6 +115,7 @@ constexpr double kAging = TDC_SERVER_AGING;
 // batched (the FP64 general path: focused alone on the side stream).
 int job_kind(const FocusPlan &pl)
 {
+    if (pl.profile) return 3 + (pl.profile == 8 ? 3 : pl.profile == 4 ? 2 : pl.profile == 2 ? 1 : 0);
     if (pl.path == TDC_PATH_FP32_BULK) return pl.seg ? 1 : (pl.anchored ? 2 : 0);
     if (pl.path == TDC_PATH_GENERAL) return 16 + pl.variant;
     return -1;
@@ -121,6 +126,20 @@ int job_kind(const FocusPlan &pl)
 double kind_cost(int kind)
 {
     return kind >= 16 ? ((kind - 16) & 2 ? 9.0 : 5.5) : 1.0;
+}
+
+// Bulk-kernel correlations one (pixel, chirp) pair of a job stands for.
+double pair_work(const FocusPlan &pl, int n_samples)
+{
+    return pl.profile ? kProfilePairCost : n_samples * kind_cost(job_kind(pl));
+}
+
+// The same before the job is planned (its size decides, barring inputs that rule profiles out).
+double pair_work_estimate(const tdc_job_desc &d)
+{
+    const bool profile = !std::isfinite(d.doppler_bandwidth) &&
+                         profile_pays((double)d.n_pix, d.n_pri, d.n_samples);
+    return profile ? kProfilePairCost : d.n_samples;
 }
 
 size_t device_footprint(const tdc_job_desc &d, int n_sm)
@@ -134,6 +153,31 @@ size_t device_footprint(const tdc_job_desc &d, int n_sm)
     if (cpg > cpg_cap) groups = (d.n_pri + cpg_cap - 1) / cpg_cap;
     const size_t n_tiles = (P + kFocusTile - 1) / kFocusTile;
     size_t b = 0;
+    if (profile_pays((double)P, (double)C, (double)S)) {
+        // range profiles: the table over the grid's ranges, and this plan's groups where they are more
+        auto g = [&](long long i, int k) { return d.grid_f64 ? d.grid_f64[3 * i + k] : (double)d.grid[3 * i + k]; };
+        double lo[3], hi[3];
+        for (int k = 0; k < 3; ++k) lo[k] = hi[k] = g(0, k);
+        for (long long i = 1; i < (long long)P; ++i)
+            for (int k = 0; k < 3; ++k) {
+                lo[k] = std::min(lo[k], g(i, k));
+                hi[k] = std::max(hi[k], g(i, k));
+            }
+        const double dx = hi[0] - lo[0], dy = hi[1] - lo[1], dz = hi[2] - lo[2];
+        const double dt = S > 1 ? ((double)d.sample_times[S - 1] - d.sample_times[0]) / (S - 1) : 0.0;
+        const double cells_per_m = 4.0 * S * 2.0 * (double)d.mod_rate * dt / kC0 * 1.01;
+        const double diag = std::sqrt(dx * dx + dy * dy + dz * dz);
+        if (cells_per_m * diag < 4.0 * S &&
+            profile_table_fits(profile_cells(cells_per_m, diag) - 4, (int)S, kServerTableRatio))
+            b += C * (size_t)profile_cells(cells_per_m, diag) * kProfileCoefs * 8 + C * 4 + 48 + S * (kProfileNodes * 8 + 4);
+        int pg = 1, pcpg = d.n_pri;
+        plan_groups(profile_tiles((long long)P, detect_run((long long)P, g)), d.n_pri, n_sm * kProfileCtasPerSm, pg,
+                    pcpg, kProfileMinUnitsPerSlot);
+        const int cap = std::max(1, (int)(kServerUnitWork / ((double)kFocusTile * kProfilePairCost)));
+        if (pcpg > cap) pg = (d.n_pri + cap - 1) / cap;
+        groups = std::max(groups, pg);
+        b += ((size_t)profile_tiles((long long)P, detect_run((long long)P, g)) + 1) * groups * sizeof(FocusUnit);
+    }
     b += C * s_pad * 8;                 // samples
     b += C * sizeof(ChirpRec);          // records
     b += ((C + kChunk - 1) / kChunk) * 9 * sizeof(SkipPoint);
@@ -183,7 +227,7 @@ struct tdc_server {
     // kAging x time waited since submission, in seconds.
     double score(const Job *j, double t_ms) const
     {
-        const double rem = j->state == kQueued ? (double)j->d.n_pix * j->d.n_pri * j->d.n_samples
+        const double rem = j->state == kQueued ? (double)j->d.n_pix * j->d.n_pri * pair_work_estimate(j->d)
                                                : (double)(j->n_units - j->next_unit) * j->unit_work;
         return rem / kRateEstimate - kAging * (t_ms - j->t_submit) / 1e3;
     }
@@ -250,12 +294,16 @@ int tdc_server::admit_one(Job *j)
     // other jobs' launches run.
     if (p->image_dev.ensure((size_t)p->P * 8) != cudaSuccess || p->image_host.ensure((size_t)p->P * 8) != cudaSuccess)
         return set_last_error(TDC_ERR_NO_MEMORY, "image buffers");
+    if (j->plan.profile) {
+        int launches = 0;
+        if ((rc = profile_build(p, j->plan, p->stream, launches))) return rc;
+    }
     // The slot's buffers come from the stream-ordered pool on the slot's stream:
     // settle them before the launch streams use them.
     if (cudaStreamSynchronize(p->stream) != cudaSuccess) return set_last_error(TDC_ERR_CUDA, "slot stream sync");
     j->n_units = p->units_host.size();
     j->next_unit = 0;
-    j->unit_work = (double)kFocusTile * j->plan.job.chirps_per_group * d.n_samples * kind_cost(job_kind(j->plan));
+    j->unit_work = (double)kFocusTile * j->plan.job.chirps_per_group * pair_work(j->plan, d.n_samples);
     return TDC_OK;
 }
 
@@ -412,8 +460,10 @@ void tdc_server::launch_batch()
     const int kind = job_kind(members[0]->plan);
     const bool seg = kind == 1;
     const bool general = kind >= 16;
+    const int profile = members[0]->plan.profile;
     const int variant = general ? members[0]->plan.variant : 0;
-    const int bps = general    ? focus_general_blocks_per_sm(variant, stage_bytes)
+    const int bps = profile    ? focus_profile_blocks_per_sm(profile)
+                    : general  ? focus_general_blocks_per_sm(variant, stage_bytes)
                     : seg      ? focus_fp32_seg_blocks_per_sm(stage_bytes)
                     : anchored ? focus_fp32_anchor_blocks_per_sm(stage_bytes)
                                : focus_fp32_blocks_per_sm(stage_bytes);
@@ -422,7 +472,9 @@ void tdc_server::launch_batch()
     const FocusJob *jobs_d = reinterpret_cast<const FocusJob *>(d + kBatchOffJobs);
     const FocusUnit *units_d = reinterpret_cast<const FocusUnit *>(d + off_units);
     int *counter_d = reinterpret_cast<int *>(d);
-    if (general)
+    if (profile)
+        err |= launch_focus_profile(profile, jobs_d, units_d, (int)n_units, counter_d, grid, st) != cudaSuccess;
+    else if (general)
         err |= launch_focus_general(variant, jobs_d, units_d, (int)n_units, counter_d, counter_d + 1, stage_bytes, grid,
                                     st) != cudaSuccess;
     else if (seg)
@@ -627,6 +679,7 @@ int tdc_server_create(int device, size_t memory_budget_bytes, int max_jobs, tdc_
             s->free_slots.push_back(p);
             s->slot_mem[p] = 0;
             rc = processor_use_slot_stream(p, greatest);
+            p->table_ratio = kServerTableRatio;
         }
     }
     if (rc) {

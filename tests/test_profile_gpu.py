@@ -1,0 +1,97 @@
+"""GPU parity of the focus through range profiles (csrc/tdc_profile.cu): focuses of at least
+5e8 correlations read each (pixel, chirp) sum from a per-chirp table of the row's spectrum
+instead of summing the samples. Checked on pixel subsets against the FP64 oracle, over the
+forms the path takes: pixels sharing an anchor in groups of 8, 4, 2 and 1, ragged runs and
+bands, one run, odd row lengths, double-float inputs, ranges too short for the range-difference
+series, an antenna on a pixel, a falling chirp, rows beyond whole-row staging.
+
+Tolerance: relative L2 <= 3e-6, from the parts of the error (each rms, radians of phase or
+relative to the row): sample frequencies as an affine fit of FP32 sample times 1.5e-6,
+interpolation 3e-7, phase difference from the anchor 1e-6 at 5 cycles, FP32 sums 5e-7,
+sincos 3e-7."""
+import numpy as np
+import pytest
+
+import oracle
+from sarlabtdc import scenes
+from tdc_testutil import rel_l2
+
+pytestmark = pytest.mark.gpu
+
+INF = float("inf")
+L2_TOL = 3e-6
+
+
+def _check(sc, group, pos64=None, grid64=False, anchored=True, api=None, seed=3):
+    import _sarlabtdc
+
+    api = sc.api_arrays() if api is None else api
+    grid = sc.grid if grid64 else sc.grid.astype(np.float32)
+    p = _sarlabtdc.TdcProcessor(0)
+    p.setRawData(*api.values())
+    if pos64 is not None:
+        p.setChirpPositionsF64(pos64)
+    (p.setFocusGridF64 if grid64 else p.setFocusGrid)(grid)
+    p.setAnchoredRanges(anchored)
+    p.start(0.0, INF, False, False, True)
+    img, st = p.getFocusedImage().ravel(), p.lastStats()
+    # (rows are staged by the direct kernels only)
+    assert st["path_name"] == "fp32_bulk" and st["stage_samples"] == 0
+    assert st["anchor_pixels"] == (group if group > 1 else 0)
+    n = img.size
+    edge = [0, 7, 8, sc.grid.shape[1] - 1, sc.grid.shape[1] % n, n - 1]
+    pix = np.unique(np.concatenate([edge, np.random.default_rng(seed).choice(n, 60, replace=False)]))
+    prob = oracle.Problem(raw=api["rawData"], sampleTimes=api["sampleTimes"],
+                          position=pos64 if pos64 is not None else api["position"], velocity=api["velocity"],
+                          attitude=api["attitude"], modRate=api["modRate"], startFreq=api["startFreq"], grid=grid)
+    ref = oracle.focus(prob, oracle.Opts(applyRangeWin=False, dopplerBandwidth=INF), pixels=pix)
+    assert np.all(np.isfinite(img))
+    err = rel_l2(img[pix], ref)
+    assert err <= L2_TOL, err
+    return img
+
+
+@pytest.mark.parametrize("nx,ny,n_pri,n_samples,spacing,group", [
+    (57, 131, 300, 256, 1e-3, 8),     # ragged groups, a last band of 3 runs
+    (8, 512, 1024, 128, 2e-3, 8),     # one group a run
+    (129, 64, 129, 500, 2e-3, 8),     # one pixel more than whole groups, one chirp past a skip chunk
+    (9000, 1, 150, 400, 0.2e-3, 8),   # one long run
+    (70, 110, 256, 256, 3.9e-3, 4),
+    (70, 110, 256, 256, 8e-3, 2),
+    (70, 110, 256, 256, 2e-2, 1),
+    (64, 65, 1000, 123, 1e-3, 8),     # odd row length, many chirps
+    (256, 256, 40, 12345, 2e-3, 8),   # rows too long for whole-row stages
+    (301, 200, 64, 160, 1e-3, 8),     # two blocks of chirp records
+])
+def test_profile_focus_against_the_oracle(cuda_device, nx, ny, n_pri, n_samples, spacing, group):
+    sc = scenes.small_scene(seed=nx + n_samples, n_pri=n_pri, n_samples=n_samples, nx=nx, ny=ny, spacing=spacing,
+                            jitter=0.2e-3, device="cuda")
+    _check(sc, group)
+
+
+def test_profile_focus_double_float_inputs_and_no_anchors(cuda_device):
+    """FP64 positions and grid; and every range in double-float with anchored ranges off."""
+    sc = scenes.small_scene(seed=7, n_pri=320, n_samples=300, nx=83, ny=77, spacing=1.3e-3, jitter=0.5e-3,
+                            device="cuda")
+    a = _check(sc, 8, pos64=sc.positions, grid64=True)
+    b = _check(sc, 0, pos64=sc.positions, grid64=True, anchored=False)
+    assert rel_l2(a, b) <= 2 * L2_TOL
+
+
+def test_profile_focus_at_short_ranges(cuda_device):
+    """The antenna 2 cm above the grid's edge and, for one chirp, on a pixel (its window is zero
+    there): every range is too short for the series of the range difference."""
+    sc = scenes.small_scene(seed=8, n_pri=300, n_samples=256, nx=72, ny=110, height=0.02, y0=0.01, device="cuda")
+    api = sc.api_arrays()
+    api["position"] = np.array(api["position"])
+    api["position"][150, :, :] = sc.grid.astype(np.float32)[40, 21]
+    _check(sc, 8, api=api)
+
+
+def test_profile_focus_of_a_falling_chirp(cuda_device):
+    """81 to 77 GHz: the cells run backwards in range."""
+    sc = scenes.small_scene(seed=9, n_pri=300, n_samples=256, nx=72, ny=110, device="cuda")
+    rng = np.random.default_rng(10)
+    sc.radar = scenes.Radar(f0=81e9, bandwidth=-4e9, n_samples=256)
+    scenes.finish_raw(sc, scenes.simulate_raw(sc.positions, sc.targets, sc.amps, sc.radar, "cuda"), 20.0, rng)
+    _check(sc, 8)
