@@ -1184,12 +1184,14 @@ int profile_cells(double cells_per_m, double diagonal)
 }
 
 // Pixels sharing an anchor of a range-profile focus of the resident acquisition and grid, or 0
-// where the direct kernels run: finite band, kept per-chirp sums, non-finite inputs, small
+// where the direct kernels run: kept per-chirp sums, non-finite inputs, small
 // focuses (profile_pays), a grid wider than the unambiguous range, ranges beyond what the cell
 // index resolves in FP32, or a table larger than half the free device memory.
 int profile_group(tdc_processor *p, ProfileBuild &b)
 {
-    if (p->keep_sums || !p->rec_finite || std::isfinite(p->opts.bw / 2.0f)) return 0;
+    const float half_bw = p->opts.bw / 2.0f;
+    const bool band = std::isfinite(half_bw);
+    if (p->keep_sums || (!band && (!p->rec_finite || !(half_bw > 0.0f)))) return 0;
     const long long P = std::max(p->P, p->plan_pixels);
     if (!profile_pays((double)P, p->C, p->S)) return 0;
     const double g1 = 2.0 * p->F1 / kC0, gc = 2.0 * p->F0 / kC0 + g1 * (p->S / 2);
@@ -1296,7 +1298,7 @@ int focus_plan(tdc_processor *p, FocusPlan &plan, double max_unit_work)
         slots = p->n_sm * 4;
     }
 
-    const int tile_cols = choose_tile_cols(p);
+    const int tile_cols = profile ? 0 : choose_tile_cols(p);
     const int run = profile ? p->grid_run : 0;
     const long long n_tiles = profile ? profile_tiles(P, run) : tile_count(P, tile_cols, p->cols);
     // (block tiles also depend on the grid's shape, not only on its pixel count)
@@ -1308,8 +1310,9 @@ int focus_plan(tdc_processor *p, FocusPlan &plan, double max_unit_work)
                                                      : tile_count(p->plan_pixels, tile_cols, p->cols);
     if (path != p->plan_path || P != p->plan_P || C != p->plan_C || slots != p->plan_slots ||
         max_unit_work != p->plan_unit_cap || tile_cols != p->plan_tile_cols || plan_cols != p->plan_cols ||
-        plan_tiles != p->plan_tiles || profile != p->plan_profile || run != p->plan_run) {
-        int min_units = profile                    ? kProfileMinUnitsPerSlot
+        plan_tiles != p->plan_tiles || profile != p->plan_profile || (profile && std::isfinite(p->opts.bw) != p->plan_band) || run != p->plan_run) {
+        int min_units = profile && std::isfinite(p->opts.bw / 2.0f) ? kProfileBandMinUnitsPerSlot
+                        : profile                                    ? kProfileMinUnitsPerSlot
                         : path == TDC_PATH_GENERAL ? kGeneralMinUnitsPerSlot
                                                    : kFocusMinUnitsPerSlot;
         if (path == TDC_PATH_FP32_BULK && !profile && max_unit_work <= 0) {
@@ -1355,6 +1358,7 @@ int focus_plan(tdc_processor *p, FocusPlan &plan, double max_unit_work)
         p->plan_C = C;
         p->plan_slots = slots;
         p->plan_profile = profile;
+        p->plan_band = std::isfinite(p->opts.bw);
         p->plan_run = run;
         p->plan_uploaded = false;
     }
@@ -1400,7 +1404,6 @@ int focus_plan(tdc_processor *p, FocusPlan &plan, double max_unit_work)
         build.cell_base = reinterpret_cast<int *>(build.job_out + 1);
         ProfileJob &job = build.job;
         const double g1 = 2.0 * p->F1 / kC0, gc = 2.0 * p->F0 / kC0 + g1 * (p->S / 2);
-        plan.job.tile_cols = 0;
         plan.job.grid_cols = run;
         plan.job.profile = build.job_out;
         job.n_cells = build.n_cells;
@@ -1410,7 +1413,12 @@ int focus_plan(tdc_processor *p, FocusPlan &plan, double max_unit_work)
         split_dd(build.cells_per_m, job.cells_hi, job.cells_lo);
         job.cells_per_cycle = (float)(build.cells_per_m / gc);
         job.inv_gc2x4 = (float)(4.0 / (gc * gc));
-        const double reach = profile == 8 ? p->group_reach[0] : profile == 4 ? p->group_reach[1] : p->group_reach[2];
+        const double reach = profile == 8   ? p->group_reach[0]
+                             : profile == 4 ? p->group_reach[1]
+                             : profile == 2 ? p->group_reach[2]
+                                            : 0.0;
+        job.inv_gc = (float)(1.0 / gc);
+        job.reach = (float)reach;
         job.r_safe = (float)(reach / 0.03);
         plan.build = build;
     }
@@ -1492,8 +1500,9 @@ int focus_resident(tdc_processor *p, float2 *image_dev, cudaStream_t st, int &la
     int *status = counter + 1;
     if (plan.profile) {
         if (int rc = profile_build(p, plan, st, launches)) return rc;
-        const int grid = std::min(n_units, p->n_sm * focus_profile_blocks_per_sm(plan.profile));
-        TDC_CK(launch_focus_profile(plan.profile, jobs_dev, units_dev, n_units, counter, grid, st),
+        const bool band = std::isfinite(job.half_bw);
+        const int grid = std::min(n_units, p->n_sm * focus_profile_blocks_per_sm(plan.profile, band));
+        TDC_CK(launch_focus_profile(plan.profile, band, jobs_dev, units_dev, n_units, counter, grid, st),
                "focus kernel (range profiles)");
     } else if (path == TDC_PATH_FP32_BULK) {
         const int grid = std::min(n_units, slots);

@@ -152,8 +152,11 @@ struct __align__(16) ProfileJob {
     int n_cells;               // cells per chirp
     const float4 *cells;       // [C][n_cells][kProfileCoefs / 2]: pairs of complex polynomial coefficients
     const int *cell_base;      // [C] absolute index of each chirp's first cell
+    float inv_gc;              // 1 / gc
+    float reach;               // largest distance of a pixel from its anchor [m]
+    float pad_[2];
 };
-static_assert(sizeof(ProfileJob) == 48, "ProfileJob layout");
+static_assert(sizeof(ProfileJob) == 64, "ProfileJob layout");
 
 // Kernels copy a FocusJob into shared memory one int per thread (128 threads); the
 // no-allocation scratch reserves 256 bytes for it.
@@ -183,6 +186,7 @@ constexpr int kProfileCtasPerSm = TDC_PROFILE_CTAS;
 #define TDC_PROFILE_MIN_UNITS 3
 #endif
 constexpr int kProfileMinUnitsPerSlot = TDC_PROFILE_MIN_UNITS;
+constexpr int kProfileBandMinUnitsPerSlot = 8;  // (units differ in their live chirps)
 
 // Inputs and outputs of profile_build_kernel.
 struct ProfileBuild {
@@ -281,12 +285,12 @@ int focus_general_smem_bytes(int stage_bytes);
 
 // Range profiles: the per-length constants (twiddle [S][kProfileNodes], factor [S]), the table
 // of the resident acquisition over the grid's ranges, and the focus that reads it, with
-// `group` (8, 4, 2 or 1) consecutive pixels sharing an anchor.
+// `group` (8, 4, 2 or 1) consecutive pixels sharing an anchor (band: a finite Doppler band).
 cudaError_t launch_profile_twiddle(float2 *twiddle, float *factor, int S, cudaStream_t st);
 cudaError_t launch_profile_build(const ProfileBuild &b, cudaStream_t st);
-cudaError_t launch_focus_profile(int group, const FocusJob *jobs_dev, const FocusUnit *units_dev, int n_units,
+cudaError_t launch_focus_profile(int group, bool band, const FocusJob *jobs_dev, const FocusUnit *units_dev, int n_units,
                                  int *counter_dev, int grid_ctas, cudaStream_t st);
-int focus_profile_blocks_per_sm(int group);
+int focus_profile_blocks_per_sm(int group, bool band);
 // out[0..2] = max(out, largest distance of a pixel from the anchor of its group of 8 / 4 / 2
 // consecutive pixels of a run) as float bits (out starts at 0; a NaN compares above any distance).
 cudaError_t launch_group_reach(const float4 *hi, long long P, int run, int *out, cudaStream_t st);

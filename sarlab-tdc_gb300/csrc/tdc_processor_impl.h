@@ -217,6 +217,7 @@ struct tdc_processor {
     long long plan_P = -1;
     int plan_C = -1, plan_groups = 0, plan_cpg = 0, plan_path = -1, plan_slots = 0, plan_tile_cols = -1,
         plan_cols = -1, plan_profile = -1, plan_run = 0;
+    bool plan_band = false;
     double plan_unit_cap = 0.0;
     long long plan_tiles = -1;   // tiles the chirp groups were planned for
     long long plan_pixels = 0;   // plan the chirp groups for a grid of this many pixels (0: the grid's own)

@@ -299,9 +299,11 @@ struct SharedSums {
     float2 dd[kPT / 2][kThreads];
 };
 
-// Chirp records of kFlush chirps at a time: position (high, low) and first cell.
+// Chirp records of kFlush chirps at a time (position high and low, with a finite band the
+// velocity) and their first cells.
+template <bool BAND>
 struct SharedChirps {
-    float4 p[kFlush][2];
+    float4 p[kFlush][BAND ? 3 : 2];
     int base[kFlush];
 };
 
@@ -378,15 +380,17 @@ __device__ __forceinline__ float2 fresh2(const float2 *p)
 // and the anchor's cell and place in it.
 struct Anchor {
     float ex, ey, ez, rh, h, turn, t0;
+    float w;  // Doppler window (BAND with every pixel its own anchor)
     float2 a[kProfileCoefs];
 };
 
 // One chirp's contributions to two pixels with phase differences psi (cycles) from their
 // anchor: e^{j (turn + 2 pi psi)} A(t0 + psi cells_per_cycle), A the cell's polynomial with
-// coefficients a. Real and imaginary part of the value h advance together; the product with
+// coefficients a, times its window (WEIGHTED). Real and imaginary part of the value h advance together; the product with
 // the phasor is kept as h cos and h sin (c_i, s_i) and combined when the sums are flushed.
+template <bool WEIGHTED>
 __device__ __forceinline__ void add_pair(float2 psi, float turn, float t0, float cells_per_cycle,
-                                         const float2 (&a)[kProfileCoefs], float2 &c0, float2 &s0, float2 &c1,
+                                         const float2 (&a)[kProfileCoefs], float w0, float w1, float2 &c0, float2 &s0, float2 &c1,
                                          float2 &s1)
 {
     const float2 n = __fadd2_rn(__fadd2_rn(psi, both(12582912.0f)), both(-12582912.0f));  // nearest integer
@@ -395,6 +399,12 @@ __device__ __forceinline__ void add_pair(float2 psi, float turn, float t0, float
     float sn0, cs0, sn1, cs1;
     __sincosf(x.x, &sn0, &cs0);
     __sincosf(x.y, &sn1, &cs1);
+    if (WEIGHTED) {
+        cs0 *= w0;
+        sn0 *= w0;
+        cs1 *= w1;
+        sn1 *= w1;
+    }
     const float2 ta = both(t.x), tb = both(t.y);
     float2 h0 = a[kProfileCoefs - 1], h1 = h0;
 #pragma unroll
@@ -425,14 +435,18 @@ __device__ __forceinline__ void add_pair(float2 psi, float turn, float t0, float
 // warp instead of 256 pixels of a run, and chirp records staged in shared memory 32 at a time,
 // 7.2-7.4 (the cells' wait for memory: 1.5 -> 0.4 cycles an instruction). 64-thread CTAs at 128
 // registers: 16 warps an SM; 12 or 18 warps are 2-6% slower.
-template <int G>
-__global__ void __launch_bounds__(kThreads, G == 1 ? 6 : TDC_PROFILE_MINB)
+//
+// BAND: a finite Doppler band. Chirps out of band for all of a warp's pixels are found first, 32
+// at a time, from the anchors' Doppler and a bound on its change over a group (about 20
+// operations an anchor and chirp); the others weight each pixel with its own window.
+template <int G, bool BAND>
+__global__ void __launch_bounds__(kThreads, G == 1 ? (BAND ? 4 : 6) : BAND ? 6 : TDC_PROFILE_MINB)
     profile_focus_kernel(const FocusJob *__restrict__ jobs, const FocusUnit *__restrict__ units, int n_units,
                          int *__restrict__ counter)
 {
     constexpr int kSub = kPT / G;  // anchors per thread
     __shared__ SharedSums sums;
-    __shared__ __align__(16) SharedChirps recs[2];
+    __shared__ __align__(16) SharedChirps<BAND> recs[2];
     __shared__ int s_unit;
     __shared__ FocusUnit un;
     __shared__ FocusJob sJ;
@@ -543,6 +557,11 @@ __global__ void __launch_bounds__(kThreads, G == 1 ? 6 : TDC_PROFILE_MINB)
             n.turn = kTwoPiF * dd_frac_mul(g.x, g.y, n.rh, rl);
             // gc / (2 R0), 1 / R0 to FP32 rounding (rsqrt is not)
             n.h = 0.5f * g.x * fmaf(rs, fmaf(-rl, rs, fmaf(-n.rh, rs, 1.0f)), rs);
+            if (BAND && G == 1) {
+                const float4 v = recs[buf].p[k][2];
+                const float fd = doppler_freq(sJ.two_over_lambda, v.x, v.y, v.z, n.ex, n.ey, n.ez, rs);
+                n.w = doppler_window(fd, ph.w, sJ.half_bw, sJ.inv_bw, (sJ.flags & kFlagTaper) != 0, sJ.az_a);
+            }
             return n;
         };
         // the next block's records are copied while this one is worked on: thread tid copies half of
@@ -550,6 +569,7 @@ __global__ void __launch_bounds__(kThreads, G == 1 ? 6 : TDC_PROFILE_MINB)
         auto copy_ahead = [&](int first, int to) {
             if (first + (tid >> 1) < c1)
                 copy_async<16>(&recs[to].p[tid >> 1][tid & 1], &chirps[first + (tid >> 1)].p_hi + (tid & 1));
+            if (BAND && tid < kFlush && first + tid < c1) copy_async<16>(&recs[to].p[tid][BAND ? 2 : 0], &chirps[first + tid].vel);
             if (tid < kFlush && first + tid < c1) copy_async<4>(&recs[to].base[tid], &cell_base[first + tid]);
         };
         copy_ahead(c0, 0);
@@ -558,7 +578,7 @@ __global__ void __launch_bounds__(kThreads, G == 1 ? 6 : TDC_PROFILE_MINB)
             copy_async_wait();
             __syncthreads();  // this block's records are in, every thread is done with the last one's
             if (skip_test && b0 >= chunk_end) {
-                // unbounded band: a chunk is dropped only where the test's first point is NaN
+                // (unbounded band: a chunk is dropped only where the test's first point is NaN)
                 const int k = b0 / sJ.chunk;
                 chunk_end = (k + 1) * sJ.chunk;
                 dropped = 0;
@@ -568,6 +588,11 @@ __global__ void __launch_bounds__(kThreads, G == 1 ? 6 : TDC_PROFILE_MINB)
 #pragma unroll 1
                 for (int i = 0; i < count; ++i) {
                     const float4 h = __ldg(&sJ.grid_hi[p0 + i]);
+                    if (BAND) {
+                        if (!chunk_is_nonzero(sJ.skip + (size_t)k * 9, h.x, h.y, h.z, sJ.two_over_lambda, sJ.half_bw))
+                            dropped |= 1u << i;
+                        continue;
+                    }
                     const float ex = pf.x - h.x, ey = pf.y - h.y, ez = pf.z - h.z;
                     const float rs = rsqrtf(ex * ex + ey * ey + ez * ez);
                     const float val =
@@ -578,9 +603,35 @@ __global__ void __launch_bounds__(kThreads, G == 1 ? 6 : TDC_PROFILE_MINB)
             int n = min(kFlush, c1 - b0);
             if (skip_test) n = min(n, chunk_end - b0);
             copy_ahead(b0 + n, buf ^ 1);
+            unsigned int todo = 0xffffffffu >> (kFlush - n);  // chirps of the block still to add
+            if constexpr (BAND) {
+                unsigned int live = 0;
+                if (dropped != (1u << count) - 1u)  // (some pixel's chunk is seen)
+                    for (int k = 0; k < n; ++k) {
+                        const float4 p = recs[buf].p[k][0], v = recs[buf].p[k][2];
+                        bool any = false;
+#pragma unroll
+                        for (int g = 0; g < kSub; ++g) {
+                            const float ex = p.x - ax[g][0], ey = p.y - ax[g][1], ez = p.z - ax[g][2];
+                            const float rs = rsqrtf(fmaf(ex, ex, fmaf(ey, ey, ez * ez)));
+                            const float tol = sJ.two_over_lambda;
+                            const float fd = doppler_freq(tol, v.x, v.y, v.z, ex, ey, ez, rs);
+                            // directions within the group differ by at most 2 sin(asin(reach / R) / 2)
+                            const float rel = sP.reach * rs;
+                            const float bound = 1.05f * tol * (fabsf(v.x) + fabsf(v.y) + fabsf(v.z)) * rel +
+                                                1e-4f * (fabsf(fd) + fabsf(p.w) + sJ.half_bw) + 1e-6f;
+                            any |= !(fabsf(fd - p.w) > sJ.half_bw + bound) || !(rel < 0.4f);
+                        }
+                        if (any) live |= 1u << k;
+                    }
+                todo &= __reduce_or_sync(0xffffffffu, live);
+            }
+            int k = __ffs(todo) - 1;
             Anchor next;
-            if (G > 2) next = anchor_of(0, ax[0]);
-            for (int k = 0; k < n; ++k) {
+            if (G > 2 && todo) next = anchor_of(k, ax[0]);
+            while (todo) {
+                todo &= todo - 1;
+                const int k_next = todo ? __ffs(todo) - 1 : k;
 #pragma unroll
                 for (int g = 0; g < kSub; ++g) {
                     // (one or two pixels an anchor: the thread's other anchors cover the latency)
@@ -590,6 +641,10 @@ __global__ void __launch_bounds__(kThreads, G == 1 ? 6 : TDC_PROFILE_MINB)
                         float sn, cs;
                         __sincosf(cur.turn, &sn, &cs);
                         if (!(cur.rh > 0.0f)) sn = cs = 0.0f;
+                        if (BAND) {
+                            sn *= cur.w;
+                            cs *= cur.w;
+                        }
                         float2 h = cur.a[kProfileCoefs - 1];
 #pragma unroll
                         for (int m = kProfileCoefs - 2; m >= 0; --m) h = __ffma2_rn(h, both(cur.t0), cur.a[m]);
@@ -636,27 +691,85 @@ __global__ void __launch_bounds__(kThreads, G == 1 ? 6 : TDC_PROFILE_MINB)
                                 if (!(r2 > 0.0f)) zero |= 1u << i;
                             }
                         }
-                        if (zero) {
+                        if (!BAND && zero) {
 #pragma unroll
                             for (int i = 0; i < G; ++i)
                                 if ((zero & ~(dropped >> (g * G))) >> i & 1u)
                                     stash(sums, g * G + i, tid, hc[g * G + i], hs[g * G + i]);
                         }
+                        // Doppler windows of the pixels, fd = -(2 / lambda) v.(e - d) / R
+                        float w[G];
+                        if constexpr (BAND) {
+                            const float4 v = recs[buf].p[k][2];
+                            const float fdc = recs[buf].p[k][0].w, tol = sJ.two_over_lambda;
+                            const float half = sJ.half_bw, inv_bw = sJ.inv_bw, az = sJ.az_a;
+                            const bool taper = (sJ.flags & kFlagTaper) != 0;
+                            const float tx = tol * v.x, ty = tol * v.y, tz = tol * v.z;
+                            const float te = -fmaf(tx, cur.ex, fmaf(ty, cur.ey, tz * cur.ez));
+                            const float slack = 2e-6f * (fabsf(tx) + fabsf(ty) + fabsf(tz)) +
+                                                1e-6f * (fabsf(fdc) + half);
+                            unsigned int edge = 0;  // pixels at the band's edge to FP32 rounding
+#pragma unroll
+                            for (int i = 0; i < G; i += 2) {
+                                const int s = (g * G + i) / 2;
+                                const float2 dot =
+                                    __ffma2_rn(dx[s], both(tx),
+                                               __ffma2_rn(dy[s], both(ty),
+                                                          __ffma2_rn(fresh2(&sums.dz[s][tid]), both(tz), both(te))));
+                                const float2 r = __ffma2_rn(psi[i / 2], both(sP.inv_gc), both(cur.rh));
+#pragma unroll
+                                for (int q = 0; q < 2; ++q) {
+                                    const float df = __fdividef(q ? dot.y : dot.x, q ? r.y : r.x) - fdc;
+                                    w[i + q] = 0.0f;
+                                    if (fabsf(df) <= half)
+                                        w[i + q] = taper ? fmaf(1.0f - az, __cosf(kTwoPiF * df * inv_bw), az) : 1.0f;
+                                    if (fabsf(fabsf(df) - half) <= slack) edge |= 1u << (i + q);
+                                }
+                            }
+                            while (edge) {
+                                // the side of the edge is decided as the direct kernels decide it
+                                const int i = __ffs(edge) - 1;
+                                edge &= edge - 1;
+                                int m;
+                                const long long p = run_pixels(sJ.P, sJ.grid_cols, un.tile, tid, m) + g * G + i;
+                                const float4 ph = recs[buf].p[k][0], pl = recs[buf].p[k][1];
+                                const float4 hi = g * G + i < m ? __ldg(&sJ.grid_hi[p]) : ph;
+                                const float4 lo = g * G + i < m && sJ.grid_lo ? __ldg(&sJ.grid_lo[p])
+                                                                              : make_float4(0.f, 0.f, 0.f, 0.f);
+                                float ex, ey, ez, exl, eyl, ezl, rh, rl, rs, dh;
+                                dd_sub(ph.x, pl.x, hi.x, lo.x, ex, exl);
+                                dd_sub(ph.y, pl.y, hi.y, lo.y, ey, eyl);
+                                dd_sub(ph.z, pl.z, hi.z, lo.z, ez, ezl);
+                                dd_range(ex, exl, ey, eyl, ez, ezl, rh, rl, rs, dh);
+                                const float fd = doppler_freq(tol, v.x, v.y, v.z, ex, ey, ez, rs);
+                                const float we = doppler_window(fd, fdc, half, inv_bw, taper, az);
+#pragma unroll
+                                for (int q = 0; q < G; ++q)
+                                    if (q == i) w[q] = we;
+                            }
+#pragma unroll
+                            for (int i = 0; i < G; ++i)
+                                if (zero >> i & 1u) w[i] = 0.0f;
+                        } else {
+#pragma unroll
+                            for (int i = 0; i < G; ++i) w[i] = 1.0f;
+                        }
                         // the next anchor's chain of dependent operations runs beside this one's pixels
-                        if (G > 2) next = anchor_of(g + 1 < kSub ? k : min(k + 1, n - 1), ax[g + 1 < kSub ? g + 1 : 0]);
+                        if (G > 2) next = anchor_of(g + 1 < kSub ? k : k_next, ax[g + 1 < kSub ? g + 1 : 0]);
 #pragma unroll
                         for (int i = 0; i < G; i += 2) {
                             const int s = g * G + i;
-                            add_pair(psi[i / 2], cur.turn, cur.t0, jc.y, cur.a, hc[s], hs[s], hc[s + 1],
-                                     hs[s + 1]);
+                            add_pair<BAND>(psi[i / 2], cur.turn, cur.t0, jc.y, cur.a, w[i], w[i + 1], hc[s], hs[s], hc[s + 1],
+                                           hs[s + 1]);
                         }
-                        if (zero) {
+                        if (!BAND && zero) {
 #pragma unroll
                             for (int i = 0; i < G; ++i)
                                 if (zero >> i & 1u) hc[g * G + i] = hs[g * G + i] = make_float2(0.f, 0.f);
                         }
                     }
                 }
+                k = k_next;
             }
             // the plain sums of these chirps (of one skip-test chunk) into the Kahan sums
 #pragma unroll
@@ -697,27 +810,29 @@ cudaError_t launch_profile_build(const ProfileBuild &b, cudaStream_t st)
 
 using ProfileFn = void (*)(const FocusJob *, const FocusUnit *, int, int *);
 
+template <bool BAND>
 static ProfileFn profile_fn(int group)
 {
     switch (group) {
-    case 8: return profile_focus_kernel<8>;
-    case 4: return profile_focus_kernel<4>;
-    case 2: return profile_focus_kernel<2>;
-    default: return profile_focus_kernel<1>;
+    case 8: return profile_focus_kernel<8, BAND>;
+    case 4: return profile_focus_kernel<4, BAND>;
+    case 2: return profile_focus_kernel<2, BAND>;
+    default: return profile_focus_kernel<1, BAND>;
     }
 }
 
-cudaError_t launch_focus_profile(int group, const FocusJob *jobs_dev, const FocusUnit *units_dev, int n_units,
+cudaError_t launch_focus_profile(int group, bool band, const FocusJob *jobs_dev, const FocusUnit *units_dev, int n_units,
                                  int *counter_dev, int grid_ctas, cudaStream_t st)
 {
-    profile_fn(group)<<<grid_ctas, kThreads, 0, st>>>(jobs_dev, units_dev, n_units, counter_dev);
+    (band ? profile_fn<true>(group) : profile_fn<false>(group))<<<grid_ctas, kThreads, 0, st>>>(jobs_dev, units_dev, n_units, counter_dev);
     return cudaGetLastError();
 }
 
-int focus_profile_blocks_per_sm(int group)
+int focus_profile_blocks_per_sm(int group, bool band)
 {
     int blocks = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, profile_fn(group), kThreads, 0) != cudaSuccess) return 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, band ? profile_fn<true>(group) : profile_fn<false>(group),
+                                                      kThreads, 0) != cudaSuccess) return 0;
     return blocks;
 }
 

@@ -115,7 +115,9 @@ constexpr double kAging = TDC_SERVER_AGING;
 // batched (the FP64 general path: focused alone on the side stream).
 int job_kind(const FocusPlan &pl)
 {
-    if (pl.profile) return 3 + (pl.profile == 8 ? 3 : pl.profile == 4 ? 2 : pl.profile == 2 ? 1 : 0);
+    if (pl.profile)
+        return 3 + (pl.profile == 8 ? 3 : pl.profile == 4 ? 2 : pl.profile == 2 ? 1 : 0) +
+               (std::isfinite(pl.job.half_bw) ? 4 : 0);
     if (pl.path == TDC_PATH_FP32_BULK) return pl.seg ? 1 : (pl.anchored ? 2 : 0);
     if (pl.path == TDC_PATH_GENERAL) return 16 + pl.variant;
     return -1;
@@ -137,8 +139,7 @@ double pair_work(const FocusPlan &pl, int n_samples)
 // The same before the job is planned (its size decides, barring inputs that rule profiles out).
 double pair_work_estimate(const tdc_job_desc &d)
 {
-    const bool profile = !std::isfinite(d.doppler_bandwidth) &&
-                         profile_pays((double)d.n_pix, d.n_pri, d.n_samples);
+    const bool profile = profile_pays((double)d.n_pix, d.n_pri, d.n_samples);
     return profile ? kProfilePairCost : d.n_samples;
 }
 
@@ -169,10 +170,10 @@ size_t device_footprint(const tdc_job_desc &d, int n_sm)
         const double diag = std::sqrt(dx * dx + dy * dy + dz * dz);
         if (cells_per_m * diag < 4.0 * S &&
             profile_table_fits(profile_cells(cells_per_m, diag) - 4, (int)S, kServerTableRatio))
-            b += C * (size_t)profile_cells(cells_per_m, diag) * kProfileCoefs * 8 + C * 4 + 48 + S * (kProfileNodes * 8 + 4);
+            b += C * (size_t)profile_cells(cells_per_m, diag) * kProfileCoefs * 8 + C * 4 + sizeof(ProfileJob) + S * (kProfileNodes * 8 + 4);
         int pg = 1, pcpg = d.n_pri;
         plan_groups(profile_tiles((long long)P, detect_run((long long)P, g)), d.n_pri, n_sm * kProfileCtasPerSm, pg,
-                    pcpg, kProfileMinUnitsPerSlot);
+                    pcpg, std::isfinite(d.doppler_bandwidth / 2.0f) ? kProfileBandMinUnitsPerSlot : kProfileMinUnitsPerSlot);
         const int cap = std::max(1, (int)(kServerUnitWork / ((double)kFocusTile * kProfilePairCost)));
         if (pcpg > cap) pg = (d.n_pri + cap - 1) / cap;
         groups = std::max(groups, pg);
@@ -462,7 +463,7 @@ void tdc_server::launch_batch()
     const bool general = kind >= 16;
     const int profile = members[0]->plan.profile;
     const int variant = general ? members[0]->plan.variant : 0;
-    const int bps = profile    ? focus_profile_blocks_per_sm(profile)
+    const int bps = profile    ? focus_profile_blocks_per_sm(profile, skip_zero)
                     : general  ? focus_general_blocks_per_sm(variant, stage_bytes)
                     : seg      ? focus_fp32_seg_blocks_per_sm(stage_bytes)
                     : anchored ? focus_fp32_anchor_blocks_per_sm(stage_bytes)
@@ -473,7 +474,7 @@ void tdc_server::launch_batch()
     const FocusUnit *units_d = reinterpret_cast<const FocusUnit *>(d + off_units);
     int *counter_d = reinterpret_cast<int *>(d);
     if (profile)
-        err |= launch_focus_profile(profile, jobs_d, units_d, (int)n_units, counter_d, grid, st) != cudaSuccess;
+        err |= launch_focus_profile(profile, skip_zero, jobs_d, units_d, (int)n_units, counter_d, grid, st) != cudaSuccess;
     else if (general)
         err |= launch_focus_general(variant, jobs_d, units_d, (int)n_units, counter_d, counter_d + 1, stage_bytes, grid,
                                     st) != cudaSuccess;

@@ -95,3 +95,45 @@ def test_profile_focus_of_a_falling_chirp(cuda_device):
     sc.radar = scenes.Radar(f0=81e9, bandwidth=-4e9, n_samples=256)
     scenes.finish_raw(sc, scenes.simulate_raw(sc.positions, sc.targets, sc.amps, sc.radar, "cuda"), 20.0, rng)
     _check(sc, 8)
+
+
+@pytest.mark.parametrize("nx,ny,spacing,group,taper,centre,band,skip", [
+    (57, 131, 1e-3, 8, True, 0.0, 14.0, True),    # ragged groups, a partial last skip chunk
+    (131, 57, 2e-3, 8, False, 3.0, 9.0, True),    # rectangular window off the centre
+    (64, 80, 3.9e-3, 4, True, -2.0, 20.0, False),
+    (64, 80, 8e-3, 2, False, 0.0, 30.0, True),
+    (64, 80, 2e-2, 1, True, 0.0, 20.0, True),
+    (72, 110, 1e-3, 8, True, 500.0, 5.0, True),   # every chirp out of band
+])
+def test_profile_focus_under_a_finite_band(cuda_device, nx, ny, spacing, group, taper, centre, band, skip):
+    """Antenna moving along the rail; most chirps are out of band for a pixel. Tolerance 2e-4, as
+    for the direct kernels: a chirp at the inclusive edge of the band may fall on either side in
+    FP32 and FP64."""
+    import _sarlabtdc
+
+    sc = scenes.small_scene(seed=nx + ny, n_pri=750, n_samples=192, nx=nx, ny=ny, spacing=spacing, rail_len=0.75,
+                            device="cuda")
+    api = sc.api_arrays()
+    vel = np.zeros_like(api["velocity"])
+    vel[..., 0] = 0.08
+    api["velocity"] = vel
+    grid = sc.grid.astype(np.float32)
+    p = _sarlabtdc.TdcProcessor(0)
+    p.setRawData(*api.values())
+    p.setFocusGrid(grid)
+    p.setSkipTest(skip)
+    p.start(centre, band, False, False, taper)
+    img, st = p.getFocusedImage().ravel(), p.lastStats()
+    assert st["path_name"] == "fp32_bulk" and st["stage_samples"] == 0
+    assert st["anchor_pixels"] == (group if group > 1 else 0)
+    pix = np.unique(np.concatenate([[0, nx - 1, nx, img.size - 1],
+                                    np.random.default_rng(5).choice(img.size, 100, replace=False)]))
+    prob = oracle.Problem(raw=api["rawData"], sampleTimes=api["sampleTimes"], position=api["position"],
+                          velocity=api["velocity"], attitude=api["attitude"], modRate=api["modRate"],
+                          startFreq=api["startFreq"], grid=grid)
+    ref = oracle.focus(prob, oracle.Opts(dopplerWinCenter=centre, dopplerBandwidth=band, applyRangeWin=False,
+                                         dopplerWinTaper=taper, skip_test=skip), pixels=pix)
+    if not np.any(ref):
+        assert not np.any(img[pix])
+    else:
+        assert rel_l2(img[pix], ref) <= 2e-4
