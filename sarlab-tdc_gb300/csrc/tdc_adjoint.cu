@@ -357,21 +357,36 @@ __global__ void __launch_bounds__(kFocusThreads, 3)
     }
 }
 
-// grad[c] = sum over tiles of gpart[tile][c], in FP64, tile order.
-__global__ void adjoint_reduce_kernel(const float4 *__restrict__ gpart, int n_tiles, int C, double *__restrict__ grad)
+// grad[c] = sum over tiles of gpart[tile][c] in FP64, in a fixed order: 32 slices of a block's
+// threads each add a run of tiles, 4 loads in flight at a time, and the slices are added in order
+// (one thread per chirp over 512 tiles would wait for a load at a time).
+constexpr int kAdjReduceChirps = 16, kAdjReduceSlices = 32;
+__global__ void __launch_bounds__(kAdjReduceChirps *kAdjReduceSlices)
+    adjoint_reduce_kernel(const float4 *__restrict__ gpart, int n_tiles, int C, double *__restrict__ grad)
 {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= C) return;
+    __shared__ double part[kAdjReduceSlices][kAdjReduceChirps][3];
+    const int c = blockIdx.x * kAdjReduceChirps + threadIdx.x;
+    const int per = (n_tiles + kAdjReduceSlices - 1) / kAdjReduceSlices;
+    const int t0 = threadIdx.y * per, t1 = min(n_tiles, t0 + per);
     double x = 0.0, y = 0.0, z = 0.0;
-    for (int t = 0; t < n_tiles; ++t) {
-        const float4 v = gpart[(size_t)t * C + c];
-        x += v.x;
-        y += v.y;
-        z += v.z;
+    if (c < C) {
+#pragma unroll 4
+        for (int t = t0; t < t1; ++t) {
+            const float4 v = __ldg(&gpart[(size_t)t * C + c]);
+            x += v.x;
+            y += v.y;
+            z += v.z;
+        }
     }
-    grad[3 * c + 0] = x;
-    grad[3 * c + 1] = y;
-    grad[3 * c + 2] = z;
+    part[threadIdx.y][threadIdx.x][0] = x;
+    part[threadIdx.y][threadIdx.x][1] = y;
+    part[threadIdx.y][threadIdx.x][2] = z;
+    __syncthreads();
+    if (threadIdx.y < 3 && c < C) {
+        double s = 0.0;
+        for (int k = 0; k < kAdjReduceSlices; ++k) s += part[k][threadIdx.x][threadIdx.y];
+        grad[3 * c + threadIdx.y] = s;
+    }
 }
 
 }  // namespace
@@ -407,7 +422,8 @@ cudaError_t launch_adjoint_fp32(const FocusJob *jobs_dev, const FocusUnit *units
 cudaError_t launch_adjoint_reduce(const float4 *gpart, int n_tiles, int C, double *grad, cudaStream_t st)
 {
     if (C <= 0) return cudaSuccess;
-    adjoint_reduce_kernel<<<(C + 127) / 128, 128, 0, st>>>(gpart, n_tiles, C, grad);
+    adjoint_reduce_kernel<<<(C + kAdjReduceChirps - 1) / kAdjReduceChirps, dim3(kAdjReduceChirps, kAdjReduceSlices), 0,
+                            st>>>(gpart, n_tiles, C, grad);
     return cudaGetLastError();
 }
 

@@ -1184,14 +1184,14 @@ int profile_cells(double cells_per_m, double diagonal)
 }
 
 // Pixels sharing an anchor of a range-profile focus of the resident acquisition and grid, or 0
-// where the direct kernels run: kept per-chirp sums, non-finite inputs, small
+// where the direct kernels run: non-finite inputs, small
 // focuses (profile_pays), a grid wider than the unambiguous range, ranges beyond what the cell
 // index resolves in FP32, or a table larger than half the free device memory.
 int profile_group(tdc_processor *p, ProfileBuild &b)
 {
     const float half_bw = p->opts.bw / 2.0f;
     const bool band = std::isfinite(half_bw);
-    if (p->keep_sums || (!band && (!p->rec_finite || !(half_bw > 0.0f)))) return 0;
+    if (!band && (!p->rec_finite || !(half_bw > 0.0f))) return 0;
     const long long P = std::max(p->P, p->plan_pixels);
     if (!profile_pays((double)P, p->C, p->S)) return 0;
     const double g1 = 2.0 * p->F1 / kC0, gc = 2.0 * p->F0 / kC0 + g1 * (p->S / 2);
@@ -1449,6 +1449,7 @@ void processor_release_memory(tdc_processor *p)
     p->plan_uploaded = false;
     p->grid_lo_valid = false;
     p->twiddle_S = 0;
+    p->table_epoch = 0;
 }
 
 size_t processor_device_bytes(tdc_processor *p)
@@ -1474,7 +1475,7 @@ int focus_resident(tdc_processor *p, float2 *image_dev, cudaStream_t st, int &la
     // Autofocus: keep the per-(chirp, pixel) sums for the adjoint when they fit in half the
     // free device memory (whole-row FP32-bulk focus only).
     bool store = false;
-    if (p->keep_sums && path == TDC_PATH_FP32_BULK && !plan.seg && p->per_chirp) {
+    if (p->keep_sums && path == TDC_PATH_FP32_BULK && !plan.profile && !plan.seg && p->per_chirp) {
         const size_t bytes = (size_t)C * (size_t)P * sizeof(float2);
         size_t free_b = 0, total_b = 0;
         if (bytes <= p->chirp_sums.cap ||
@@ -1500,6 +1501,7 @@ int focus_resident(tdc_processor *p, float2 *image_dev, cudaStream_t st, int &la
     int *status = counter + 1;
     if (plan.profile) {
         if (int rc = profile_build(p, plan, st, launches)) return rc;
+        p->table_epoch = p->state_epoch;
         const bool band = std::isfinite(job.half_bw);
         const int grid = std::min(n_units, p->n_sm * focus_profile_blocks_per_sm(plan.profile, band));
         TDC_CK(launch_focus_profile(plan.profile, band, jobs_dev, units_dev, n_units, counter, grid, st),
@@ -1546,6 +1548,40 @@ int focus_resident(tdc_processor *p, float2 *image_dev, cudaStream_t st, int &la
     if (path == TDC_PATH_FP32_BULK && !plan.seg && plan.anchored && !store && !std::isfinite(job.half_bw) &&
         job.tile_cols == 0)
         p->stats.anchor_pixels = 32;
+    return TDC_OK;
+}
+
+// Adjoint through range profiles. The table is the forward's where it was built for the current
+// acquisition, trajectory and grid (stream-ordered before this call, as kept sums are), else
+// built here.
+int adjoint_profile(tdc_processor *p, const FocusPlan &plan, const float2 *gimg, double *grad, cudaStream_t st)
+{
+    const int C = p->C, n_units = (int)p->units_host.size(), n_tiles = plan.job.n_tiles;
+    int launches = 0;
+    if (p->table_epoch != p->state_epoch) {
+        if (int rc = profile_build(p, plan, st, launches)) return rc;
+        p->table_epoch = p->state_epoch;
+    }
+    const size_t off_job = 256;
+    const size_t off_units = round_up(off_job + sizeof(FocusJob), 256);
+    const size_t off_gpart = round_up(off_units + (size_t)n_units * sizeof(FocusUnit), 256);
+    TDC_CK(p->adj_scratch.ensure(off_gpart + (size_t)n_tiles * C * 16), "alloc adjoint scratch");
+    unsigned char *scr = p->adj_scratch.as<unsigned char>();
+    TDC_CK(cudaMemcpyAsync(scr + off_job, &plan.job, sizeof(FocusJob), cudaMemcpyHostToDevice, st), "copy job");
+    TDC_CK(cudaMemcpyAsync(scr + off_units, p->units_host.data(), (size_t)n_units * sizeof(FocusUnit),
+                           cudaMemcpyHostToDevice, st),
+           "copy units");
+    TDC_CK(cudaMemsetAsync(scr, 0, 8, st), "reset counter");
+    float4 *gpart = reinterpret_cast<float4 *>(scr + off_gpart);
+    const bool band = std::isfinite(plan.job.half_bw);
+    const int grid = std::min(n_units, p->n_sm * focus_profile_blocks_per_sm(plan.profile, band, true));
+    TDC_CK(launch_adjoint_profile(plan.profile, band, reinterpret_cast<const FocusJob *>(scr + off_job),
+                                  reinterpret_cast<const FocusUnit *>(scr + off_units), n_units,
+                                  reinterpret_cast<int *>(scr), grid, gimg, gpart, st),
+           "adjoint kernel (range profiles)");
+    TDC_CK(launch_adjoint_reduce(gpart, n_tiles, C, grad, st), "adjoint reduce kernel");
+    TDC_CK(cudaStreamSynchronize(st), "adjoint sync");
+    p->stats.adjoint_stored = 0;
     return TDC_OK;
 }
 
@@ -1951,10 +1987,14 @@ int tdc_processor_adjoint_device(tdc_processor *p, const float *grad_image_dev, 
     if (!p->per_chirp || choose_path(p) != TDC_PATH_FP32_BULK)
         return fail(TDC_ERR_UNSUPPORTED, "the adjoint needs the FP32-bulk path (per-chirp trajectory, uniform "
                                          "sample spacing)");
-    if (needs_segments(p->s_pad))
-        return fail(TDC_ERR_UNSUPPORTED, "the adjoint stages whole chirps: these chirps are too long");
     TDC_CK(cudaSetDevice(p->device), "cudaSetDevice");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (needs_segments(p->s_pad))
+        return fail(TDC_ERR_UNSUPPORTED, "the adjoint stages whole chirps: these chirps are too long");
+    FocusPlan plan;
+    if (int rc = focus_plan(p, plan)) return rc;
+    if (plan.profile)
+        return adjoint_profile(p, plan, reinterpret_cast<const float2 *>(grad_image_dev), grad_offsets_dev, st);
     const long long P = p->P;
     const int C = p->C;
     int cb = 1;

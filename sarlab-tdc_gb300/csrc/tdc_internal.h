@@ -290,7 +290,12 @@ cudaError_t launch_profile_twiddle(float2 *twiddle, float *factor, int S, cudaSt
 cudaError_t launch_profile_build(const ProfileBuild &b, cudaStream_t st);
 cudaError_t launch_focus_profile(int group, bool band, const FocusJob *jobs_dev, const FocusUnit *units_dev, int n_units,
                                  int *counter_dev, int grid_ctas, cudaStream_t st);
-int focus_profile_blocks_per_sm(int group, bool band);
+// Its adjoint: gpart[tile][C] = (d/dx, d/dy, d/dz) of each chirp over the tile's pixels (sums of
+// Re(conj(G) dI/dR) (P - T) / R; .w is not written).
+cudaError_t launch_adjoint_profile(int group, bool band, const FocusJob *jobs_dev, const FocusUnit *units_dev,
+                                   int n_units, int *counter_dev, int grid_ctas, const float2 *gimg, float4 *gpart,
+                                   cudaStream_t st);
+int focus_profile_blocks_per_sm(int group, bool band, bool adjoint = false);
 // out[0..2] = max(out, largest distance of a pixel from the anchor of its group of 8 / 4 / 2
 // consecutive pixels of a run) as float bits (out starts at 0; a NaN compares above any distance).
 cudaError_t launch_group_reach(const float4 *hi, long long P, int run, int *out, cudaStream_t st);

@@ -418,6 +418,51 @@ __device__ __forceinline__ void add_pair(float2 psi, float turn, float t0, float
     s1 = __ffma2_rn(h1, both(sn1), s1);
 }
 
+// Coefficients of D = A - j kappa A', kappa = cells per cycle / 2 pi (the adjoint).
+__device__ __forceinline__ void adjoint_coefs(const float2 (&a)[kProfileCoefs], float cells_per_cycle,
+                                              float2 (&d)[kProfileCoefs - 1])
+{
+    const float kappa = cells_per_cycle * (0.5f / kPiF);
+#pragma unroll
+    for (int m = 0; m < kProfileCoefs - 1; ++m) {
+        const float c = kappa * (float)(m + 1);
+        d[m] = make_float2(fmaf(c, a[m + 1].y, a[m].x), fmaf(-c, a[m + 1].x, a[m].y));
+    }
+}
+
+// One chirp's terms of the adjoint for two pixels: with D = (dF/dR) / (j 2 pi gc e^{j phase}) given
+// by the coefficients d, gi the image gradient (re, im) and range = R, adds
+// dl = Im(conj(gi) e^{j phase} D) / R and dl x offset to the sums.
+__device__ __forceinline__ void adjoint_pair(float2 psi, float turn, float t0, float cells_per_cycle,
+                                             const float2 (&d)[kProfileCoefs - 1], float w0, float w1, float2 g0,
+                                             float2 g1, float2 range, float2 dx, float2 dy, float2 dz, float2 &s,
+                                             float2 &sx, float2 &sy, float2 &sz)
+{
+    const float2 n = __fadd2_rn(__fadd2_rn(psi, both(12582912.0f)), both(-12582912.0f));
+    const float2 x = __ffma2_rn(__fadd2_rn(psi, make_float2(-n.x, -n.y)), both(kTwoPiF), both(turn));
+    const float2 t = __ffma2_rn(psi, both(cells_per_cycle), both(t0));
+    float sn0, cs0, sn1, cs1;
+    __sincosf(x.x, &sn0, &cs0);
+    __sincosf(x.y, &sn1, &cs1);
+    const float2 ta = both(t.x), tb = both(t.y);
+    float2 h0 = d[kProfileCoefs - 2], h1 = h0;
+#pragma unroll
+    for (int m = kProfileCoefs - 3; m >= 0; --m) {
+        h0 = __ffma2_rn(h0, ta, d[m]);
+        h1 = __ffma2_rn(h1, tb, d[m]);
+    }
+    // Im(conj(g) e^{j x} h) = (g.im cos - g.re sin)... written out: g = gi, t = e^{j x} h,
+    // g.im t.re - g.re t.im
+    const float p0 = g0.y * cs0 - g0.x * sn0, q0 = g0.y * sn0 + g0.x * cs0;
+    const float p1 = g1.y * cs1 - g1.x * sn1, q1 = g1.y * sn1 + g1.x * cs1;
+    const float2 dl = make_float2(w0 * __fdividef(p0 * h0.x - q0 * h0.y, range.x),
+                                  w1 * __fdividef(p1 * h1.x - q1 * h1.y, range.y));
+    s = __fadd2_rn(s, dl);
+    sx = __ffma2_rn(dl, dx, sx);
+    sy = __ffma2_rn(dl, dy, sy);
+    sz = __ffma2_rn(dl, dz, sz);
+}
+
 // Persistent CTAs of 64 threads over units (tile x chirp group) from an atomic counter, 8
 // pixels a thread. Per chirp, each G consecutive pixels share an anchor pixel: its range R0,
 // the carrier phase frac(gc R0) and the cell it reads (64 bytes, from L1 / L2: neighbouring
@@ -439,14 +484,20 @@ __device__ __forceinline__ void add_pair(float2 psi, float turn, float t0, float
 // BAND: a finite Doppler band. Chirps out of band for all of a warp's pixels are found first, 32
 // at a time, from the anchors' Doppler and a bound on its change over a group (about 20
 // operations an anchor and chirp); the others weight each pixel with its own window.
-template <int G, bool BAND>
-__global__ void __launch_bounds__(kThreads, G == 1 ? (BAND ? 4 : 6) : BAND ? 6 : TDC_PROFILE_MINB)
+//
+// ADJ: the adjoint with respect to the chirps' positions. F(R) = e^{j 2 pi gc R} A(t), so
+// dF/dR = j 2 pi gc e^{j ...} D, D = A - j (cells per cycle / 2 pi) A'(t): the same evaluation with
+// the coefficients of D, formed once an anchor. Each chirp's sum over the tile's pixels (two
+// shuffle steps, then shared memory, 32 chirps at a time) goes to gpart[tile][chirp].
+template <int G, bool BAND, bool ADJ>
+__global__ void __launch_bounds__(kThreads, G == 1 ? (BAND || ADJ ? 4 : 6) : BAND || (ADJ && G == 2) ? 6 : TDC_PROFILE_MINB)
     profile_focus_kernel(const FocusJob *__restrict__ jobs, const FocusUnit *__restrict__ units, int n_units,
-                         int *__restrict__ counter)
+                         int *__restrict__ counter, const float2 *__restrict__ gimg, float4 *__restrict__ gpart)
 {
     constexpr int kSub = kPT / G;  // anchors per thread
     __shared__ SharedSums sums;
     __shared__ __align__(16) SharedChirps<BAND> recs[2];
+    __shared__ float red[ADJ ? kFlush : 1][3][kThreads / 4];  // (ADJ) 8 partial sums a warp
     __shared__ int s_unit;
     __shared__ FocusUnit un;
     __shared__ FocusJob sJ;
@@ -521,6 +572,14 @@ __global__ void __launch_bounds__(kThreads, G == 1 ? (BAND ? 4 : 6) : BAND ? 6 :
             hc[i] = hs[i] = make_float2(0.f, 0.f);
             sums.s[i][tid] = make_float4(0.f, 0.f, 0.f, 0.f);
         }
+
+        float2 gi[kPT];  // (ADJ) image gradient of the pixels
+        auto load_gradient = [&](unsigned int without) {
+#pragma unroll
+            for (int i = 0; i < kPT; ++i)
+                gi[i] = i < count && !(without >> i & 1u) ? __ldg(&gimg[p0 + i]) : make_float2(0.f, 0.f);
+        };
+        if (ADJ) load_gradient(0);
 
         const ChirpRec *__restrict__ chirps = sJ.chirps;
         const int *__restrict__ cell_base = sP.cell_base;
@@ -599,10 +658,16 @@ __global__ void __launch_bounds__(kThreads, G == 1 ? (BAND ? 4 : 6) : BAND ? 6 :
                         fabsf(doppler_freq(sJ.two_over_lambda, v.x, v.y, v.z, ex, ey, ez, rs) - pf.w);
                     if (!(val <= sJ.half_bw)) dropped |= 1u << i;
                 }
+                if (ADJ) load_gradient(dropped);
             }
             int n = min(kFlush, c1 - b0);
             if (skip_test) n = min(n, chunk_end - b0);
             copy_ahead(b0 + n, buf ^ 1);
+            if (ADJ && BAND) {  // (chirps out of band keep zero sums)
+                if ((tid & 31) < 8)
+                    for (int i = 0; i < kFlush * 3; ++i) red[i / 3][i % 3][(tid >> 5) * 8 + (tid & 31)] = 0.f;
+                __syncwarp();
+            }
             unsigned int todo = 0xffffffffu >> (kFlush - n);  // chirps of the block still to add
             if constexpr (BAND) {
                 unsigned int live = 0;
@@ -632,6 +697,7 @@ __global__ void __launch_bounds__(kThreads, G == 1 ? (BAND ? 4 : 6) : BAND ? 6 :
             while (todo) {
                 todo &= todo - 1;
                 const int k_next = todo ? __ffs(todo) - 1 : k;
+                float grad[3] = {0.f, 0.f, 0.f};
 #pragma unroll
                 for (int g = 0; g < kSub; ++g) {
                     // (one or two pixels an anchor: the thread's other anchors cover the latency)
@@ -644,6 +710,19 @@ __global__ void __launch_bounds__(kThreads, G == 1 ? (BAND ? 4 : 6) : BAND ? 6 :
                         if (BAND) {
                             sn *= cur.w;
                             cs *= cur.w;
+                        }
+                        if constexpr (ADJ) {
+                            float2 d[kProfileCoefs - 1];
+                            adjoint_coefs(cur.a, fresh(&sP.inv_gc2x4).y, d);
+                            float2 h = d[kProfileCoefs - 2];
+#pragma unroll
+                            for (int m = kProfileCoefs - 3; m >= 0; --m) h = __ffma2_rn(h, both(cur.t0), d[m]);
+                            const float p = gi[g].y * cs - gi[g].x * sn, q = gi[g].y * sn + gi[g].x * cs;
+                            const float dl = cur.rh > 0.0f ? __fdividef(p * h.x - q * h.y, cur.rh) : 0.0f;
+                            grad[0] = fmaf(dl, cur.ex, grad[0]);
+                            grad[1] = fmaf(dl, cur.ey, grad[1]);
+                            grad[2] = fmaf(dl, cur.ez, grad[2]);
+                            continue;
                         }
                         float2 h = cur.a[kProfileCoefs - 1];
 #pragma unroll
@@ -691,7 +770,7 @@ __global__ void __launch_bounds__(kThreads, G == 1 ? (BAND ? 4 : 6) : BAND ? 6 :
                                 if (!(r2 > 0.0f)) zero |= 1u << i;
                             }
                         }
-                        if (!BAND && zero) {
+                        if (!BAND && !ADJ && zero) {
 #pragma unroll
                             for (int i = 0; i < G; ++i)
                                 if ((zero & ~(dropped >> (g * G))) >> i & 1u)
@@ -752,28 +831,69 @@ __global__ void __launch_bounds__(kThreads, G == 1 ? (BAND ? 4 : 6) : BAND ? 6 :
                                 if (zero >> i & 1u) w[i] = 0.0f;
                         } else {
 #pragma unroll
-                            for (int i = 0; i < G; ++i) w[i] = 1.0f;
+                            for (int i = 0; i < G; ++i) w[i] = ADJ && (zero >> i & 1u) ? 0.0f : 1.0f;
                         }
                         // the next anchor's chain of dependent operations runs beside this one's pixels
                         if (G > 2) next = anchor_of(g + 1 < kSub ? k : k_next, ax[g + 1 < kSub ? g + 1 : 0]);
+                        if constexpr (ADJ) {
+                            float2 d[kProfileCoefs - 1];
+                            adjoint_coefs(cur.a, jc.y, d);
+                            float2 sum = both(0.f), sx = sum, sy = sum, sz = sum;
+#pragma unroll
+                            for (int i = 0; i < G; i += 2) {
+                                const int s = (g * G + i) / 2;
+                                float2 r = __ffma2_rn(psi[i / 2], both(sP.inv_gc), both(cur.rh));
+                                if (zero >> i & 1u) r.x = 1.0f;
+                                if (zero >> (i + 1) & 1u) r.y = 1.0f;
+                                adjoint_pair(psi[i / 2], cur.turn, cur.t0, jc.y, d, w[i], w[i + 1], gi[g * G + i],
+                                             gi[g * G + i + 1], r, dx[s], dy[s], fresh2(&sums.dz[s][tid]), sum, sx, sy,
+                                             sz);
+                            }
+                            // sum over the pixels of dl (e - d)
+                            const float all = sum.x + sum.y;
+                            grad[0] += fmaf(all, cur.ex, -(sx.x + sx.y));
+                            grad[1] += fmaf(all, cur.ey, -(sy.x + sy.y));
+                            grad[2] += fmaf(all, cur.ez, -(sz.x + sz.y));
+                            continue;
+                        }
 #pragma unroll
                         for (int i = 0; i < G; i += 2) {
                             const int s = g * G + i;
                             add_pair<BAND>(psi[i / 2], cur.turn, cur.t0, jc.y, cur.a, w[i], w[i + 1], hc[s], hs[s], hc[s + 1],
                                            hs[s + 1]);
                         }
-                        if (!BAND && zero) {
+                        if (!BAND && !ADJ && zero) {
 #pragma unroll
                             for (int i = 0; i < G; ++i)
                                 if (zero >> i & 1u) hc[g * G + i] = hs[g * G + i] = make_float2(0.f, 0.f);
                         }
                     }
                 }
+                if constexpr (ADJ) {
+#pragma unroll
+                    for (int v = 0; v < 3; ++v) {
+                        grad[v] += __shfl_xor_sync(0xffffffffu, grad[v], 16);
+                        grad[v] += __shfl_xor_sync(0xffffffffu, grad[v], 8);
+                    }
+                    if ((tid & 31) < 8)
+#pragma unroll
+                        for (int v = 0; v < 3; ++v) red[k][v][(tid >> 5) * 8 + (tid & 31)] = grad[v];
+                }
                 k = k_next;
+            }
+            if constexpr (ADJ) {
+                __syncthreads();
+                float *__restrict__ out = reinterpret_cast<float *>(gpart + (size_t)un.tile * sJ.C + b0);
+                for (int i = tid; i < 3 * n; i += kThreads) {
+                    float s = 0.f;
+#pragma unroll
+                    for (int j = 0; j < kThreads / 4; ++j) s += red[i / 3][i % 3][j];
+                    out[4 * (i / 3) + i % 3] = kTwoPiF * sP.gc_hi * s;
+                }
             }
             // the plain sums of these chirps (of one skip-test chunk) into the Kahan sums
 #pragma unroll
-            for (int i = 0; i < kPT; ++i) {
+            for (int i = 0; i < (ADJ ? 0 : kPT); ++i) {
                 if (!(dropped >> i & 1u)) stash(sums, i, tid, hc[i], hs[i]);
                 hc[i] = hs[i] = make_float2(0.f, 0.f);
             }
@@ -781,6 +901,7 @@ __global__ void __launch_bounds__(kThreads, G == 1 ? (BAND ? 4 : 6) : BAND ? 6 :
             buf ^= 1;
         }
 
+        if (ADJ) continue;
         p0 = run_pixels(sJ.P, sJ.grid_cols, un.tile, tid, count);
         float4 *__restrict__ part = sJ.partial + (size_t)un.group * sJ.P;
 #pragma unroll
@@ -808,31 +929,42 @@ cudaError_t launch_profile_build(const ProfileBuild &b, cudaStream_t st)
     return cudaGetLastError();
 }
 
-using ProfileFn = void (*)(const FocusJob *, const FocusUnit *, int, int *);
+using ProfileFn = void (*)(const FocusJob *, const FocusUnit *, int, int *, const float2 *, float4 *);
 
-template <bool BAND>
+template <bool BAND, bool ADJ>
 static ProfileFn profile_fn(int group)
 {
     switch (group) {
-    case 8: return profile_focus_kernel<8, BAND>;
-    case 4: return profile_focus_kernel<4, BAND>;
-    case 2: return profile_focus_kernel<2, BAND>;
-    default: return profile_focus_kernel<1, BAND>;
+    case 8: return profile_focus_kernel<8, BAND, ADJ>;
+    case 4: return profile_focus_kernel<4, BAND, ADJ>;
+    case 2: return profile_focus_kernel<2, BAND, ADJ>;
+    default: return profile_focus_kernel<1, BAND, ADJ>;
     }
 }
 
-cudaError_t launch_focus_profile(int group, bool band, const FocusJob *jobs_dev, const FocusUnit *units_dev, int n_units,
-                                 int *counter_dev, int grid_ctas, cudaStream_t st)
+cudaError_t launch_focus_profile(int group, bool band, const FocusJob *jobs_dev, const FocusUnit *units_dev,
+                                 int n_units, int *counter_dev, int grid_ctas, cudaStream_t st)
 {
-    (band ? profile_fn<true>(group) : profile_fn<false>(group))<<<grid_ctas, kThreads, 0, st>>>(jobs_dev, units_dev, n_units, counter_dev);
+    const ProfileFn fn = band ? profile_fn<true, false>(group) : profile_fn<false, false>(group);
+    fn<<<grid_ctas, kThreads, 0, st>>>(jobs_dev, units_dev, n_units, counter_dev, nullptr, nullptr);
     return cudaGetLastError();
 }
 
-int focus_profile_blocks_per_sm(int group, bool band)
+cudaError_t launch_adjoint_profile(int group, bool band, const FocusJob *jobs_dev, const FocusUnit *units_dev,
+                                   int n_units, int *counter_dev, int grid_ctas, const float2 *gimg, float4 *gpart,
+                                   cudaStream_t st)
 {
+    const ProfileFn fn = band ? profile_fn<true, true>(group) : profile_fn<false, true>(group);
+    fn<<<grid_ctas, kThreads, 0, st>>>(jobs_dev, units_dev, n_units, counter_dev, gimg, gpart);
+    return cudaGetLastError();
+}
+
+int focus_profile_blocks_per_sm(int group, bool band, bool adjoint)
+{
+    const ProfileFn fn = adjoint ? (band ? profile_fn<true, true>(group) : profile_fn<false, true>(group))
+                                 : (band ? profile_fn<true, false>(group) : profile_fn<false, false>(group));
     int blocks = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, band ? profile_fn<true>(group) : profile_fn<false>(group),
-                                                      kThreads, 0) != cudaSuccess) return 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, fn, kThreads, 0) != cudaSuccess) return 0;
     return blocks;
 }
 

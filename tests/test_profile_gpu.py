@@ -137,3 +137,67 @@ def test_profile_focus_under_a_finite_band(cuda_device, nx, ny, spacing, group, 
         assert not np.any(img[pix])
     else:
         assert rel_l2(img[pix], ref) <= 2e-4
+
+
+@pytest.mark.parametrize("nx,ny,spacing,group,band,anchored", [
+    (57, 131, 1e-3, 8, INF, True),
+    (64, 80, 3.9e-3, 4, INF, True),
+    (64, 80, 8e-3, 2, INF, True),
+    (64, 80, 1e-3, 1, INF, False),
+    (57, 131, 1e-3, 8, 14.0, True),
+    (64, 80, 1e-3, 1, 14.0, False),
+])
+def test_profile_adjoint_against_the_oracle(cuda_device, nx, ny, spacing, group, band, anchored):
+    """Gradient of a real loss of the image for every chirp's position, at offsets from the base
+    trajectory, with and without a forward before it: against the FP64 oracle to 3e-6 relative
+    L2, as the image (its parts scale alike); under a finite band, where FP32 and FP64 can put a
+    chirp on either side of the edge, against the direct adjoint of the grid's two halves (too
+    small for profiles; the gradient is a sum over pixels) to twice that."""
+    import torch
+
+    import _sarlabtdc
+
+    sc = scenes.small_scene(seed=nx + ny, n_pri=520, n_samples=192, nx=nx, ny=ny, spacing=spacing, rail_len=0.52,
+                            jitter=0.2e-3, device="cuda")
+    api = sc.api_arrays()
+    vel = np.zeros_like(api["velocity"])
+    vel[..., 0] = 0.08
+    api["velocity"] = vel
+    p = _sarlabtdc.TdcProcessor(0)
+    p.setRawData(*api.values())
+    p.setChirpPositionsF64(sc.positions)
+    p.setFocusGridF64(sc.grid)
+    p.setAnchoredRanges(anchored)
+    p.prepare(0.0, band, False, False, True)
+    p.uploadGrid()
+    p.keepChirpSums(True)
+    rng = np.random.default_rng(11)
+    off = rng.normal(0, 0.1e-3, (sc.n_pri, 3))
+    g = (rng.normal(size=nx * ny) + 1j * rng.normal(size=nx * ny)).astype(np.complex64)
+    off_d, g_d = torch.from_numpy(off).cuda(), torch.from_numpy(g).cuda()
+    p.setChirpOffsetsDevice(off_d)
+    grad = torch.empty((sc.n_pri, 3), dtype=torch.float64, device="cuda")
+    p.adjointDevice(g_d, grad)
+    alone = grad.cpu().numpy()
+    img = torch.empty(nx * ny, dtype=torch.complex64, device="cuda")
+    p.focusDevice(img)
+    assert p.lastStats()["anchor_pixels"] == (group if group > 1 else 0)
+    p.adjointDevice(g_d, grad)
+    assert p.lastStats()["adjoint_stored"] == 0
+    np.testing.assert_array_equal(grad.cpu().numpy(), alone)
+    if np.isinf(band):
+        prob = oracle.Problem(raw=api["rawData"], sampleTimes=api["sampleTimes"], position=sc.positions,
+                              velocity=vel[:, 0, :], modRate=api["modRate"], startFreq=api["startFreq"], grid=sc.grid)
+        ref = oracle.adjoint_offsets(prob, oracle.Opts(applyRangeWin=False), off, g.astype(np.complex128))
+        assert rel_l2(alone, ref) <= 3e-6
+        return
+    ref = np.zeros_like(alone)
+    half = ny // 2
+    for rows in (slice(0, half), slice(half, ny)):
+        part = np.ascontiguousarray(sc.grid[rows])
+        p.setFocusGridF64(part)
+        p.uploadGrid()
+        g_part = torch.from_numpy(np.ascontiguousarray(g.reshape(ny, nx)[rows].ravel())).cuda()
+        p.adjointDevice(g_part, grad)
+        ref += grad.cpu().numpy()
+    assert rel_l2(alone, ref) <= 6e-6
