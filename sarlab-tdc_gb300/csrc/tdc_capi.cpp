@@ -407,10 +407,12 @@ int prepare(tdc_processor *p, const StartOpts &o, int &launches)
     // ulp of the chirp's largest FP32 coordinate on that axis, i.e. what remains is the rounding
     // of the input (up to half an ulp per sample, spread a little further by the fit).
     std::vector<MotionRec> mrecs;
+    std::vector<MoveRec> vrecs;  // the same fits about the middle sample (range profiles)
     p->motion_fit_ok = false;
     p->motion_v1max = p->motion_v2max = 0.0;
     if (p->traj_varies && !p->win_varies && S >= 3) {
         mrecs.resize(C);
+        vrecs.resize(C);
         const double hs = 0.5 * (S - 1);
         double sxx = 0.0, m2 = 0.0, sqq = 0.0;
         for (int s = 0; s < S; ++s) m2 += (s - hs) * (s - hs);
@@ -465,6 +467,18 @@ int prepare(tdc_processor *p, const StartOpts &o, int &launches)
                                     (float)(2.0 * (V1[0] * V2[0] + V1[1] * V2[1] + V1[2] * V2[2])));
                 m.v1 = make_float4((float)V1[0], (float)V1[1], (float)V1[2], (float)(n1 * n1));
                 m.v2 = make_float4((float)V2[0], (float)V2[1], (float)V2[2], (float)(n2 * n2));
+                MoveRec &mv = vrecs[c];
+                const double sc = S / 2;
+                double w1[3], n2w = 0.0;
+                for (int k = 0; k < 3; ++k) {
+                    split_dd((double)p0[k] + V0[k] + sc * (V1[k] + sc * V2[k]), h[k], l[k]);
+                    w1[k] = V1[k] + 2.0 * sc * V2[k];
+                    n2w += w1[k] * w1[k];
+                }
+                mv.p_hi = make_float4(h[0], h[1], h[2], 0.f);
+                mv.p_lo = make_float4(l[0], l[1], l[2], 0.f);
+                mv.w1 = make_float4((float)w1[0], (float)w1[1], (float)w1[2], (float)n2w);
+                mv.v2 = make_float4((float)V2[0], (float)V2[1], (float)V2[2], 0.f);
                 v1m = std::max(v1m, n1);
                 v2m = std::max(v2m, n2);
             }
@@ -583,7 +597,11 @@ int prepare(tdc_processor *p, const StartOpts &o, int &launches)
         TDC_CK(cudaMemcpyAsync(p->motion_rec.p, mrecs.data(), mrecs.size() * sizeof(MotionRec),
                                cudaMemcpyHostToDevice, st),
                "copy motion records");
-        p->stats.h2d_bytes += (int64_t)(mrecs.size() * sizeof(MotionRec));
+        TDC_CK(p->move_rec.ensure(vrecs.size() * sizeof(MoveRec)), "alloc motion records");
+        TDC_CK(cudaMemcpyAsync(p->move_rec.p, vrecs.data(), vrecs.size() * sizeof(MoveRec), cudaMemcpyHostToDevice,
+                               st),
+               "copy motion records");
+        p->stats.h2d_bytes += (int64_t)(mrecs.size() * sizeof(MotionRec) + vrecs.size() * sizeof(MoveRec));
     }
     if (!wdot.empty()) {
         TDC_CK(p->wdot.ensure(wdot.size() * sizeof(float)), "alloc per-sample window offsets");
@@ -1171,6 +1189,11 @@ bool profile_pays(double n_pix, double n_pri, double n_samples)
     return n_pix >= 4.0 * n_samples && n_pix * n_pri * n_samples >= TDC_PROFILE_MIN_WORK;
 }
 
+// Smooth motion through range profiles: largest bend of the phase at a row's ends [rad].
+constexpr double kMoveMaxBend = 0.1;
+// ... and of its difference within a group [rad] (the neglected second order is half its square).
+constexpr double kMoveMaxTurn = 4e-3;
+
 bool profile_table_fits(int n_cells, int n_samples, double table_ratio)
 {
     return table_ratio <= 0.0 || n_cells * (kProfileCoefs * 8.0) <= table_ratio * (n_samples * 8.0);
@@ -1187,7 +1210,7 @@ int profile_cells(double cells_per_m, double diagonal)
 // where the direct kernels run: non-finite inputs, small
 // focuses (profile_pays), a grid wider than the unambiguous range, ranges beyond what the cell
 // index resolves in FP32, or a table larger than half the free device memory.
-int profile_group(tdc_processor *p, ProfileBuild &b)
+int profile_group(tdc_processor *p, int path, ProfileBuild &b)
 {
     const float half_bw = p->opts.bw / 2.0f;
     const bool band = std::isfinite(half_bw);
@@ -1205,6 +1228,24 @@ int profile_group(tdc_processor *p, ProfileBuild &b)
     const double rmax = max_range(p->ant_min, p->ant_max, p->grid_min, p->grid_max);
     if (!(std::fabs(b.cells_per_m) * rmax < 2097152.0) || !(diag2 >= 0.0) || !(std::fabs(gc) > 0.0)) return 0;
     b.n_cells = profile_cells(b.cells_per_m, std::sqrt(diag2));
+    b.margin = 0;
+    b.chirp_words = 3;
+    const bool motion = path == TDC_PATH_FP32_MOTION;
+    double slack = 0.0, max_bend = 0.0;  // largest shift of a pixel's cell [cells], bend [rad]
+    const double rmin = min_range(p->ant_min, p->ant_max, p->grid_min, p->grid_max);
+    const double w1 = p->motion_v1max + 2.0 * p->motion_v2max * p->S, h = 0.5 * p->S;
+    if (motion) {
+        // (motion_segment has bounded the motion: rmin > 0)
+        const double bend = 2.0 * M_PI * h * h *
+                            (std::fabs(g1) * w1 + std::fabs(gc) * (w1 * w1 / (2.0 * rmin) + p->motion_v2max));
+        const double shift = 4.0 * p->S * std::fabs(gc) * w1;
+        if (band || !(bend <= kMoveMaxBend) || !(shift <= 64.0)) return 0;
+        b.margin = 2 * (int)std::ceil(0.5 * shift) + 2;
+        b.n_cells += 2 * b.margin;
+        b.chirp_words = 4;
+        slack = shift;
+        max_bend = bend;
+    }
     if (b.n_cells > 4LL * p->S || !profile_table_fits(b.n_cells, p->S, p->table_ratio)) return 0;
     b.C = p->C;
     b.S = p->S;
@@ -1222,7 +1263,15 @@ int profile_group(tdc_processor *p, ProfileBuild &b)
     if (!p->anchor_enabled) return 1;
     // |t| <= 1/2 (the anchor's place in its cell) + the group's reach
     for (int k = 0; k < 3; ++k)
-        if (std::fabs(b.cells_per_m) * p->group_reach[k] <= kProfileReach - 0.52) return 8 >> k;
+    {
+        const double reach = p->group_reach[k], turn = motion ? 2.0 * reach / rmin : 0.0;
+        // moving antennas: the group's spread of directions (turn) changes its pixels' shifts, their
+        // bends (kept to first order) and the part of the bend from V2 (taken as the anchor's)
+        if (motion && !(turn * max_bend <= kMoveMaxTurn &&
+                        2.0 * M_PI * h * h * std::fabs(gc) * p->motion_v2max * turn <= 2e-6))
+            continue;
+        if (std::fabs(b.cells_per_m) * reach + slack * turn <= kProfileReach - 0.52) return 8 >> k;
+    }
     return 1;
 }
 
@@ -1278,7 +1327,7 @@ int focus_plan(tdc_processor *p, FocusPlan &plan, double max_unit_work)
     int slots;
     bool anchored = false;
     ProfileBuild build{};
-    const int profile = path == TDC_PATH_FP32_BULK ? profile_group(p, build) : 0;
+    const int profile = path == TDC_PATH_FP32_BULK || path == TDC_PATH_FP32_MOTION ? profile_group(p, path, build) : 0;
     if (profile) {
         slots = p->n_sm * kProfileCtasPerSm;
     } else if (path == TDC_PATH_FP32_MOTION) {
@@ -1396,7 +1445,8 @@ int focus_plan(tdc_processor *p, FocusPlan &plan, double max_unit_work)
     plan.job.n_tiles = (int)n_tiles;
     if (profile) {
         build.rows = p->xw.as<const float2>();
-        build.chirps = plan.job.chirps;
+        if (path == TDC_PATH_FP32_MOTION) plan.job.chirps = reinterpret_cast<const ChirpRec *>(p->move_rec.p);
+        build.chirps = reinterpret_cast<const float4 *>(plan.job.chirps);
         build.twiddle = p->twiddle.as<const float2>();
         build.factor = reinterpret_cast<const float *>(build.twiddle + (size_t)p->S * kProfileNodes);
         build.cells = p->cells.as<float4>();
@@ -1418,6 +1468,11 @@ int focus_plan(tdc_processor *p, FocusPlan &plan, double max_unit_work)
                              : profile == 2 ? p->group_reach[2]
                                             : 0.0;
         job.inv_gc = (float)(1.0 / gc);
+        const double h = 0.5 * p->S;
+        job.rate_cells = (float)(4.0 * p->S * gc);
+        job.bend1 = (float)(2.0 * M_PI * h * h * g1);
+        job.bend2 = (float)(M_PI * h * h * gc);
+        job.bend3 = (float)(2.0 * M_PI * h * h * h * g1);
         job.reach = (float)reach;
         job.r_safe = (float)(reach / 0.03);
         plan.build = build;
@@ -1503,8 +1558,9 @@ int focus_resident(tdc_processor *p, float2 *image_dev, cudaStream_t st, int &la
         if (int rc = profile_build(p, plan, st, launches)) return rc;
         p->table_epoch = p->state_epoch;
         const bool band = std::isfinite(job.half_bw);
-        const int grid = std::min(n_units, p->n_sm * focus_profile_blocks_per_sm(plan.profile, band));
-        TDC_CK(launch_focus_profile(plan.profile, band, jobs_dev, units_dev, n_units, counter, grid, st),
+        const bool motion = path == TDC_PATH_FP32_MOTION;
+        const int grid = std::min(n_units, p->n_sm * focus_profile_blocks_per_sm(plan.profile, band, false, motion));
+        TDC_CK(launch_focus_profile(plan.profile, band, motion, jobs_dev, units_dev, n_units, counter, grid, st),
                "focus kernel (range profiles)");
     } else if (path == TDC_PATH_FP32_BULK) {
         const int grid = std::min(n_units, slots);
@@ -1536,13 +1592,14 @@ int focus_resident(tdc_processor *p, float2 *image_dev, cudaStream_t st, int &la
     p->sums_epoch = store ? p->state_epoch : 0;
     p->stats.path = path;
     p->stats.correlations = (int64_t)P * C * p->S;
-    const bool staged = (path == TDC_PATH_FP32_BULK && !plan.profile) || path == TDC_PATH_GENERAL || path == TDC_PATH_FP32_MOTION;
+    const bool staged = !plan.profile && (path == TDC_PATH_FP32_BULK || path == TDC_PATH_GENERAL ||
+                                          path == TDC_PATH_FP32_MOTION);
     const int row = path == TDC_PATH_GENERAL ? job.seg_len : plan.seg ? kSegmentSamples : p->s_pad;
     p->stats.stage_samples = staged ? std::min(row, p->s_pad) : 0;
     p->stats.stage_chirps = staged ? (row < p->s_pad ? 1 : plan.cb) : 0;
     p->stats.general_variant = path == TDC_PATH_GENERAL ? plan.variant : 0;
     p->stats.tile_cols = job.tile_cols;
-    p->stats.motion_segment = path == TDC_PATH_FP32_MOTION ? job.seg_len : 0;
+    p->stats.motion_segment = path == TDC_PATH_FP32_MOTION && !plan.profile ? job.seg_len : 0;
     p->stats.span_permille = path == TDC_PATH_FP32_BULK && !plan.seg && !store ? p->span_permille : 1000;
     p->stats.anchor_pixels = plan.profile > 1 ? plan.profile : 0;
     if (path == TDC_PATH_FP32_BULK && !plan.seg && plan.anchored && !store && !std::isfinite(job.half_bw) &&
@@ -1574,7 +1631,7 @@ int adjoint_profile(tdc_processor *p, const FocusPlan &plan, const float2 *gimg,
     TDC_CK(cudaMemsetAsync(scr, 0, 8, st), "reset counter");
     float4 *gpart = reinterpret_cast<float4 *>(scr + off_gpart);
     const bool band = std::isfinite(plan.job.half_bw);
-    const int grid = std::min(n_units, p->n_sm * focus_profile_blocks_per_sm(plan.profile, band, true));
+    const int grid = std::min(n_units, p->n_sm * focus_profile_blocks_per_sm(plan.profile, band, true, false));
     TDC_CK(launch_adjoint_profile(plan.profile, band, reinterpret_cast<const FocusJob *>(scr + off_job),
                                   reinterpret_cast<const FocusUnit *>(scr + off_units), n_units,
                                   reinterpret_cast<int *>(scr), grid, gimg, gpart, st),

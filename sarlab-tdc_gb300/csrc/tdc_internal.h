@@ -81,6 +81,19 @@ struct __align__(16) MotionRec {
 };
 static_assert(sizeof(MotionRec) == 80, "MotionRec must be 80 bytes");
 
+// One chirp's record for the smooth motion through range profiles, 64 bytes: the same positions
+// about the middle sample sc = S / 2, P[c, s] = P(sc) + W1 (s - sc) + V2 (s - sc)^2.
+//   p_hi.xyz, p_lo.xyz  P(sc) as double-float pairs
+//   w1.xyz              W1 = V1 + 2 sc V2 [m / sample]; w1.w = |W1|^2
+//   v2.xyz              V2 [m / sample^2]
+struct __align__(16) MoveRec {
+    float4 p_hi;
+    float4 p_lo;
+    float4 w1;
+    float4 v2;
+};
+static_assert(sizeof(MoveRec) == 64, "MoveRec must be 64 bytes");
+
 // One sample point of the reference's chunk skip test (tdcprocessor.cpp:355-378).
 struct __align__(16) SkipPoint {
     float4 pos_fdc;  // position xyz, window centre
@@ -155,8 +168,15 @@ struct __align__(16) ProfileJob {
     float inv_gc;              // 1 / gc
     float reach;               // largest distance of a pixel from its anchor [m]
     float pad_[2];
+    // smooth motion: cells per (m / sample) of range rate, 4 S gc; with h = S / 2, the bend of the
+    // phase at the row's ends is bend1 a + bend2 (|W1|^2 - a^2) / R + 2 bend2 e.V2 / R radians
+    // (a = e.W1 / R), and its cubic part bend3 d2R/ds2 / 2
+    float rate_cells;
+    float bend1;               // 2 pi h^2 g1
+    float bend2;               // pi h^2 gc
+    float bend3;               // 2 pi h^3 g1
 };
-static_assert(sizeof(ProfileJob) == 64, "ProfileJob layout");
+static_assert(sizeof(ProfileJob) == 80, "ProfileJob layout");
 
 // Kernels copy a FocusJob into shared memory one int per thread (128 threads); the
 // no-allocation scratch reserves 256 bytes for it.
@@ -191,7 +211,7 @@ constexpr int kProfileBandMinUnitsPerSlot = 8;  // (units differ in their live c
 // Inputs and outputs of profile_build_kernel.
 struct ProfileBuild {
     const float2 *rows;      // [C][s_pad] windowed samples
-    const ChirpRec *chirps;  // [C]
+    const float4 *chirps;    // [C] records of chirp_words float4: position high, low, ...
     const float2 *twiddle;   // [S][kProfileNodes], launch_profile_twiddle
     const float *factor;     // [S]
     float4 *cells;           // [C][n_cells][kProfileCoefs / 2]
@@ -201,6 +221,8 @@ struct ProfileBuild {
     double box_min[3], box_max[3];  // bounding box of the grid
     double cells_per_m;
     int C, S, s_pad, n_cells;
+    int chirp_words;
+    int margin;              // cells the table starts early (even; smooth motion)
 };
 
 // Tiles of a P-pixel grid whose runs are `run` pixels long: groups of kProfilePixels
@@ -288,14 +310,15 @@ int focus_general_smem_bytes(int stage_bytes);
 // `group` (8, 4, 2 or 1) consecutive pixels sharing an anchor (band: a finite Doppler band).
 cudaError_t launch_profile_twiddle(float2 *twiddle, float *factor, int S, cudaStream_t st);
 cudaError_t launch_profile_build(const ProfileBuild &b, cudaStream_t st);
-cudaError_t launch_focus_profile(int group, bool band, const FocusJob *jobs_dev, const FocusUnit *units_dev, int n_units,
+// motion: the records are MoveRec, every sample of a chirp at a range of its own.
+cudaError_t launch_focus_profile(int group, bool band, bool motion, const FocusJob *jobs_dev, const FocusUnit *units_dev, int n_units,
                                  int *counter_dev, int grid_ctas, cudaStream_t st);
 // Its adjoint: gpart[tile][C] = (d/dx, d/dy, d/dz) of each chirp over the tile's pixels (sums of
 // Re(conj(G) dI/dR) (P - T) / R; .w is not written).
 cudaError_t launch_adjoint_profile(int group, bool band, const FocusJob *jobs_dev, const FocusUnit *units_dev,
                                    int n_units, int *counter_dev, int grid_ctas, const float2 *gimg, float4 *gpart,
                                    cudaStream_t st);
-int focus_profile_blocks_per_sm(int group, bool band, bool adjoint = false);
+int focus_profile_blocks_per_sm(int group, bool band, bool adjoint, bool motion);
 // out[0..2] = max(out, largest distance of a pixel from the anchor of its group of 8 / 4 / 2
 // consecutive pixels of a run) as float bits (out starts at 0; a NaN compares above any distance).
 cudaError_t launch_group_reach(const float4 *hi, long long P, int run, int *out, cudaStream_t st);

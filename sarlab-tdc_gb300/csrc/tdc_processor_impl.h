@@ -170,7 +170,7 @@ struct tdc_processor {
     // per-sample offsets / windows, residual frequency table.
     tdc::impl::DevBuf gen_rec, traj, wins, wdot, gres;
     // Smooth-motion kernel: one MotionRec per chirp.
-    tdc::impl::DevBuf motion_rec;
+    tdc::impl::DevBuf motion_rec, move_rec;
     // Autofocus: the forward's per-(chirp, pixel) sums and the rows pre-scaled by the sample
     // index, so the adjoint computes only the index-weighted sums (keep_sums on).
     tdc::impl::DevBuf chirp_sums, xs_scaled;
@@ -241,7 +241,7 @@ struct tdc_processor {
     {
         return {&xw,      &chirps,     &skip,    &gs,      &pos_base, &wr,      &offsets,     &flag,     &gen_rec,
                 &traj,    &wins,       &wdot,    &gres,    &grid_stage, &grid_hi, &grid_lo, &scratch, &adj_scratch,
-                &chirp_sums, &xs_scaled, &motion_rec, &cells, &cell_base, &twiddle,
+                &chirp_sums, &xs_scaled, &motion_rec, &move_rec, &cells, &cell_base, &twiddle,
                 &image_dev};
     }
 };

@@ -150,8 +150,8 @@ __global__ void __launch_bounds__(kBuildThreads)
     if (tid < kBuildChirps) {
         // first cell: the smallest cell coordinate of any point in the grid's bounding box
         const int c = min(c0 + tid, b.C - 1);
-        const ChirpRec r = b.chirps[c];
-        const double p[3] = {(double)r.p_hi.x + r.p_lo.x, (double)r.p_hi.y + r.p_lo.y, (double)r.p_hi.z + r.p_lo.z};
+        const float4 ph = b.chirps[(size_t)c * b.chirp_words], pl = b.chirps[(size_t)c * b.chirp_words + 1];
+        const double p[3] = {(double)ph.x + pl.x, (double)ph.y + pl.y, (double)ph.z + pl.z};
         double near2 = 0.0, far2 = 0.0;
         for (int k = 0; k < 3; ++k) {
             const double lo = b.box_min[k] - p[k], hi = p[k] - b.box_max[k];
@@ -161,7 +161,7 @@ __global__ void __launch_bounds__(kBuildThreads)
         }
         const double u = fmin(b.cells_per_m * sqrt(near2), b.cells_per_m * sqrt(far2));
         // (positions far outside what the table can index: any base will do, reads are clamped)
-        const int base = fabs(u) < 1e9 ? 2 * (int)floor(0.5 * u) - 2 : 0;
+        const int base = fabs(u) < 1e9 ? 2 * (int)floor(0.5 * u) - 2 - b.margin : 0;
         if (blockIdx.y == 0 && c0 + tid < b.C) b.cell_base[c0 + tid] = base;
         const int node = base >> 1;
         const int block = (node >= 0 ? node / kOwn : -((kOwn - 1 - node) / kOwn)) + (int)blockIdx.y;
@@ -299,11 +299,11 @@ struct SharedSums {
     float2 dd[kPT / 2][kThreads];
 };
 
-// Chirp records of kFlush chirps at a time (position high and low, with a finite band the
-// velocity) and their first cells.
-template <bool BAND>
+// Chirp records of kFlush chirps at a time (position high and low; the velocity with a finite
+// band; W1 and V2 with smooth motion) and their first cells.
+template <int WORDS>
 struct SharedChirps {
-    float4 p[kFlush][BAND ? 3 : 2];
+    float4 p[kFlush][WORDS];
     int base[kFlush];
 };
 
@@ -380,7 +380,7 @@ __device__ __forceinline__ float2 fresh2(const float2 *p)
 // and the anchor's cell and place in it.
 struct Anchor {
     float ex, ey, ez, rh, h, turn, t0;
-    float w;  // Doppler window (BAND with every pixel its own anchor)
+    float w;  // Doppler window (BAND with every pixel its own anchor); cell shift of its motion (MOVE)
     float2 a[kProfileCoefs];
 };
 
@@ -412,6 +412,74 @@ __device__ __forceinline__ void add_pair(float2 psi, float turn, float t0, float
         h0 = __ffma2_rn(h0, ta, a[m]);
         h1 = __ffma2_rn(h1, tb, a[m]);
     }
+    c0 = __ffma2_rn(h0, both(cs0), c0);
+    s0 = __ffma2_rn(h0, both(sn0), s0);
+    c1 = __ffma2_rn(h1, both(cs1), c1);
+    s1 = __ffma2_rn(h1, both(sn1), s1);
+}
+
+// Smooth motion: the anchor's bend eps0 [rad at the row's ends]; a := coefficients of
+// e^{j (eps0 s^2 + cubic s^3)} A, bend := of the pixel's first-order term, s^2 (1 + j eps0 s^2) A
+// (s = s~ / (S / 2) = -j (4 / pi) d/dt).
+__device__ __forceinline__ float move_coefs(const Anchor &n, float4 w1, float4 v2, const ProfileJob &job,
+                                            float2 (&a)[kProfileCoefs], float2 (&bend)[kProfileCoefs - 2])
+{
+    const float ri = n.rh > 0.0f ? 2.0f * n.h * job.inv_gc : 0.0f;
+    const float rate = fmaf(n.ex, w1.x, fmaf(n.ey, w1.y, n.ez * w1.z)) * ri;
+    const float ev = fmaf(n.ex, v2.x, fmaf(n.ey, v2.y, n.ez * v2.z));
+    const float curve = ri * fmaf(0.5f, fmaf(-rate, rate, w1.w), ev);  // b
+    const float eps = fmaf(job.bend1, rate, 2.0f * job.bend2 * curve);
+    const float cubic = job.bend3 * curve;
+    constexpr float q = -16.0f / (kPiF * kPiF);
+    float2 b[kProfileCoefs - 2], c[kProfileCoefs - 4], e[kProfileCoefs - 6];
+#pragma unroll
+    for (int m = 0; m < kProfileCoefs - 2; ++m) b[m] = __fmul2_rn(a[m + 2], both(q * (float)((m + 2) * (m + 1))));
+#pragma unroll
+    for (int m = 0; m < kProfileCoefs - 4; ++m) c[m] = __fmul2_rn(b[m + 2], both(q * (float)((m + 2) * (m + 1))));
+#pragma unroll
+    for (int m = 0; m < kProfileCoefs - 6; ++m) e[m] = __fmul2_rn(c[m + 2], both(q * (float)((m + 2) * (m + 1))));
+    const float e2 = -0.5f * eps * eps, e3 = -eps * eps * eps * (1.0f / 6.0f);
+#pragma unroll
+    for (int m = 0; m < kProfileCoefs - 2; ++m) {
+        // + j eps b; + j cubic s b = cubic (4 / pi) b'
+        a[m] = make_float2(fmaf(-eps, b[m].y, a[m].x), fmaf(eps, b[m].x, a[m].y));
+        if (m + 1 < kProfileCoefs - 2)
+            a[m] = __ffma2_rn(b[m + 1], both(cubic * (4.0f / kPiF) * (float)(m + 1)), a[m]);
+        bend[m] = b[m];
+        if (m < kProfileCoefs - 4) {
+            a[m] = __ffma2_rn(c[m], both(e2), a[m]);
+            bend[m] = make_float2(fmaf(-eps, c[m].y, b[m].x), fmaf(eps, c[m].x, b[m].y));
+        }
+        if (m < kProfileCoefs - 6) a[m] = make_float2(fmaf(-e3, e[m].y, a[m].x), fmaf(e3, e[m].x, a[m].y));
+    }
+    return eps;
+}
+
+// add_pair with the pixels' places t in the cell and bends eps beside the anchor's.
+__device__ __forceinline__ void add_moving_pair(float2 psi, float turn, float2 t, float2 eps,
+                                                const float2 (&a)[kProfileCoefs],
+                                                const float2 (&bend)[kProfileCoefs - 2], float2 &c0, float2 &s0,
+                                                float2 &c1, float2 &s1)
+{
+    const float2 n = __fadd2_rn(__fadd2_rn(psi, both(12582912.0f)), both(-12582912.0f));  // nearest integer
+    const float2 x = __ffma2_rn(__fadd2_rn(psi, make_float2(-n.x, -n.y)), both(kTwoPiF), both(turn));
+    float sn0, cs0, sn1, cs1;
+    __sincosf(x.x, &sn0, &cs0);
+    __sincosf(x.y, &sn1, &cs1);
+    const float2 ta = both(t.x), tb = both(t.y);
+    float2 h0 = a[kProfileCoefs - 1], h1 = h0, b0 = bend[kProfileCoefs - 3], b1 = b0;
+#pragma unroll
+    for (int m = kProfileCoefs - 2; m >= 0; --m) {
+        h0 = __ffma2_rn(h0, ta, a[m]);
+        h1 = __ffma2_rn(h1, tb, a[m]);
+    }
+#pragma unroll
+    for (int m = kProfileCoefs - 4; m >= 0; --m) {
+        b0 = __ffma2_rn(b0, ta, bend[m]);
+        b1 = __ffma2_rn(b1, tb, bend[m]);
+    }
+    h0 = make_float2(fmaf(-eps.x, b0.y, h0.x), fmaf(eps.x, b0.x, h0.y));  // + j eps b
+    h1 = make_float2(fmaf(-eps.y, b1.y, h1.x), fmaf(eps.y, b1.x, h1.y));
     c0 = __ffma2_rn(h0, both(cs0), c0);
     s0 = __ffma2_rn(h0, both(sn0), s0);
     c1 = __ffma2_rn(h1, both(cs1), c1);
@@ -489,14 +557,27 @@ __device__ __forceinline__ void adjoint_pair(float2 psi, float turn, float t0, f
 // dF/dR = j 2 pi gc e^{j ...} D, D = A - j (cells per cycle / 2 pi) A'(t): the same evaluation with
 // the coefficients of D, formed once an anchor. Each chirp's sum over the tile's pixels (two
 // shuffle steps, then shared memory, 32 chirps at a time) goes to gpart[tile][chirp].
-template <int G, bool BAND, bool ADJ>
-__global__ void __launch_bounds__(kThreads, G == 1 ? (BAND || ADJ ? 4 : 6) : BAND || (ADJ && G == 2) ? 6 : TDC_PROFILE_MINB)
+//
+// MOVE: positions moving within each chirp, R_s = R + a s~ + b s~^2 about the middle sample (s~ = s -
+// sc, a = e.W1 / R, b = (|W1|^2 - a^2) / (2 R) + e.V2 / R), so the phase of sample s is
+//   gc R + s~ (g1 R + gc a) + s~^2 (g1 a + gc b) + s~^3 g1 b  cycles.
+// The linear part is a shift of the cell coordinate by 4 S gc a. The rest is small (the host
+// bounds it to 0.1 rad at the row's ends, eps there): s~ is -j (2 S / pi) d/dt on A(t), so with
+// B = s~^2 A (in units of the half row) and so on, e^{j eps s~^2} A = A + j eps B - eps^2 / 2 C
+// - j eps^3 / 6 E, all polynomials of the cell formed once an anchor; the pixel's difference in
+// eps from its anchor, at most a few per cent of it, enters to first order. 64 x 512 pixels x 512
+// chirps x 1024 samples: 2.64 ms in the per-segment kernel of tdc_motion.cu, 0.21 ms here.
+template <int G, bool BAND, bool ADJ, bool MOVE>
+__global__ void __launch_bounds__(kThreads, G == 1 ? (BAND || ADJ ? 4 : 6) : BAND || MOVE || (ADJ && G == 2) ? 6 : TDC_PROFILE_MINB)
     profile_focus_kernel(const FocusJob *__restrict__ jobs, const FocusUnit *__restrict__ units, int n_units,
                          int *__restrict__ counter, const float2 *__restrict__ gimg, float4 *__restrict__ gpart)
 {
     constexpr int kSub = kPT / G;  // anchors per thread
     __shared__ SharedSums sums;
-    __shared__ __align__(16) SharedChirps<BAND> recs[2];
+    static_assert(!MOVE || (!BAND && !ADJ), "smooth motion: unbounded band, forward only");
+    constexpr int kWords = MOVE ? 4 : BAND ? 3 : 2;  // float4 staged per record
+    constexpr int kStride = MOVE ? 4 : 3;            // float4 per record in memory
+    __shared__ __align__(16) SharedChirps<kWords> recs[2];
     __shared__ float red[ADJ ? kFlush : 1][3][kThreads / 4];  // (ADJ) 8 partial sums a warp
     __shared__ int s_unit;
     __shared__ FocusUnit un;
@@ -581,7 +662,7 @@ __global__ void __launch_bounds__(kThreads, G == 1 ? (BAND || ADJ ? 4 : 6) : BAN
         };
         if (ADJ) load_gradient(0);
 
-        const ChirpRec *__restrict__ chirps = sJ.chirps;
+        const float4 *__restrict__ chirps = reinterpret_cast<const float4 *>(sJ.chirps);
         const int *__restrict__ cell_base = sP.cell_base;
         const float4 *__restrict__ cells = sP.cells;
         const bool skip_test = (sJ.flags & kFlagSkipTest) != 0;
@@ -600,11 +681,21 @@ __global__ void __launch_bounds__(kThreads, G == 1 ? (BAND || ADJ ? 4 : 6) : BAN
             dd_sub(ph.y, pl.y, p[1], p[4], n.ey, eyl);
             dd_sub(ph.z, pl.z, p[2], p[5], n.ez, ezl);
             dd_range(n.ex, exl, n.ey, eyl, n.ez, ezl, n.rh, rl, rs, dh);
+            // gc / (2 R0), 1 / R0 to FP32 rounding (rsqrt is not)
+            const float rinv = fmaf(rs, fmaf(-rl, rs, fmaf(-n.rh, rs, 1.0f)), rs);
+            n.h = 0.5f * g.x * rinv;
             // its cell, and its place in it
-            const float kf = rintf(g.z * n.rh);
+            float shift = 0.f;
+            if (MOVE) {
+                const float4 w1 = recs[buf].p[k][kWords - 2];
+                shift = sP.rate_cells * (fmaf(n.ex, w1.x, fmaf(n.ey, w1.y, n.ez * w1.z)) * rinv);
+                if (!(n.rh > 0.0f)) shift = 0.f;
+            }
+            const float kf = rintf(fmaf(g.z, n.rh, shift));
             n.t0 = fmaf(g.z, n.rh, -kf);
             n.t0 = fmaf(g.z, rl, n.t0);
             n.t0 = fmaf(g.w, n.rh, n.t0);
+            if (MOVE) n.t0 += shift;
             const int cell = min(max((int)kf - base, 0), n_cells - 1);
             const float4 *__restrict__ pc = cells + ((size_t)(b0 + k) * n_cells + cell) * (kProfileCoefs / 2);
 #pragma unroll
@@ -614,8 +705,7 @@ __global__ void __launch_bounds__(kThreads, G == 1 ? (BAND || ADJ ? 4 : 6) : BAN
                 n.a[2 * m + 1] = make_float2(v.z, v.w);
             }
             n.turn = kTwoPiF * dd_frac_mul(g.x, g.y, n.rh, rl);
-            // gc / (2 R0), 1 / R0 to FP32 rounding (rsqrt is not)
-            n.h = 0.5f * g.x * fmaf(rs, fmaf(-rl, rs, fmaf(-n.rh, rs, 1.0f)), rs);
+            if (MOVE) n.w = shift;
             if (BAND && G == 1) {
                 const float4 v = recs[buf].p[k][2];
                 const float fd = doppler_freq(sJ.two_over_lambda, v.x, v.y, v.z, n.ex, n.ey, n.ez, rs);
@@ -627,8 +717,11 @@ __global__ void __launch_bounds__(kThreads, G == 1 ? (BAND || ADJ ? 4 : 6) : BAN
         // record tid / 2
         auto copy_ahead = [&](int first, int to) {
             if (first + (tid >> 1) < c1)
-                copy_async<16>(&recs[to].p[tid >> 1][tid & 1], &chirps[first + (tid >> 1)].p_hi + (tid & 1));
-            if (BAND && tid < kFlush && first + tid < c1) copy_async<16>(&recs[to].p[tid][BAND ? 2 : 0], &chirps[first + tid].vel);
+                copy_async<16>(&recs[to].p[tid >> 1][tid & 1], chirps + (size_t)(first + (tid >> 1)) * kStride + (tid & 1));
+            if (kWords > 2 && tid < kFlush && first + tid < c1)
+#pragma unroll
+                for (int v = 2; v < kWords; ++v)
+                    copy_async<16>(&recs[to].p[tid][v], chirps + (size_t)(first + tid) * kStride + v);
             if (tid < kFlush && first + tid < c1) copy_async<4>(&recs[to].base[tid], &cell_base[first + tid]);
         };
         copy_ahead(c0, 0);
@@ -724,9 +817,16 @@ __global__ void __launch_bounds__(kThreads, G == 1 ? (BAND || ADJ ? 4 : 6) : BAN
                             grad[2] = fmaf(dl, cur.ez, grad[2]);
                             continue;
                         }
-                        float2 h = cur.a[kProfileCoefs - 1];
+                        float2 a[kProfileCoefs];
 #pragma unroll
-                        for (int m = kProfileCoefs - 2; m >= 0; --m) h = __ffma2_rn(h, both(cur.t0), cur.a[m]);
+                        for (int m = 0; m < kProfileCoefs; ++m) a[m] = cur.a[m];
+                        if constexpr (MOVE) {
+                            float2 bend[kProfileCoefs - 2];
+                            move_coefs(cur, recs[buf].p[k][kWords - 2], recs[buf].p[k][kWords - 1], sP, a, bend);
+                        }
+                        float2 h = a[kProfileCoefs - 1];
+#pragma unroll
+                        for (int m = kProfileCoefs - 2; m >= 0; --m) h = __ffma2_rn(h, both(cur.t0), a[m]);
                         hc[g].x = fmaf(cs, h.x, fmaf(-sn, h.y, hc[g].x));
                         hc[g].y = fmaf(cs, h.y, fmaf(sn, h.x, hc[g].y));
                     } else {
@@ -856,6 +956,46 @@ __global__ void __launch_bounds__(kThreads, G == 1 ? (BAND || ADJ ? 4 : 6) : BAN
                             grad[2] += fmaf(all, cur.ez, -(sz.x + sz.y));
                             continue;
                         }
+                        if constexpr (MOVE) {
+                            const float4 w1 = recs[buf].p[k][kWords - 2], v2 = recs[buf].p[k][kWords - 1];
+                            float2 a[kProfileCoefs], bend[kProfileCoefs - 2];
+#pragma unroll
+                            for (int m = 0; m < kProfileCoefs; ++m) a[m] = cur.a[m];
+                            const float eps0 = move_coefs(cur, w1, v2, sP, a, bend);
+                            const float ew = fmaf(cur.ex, w1.x, fmaf(cur.ey, w1.y, cur.ez * w1.z));
+                            const float bend_v = 2.0f * sP.bend2 * fmaf(cur.ex, v2.x, fmaf(cur.ey, v2.y, cur.ez * v2.z));
+#pragma unroll
+                            for (int i = 0; i < G; i += 2) {
+                                const int s = g * G + i, q = s / 2;
+                                const float2 dot = __ffma2_rn(dx[q], both(-w1.x),
+                                                              __ffma2_rn(dy[q], both(-w1.y),
+                                                                         __ffma2_rn(fresh2(&sums.dz[q][tid]),
+                                                                                    both(-w1.z), both(ew))));
+                                const float2 r = __ffma2_rn(psi[i / 2], both(sP.inv_gc), both(cur.rh));
+                                float2 ri = make_float2(__frcp_rn(r.x), __frcp_rn(r.y));
+                                if (zero) {
+                                    if (zero >> i & 1u) ri.x = 0.f;
+                                    if (zero >> (i + 1) & 1u) ri.y = 0.f;
+                                }
+                                const float2 rate = __fmul2_rn(dot, ri);
+                                // place in the cell: the anchor's, less its shift, plus the pixel's
+                                const float2 t = __ffma2_rn(rate, both(sP.rate_cells),
+                                                            __ffma2_rn(psi[i / 2], both(jc.y), both(cur.t0 - cur.w)));
+                                const float2 bow = __fmul2_rn(
+                                    __ffma2_rn(both(sP.bend2), __ffma2_rn(rate, make_float2(-rate.x, -rate.y), both(w1.w)),
+                                               both(bend_v)),
+                                    ri);
+                                const float2 eps = __ffma2_rn(both(sP.bend1), rate, bow);
+                                add_moving_pair(psi[i / 2], cur.turn, t, __fadd2_rn(eps, both(-eps0)), a, bend, hc[s],
+                                                hs[s], hc[s + 1], hs[s + 1]);
+                            }
+                            if (zero) {
+#pragma unroll
+                                for (int i = 0; i < G; ++i)
+                                    if (zero >> i & 1u) hc[g * G + i] = hs[g * G + i] = make_float2(0.f, 0.f);
+                            }
+                            continue;
+                        }
 #pragma unroll
                         for (int i = 0; i < G; i += 2) {
                             const int s = g * G + i;
@@ -931,22 +1071,31 @@ cudaError_t launch_profile_build(const ProfileBuild &b, cudaStream_t st)
 
 using ProfileFn = void (*)(const FocusJob *, const FocusUnit *, int, int *, const float2 *, float4 *);
 
-template <bool BAND, bool ADJ>
+template <bool BAND, bool ADJ, bool MOVE>
 static ProfileFn profile_fn(int group)
 {
     switch (group) {
-    case 8: return profile_focus_kernel<8, BAND, ADJ>;
-    case 4: return profile_focus_kernel<4, BAND, ADJ>;
-    case 2: return profile_focus_kernel<2, BAND, ADJ>;
-    default: return profile_focus_kernel<1, BAND, ADJ>;
+    case 8: return profile_focus_kernel<8, BAND, ADJ, MOVE>;
+    case 4: return profile_focus_kernel<4, BAND, ADJ, MOVE>;
+    case 2: return profile_focus_kernel<2, BAND, ADJ, MOVE>;
+    default: return profile_focus_kernel<1, BAND, ADJ, MOVE>;
     }
 }
 
-cudaError_t launch_focus_profile(int group, bool band, const FocusJob *jobs_dev, const FocusUnit *units_dev,
-                                 int n_units, int *counter_dev, int grid_ctas, cudaStream_t st)
+static ProfileFn profile_fn(int group, bool band, bool adjoint, bool motion)
 {
-    const ProfileFn fn = band ? profile_fn<true, false>(group) : profile_fn<false, false>(group);
-    fn<<<grid_ctas, kThreads, 0, st>>>(jobs_dev, units_dev, n_units, counter_dev, nullptr, nullptr);
+    if (motion) return profile_fn<false, false, true>(group);
+    if (adjoint) return band ? profile_fn<true, true, false>(group) : profile_fn<false, true, false>(group);
+    return band ? profile_fn<true, false, false>(group) : profile_fn<false, false, false>(group);
+}
+
+cudaError_t launch_focus_profile(int group, bool band, bool motion, const FocusJob *jobs_dev,
+                                 const FocusUnit *units_dev, int n_units, int *counter_dev, int grid_ctas,
+                                 cudaStream_t st)
+{
+    if (band && motion) return cudaErrorInvalidValue;
+    profile_fn(group, band, false, motion)<<<grid_ctas, kThreads, 0, st>>>(jobs_dev, units_dev, n_units, counter_dev,
+                                                                           nullptr, nullptr);
     return cudaGetLastError();
 }
 
@@ -954,17 +1103,17 @@ cudaError_t launch_adjoint_profile(int group, bool band, const FocusJob *jobs_de
                                    int n_units, int *counter_dev, int grid_ctas, const float2 *gimg, float4 *gpart,
                                    cudaStream_t st)
 {
-    const ProfileFn fn = band ? profile_fn<true, true>(group) : profile_fn<false, true>(group);
-    fn<<<grid_ctas, kThreads, 0, st>>>(jobs_dev, units_dev, n_units, counter_dev, gimg, gpart);
+    profile_fn(group, band, true, false)<<<grid_ctas, kThreads, 0, st>>>(jobs_dev, units_dev, n_units, counter_dev,
+                                                                         gimg, gpart);
     return cudaGetLastError();
 }
 
-int focus_profile_blocks_per_sm(int group, bool band, bool adjoint)
+int focus_profile_blocks_per_sm(int group, bool band, bool adjoint, bool motion)
 {
-    const ProfileFn fn = adjoint ? (band ? profile_fn<true, true>(group) : profile_fn<false, true>(group))
-                                 : (band ? profile_fn<true, false>(group) : profile_fn<false, false>(group));
     int blocks = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, fn, kThreads, 0) != cudaSuccess) return 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, profile_fn(group, band, adjoint, motion), kThreads, 0) !=
+        cudaSuccess)
+        return 0;
     return blocks;
 }
 

@@ -463,7 +463,7 @@ void tdc_server::launch_batch()
     const bool general = kind >= 16;
     const int profile = members[0]->plan.profile;
     const int variant = general ? members[0]->plan.variant : 0;
-    const int bps = profile    ? focus_profile_blocks_per_sm(profile, skip_zero)
+    const int bps = profile    ? focus_profile_blocks_per_sm(profile, skip_zero, false, false)
                     : general  ? focus_general_blocks_per_sm(variant, stage_bytes)
                     : seg      ? focus_fp32_seg_blocks_per_sm(stage_bytes)
                     : anchored ? focus_fp32_anchor_blocks_per_sm(stage_bytes)
@@ -474,7 +474,7 @@ void tdc_server::launch_batch()
     const FocusUnit *units_d = reinterpret_cast<const FocusUnit *>(d + off_units);
     int *counter_d = reinterpret_cast<int *>(d);
     if (profile)
-        err |= launch_focus_profile(profile, skip_zero, jobs_d, units_d, (int)n_units, counter_d, grid, st) != cudaSuccess;
+        err |= launch_focus_profile(profile, skip_zero, false, jobs_d, units_d, (int)n_units, counter_d, grid, st) != cudaSuccess;
     else if (general)
         err |= launch_focus_general(variant, jobs_d, units_d, (int)n_units, counter_d, counter_d + 1, stage_bytes, grid,
                                     st) != cudaSuccess;

@@ -201,3 +201,47 @@ def test_profile_adjoint_against_the_oracle(cuda_device, nx, ny, spacing, group,
         p.adjointDevice(g_part, grad)
         ref += grad.cpu().numpy()
     assert rel_l2(alone, ref) <= 6e-6
+
+
+@pytest.mark.parametrize("nx,ny,n_pri,n_samples,spacing,drift,accel", [
+    (57, 131, 300, 256, 1e-3, 0.3e-3, 0.0),
+    (131, 57, 129, 777, 1e-3, 0.5e-3, 0.0),
+    (64, 80, 400, 300, 2e-3, 0.2e-3, 0.0),
+    (64, 80, 400, 300, 3.9e-3, 0.3e-3, 0.0),
+    (64, 80, 400, 300, 2e-2, 0.3e-3, 0.0),
+    (57, 131, 300, 256, 1e-3, 0.2e-3, 1e-6),   # a little acceleration
+])
+def test_profile_focus_of_smooth_motion(cuda_device, nx, ny, n_pri, n_samples, spacing, drift, accel):
+    """Positions moving within each chirp, at least 5e8 correlations. The oracle reads every
+    sample's FP32 position; the fit smooths their rounding, 1.7e-8 m rms a coordinate or 5e-5 rad
+    a sample, which the sum over samples averages: tolerance 2e-5. The FP32 general kernel, which
+    follows each position, and this path agree to the same."""
+    import _sarlabtdc
+
+    sc = scenes.small_scene(seed=nx + n_samples, n_pri=n_pri, n_samples=n_samples, nx=nx, ny=ny, spacing=spacing,
+                            rail_len=0.3, device="cuda")
+    rng = np.random.default_rng(4)
+    api = sc.api_arrays()
+    u = (np.arange(n_samples) / n_samples)[None, :, None]
+    pos = api["position"].astype(np.float64) + u * rng.normal(0.0, drift, (n_pri, 1, 3))
+    pos = pos + u * u * rng.normal(0.0, accel, (n_pri, 1, 3)) if accel else pos
+    api["position"] = pos.astype(np.float32)
+    grid = sc.grid.astype(np.float32)
+    p = _sarlabtdc.TdcProcessor(0)
+    p.setRawData(*api.values())
+    p.setFocusGrid(grid)
+    p.start(0.0, INF, False, False, True)
+    img, st = p.getFocusedImage().ravel(), p.lastStats()
+    assert st["path_name"] == "fp32_motion" and st["stage_samples"] == 0 and st["motion_segment"] == 0
+    pix = np.unique(np.concatenate([[0, nx - 1, nx, img.size - 1],
+                                    np.random.default_rng(5).choice(img.size, 60, replace=False)]))
+    prob = oracle.Problem(raw=api["rawData"], sampleTimes=api["sampleTimes"], position=api["position"],
+                          velocity=api["velocity"], attitude=api["attitude"], modRate=api["modRate"],
+                          startFreq=api["startFreq"], grid=grid)
+    ref = oracle.focus(prob, oracle.Opts(applyRangeWin=False, dopplerBandwidth=INF), pixels=pix)
+    err = rel_l2(img[pix], ref)
+    assert err <= 2e-5, err
+    p.setMotionPath(False)
+    p.start(0.0, INF, False, False, True)
+    assert p.lastStats()["path_name"] == "general"
+    assert rel_l2(img, p.getFocusedImage().ravel()) <= 2e-5
