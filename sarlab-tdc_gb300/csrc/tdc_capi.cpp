@@ -631,17 +631,6 @@ int prepare(tdc_processor *p, const StartOpts &o, int &launches)
     return TDC_OK;
 }
 
-// Reach of the anchored pixel groups of the resident grid (range profiles): flag[10..12] on the
-// device, as float bits.
-int enqueue_group_reach(tdc_processor *p, cudaStream_t st, int &launches)
-{
-    int *reach = p->flag.as<int>() + 10;
-    TDC_CK(cudaMemsetAsync(reach, 0, 12, st), "reset reach");
-    TDC_CK(launch_group_reach(p->grid_hi.as<float4>(), p->P, p->grid_run, reach, st), "reach kernel");
-    launches += 1;
-    return TDC_OK;
-}
-
 void set_group_reach(tdc_processor *p, const int *bits)
 {
     for (int k = 0; k < 3; ++k) {
@@ -652,12 +641,35 @@ void set_group_reach(tdc_processor *p, const int *bits)
     p->reach_known = true;
 }
 
-int read_group_reach(tdc_processor *p, cudaStream_t st)
+// Reach of the anchored pixel groups of the resident grid (range profiles), measured now.
+int measure_group_reach(tdc_processor *p)
 {
-    int bits[3];
-    TDC_CK(cudaMemcpyAsync(bits, p->flag.as<int>() + 10, sizeof(bits), cudaMemcpyDeviceToHost, st), "read reach");
-    TDC_CK(cudaStreamSynchronize(st), "reach sync");
+    int bits[3], *reach = p->flag.as<int>() + 10;
+    TDC_CK(cudaMemsetAsync(reach, 0, sizeof(bits), p->stream), "reset reach");
+    TDC_CK(launch_group_reach(p->grid_hi.as<float4>(), p->P, p->grid_run, reach, p->stream), "reach kernel");
+    TDC_CK(cudaMemcpyAsync(bits, reach, sizeof(bits), cudaMemcpyDeviceToHost, p->stream), "read reach");
+    TDC_CK(cudaStreamSynchronize(p->stream), "reach sync");
     set_group_reach(p, bits);
+    return TDC_OK;
+}
+
+// Radii of the resident grid's work tiles, flat and block (unit spans), measured now.
+int measure_tile_radii(tdc_processor *p)
+{
+    const int n_flat = (int)(p->tile_centre_flat.size() / 3), n_block = (int)(p->tile_centre_block.size() / 3);
+    std::vector<float> r((size_t)n_flat + n_block);
+    TDC_CK(p->tile_radius.ensure(r.size() * 4), "alloc tile radii");
+    float *dev = p->tile_radius.as<float>();
+    TDC_CK(launch_tile_radius(p->grid_hi.as<float4>(), p->P, p->rows, p->cols, 0, n_flat, dev, p->stream),
+           "tile radius kernel");
+    TDC_CK(launch_tile_radius(p->grid_hi.as<float4>(), p->P, p->rows, p->cols, kBlockTileCols, n_block, dev + n_flat,
+                              p->stream),
+           "tile radius kernel");
+    TDC_CK(cudaMemcpyAsync(r.data(), dev, r.size() * 4, cudaMemcpyDeviceToHost, p->stream), "read tile radii");
+    TDC_CK(cudaStreamSynchronize(p->stream), "tile radius sync");
+    p->tile_radius_flat.assign(r.begin(), r.begin() + n_flat);
+    p->tile_radius_block.assign(r.begin() + n_flat, r.end());
+    p->tile_radius_known = true;
     return TDC_OK;
 }
 
@@ -681,73 +693,31 @@ int upload_grid(tdc_processor *p, int &launches)
             p->axis_r[k] = p->rows > 1 ? g(p->cols, k) - g(0, k) : 0.0;
         }
         // centre pixel of every work tile, flat and block (the planner's cost estimate under
-        // a finite Doppler band)
+        // a finite Doppler band; the tiles' radii are measured when a plan asks for them)
         p->tile_centre_flat.clear();
         p->tile_centre_block.clear();
+        p->tile_radius_known = false;
         if (P > 0) {
             const long long n_flat = (P + kFocusTile - 1) / kFocusTile;
             p->tile_centre_flat.resize((size_t)n_flat * 3);
-            p->tile_radius_flat.assign((size_t)n_flat, 0.0);
             for (long long t = 0; t < n_flat; ++t) {
                 const long long i = std::min(P - 1, t * kFocusTile + kFocusTile / 2);
                 for (int k = 0; k < 3; ++k) p->tile_centre_flat[3 * t + k] = g(i, k);
-                double r2 = 0.0;
-                for (long long q = t * kFocusTile; q < std::min(P, (t + 1) * kFocusTile); ++q) {
-                    const double dx = g(q, 0) - g(i, 0), dy = g(q, 1) - g(i, 1), dz = g(q, 2) - g(i, 2);
-                    const double d2 = dx * dx + dy * dy + dz * dz;
-                    r2 = d2 > r2 || d2 != d2 ? d2 : r2;
-                }
-                p->tile_radius_flat[t] = std::sqrt(r2);
             }
-            // anchored ranges: distance of each pixel from its group's anchor (groups of 32
-            // consecutive pixels; the anchor is the 17th pixel or the group's last)
-            double span2 = 0.0;
-            for (long long b = 0; b < P; b += 32) {
-                const long long a = std::min(P - 1, b + 16);
-                const double ax = g(a, 0), ay = g(a, 1), az = g(a, 2);
-                for (long long i = b; i < std::min(P, b + 32); ++i) {
-                    const double dx = g(i, 0) - ax, dy = g(i, 1) - ay, dz = g(i, 2) - az;
-                    const double d2 = dx * dx + dy * dy + dz * dz;
-                    span2 = d2 > span2 || d2 != d2 ? d2 : span2;
-                }
-            }
-            p->anchor_span = std::sqrt(span2);
             const int tile_rows = kFocusTile / kBlockTileCols;
             const long long n_tr = (p->rows + tile_rows - 1) / tile_rows;
             const long long n_tc = (p->cols + kBlockTileCols - 1) / kBlockTileCols;
             p->tile_centre_block.resize((size_t)(n_tr * n_tc) * 3);
-            p->tile_radius_block.assign((size_t)(n_tr * n_tc), 0.0);
             for (long long tr = 0; tr < n_tr; ++tr)
                 for (long long tc = 0; tc < n_tc; ++tc) {
                     const long long r = std::min<long long>(p->rows - 1, tr * tile_rows + tile_rows / 2);
                     const long long c = std::min<long long>(p->cols - 1, tc * kBlockTileCols + kBlockTileCols / 2);
-                    const long long ci = r * p->cols + c;
-                    for (int k = 0; k < 3; ++k) p->tile_centre_block[3 * (tr * n_tc + tc) + k] = g(ci, k);
-                    double r2 = 0.0;
-                    for (long long rr = tr * tile_rows; rr < std::min<long long>(p->rows, (tr + 1) * tile_rows); ++rr)
-                        for (long long cc = tc * kBlockTileCols;
-                             cc < std::min<long long>(p->cols, (tc + 1) * kBlockTileCols); ++cc) {
-                            const long long q = rr * p->cols + cc;
-                            if (q >= P) continue;
-                            const double dx = g(q, 0) - g(ci, 0), dy = g(q, 1) - g(ci, 1), dz = g(q, 2) - g(ci, 2);
-                            const double d2 = dx * dx + dy * dy + dz * dz;
-                            r2 = d2 > r2 || d2 != d2 ? d2 : r2;
-                        }
-                    p->tile_radius_block[tr * n_tc + tc] = std::sqrt(r2);
+                    for (int k = 0; k < 3; ++k)
+                        p->tile_centre_block[3 * (tr * n_tc + tc) + k] = g(r * p->cols + c, k);
                 }
         }
     }
     if (!p->host_reads) {
-        for (int k = 0; k < 3; ++k) {
-            p->grid_min[k] = std::numeric_limits<double>::infinity();
-            p->grid_max[k] = -std::numeric_limits<double>::infinity();
-        }
-        for (long long i = 0; i < P; ++i)
-            for (int k = 0; k < 3; ++k) {
-                const double v = p->grid64 ? p->grid64[3 * i + k] : (double)p->grid[3 * i + k];
-                p->grid_min[k] = std::min(p->grid_min[k], v);
-                p->grid_max[k] = std::max(p->grid_max[k], v);
-            }
         TDC_CK(p->grid_stage.ensure((size_t)P * 3 * elt), "alloc grid staging");
         TDC_CK(cudaMemcpyAsync(p->grid_stage.p, src, (size_t)P * 3 * elt, cudaMemcpyHostToDevice, st), "copy grid");
         src = p->grid_stage.p;
@@ -767,30 +737,32 @@ int upload_grid(tdc_processor *p, int &launches)
     TDC_CK(p->flag.ensure(64), "alloc flag");
     p->grid_run = detect_run(
         P, [&](long long i, int k) { return p->grid64 ? p->grid64[3 * i + k] : (double)p->grid[3 * i + k]; });
-    // (small focuses do not ask for it: measured when a plan first does)
+    // (small focuses do not ask for the reach: measured when a plan first does)
     p->reach_known = p->has_raw && profile_pays((double)std::max(P, p->plan_pixels), p->C, p->S);
-    if (p->reach_known)
-        if (int rc = enqueue_group_reach(p, st, launches)) return rc;
-    if (p->host_reads && P > 0) {
-        // bounding box of the grid on the device (order-preserving integer keys of the floats)
-        const int init[6] = {0x7fffffff, 0x7fffffff, 0x7fffffff, (int)0x80000000, (int)0x80000000,
-                             (int)0x80000000};
-        int keys[9];
+    if (P > 0) {
+        // bounding box, reach and anchor span of the grid, measured on the device (the box as
+        // order-preserving integer keys of the floats)
+        const int init[10] = {0x7fffffff, 0x7fffffff, 0x7fffffff, (int)0x80000000, (int)0x80000000,
+                              (int)0x80000000, 0, 0, 0, 0};
+        int keys[10];
         int *box = p->flag.as<int>() + 4;
         TDC_CK(cudaMemcpyAsync(box, init, sizeof(init), cudaMemcpyHostToDevice, st), "init bbox");
+        if (p->reach_known)
+            TDC_CK(launch_group_reach(p->grid_hi.as<float4>(), P, p->grid_run, box + 6, st), "reach kernel");
         TDC_CK(launch_grid_bbox(p->grid_hi.as<float4>(), P, box, st), "bbox kernel");
         TDC_CK(cudaMemcpyAsync(keys, box, sizeof(keys), cudaMemcpyDeviceToHost, st), "read bbox");
         TDC_CK(cudaStreamSynchronize(st), "grid sync");
-        launches += 1;
-        set_group_reach(p, keys + 6);
+        launches += p->reach_known ? 2 : 1;
+        if (p->reach_known) set_group_reach(p, keys + 6);
+        float span;
+        std::memcpy(&span, &keys[9], 4);
+        p->anchor_span = span;
         for (int k = 0; k < 6; ++k) {
             const int bits = keys[k] >= 0 ? keys[k] : keys[k] ^ 0x7fffffff;
             float f;
             std::memcpy(&f, &bits, 4);
             (k < 3 ? p->grid_min[k] : p->grid_max[k - 3]) = f;
         }
-    } else if (p->reach_known) {
-        return read_group_reach(p, st);
     }
     return TDC_OK;
 }
@@ -930,6 +902,7 @@ int choose_tile_cols(const tdc_processor *p)
 void plan_unit_order_and_spans(tdc_processor *p, int tile_cols, bool narrow)
 {
     if (!std::isfinite(p->opts.bw) || p->rec_host.size() != (size_t)p->C || p->units_host.size() < 2) return;
+    if (narrow && !p->tile_radius_known && measure_tile_radii(p)) narrow = false;
     const std::vector<double> &centres = tile_cols ? p->tile_centre_block : p->tile_centre_flat;
     const std::vector<double> &radii = tile_cols ? p->tile_radius_block : p->tile_radius_flat;
     const long long n_tiles = (long long)centres.size() / 3;
@@ -1255,10 +1228,7 @@ int profile_group(tdc_processor *p, int path, ProfileBuild &b)
         size_t free_b = 0, total_b = 0;
         if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || bytes > free_b / 2) return 0;
     }
-    if (!p->reach_known) {
-        int launches = 0;
-        if (enqueue_group_reach(p, p->stream, launches) || read_group_reach(p, p->stream)) return 0;
-    }
+    if (!p->reach_known && measure_group_reach(p)) return 0;
     if (!std::isfinite(p->group_reach[0])) return 0;
     if (!p->anchor_enabled) return 1;
     // |t| <= 1/2 (the anchor's place in its cell) + the group's reach

@@ -113,6 +113,8 @@ __global__ void scale_rows_kernel(const float2 *__restrict__ rows, long long tot
 
 // Bounding box of the grid's high floats: out = (min x, min y, min z, max x, max y, max z),
 // each as an order-preserving int (see float_key); out must start at (INT_MAX x3, INT_MIN x3).
+// out[9] = largest distance of a pixel from the anchor of its 32 consecutive pixels (the 17th, or
+// the last), as float bits (starts at 0; a NaN compares above any distance).
 __device__ __forceinline__ int float_key(float f)
 {
     const int i = __float_as_int(f);
@@ -122,6 +124,7 @@ __device__ __forceinline__ int float_key(float f)
 __global__ void grid_bbox_kernel(const float4 *__restrict__ hi, long long P, int *__restrict__ out)
 {
     int mn[3] = {0x7fffffff, 0x7fffffff, 0x7fffffff}, mx[3] = {(int)0x80000000, (int)0x80000000, (int)0x80000000};
+    float span2 = 0.f;
     for (long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x; p < P; p += (long long)gridDim.x * blockDim.x) {
         const float4 v = hi[p];
         const int k[3] = {float_key(v.x), float_key(v.y), float_key(v.z)};
@@ -129,7 +132,13 @@ __global__ void grid_bbox_kernel(const float4 *__restrict__ hi, long long P, int
             mn[d] = min(mn[d], k[d]);
             mx[d] = max(mx[d], k[d]);
         }
+        const float4 a = hi[min(P - 1, (p & ~31LL) + 16)];
+        const float dx = v.x - a.x, dy = v.y - a.y, dz = v.z - a.z;
+        const float d2 = dx * dx + dy * dy + dz * dz;
+        span2 = d2 > span2 || d2 != d2 ? d2 : span2;
     }
+    const int span = __reduce_max_sync(0xffffffffu, __float_as_int(fabsf(sqrtf(span2))));
+    if ((threadIdx.x & 31) == 0 && span > 0) atomicMax(&out[9], span);
     for (int d = 0; d < 3; ++d) {
         for (int off = 16; off > 0; off >>= 1) {
             mn[d] = min(mn[d], __shfl_xor_sync(0xffffffffu, mn[d], off));
@@ -140,6 +149,36 @@ __global__ void grid_bbox_kernel(const float4 *__restrict__ hi, long long P, int
             atomicMax(&out[3 + d], mx[d]);
         }
     }
+}
+
+// Largest distance from each work tile's centre pixel to its other pixels (see FocusJob::tile_cols);
+// one warp a tile.
+__global__ void tile_radius_kernel(const float4 *__restrict__ hi, long long P, int rows, int cols, int tile_cols,
+                                   int n_tiles, float *__restrict__ radius)
+{
+    const int t = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+    if (t >= n_tiles) return;
+    long long centre;
+    if (tile_cols) {
+        const int n_tc = (cols + tile_cols - 1) / tile_cols, tile_rows = kFocusTile / tile_cols;
+        const long long r = min((long long)rows - 1, (long long)(t / n_tc) * tile_rows + tile_rows / 2);
+        const long long c = min((long long)cols - 1, (long long)(t % n_tc) * tile_cols + tile_cols / 2);
+        centre = r * cols + c;
+    } else {
+        centre = min(P - 1, (long long)t * kFocusTile + kFocusTile / 2);
+    }
+    const float4 a = hi[centre];
+    float r2 = 0.f;
+    for (int s = lane; s < kFocusTile; s += 32) {
+        const long long p = tile_pixel(tile_cols, cols, P, t, s);
+        if (p < 0) continue;
+        const float4 v = hi[p];
+        const float dx = v.x - a.x, dy = v.y - a.y, dz = v.z - a.z;
+        const float d2 = dx * dx + dy * dy + dz * dz;
+        r2 = d2 > r2 || d2 != d2 ? d2 : r2;
+    }
+    const int m = __reduce_max_sync(0xffffffffu, __float_as_int(fabsf(r2)));
+    if (lane == 0) radius[t] = sqrtf(__int_as_float(m));
 }
 
 // Reach of the anchored pixel groups of the range-profile focus: the largest distance from a
@@ -281,6 +320,15 @@ cudaError_t launch_grid_bbox(const float4 *hi, long long P, int *out, cudaStream
     long long blocks = (P + 255) / 256;
     if (blocks > 152 * 8) blocks = 152 * 8;
     grid_bbox_kernel<<<(unsigned)blocks, 256, 0, st>>>(hi, P, out);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_tile_radius(const float4 *hi, long long P, int rows, int cols, int tile_cols, int n_tiles,
+                               float *radius, cudaStream_t st)
+{
+    if (n_tiles <= 0) return cudaSuccess;
+    tile_radius_kernel<<<(unsigned)((n_tiles * 32LL + 255) / 256), 256, 0, st>>>(hi, P, rows, cols, tile_cols, n_tiles,
+                                                                                radius);
     return cudaGetLastError();
 }
 

@@ -205,6 +205,8 @@ struct tdc_processor {
     std::vector<double> tile_centre_flat, tile_centre_block;
     // Largest distance from each tile's centre pixel to its other pixels (flat, block tiles).
     std::vector<double> tile_radius_flat, tile_radius_block;
+    bool tile_radius_known = false;  // ... measured for the resident grid
+    tdc::impl::DevBuf tile_radius;
     // Chirp offsets applied on the device since the last prepare (rec_host's positions are then
     // not the ones the kernels use: no unit spans from them).
     bool offsets_applied = false;
@@ -241,7 +243,7 @@ struct tdc_processor {
     {
         return {&xw,      &chirps,     &skip,    &gs,      &pos_base, &wr,      &offsets,     &flag,     &gen_rec,
                 &traj,    &wins,       &wdot,    &gres,    &grid_stage, &grid_hi, &grid_lo, &scratch, &adj_scratch,
-                &chirp_sums, &xs_scaled, &motion_rec, &move_rec, &cells, &cell_base, &twiddle,
+                &chirp_sums, &xs_scaled, &motion_rec, &move_rec, &cells, &cell_base, &twiddle, &tile_radius,
                 &image_dev};
     }
 };

@@ -68,6 +68,7 @@ struct Job {
     size_t n_units = 0;
     double unit_work = 0;  // correlations per unit, in FP32-bulk kernel time (kind_cost)
     size_t footprint = 0;
+    bool profile = true;  // range profiles where they pay: their table fits the budget
     int state = kQueued;
     int rc = TDC_OK;
     std::string err;
@@ -143,8 +144,10 @@ double pair_work_estimate(const tdc_job_desc &d)
     return profile ? kProfilePairCost : d.n_samples;
 }
 
-size_t device_footprint(const tdc_job_desc &d, int n_sm)
+// Device bytes of a job; `table`: what range profiles take beside them (0: the job is too small).
+size_t device_footprint(const tdc_job_desc &d, int n_sm, size_t &table)
 {
+    table = 0;
     const size_t C = (size_t)d.n_pri, S = (size_t)d.n_samples, P = (size_t)d.n_pix;
     const size_t s_pad = round_up(S, kSampleAlign);
     int groups = 1, cpg = d.n_pri;
@@ -155,29 +158,18 @@ size_t device_footprint(const tdc_job_desc &d, int n_sm)
     const size_t n_tiles = (P + kFocusTile - 1) / kFocusTile;
     size_t b = 0;
     if (profile_pays((double)P, (double)C, (double)S)) {
-        // range profiles: the table over the grid's ranges, and this plan's groups where they are more
+        // range profiles: the table, bounded by its ratio to the samples whatever the grid, and
+        // this plan's groups where they are more
         auto g = [&](long long i, int k) { return d.grid_f64 ? d.grid_f64[3 * i + k] : (double)d.grid[3 * i + k]; };
-        double lo[3], hi[3];
-        for (int k = 0; k < 3; ++k) lo[k] = hi[k] = g(0, k);
-        for (long long i = 1; i < (long long)P; ++i)
-            for (int k = 0; k < 3; ++k) {
-                lo[k] = std::min(lo[k], g(i, k));
-                hi[k] = std::max(hi[k], g(i, k));
-            }
-        const double dx = hi[0] - lo[0], dy = hi[1] - lo[1], dz = hi[2] - lo[2];
-        const double dt = S > 1 ? ((double)d.sample_times[S - 1] - d.sample_times[0]) / (S - 1) : 0.0;
-        const double cells_per_m = 4.0 * S * 2.0 * (double)d.mod_rate * dt / kC0 * 1.01;
-        const double diag = std::sqrt(dx * dx + dy * dy + dz * dz);
-        if (cells_per_m * diag < 4.0 * S &&
-            profile_table_fits(profile_cells(cells_per_m, diag) - 4, (int)S, kServerTableRatio))
-            b += C * (size_t)profile_cells(cells_per_m, diag) * kProfileCoefs * 8 + C * 4 + sizeof(ProfileJob) + S * (kProfileNodes * 8 + 4);
+        const long long tiles = profile_tiles((long long)P, detect_run((long long)P, g));
         int pg = 1, pcpg = d.n_pri;
-        plan_groups(profile_tiles((long long)P, detect_run((long long)P, g)), d.n_pri, n_sm * kProfileCtasPerSm, pg,
-                    pcpg, std::isfinite(d.doppler_bandwidth / 2.0f) ? kProfileBandMinUnitsPerSlot : kProfileMinUnitsPerSlot);
+        plan_groups(tiles, d.n_pri, n_sm * kProfileCtasPerSm, pg, pcpg,
+                    std::isfinite(d.doppler_bandwidth / 2.0f) ? kProfileBandMinUnitsPerSlot : kProfileMinUnitsPerSlot);
         const int cap = std::max(1, (int)(kServerUnitWork / ((double)kFocusTile * kProfilePairCost)));
         if (pcpg > cap) pg = (d.n_pri + cap - 1) / cap;
-        groups = std::max(groups, pg);
-        b += ((size_t)profile_tiles((long long)P, detect_run((long long)P, g)) + 1) * groups * sizeof(FocusUnit);
+        table = (size_t)(kServerTableRatio * (double)(C * S * 8)) + C * 4 + sizeof(ProfileJob) +
+                S * (kProfileNodes * 8 + 4) + (size_t)(tiles + 1) * pg * sizeof(FocusUnit) +
+                (size_t)std::max(0, pg - groups) * P * 16;
     }
     b += C * s_pad * 8;                 // samples
     b += C * sizeof(ChirpRec);          // records
@@ -288,6 +280,7 @@ int tdc_server::admit_one(Job *j)
     if (!rc) rc = tdc_processor_prepare(p, d.doppler_win_center, d.doppler_bandwidth, d.dop_centroid_win,
                                         d.apply_range_win, d.doppler_win_taper);
     if (!rc) rc = tdc_processor_upload_grid(p);
+    p->table_ratio = j->profile ? kServerTableRatio : 1e-9;
     if (!rc) rc = focus_plan(p, j->plan, kServerUnitWork);
     if (rc) return rc;
     // Images go through device + pinned buffers: a kernel writing the caller's freshly
@@ -680,7 +673,6 @@ int tdc_server_create(int device, size_t memory_budget_bytes, int max_jobs, tdc_
             s->free_slots.push_back(p);
             s->slot_mem[p] = 0;
             rc = processor_use_slot_stream(p, greatest);
-            p->table_ratio = kServerTableRatio;
         }
     }
     if (rc) {
@@ -709,7 +701,11 @@ int tdc_server_submit(tdc_server *s, const tdc_job_desc *job, uint64_t *job_id)
         j->pos32.resize((size_t)job->n_pri * 3);
         for (size_t i = 0; i < j->pos32.size(); ++i) j->pos32[i] = (float)job->position_f64[i];
     }
-    j->footprint = device_footprint(*job, s->n_sm);
+    size_t table = 0;
+    j->footprint = device_footprint(*job, s->n_sm, table);
+    // (a job that fits the budget only without a table keeps the direct kernels)
+    j->profile = j->footprint + table <= s->budget;
+    if (j->profile) j->footprint += table;
     if (cudaEventCreateWithFlags(&j->done_ev, cudaEventDisableTiming) != cudaSuccess)
         return set_last_error(TDC_ERR_CUDA, "event creation failed");
     std::lock_guard<std::mutex> lk(s->mu);
