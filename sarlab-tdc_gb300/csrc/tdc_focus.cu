@@ -884,8 +884,9 @@ __global__ void __launch_bounds__(kFocusThreads, TDC_FOCUS_MINB)
 constexpr int kReducePixels = 32, kReduceSlices = 8;
 __global__ void __launch_bounds__(kReducePixels *kReduceSlices)
     focus_reduce_sliced_kernel(const float4 *__restrict__ partial, int n_groups, long long P,
-                               float2 *__restrict__ image)
+                               float2 *__restrict__ image, const int *__restrict__ enabled, int want)
 {
+    if (enabled && *enabled != want) return;
     __shared__ double2 part[kReduceSlices][kReducePixels];
     const long long p = (long long)blockIdx.x * kReducePixels + threadIdx.x;
     const int per = (n_groups + kReduceSlices - 1) / kReduceSlices;
@@ -913,8 +914,9 @@ __global__ void __launch_bounds__(kReducePixels *kReduceSlices)
 
 // The same for a few groups: one thread a pixel, the groups in order.
 __global__ void focus_reduce_kernel(const float4 *__restrict__ partial, int n_groups, long long P,
-                                    float2 *__restrict__ image)
+                                    float2 *__restrict__ image, const int *__restrict__ enabled, int want)
 {
+    if (enabled && *enabled != want) return;
     const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= P) return;
     double re = 0.0, im = 0.0;
@@ -1008,18 +1010,19 @@ cudaError_t launch_focus_fp32_seg(const FocusJob *jobs_dev, const FocusUnit *uni
     return cudaGetLastError();
 }
 
-cudaError_t launch_focus_reduce(const float4 *partial, int n_groups, long long P, float2 *image, cudaStream_t st)
+cudaError_t launch_focus_reduce(const float4 *partial, int n_groups, long long P, float2 *image, cudaStream_t st,
+                                const int *enabled, int want)
 {
     if (P <= 0) return cudaSuccess;
     if (n_groups >= 2 * kReduceSlices) {
         const long long blocks = (P + kReducePixels - 1) / kReducePixels;
-        focus_reduce_sliced_kernel<<<(unsigned)blocks, dim3(kReducePixels, kReduceSlices), 0, st>>>(partial, n_groups,
-                                                                                                    P, image);
+        focus_reduce_sliced_kernel<<<(unsigned)blocks, dim3(kReducePixels, kReduceSlices), 0, st>>>(
+            partial, n_groups, P, image, enabled, want);
         return cudaGetLastError();
     }
     const int threads = 256;
     const long long blocks = (P + threads - 1) / threads;
-    focus_reduce_kernel<<<(unsigned)blocks, threads, 0, st>>>(partial, n_groups, P, image);
+    focus_reduce_kernel<<<(unsigned)blocks, threads, 0, st>>>(partial, n_groups, P, image, enabled, want);
     return cudaGetLastError();
 }
 

@@ -294,8 +294,9 @@ int focus_motion_smem_bytes(int stage_bytes);
 // Plain FP64-phase focus (comparator and general fallback), one CTA per unit.
 cudaError_t launch_focus_fp64(const FocusJob *jobs_dev, const FocusUnit *units_dev, int n_units,
                               int *status_dev, int per_sample, cudaStream_t st);
+// (enabled, when given: the launch does nothing unless *enabled == want.)
 cudaError_t launch_focus_reduce(const float4 *partial, int n_groups, long long P, float2 *image,
-                                cudaStream_t st);
+                                cudaStream_t st, const int *enabled = nullptr, int want = 0);
 // FP32 general focus (tdc_general.cu). variant bits: 1 per-sample positions, 2 per-sample
 // windows, 4 wide (non-uniform sampling residual, large intra-chirp motion: reduced phase
 // correction, longer range-change series); at least one set. Rows are staged job.seg_len
@@ -312,6 +313,9 @@ int focus_general_smem_bytes(int stage_bytes);
 // `group` (8, 4, 2 or 1) consecutive pixels sharing an anchor (band: a finite Doppler band).
 cudaError_t launch_profile_twiddle(float2 *twiddle, float *factor, int S, cudaStream_t st);
 cudaError_t launch_profile_build(const ProfileBuild &b, cudaStream_t st);
+// The same with its inputs in device memory, of at most max_cells cells; nothing where *enabled is 0.
+cudaError_t launch_profile_build_indirect(const ProfileBuild *dev, const int *enabled, int C, int max_cells,
+                                          cudaStream_t st);
 // motion: the records are MoveRec, every sample of a chirp at a range of its own.
 cudaError_t launch_focus_profile(int group, bool band, bool motion, const FocusJob *jobs_dev, const FocusUnit *units_dev, int n_units,
                                  int *counter_dev, int grid_ctas, cudaStream_t st);

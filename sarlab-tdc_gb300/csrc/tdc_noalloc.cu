@@ -12,6 +12,12 @@
 // taken from a file-scope __device__ array of TDC_NOALLOC_SCRATCH_BYTES instead
 // of cudaMalloc. Every GPU that loads this library holds that array until the
 // process exits.
+//
+// Large calls take range profiles (tdc_profile.cu, every range in double-float) when the table
+// fits the array. The host knows neither the grid's extent nor the trajectory, so a kernel
+// decides from the inputs on the device (noalloc_decide_kernel): both forms are enqueued, and
+// the one not taken finds its work counter already past its last unit. 200 x 150 pixels x 300
+// chirps x 256 samples: 395 -> 174 us.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -42,6 +48,9 @@ size_t round_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 constexpr size_t kOffStatus = 0;    // int counter, int status
 constexpr size_t kOffJob = 256;     // FocusJob
 constexpr size_t kOffUnits = 512;   // FocusUnit[n_units]
+// Words at kOffStatus.
+constexpr int kWordCounter = 0, kWordStatus = 1, kWordProfile = 2, kWordProfileCounter = 3, kWordBox = 8;
+constexpr int kSpent = 1 << 30;  // a work counter past every unit
 
 size_t layout_bytes(long long P, long long n_units, int n_groups, size_t &off_partial)
 {
@@ -57,14 +66,92 @@ __global__ void noalloc_setup_kernel(FocusJob job, int n_tiles, int n_groups, un
     const long long i0 = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i0 == 0) {
         int *words = reinterpret_cast<int *>(base + kOffStatus);
-        words[0] = 0;
-        words[1] = 0;
+        words[kWordCounter] = 0;
+        words[kWordStatus] = 0;
+        words[kWordProfile] = 0;
+        for (int k = 0; k < 10; ++k) words[kWordBox + k] = k < 3 ? 0x7fffffff : k < 6 ? (int)0x80000000 : 0;
         *reinterpret_cast<FocusJob *>(base + kOffJob) = job;
     }
     FocusUnit *units = reinterpret_cast<FocusUnit *>(base + kOffUnits);
     for (long long u = i0; u < n_units; u += (long long)gridDim.x * blockDim.x) {
         units[u] = FocusUnit{0, (int)(u / n_groups), (int)(u % n_groups), 0};
     }
+}
+
+// The profile form of a call: its job, its unit table and what its table is built from, in the
+// scratch array.
+struct ProfilePlan {
+    FocusJob job;
+    ProfileBuild build;  // box, n_cells and the job record are filled in on the device
+    FocusJob *job_out;
+    ProfileBuild *build_out;
+    FocusUnit *units;
+    int n_tiles, n_groups, max_cells;
+    double g1, gc;
+};
+
+// Whether range profiles apply, from the grid's bounding box (words, from grid_bbox_kernel) and
+// the chirp records, as the processor decides it from its host copies: finite inputs, a grid
+// within the unambiguous range, ranges the cell index resolves, a table that fits. Fills in the
+// build inputs and leaves one of the two work counters spent. One block.
+__global__ void noalloc_decide_kernel(ProfilePlan plan, int *__restrict__ words, bool band)
+{
+    __shared__ double far2[256];
+    __shared__ float box[6];
+    const int tid = threadIdx.x;
+    if (tid < 6) {
+        const int key = words[kWordBox + tid];
+        box[tid] = __int_as_float(key >= 0 ? key : key ^ 0x7fffffff);
+    }
+    __syncthreads();
+    double most = 0.0;
+    bool finite = true;
+    const ChirpRec *recs = reinterpret_cast<const ChirpRec *>(plan.build.chirps);
+    for (int c = tid; c < plan.build.C; c += blockDim.x) {
+        const ChirpRec r = recs[c];
+        double f = 0.0;
+        const double p[3] = {(double)r.p_hi.x + r.p_lo.x, (double)r.p_hi.y + r.p_lo.y, (double)r.p_hi.z + r.p_lo.z};
+        for (int k = 0; k < 3; ++k) {
+            const double d = fmax(fabs(box[k] - p[k]), fabs(p[k] - box[3 + k]));
+            f += d * d;
+        }
+        finite = finite && f < 1e30 &&
+                 (band || (isfinite(r.vel.x) && isfinite(r.vel.y) && isfinite(r.vel.z) && isfinite(r.p_hi.w)));
+        most = fmax(most, f);
+    }
+    far2[tid] = most;
+    finite = __syncthreads_and(finite);
+    for (int s = blockDim.x / 2; s > 0; s >>= 1) {
+        if (tid < s) far2[tid] = fmax(far2[tid], far2[tid + s]);
+        __syncthreads();
+    }
+    if (tid) return;
+    ProfileBuild &b = plan.build;
+    double diag2 = 0.0;
+    for (int k = 0; k < 3; ++k) {
+        b.box_min[k] = box[k];
+        b.box_max[k] = box[3 + k];
+        diag2 += (b.box_max[k] - b.box_min[k]) * (b.box_max[k] - b.box_min[k]);
+    }
+    const double span = fabs(b.cells_per_m) * sqrt(diag2);
+    const bool take = finite && diag2 < 1e30 && fabs(b.cells_per_m) * sqrt(far2[0]) < 2097152.0 &&
+                      span + 7.0 <= (double)plan.max_cells && span + 7.0 <= 4.0 * b.S;
+    if (take) {
+        b.n_cells = ((int)ceil(span) + 7) / 2 * 2;
+        b.job.n_cells = b.n_cells;
+        *plan.build_out = b;
+        *plan.job_out = plan.job;
+    }
+    words[kWordProfile] = take;
+    words[kWordCounter] = take ? kSpent : 0;
+    words[kWordProfileCounter] = take ? 0 : kSpent;
+}
+
+__global__ void noalloc_units_kernel(FocusUnit *units, int n_tiles, int n_groups)
+{
+    const int n = n_tiles * n_groups;
+    for (int u = blockIdx.x * blockDim.x + threadIdx.x; u < n; u += gridDim.x * blockDim.x)
+        units[u] = FocusUnit{0, u % n_tiles, u / n_tiles, 0};
 }
 
 int fail(int code, const std::string &msg) { return set_last_error(code, msg); }
@@ -210,13 +297,97 @@ int enqueue(const tdc_noalloc_focus_args *a, float *image_dev, cudaStream_t st, 
     noalloc_setup_kernel<<<setup_blocks, 256, 0, st>>>(job, (int)n_tiles, n_groups, base);
     e = cudaGetLastError();
     if (e != cudaSuccess) return fail(TDC_ERR_CUDA, std::string("setup kernel: ") + cudaGetErrorString(e));
+    int *words = reinterpret_cast<int *>(base + kOffStatus);
+
+    // ---- range profiles, where the call is large enough and a table may fit ----
+    const bool band = std::isfinite(job.half_bw);
+    ProfilePlan pp{};
+    bool profile = impl::profile_pays((double)P, C, S) && (band || job.half_bw > 0.0f);
+    if (profile) {
+        const double gc = a->g0 + a->g1 * (S / 2), cells_per_m = 4.0 * S * a->g1;
+        const int tiles = (int)profile_tiles(P, (int)std::min<long long>(P, 1 << 30));
+        // two units per CTA, partials in at most a third of the array
+        const int pslots = n_sm * focus_profile_blocks_per_sm(1, band, false, false);
+        const long long fit = (long long)(TDC_NOALLOC_SCRATCH_BYTES / 3) / (P * 16);
+        int pg = (int)std::max<long long>(1, std::min<long long>({(long long)C, fit, (2LL * pslots + tiles - 1) / tiles}));
+        const int pcpg = (C + pg - 1) / pg;
+        pg = (C + pcpg - 1) / pcpg;
+        // (laid over the direct form's partials: one of the two runs)
+        size_t off = round_up(kOffUnits + (size_t)n_units * sizeof(FocusUnit), 256);
+        auto take = [&](size_t bytes) {
+            const size_t at = off;
+            off = round_up(off + bytes, 256);
+            return at;
+        };
+        const size_t o_job = take(sizeof(FocusJob)), o_pjob = take(sizeof(ProfileJob)),
+                     o_build = take(sizeof(ProfileBuild)), o_units = take((size_t)tiles * pg * sizeof(FocusUnit)),
+                     o_base = take((size_t)C * 4), o_tw = take((size_t)S * (kProfileNodes * 8 + 4)),
+                     o_part = take((size_t)pg * P * 16);
+        const long long left = (long long)TDC_NOALLOC_SCRATCH_BYTES - (long long)off;
+        pp.max_cells = (int)std::max<long long>(0, std::min<long long>(4LL * S, left / ((long long)C * kProfileCoefs * 8)));
+        profile = pp.max_cells >= 16 && std::isfinite(gc) && std::fabs(gc) > 0.0 && std::isfinite(cells_per_m);
+        pp.n_tiles = tiles;
+        pp.n_groups = pg;
+        pp.job_out = reinterpret_cast<FocusJob *>(base + o_job);
+        pp.build_out = reinterpret_cast<ProfileBuild *>(base + o_build);
+        pp.units = reinterpret_cast<FocusUnit *>(base + o_units);
+        pp.job = job;
+        pp.job.partial = reinterpret_cast<float4 *>(base + o_part);
+        pp.job.n_groups = pg;
+        pp.job.chirps_per_group = pcpg;
+        pp.job.n_tiles = tiles;
+        pp.job.grid_cols = (int)std::min<long long>(P, 1 << 30);
+        ProfileBuild &b = pp.build;
+        b.job_out = reinterpret_cast<ProfileJob *>(base + o_pjob);
+        pp.job.profile = b.job_out;
+        b.rows = reinterpret_cast<const float2 *>(a->samples);
+        b.chirps = reinterpret_cast<const float4 *>(a->chirps);
+        b.twiddle = reinterpret_cast<const float2 *>(base + o_tw);
+        b.factor = reinterpret_cast<const float *>(b.twiddle + (size_t)S * kProfileNodes);
+        b.cells = reinterpret_cast<float4 *>(base + off);
+        b.cell_base = reinterpret_cast<int *>(base + o_base);
+        b.cells_per_m = cells_per_m;
+        b.C = C;
+        b.S = S;
+        b.s_pad = s_pad;
+        b.chirp_words = (int)(sizeof(ChirpRec) / 16);
+        split_dd(gc, b.job.gc_hi, b.job.gc_lo);
+        split_dd(cells_per_m, b.job.cells_hi, b.job.cells_lo);
+        b.job.inv_gc2x4 = (float)(4.0 / (gc * gc));
+        b.job.cells_per_cycle = (float)(cells_per_m / gc);
+        b.job.cells = b.cells;
+        b.job.cell_base = b.cell_base;
+        b.job.inv_gc = (float)(1.0 / gc);
+    }
+    if (profile) {
+        e = launch_grid_bbox(job.grid_hi, P, words + kWordBox, st);
+        if (e == cudaSuccess) {
+            noalloc_decide_kernel<<<1, 256, 0, st>>>(pp, words, band);
+            noalloc_units_kernel<<<8, 256, 0, st>>>(pp.units, pp.n_tiles, pp.n_groups);
+            e = cudaGetLastError();
+        }
+        if (e == cudaSuccess)
+            e = launch_profile_twiddle(const_cast<float2 *>(pp.build.twiddle), const_cast<float *>(pp.build.factor), S, st);
+        if (e == cudaSuccess)
+            e = launch_profile_build_indirect(pp.build_out, words + kWordProfile, C, pp.max_cells, st);
+        const int n = pp.n_tiles * pp.n_groups;
+        const int ctas = std::min(n, n_sm * focus_profile_blocks_per_sm(1, band, false, false));
+        if (e == cudaSuccess)
+            e = launch_focus_profile(1, band, false, pp.job_out, pp.units, n, words + kWordProfileCounter, ctas, st);
+        if (e == cudaSuccess)
+            e = launch_focus_reduce(pp.job.partial, pp.n_groups, P, reinterpret_cast<float2 *>(image_dev), st,
+                                    words + kWordProfile, 1);
+        if (e != cudaSuccess)
+            return fail(TDC_ERR_CUDA, std::string("range profile kernels: ") + cudaGetErrorString(e));
+    }
     const int grid = (int)std::min<long long>(n_units, slots);
     e = launch_focus_fp32(reinterpret_cast<const FocusJob *>(base + kOffJob),
                           reinterpret_cast<const FocusUnit *>(base + kOffUnits), (int)n_units,
                           reinterpret_cast<int *>(base + kOffStatus), reinterpret_cast<int *>(base + kOffStatus) + 1,
                           stage_bytes, grid, std::isfinite(job.half_bw), false, false, st);
     if (e != cudaSuccess) return fail(TDC_ERR_CUDA, std::string("focus kernel: ") + cudaGetErrorString(e));
-    e = launch_focus_reduce(job.partial, n_groups, P, reinterpret_cast<float2 *>(image_dev), st);
+    e = launch_focus_reduce(job.partial, n_groups, P, reinterpret_cast<float2 *>(image_dev), st,
+                            words + kWordProfile, 0);
     if (e != cudaSuccess) return fail(TDC_ERR_CUDA, std::string("reduce kernel: ") + cudaGetErrorString(e));
     *status_word = reinterpret_cast<int *>(base + kOffStatus) + 1;
     return TDC_OK;

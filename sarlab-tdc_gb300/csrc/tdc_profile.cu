@@ -133,9 +133,21 @@ __global__ void profile_twiddle_kernel(float2 *__restrict__ tw, float *__restric
 // not grow with the row, and the cells' coefficients are formed from the nodes in shared memory.
 // Bound: FP32 FMA; C x S x (nodes the grid spans + up to one block) complex MACs, a few per cent
 // of the focus it serves.
+// INDIRECT: the inputs come from device memory (`dev`, written by an earlier kernel of the stream)
+// and the CTAs return at once where *enabled is 0.
+template <bool INDIRECT>
 __global__ void __launch_bounds__(kBuildThreads)
-    profile_build_kernel(const ProfileBuild b, const __grid_constant__ ProfileStencil stencil)
+    profile_build_kernel(const __grid_constant__ ProfileBuild direct, const __grid_constant__ ProfileStencil stencil,
+                         const ProfileBuild *__restrict__ dev, const int *__restrict__ enabled)
 {
+    __shared__ ProfileBuild sb;
+    if (INDIRECT) {
+        if (*enabled == 0) return;
+        for (int i = threadIdx.x; i < (int)(sizeof(ProfileBuild) / sizeof(int)); i += kBuildThreads)
+            reinterpret_cast<int *>(&sb)[i] = reinterpret_cast<const int *>(dev)[i];
+        __syncthreads();
+    }
+    const ProfileBuild &b = INDIRECT ? sb : direct;
     __shared__ __align__(16) float2 sx[kBuildStep][kBuildChirps];
     __shared__ __align__(16) float2 sv[kBuildStep * kNodes];  // phasors of a tile; then the nodes' values
     __shared__ int s_base[kBuildChirps];            // the chirp's first cell (absolute, even)
@@ -1065,7 +1077,16 @@ cudaError_t launch_profile_build(const ProfileBuild &b, cudaStream_t st)
     // nodes of n_cells / 2 from an even cell on, wherever the first block starts
     const int blocks = (b.n_cells / 2 + kOwn - 2) / kOwn + 1;
     const dim3 grid((b.C + kBuildChirps - 1) / kBuildChirps, blocks);
-    profile_build_kernel<<<grid, kBuildThreads, 0, st>>>(b, stencil);
+    profile_build_kernel<false><<<grid, kBuildThreads, 0, st>>>(b, stencil, nullptr, nullptr);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_profile_build_indirect(const ProfileBuild *dev, const int *enabled, int C, int max_cells,
+                                          cudaStream_t st)
+{
+    static const ProfileStencil stencil = make_stencil();
+    const dim3 grid((C + kBuildChirps - 1) / kBuildChirps, (max_cells / 2 + kOwn - 2) / kOwn + 1);
+    profile_build_kernel<true><<<grid, kBuildThreads, 0, st>>>(ProfileBuild{}, stencil, dev, enabled);
     return cudaGetLastError();
 }
 
