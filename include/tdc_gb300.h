@@ -190,8 +190,7 @@ int tdc_processor_set_plan_pixels(tdc_processor *proc, int64_t n_pix);
  * next focus. */
 int tdc_processor_set_motion_path(tdc_processor *proc, int enable);
 
-/* Large focuses on the FP32-bulk path (at least 5e8 correlations and 4 pixels a sample, an
- * unbounded Doppler band) read each (pixel, chirp) sum from a table of the chirp's spectrum
+/* Large focuses on the FP32-bulk path (at least 3e8 correlations and 4 pixels a sample) read each (pixel, chirp) sum from a table of the chirp's spectrum
  * over the grid's ranges instead of adding up its samples (range profiles): the same sums to
  * FP32 rounding, at a cost that does not grow with the row's length.
  *

@@ -989,6 +989,35 @@ void plan_groups(long long n_tiles, int C, int slots, int &n_groups, int &cpg, i
     }
 }
 
+// The same for a focus through range profiles: units of whole blocks of chirp records where that
+// costs no wave. In units of one chirp of one tile (0.8 us of a CTA): each block of
+// kProfileBlock chirps exposes about 1.5 (its first anchors), each unit about 3 (its pixels, its
+// partial sums), and the reduction reads every group's partial sums.
+void plan_profile_groups(long long n_tiles, int C, int slots, int min_units_per_slot, int &n_groups, int &cpg)
+{
+    const int gmax = std::max(1, std::min(C, 1024));
+    double best = std::numeric_limits<double>::infinity();
+    n_groups = 1;
+    cpg = C;
+    for (int pass = 0; pass < 2 && !(best < std::numeric_limits<double>::infinity()); ++pass)
+        for (int g = 1; g <= gmax; ++g) {
+            const int c = (C + g - 1) / g;
+            const int geff = (C + c - 1) / c;
+            if (geff != g) continue;
+            const long long units = n_tiles * geff;
+            if (units > (1LL << 24)) break;
+            if (pass == 0 && units < (long long)min_units_per_slot * slots) continue;
+            const double waves = (double)((units + slots - 1) / slots);
+            const double cost = waves * (c + 1.5 * ((c + kProfileBlock - 1) / kProfileBlock) + 3.0) +
+                                2.7e-3 * (double)units;
+            if (cost < best - 1e-9) {
+                best = cost;
+                n_groups = geff;
+                cpg = c;
+            }
+        }
+}
+
 // Scratch layout of one focus: [status words | job | units | partials].
 struct ScratchLayout {
     size_t off_job, off_units, off_partial, total;
@@ -1151,11 +1180,13 @@ bool anchor_eligible(const tdc_processor *p, int cb)
 // Range profiles (tdc_profile.cu). The table costs about S x (nodes the grid spans, at most 2 S)
 // complex MACs a chirp, so it needs pixels enough to share it (a direct focus costs S a pixel),
 // and a launch large enough for one more kernel. Whole focus, direct / profiles, 2 mm grids: at
-// 0.54 Gcorr 211 / 157 us (128^2 pixels x 128 chirps x 256 samples), 206 / 139 (256^2 x 128 x 64),
-// 429 / 373 (64^2 x 512 x 256); at 0.27 Gcorr 175 / 151 (128^2 x 128 x 128), 104 / 128 (64^2 x 256 x
-// 256); 64^2 pixels = 4 x 1024 samples, 1024 chirps: 885 / 413.
+// 0.54 Gcorr 140 / 66 us (128^2 pixels x 128 chirps x 256 samples), 173 / 71 (256^2 x 128 x 64),
+// 144 / 69 (64^2 x 512 x 256); at 0.27 Gcorr 106 / 63 (128^2 x 128 x 128), 74 / 67 (64^2 x 256 x
+// 256); at 0.03 Gcorr 40 / 50. Below the line the gain is at most 50 us, and callers that choose
+// between anchored and double-float ranges keep the direct kernels. 64^2 pixels = 4 x 1024
+// samples, 1024 chirps: 601 / 102.
 #ifndef TDC_PROFILE_MIN_WORK
-#define TDC_PROFILE_MIN_WORK 5e8
+#define TDC_PROFILE_MIN_WORK 3e8
 #endif
 bool profile_pays(double n_pix, double n_pri, double n_samples)
 {
@@ -1343,7 +1374,8 @@ int focus_plan(tdc_processor *p, FocusPlan &plan, double max_unit_work)
             const double by_work = std::floor(work / ((double)slots * kUnitTargetCorr));
             min_units = std::max(min_units, (int)std::min(32.0, by_work));
         }
-        plan_groups(plan_tiles, C, slots, p->plan_groups, p->plan_cpg, min_units);
+        if (profile) plan_profile_groups(plan_tiles, C, slots, min_units, p->plan_groups, p->plan_cpg);
+        else plan_groups(plan_tiles, C, slots, p->plan_groups, p->plan_cpg, min_units);
         p->plan_tiles = plan_tiles;
         if (max_unit_work > 0) {
             // bound the work of one unit (tile x chirp group): at most cap / (tile x S) chirps per group

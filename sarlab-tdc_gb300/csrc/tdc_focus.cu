@@ -875,40 +875,55 @@ __global__ void __launch_bounds__(kFocusThreads, TDC_FOCUS_MINB)
     }
 }
 
-// image[p] = sum over groups of (sum - comp) in FP64, in a fixed order that depends on n_groups
-// alone. Eight slices of a block's threads each add a run of groups, 4 loads in flight at a time,
-// and the slices are added in order: small focuses are planned with up to a group per chirp, and
-// one thread adding them one after another waited for a load at a time (147 us for 480 pixels x
-// 256 groups; whole start() of 480 pixels x 256 chirps x 128 samples 354 -> 229 us, focus of
-// 4,096 pixels x 256 x 256 104 -> 77 us).
+// image[p] = sum over groups of (sum - comp) in double-float, in a fixed order that depends on
+// n_groups alone (relative error below 2^-44 before the rounding to FP32; adding in FP64 gave the
+// same images, but its conversions and adds run at 1/64 rate here: 43 us instead of 10 for 256^2
+// pixels x 29 groups). Eight slices of a block's threads each add a run of groups, 4 loads in flight
+// at a time, and the slices are added in order: small focuses are planned with up to a group per
+// chirp, and one thread adding them one after another waited for a load at a time (whole start()
+// of 480 pixels x 256 chirps x 128 samples 354 -> 229 us with the slices).
+struct DoubleFloat {
+    float h, l;
+    // += x + y
+    __device__ __forceinline__ void add(float x, float y)
+    {
+        float s, e;
+        two_sum(h, x, s, e);
+        l += e + y;
+        h = s;
+    }
+    __device__ __forceinline__ float value() const { return h + l; }
+};
+
 constexpr int kReducePixels = 32, kReduceSlices = 8;
 __global__ void __launch_bounds__(kReducePixels *kReduceSlices)
     focus_reduce_sliced_kernel(const float4 *__restrict__ partial, int n_groups, long long P,
                                float2 *__restrict__ image, const int *__restrict__ enabled, int want)
 {
     if (enabled && *enabled != want) return;
-    __shared__ double2 part[kReduceSlices][kReducePixels];
+    __shared__ float4 part[kReduceSlices][kReducePixels];
     const long long p = (long long)blockIdx.x * kReducePixels + threadIdx.x;
     const int per = (n_groups + kReduceSlices - 1) / kReduceSlices;
     const int g0 = threadIdx.y * per, g1 = min(n_groups, g0 + per);
-    double re = 0.0, im = 0.0;
+    DoubleFloat re{0.f, 0.f}, im{0.f, 0.f};
     if (p < P) {
 #pragma unroll 4
         for (int g = g0; g < g1; ++g) {
             const float4 v = __ldg(&partial[(size_t)g * P + p]);
-            re += (double)v.x - (double)v.z;
-            im += (double)v.y - (double)v.w;
+            re.add(v.x, -v.z);
+            im.add(v.y, -v.w);
         }
     }
-    part[threadIdx.y][threadIdx.x] = make_double2(re, im);
+    part[threadIdx.y][threadIdx.x] = make_float4(re.h, im.h, re.l, im.l);
     __syncthreads();
     if (threadIdx.y == 0 && p < P) {
 #pragma unroll
         for (int k = 1; k < kReduceSlices; ++k) {
-            re += part[k][threadIdx.x].x;
-            im += part[k][threadIdx.x].y;
+            const float4 v = part[k][threadIdx.x];
+            re.add(v.x, v.z);
+            im.add(v.y, v.w);
         }
-        image[p] = make_float2((float)re, (float)im);
+        image[p] = make_float2(re.value(), im.value());
     }
 }
 
@@ -919,14 +934,14 @@ __global__ void focus_reduce_kernel(const float4 *__restrict__ partial, int n_gr
     if (enabled && *enabled != want) return;
     const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= P) return;
-    double re = 0.0, im = 0.0;
+    DoubleFloat re{0.f, 0.f}, im{0.f, 0.f};
 #pragma unroll 4
     for (int g = 0; g < n_groups; ++g) {
         const float4 v = __ldg(&partial[(size_t)g * P + p]);
-        re += (double)v.x - (double)v.z;
-        im += (double)v.y - (double)v.w;
+        re.add(v.x, -v.z);
+        im.add(v.y, -v.w);
     }
-    image[p] = make_float2((float)re, (float)im);
+    image[p] = make_float2(re.value(), im.value());
 }
 
 }  // namespace

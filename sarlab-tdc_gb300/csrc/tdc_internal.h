@@ -195,6 +195,7 @@ inline long long tile_count(long long P, int tile_cols, int grid_cols)
 constexpr int kProfileThreads = 64;     // a tile's kFocusTile pixels, 8 consecutive pixels a thread
 constexpr int kProfilePixels = kFocusTile / kProfileThreads;
 constexpr int kProfileNodes = 64;       // nodes one CTA of the table's construction forms
+constexpr int kProfileBlock = 32;       // chirp records the focus stages at a time
 constexpr int kProfileCoefs = 8;        // complex coefficients per cell
 constexpr double kProfileReach = 1.5;   // |t| a cell's polynomial is made for [cells]
 // CTAs per SM the planner counts on (the focus kernel's launch bound), and units per CTA.
@@ -203,7 +204,7 @@ constexpr double kProfileReach = 1.5;   // |t| a cell's polynomial is made for [
 #endif
 constexpr int kProfileCtasPerSm = TDC_PROFILE_CTAS;
 #ifndef TDC_PROFILE_MIN_UNITS
-#define TDC_PROFILE_MIN_UNITS 3
+#define TDC_PROFILE_MIN_UNITS 1
 #endif
 constexpr int kProfileMinUnitsPerSlot = TDC_PROFILE_MIN_UNITS;
 constexpr int kProfileBandMinUnitsPerSlot = 8;  // (units differ in their live chirps)

@@ -138,16 +138,27 @@ __global__ void grid_bbox_kernel(const float4 *__restrict__ hi, long long P, int
         span2 = d2 > span2 || d2 != d2 ? d2 : span2;
     }
     const int span = __reduce_max_sync(0xffffffffu, __float_as_int(fabsf(sqrtf(span2))));
-    if ((threadIdx.x & 31) == 0 && span > 0) atomicMax(&out[9], span);
+    __shared__ int part[8][7];  // one row a warp: the block's atomics are 7, not 7 a warp
     for (int d = 0; d < 3; ++d) {
-        for (int off = 16; off > 0; off >>= 1) {
-            mn[d] = min(mn[d], __shfl_xor_sync(0xffffffffu, mn[d], off));
-            mx[d] = max(mx[d], __shfl_xor_sync(0xffffffffu, mx[d], off));
+        mn[d] = __reduce_min_sync(0xffffffffu, mn[d]);
+        mx[d] = __reduce_max_sync(0xffffffffu, mx[d]);
+    }
+    const int warp = threadIdx.x >> 5;
+    if ((threadIdx.x & 31) == 0) {
+        for (int d = 0; d < 3; ++d) {
+            part[warp][d] = mn[d];
+            part[warp][3 + d] = mx[d];
         }
-        if ((threadIdx.x & 31) == 0) {
-            atomicMin(&out[d], mn[d]);
-            atomicMax(&out[3 + d], mx[d]);
-        }
+        part[warp][6] = span;
+    }
+    __syncthreads();
+    if (threadIdx.x < 7) {
+        const int d = threadIdx.x, n_warps = blockDim.x >> 5;
+        int v = part[0][d];
+        for (int w = 1; w < n_warps; ++w) v = d < 3 ? min(v, part[w][d]) : max(v, part[w][d]);
+        if (d < 3) atomicMin(&out[d], v);
+        else if (d < 6) atomicMax(&out[d], v);
+        else if (v > 0) atomicMax(&out[9], v);
     }
 }
 

@@ -270,6 +270,7 @@ struct FocusPlan {
 int prepare(tdc_processor *p, const StartOpts &o, int &launches);
 int upload_grid(tdc_processor *p, int &launches);
 int choose_path(const tdc_processor *p);
+void plan_profile_groups(long long n_tiles, int C, int slots, int min_units_per_slot, int &n_groups, int &cpg);
 void plan_groups(long long n_tiles, int C, int slots, int &n_groups, int &cpg, int min_units_per_slot);
 // Tile shape of the resident grid: 0 (flat tiles) or the columns of a block tile.
 int choose_tile_cols(const tdc_processor *p);

@@ -191,40 +191,66 @@ __global__ void __launch_bounds__(kBuildThreads)
 #pragma unroll
         for (int k = 0; k < 2; ++k) acc[i][k] = run[i][k] = make_float2(0.f, 0.f);
 
+    // A tile's samples and phasors are loaded into registers while the tile before it is worked on.
+    constexpr int kRowsEach = kBuildStep * kBuildChirps / kBuildThreads;
+    constexpr int kPhasorsEach = kBuildStep * kNodes / 2 / kBuildThreads;
+    float2 ahead_x[kRowsEach];
+    float4 ahead_z[kPhasorsEach];
+    float ahead_f = 0.f;
+    const int si_mine = (warp & 1) * 32 + lane;  // this thread's sample of a tile, for kRowsEach chirps
+    auto load_ahead = [&](int s0) {
+        const int s = s0 + si_mine;
+        ahead_f = s < b.S ? b.factor[s] : 0.f;
+#pragma unroll
+        for (int i = 0; i < kRowsEach; ++i) {
+            const int q = (warp >> 1) + 4 * i;
+            ahead_x[i] = s < b.S && c0 + q < b.C ? b.rows[(size_t)(c0 + q) * b.s_pad + s] : make_float2(0.f, 0.f);
+        }
+        // phasors: kBuildStep x kNodes, contiguous in memory (rows past the end meet zero samples)
+        const int ns = min(kBuildStep, b.S - s0);
+        const float4 *src = reinterpret_cast<const float4 *>(b.twiddle + (size_t)s0 * kNodes);
+#pragma unroll
+        for (int i = 0; i < kPhasorsEach; ++i) {
+            const int e = tid + i * kBuildThreads;
+            ahead_z[i] = e < ns * kNodes / 2 ? __ldg(&src[e]) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+    };
+    // shift's turns at this thread's sample, modulo 2 S: (first node) x (s - sc), advanced a tile at a time
+    unsigned int turn[kRowsEach], turn_step[kRowsEach];
+    {
+        const int d = si_mine - b.S / 2;
+        const long long dm = d < 0 ? d + (long long)nn : d;
+#pragma unroll
+        for (int i = 0; i < kRowsEach; ++i) {
+            const unsigned long long sh = s_shift[(warp >> 1) + 4 * i];
+            turn[i] = (unsigned)((sh * (unsigned long long)(dm % nn)) % nn);
+            turn_step[i] = (unsigned)((sh * kBuildStep) % nn);
+        }
+    }
+    const float fnn = (float)nn, inv_nn = 1.0f / fnn;
+    load_ahead(0);
+
     for (int s0 = 0, tile = 0; s0 < b.S; s0 += kBuildStep, ++tile) {
         // rows: shifted by the block's first node, scaled, zero past the row's end
 #pragma unroll
-        for (int i = 0; i < kBuildStep * kBuildChirps / kBuildThreads; ++i) {
-            const int q = (warp >> 1) + 4 * i, si = (warp & 1) * 32 + lane;
-            const int s = s0 + si;
-            float2 v = make_float2(0.f, 0.f);
-            if (s < b.S && c0 + q < b.C) {
-                const float2 x = b.rows[(size_t)(c0 + q) * b.s_pad + s];
-                const float f = b.factor[s];
-                const int d = s - b.S / 2;
-                const unsigned int dm = d < 0 ? (unsigned)(d + (int)nn) : (unsigned)d;
-                // (nn < 2^16: the product fits 32 bits)
-                const unsigned int r = nn < 65536u ? (s_shift[q] * dm) % nn
-                                                   : (unsigned)(((unsigned long long)s_shift[q] * dm) % nn);
-                const int rc = r > nn / 2 ? (int)r - (int)nn : (int)r;
-                float sn, cs;
-                sincospif(2.0f * __fdiv_rn((float)rc, (float)nn), &sn, &cs);
-                v = make_float2(f * fmaf(x.x, cs, -x.y * sn), f * fmaf(x.x, sn, x.y * cs));
-            }
-            sx[si][q] = v;
+        for (int i = 0; i < kRowsEach; ++i) {
+            const int rc = turn[i] > nn / 2 ? (int)turn[i] - (int)nn : (int)turn[i];
+            turn[i] += turn_step[i];
+            if (turn[i] >= nn) turn[i] -= nn;
+            // rc / nn to FP32 rounding
+            const float fr = (float)rc;
+            float ratio = fr * inv_nn;
+            ratio = fmaf(fmaf(-ratio, fnn, fr), inv_nn, ratio);
+            float sn, cs;
+            sincospif(2.0f * ratio, &sn, &cs);
+            const float2 x = ahead_x[i];
+            sx[si_mine][(warp >> 1) + 4 * i] =
+                make_float2(ahead_f * fmaf(x.x, cs, -x.y * sn), ahead_f * fmaf(x.x, sn, x.y * cs));
         }
-        // phasors: kBuildStep x kNodes, contiguous in memory (rows past the end meet zero samples)
-        {
-            const int ns = min(kBuildStep, b.S - s0);
-            const float4 *src = reinterpret_cast<const float4 *>(b.twiddle + (size_t)s0 * kNodes);
-            float4 *dst = reinterpret_cast<float4 *>(sv);
 #pragma unroll
-            for (int i = 0; i < kBuildStep * kNodes / 2 / kBuildThreads; ++i) {
-                const int e = tid + i * kBuildThreads;
-                dst[e] = e < ns * kNodes / 2 ? __ldg(&src[e]) : make_float4(0.f, 0.f, 0.f, 0.f);
-            }
-        }
+        for (int i = 0; i < kPhasorsEach; ++i) reinterpret_cast<float4 *>(sv)[tid + i * kBuildThreads] = ahead_z[i];
         __syncthreads();
+        if (s0 + kBuildStep < b.S) load_ahead(s0 + kBuildStep);
 #pragma unroll 8
         for (int si = 0; si < kBuildStep / 2; ++si) {
             const int s = half * (kBuildStep / 2) + si;
@@ -303,7 +329,7 @@ constexpr int kPT = kFocusTile / kProfileThreads;  // pixels per thread: consecu
 #ifndef TDC_PROFILE_MINB
 #define TDC_PROFILE_MINB 8
 #endif
-constexpr int kFlush = 32;                         // chirps summed in plain FP32 between Kahan steps
+constexpr int kFlush = kProfileBlock;                         // chirps summed in plain FP32 between Kahan steps
 
 struct SharedSums {
     float4 s[kPT][kThreads];       // (sum.re, sum.im, comp.re, comp.im)

@@ -163,8 +163,10 @@ size_t device_footprint(const tdc_job_desc &d, int n_sm, size_t &table)
         auto g = [&](long long i, int k) { return d.grid_f64 ? d.grid_f64[3 * i + k] : (double)d.grid[3 * i + k]; };
         const long long tiles = profile_tiles((long long)P, detect_run((long long)P, g));
         int pg = 1, pcpg = d.n_pri;
-        plan_groups(tiles, d.n_pri, n_sm * kProfileCtasPerSm, pg, pcpg,
-                    std::isfinite(d.doppler_bandwidth / 2.0f) ? kProfileBandMinUnitsPerSlot : kProfileMinUnitsPerSlot);
+        plan_profile_groups(tiles, d.n_pri, n_sm * kProfileCtasPerSm,
+                            std::isfinite(d.doppler_bandwidth / 2.0f) ? kProfileBandMinUnitsPerSlot
+                                                                      : kProfileMinUnitsPerSlot,
+                            pg, pcpg);
         const int cap = std::max(1, (int)(kServerUnitWork / ((double)kFocusTile * kProfilePairCost)));
         if (pcpg > cap) pg = (d.n_pri + cap - 1) / cap;
         table = (size_t)(kServerTableRatio * (double)(C * S * 8)) + C * 4 + sizeof(ProfileJob) +
