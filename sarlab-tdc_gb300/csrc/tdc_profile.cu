@@ -331,6 +331,12 @@ constexpr int kPT = kFocusTile / kProfileThreads;  // pixels per thread: consecu
 #endif
 constexpr int kFlush = kProfileBlock;                         // chirps summed in plain FP32 between Kahan steps
 
+// (sqrt(1 + y) - 1) / (y / 2) = 1 - y / 4 + kRoot2 y^2 + kRoot3 y^3 on |y| <= Y = 0.061: the Taylor
+// terms 1/8 and -5/64, with 7/128 y^4 replaced by its best multiple of y^2 there, 0.828 Y^2 y^2
+// (error below 1.3e-7 at the end of the range, 4e-8 at 0.045, vanishing with y).
+constexpr float kRootRange = 0.061f;
+constexpr float kRoot2 = 0.125f + 7.0f / 128.0f * 0.828f * kRootRange * kRootRange, kRoot3 = -5.0f / 64.0f;
+
 struct SharedSums {
     float4 s[kPT][kThreads];       // (sum.re, sum.im, comp.re, comp.im)
     float2 dz[kPT / 2][kThreads];  // z offsets and |d|^2 of the thread's pixel pairs
@@ -575,8 +581,8 @@ __device__ __forceinline__ void adjoint_pair(float2 psi, float turn, float t0, f
 // threads read the same few cells) are formed once in double-float. A pixel then takes its
 // phase difference from the anchor, psi = gc (R - R0) cycles, from
 //   Q = gc (R^2 - R0^2) / (2 R0) = d.e' + |d|^2 h     (d = pixel - anchor, 4 operations),
-//   psi = Q (1 + b1 Q + b2 Q^2 + b3 Q^3 + b4 Q^4)     (sqrt(1 + y) - 1, y = Q k2 small),
-// where y is small (relative error below 3e-8 for reach / R0 <= 0.03), or from the exact
+//   psi = Q (1 + b1 Q + b2 Q^2 + b3 Q^3)              (sqrt(1 + y) - 1, y = Q k2 small),
+// where y is small (|y| <= 0.061, reach / R0 <= 0.03), or from the exact
 // quotient otherwise, and the cell's polynomial at t0 + psi x cells per cycle. About 36
 // operations a pixel and chirp plus 100 per anchor, whatever the row's length.
 //
@@ -585,7 +591,8 @@ __device__ __forceinline__ void adjoint_pair(float2 psi, float turn, float t0, f
 // slots) 7.7; the next anchor formed beside this one's pixels 7.5; blocks of 8 runs x 32 pixels a
 // warp instead of 256 pixels of a run, and chirp records staged in shared memory 32 at a time,
 // 7.2-7.4 (the cells' wait for memory: 1.5 -> 0.4 cycles an instruction). 64-thread CTAs at 128
-// registers: 16 warps an SM; 12 or 18 warps are 2-6% slower.
+// registers: 16 warps an SM; 12 or 18 warps are 2-6% slower. With the cells in L1, forming the next
+// anchor ahead costs more registers than it hides (7.05 -> 6.72 ms without).
 //
 // BAND: a finite Doppler band. Chirps out of band for all of a warp's pixels are found first, 32
 // at a time, from the anchors' Doppler and a bound on its change over a group (about 20
@@ -823,16 +830,13 @@ __global__ void __launch_bounds__(kThreads, G == 1 ? (BAND || ADJ ? 4 : 6) : BAN
                 todo &= __reduce_or_sync(0xffffffffu, live);
             }
             int k = __ffs(todo) - 1;
-            Anchor next;
-            if (G > 2 && todo) next = anchor_of(k, ax[0]);
             while (todo) {
                 todo &= todo - 1;
-                const int k_next = todo ? __ffs(todo) - 1 : k;
+                const int k_next = __ffs(todo) - 1;
                 float grad[3] = {0.f, 0.f, 0.f};
 #pragma unroll
                 for (int g = 0; g < kSub; ++g) {
-                    // (one or two pixels an anchor: the thread's other anchors cover the latency)
-                    const Anchor cur = G > 2 ? next : anchor_of(k, ax[g]);
+                    const Anchor cur = anchor_of(k, ax[g]);
                     if constexpr (G == 1) {
                         // (the antenna on the pixel: NaN Doppler, zero window)
                         float sn, cs;
@@ -875,8 +879,8 @@ __global__ void __launch_bounds__(kThreads, G == 1 ? (BAND || ADJ ? 4 : 6) : BAN
                             const float h = cur.h, h2 = -2.0f * h;
                             const float e2x = h2 * cur.ex, e2y = h2 * cur.ey, e2z = h2 * cur.ez;
                             const float k2 = h * jc.x;
-                            const float b1 = -0.25f * k2, b2 = 0.125f * k2 * k2;
-                            const float b3 = -0.625f * b2 * k2, b4 = 0.4375f * b2 * k2 * k2;
+                            const float b1 = -0.25f * k2, b2 = kRoot2 * k2 * k2;
+                            const float b3 = kRoot3 * k2 * k2 * k2;
 #pragma unroll
                             for (int i = 0; i < G / 2; ++i) {
                                 const int s = g * (G / 2) + i;
@@ -884,8 +888,7 @@ __global__ void __launch_bounds__(kThreads, G == 1 ? (BAND || ADJ ? 4 : 6) : BAN
                                     __ffma2_rn(dx[s], both(e2x),
                                                __ffma2_rn(dy[s], both(e2y),
                                                           __ffma2_rn(fresh2(&sums.dz[s][tid]), both(e2z), __fmul2_rn(fresh2(&sums.dd[s][tid]), both(h)))));
-                                float2 f = __ffma2_rn(q, both(b4), both(b3));
-                                f = __ffma2_rn(q, f, both(b2));
+                                float2 f = __ffma2_rn(q, both(b3), both(b2));
                                 f = __ffma2_rn(q, f, both(b1));
                                 psi[i] = __ffma2_rn(__fmul2_rn(q, q), f, q);
                             }
@@ -971,8 +974,6 @@ __global__ void __launch_bounds__(kThreads, G == 1 ? (BAND || ADJ ? 4 : 6) : BAN
 #pragma unroll
                             for (int i = 0; i < G; ++i) w[i] = ADJ && (zero >> i & 1u) ? 0.0f : 1.0f;
                         }
-                        // the next anchor's chain of dependent operations runs beside this one's pixels
-                        if (G > 2) next = anchor_of(g + 1 < kSub ? k : k_next, ax[g + 1 < kSub ? g + 1 : 0]);
                         if constexpr (ADJ) {
                             float2 d[kProfileCoefs - 1];
                             adjoint_coefs(cur.a, jc.y, d);

@@ -212,7 +212,7 @@ def test_profile_adjoint_against_the_oracle(cuda_device, nx, ny, spacing, group,
     (57, 131, 300, 256, 1e-3, 0.2e-3, 1e-6),   # a little acceleration
 ])
 def test_profile_focus_of_smooth_motion(cuda_device, nx, ny, n_pri, n_samples, spacing, drift, accel):
-    """Positions moving within each chirp, at least 5e8 correlations. The oracle reads every
+    """Positions moving within each chirp, at least 3e8 correlations. The oracle reads every
     sample's FP32 position; the fit smooths their rounding, 1.7e-8 m rms a coordinate or 5e-5 rad
     a sample, which the sum over samples averages: tolerance 2e-5. The FP32 general kernel, which
     follows each position, and this path agree to the same."""

@@ -1,4 +1,4 @@
-"""GPU parity of tdc_focus_noalloc where it may take range profiles (at least 5e8 correlations):
+"""GPU parity of tdc_focus_noalloc where it may take range profiles (at least 3e8 correlations):
 the form is decided on the device from the grid and the trajectory. Tables that fit the fixed
 scratch, a finite band with skip points, double-float inputs, and a captured call replayed on a
 grid changed in place so that its table does not fit and the direct form is taken. Tolerances: relative L2 <= 3e-6 against the FP64 oracle as for the processor's
