@@ -738,7 +738,7 @@ int upload_grid(tdc_processor *p, int &launches)
     p->grid_run = detect_run(
         P, [&](long long i, int k) { return p->grid64 ? p->grid64[3 * i + k] : (double)p->grid[3 * i + k]; });
     // (small focuses do not ask for the reach: measured when a plan first does)
-    p->reach_known = p->has_raw && profile_pays((double)std::max(P, p->plan_pixels), p->C, p->S);
+    p->reach_known = p->has_raw && profile_pays((double)std::max(P, p->plan_pixels), p->C, p->S, false);
     if (P > 0) {
         // bounding box, reach and anchor span of the grid, measured on the device (the box as
         // order-preserving integer keys of the floats)
@@ -992,21 +992,24 @@ void plan_groups(long long n_tiles, int C, int slots, int &n_groups, int &cpg, i
 // The same for a focus through range profiles: units of whole blocks of chirp records where that
 // costs no wave. In units of one chirp of one tile (0.8 us of a CTA): each block of
 // kProfileBlock chirps exposes about 1.5 (its first anchors), each unit about 3 (its pixels, its
-// partial sums), and the reduction reads every group's partial sums.
+// partial sums), and the reduction reads every group's partial sums. At least min_units_per_slot
+// units a slot, or as many as units of half a block leave (128^2 pixels x 512 chirps x 128 samples
+// under a finite band: 262 us in units of one chirp, 80 us so); a second wave to reach one unit a
+// slot costs more than a few idle slots (128^2 x 256 x 256: 60 -> 54 us).
 void plan_profile_groups(long long n_tiles, int C, int slots, int min_units_per_slot, int &n_groups, int &cpg)
 {
     const int gmax = std::max(1, std::min(C, 1024));
     double best = std::numeric_limits<double>::infinity();
     n_groups = 1;
     cpg = C;
-    for (int pass = 0; pass < 2 && !(best < std::numeric_limits<double>::infinity()); ++pass)
+    for (int want = min_units_per_slot;; want /= 2) {
         for (int g = 1; g <= gmax; ++g) {
             const int c = (C + g - 1) / g;
             const int geff = (C + c - 1) / c;
             if (geff != g) continue;
             const long long units = n_tiles * geff;
             if (units > (1LL << 24)) break;
-            if (pass == 0 && units < (long long)min_units_per_slot * slots) continue;
+            if (want > 1 && (units < (long long)want * slots || c < kProfileBlock / 2)) continue;
             const double waves = (double)((units + slots - 1) / slots);
             const double cost = waves * (c + 1.5 * ((c + kProfileBlock - 1) / kProfileBlock) + 3.0) +
                                 2.7e-3 * (double)units;
@@ -1016,6 +1019,8 @@ void plan_profile_groups(long long n_tiles, int C, int slots, int min_units_per_
                 cpg = c;
             }
         }
+        if (best < std::numeric_limits<double>::infinity() || want <= 1) return;
+    }
 }
 
 // Scratch layout of one focus: [status words | job | units | partials].
@@ -1184,13 +1189,14 @@ bool anchor_eligible(const tdc_processor *p, int cb)
 // 144 / 69 (64^2 x 512 x 256); at 0.27 Gcorr 106 / 63 (128^2 x 128 x 128), 74 / 67 (64^2 x 256 x
 // 256); at 0.03 Gcorr 40 / 50. Below the line the gain is at most 50 us, and callers that choose
 // between anchored and double-float ranges keep the direct kernels. 64^2 pixels = 4 x 1024
-// samples, 1024 chirps: 601 / 102.
+// samples, 1024 chirps: 601 / 102. Under a finite band the line is at 0.5 Gcorr: callers that read
+// the direct kernel's block tiles and unit spans do so at 0.47 (there 490-530 / 66-78 us).
 #ifndef TDC_PROFILE_MIN_WORK
 #define TDC_PROFILE_MIN_WORK 3e8
 #endif
-bool profile_pays(double n_pix, double n_pri, double n_samples)
+bool profile_pays(double n_pix, double n_pri, double n_samples, bool band)
 {
-    return n_pix >= 4.0 * n_samples && n_pix * n_pri * n_samples >= TDC_PROFILE_MIN_WORK;
+    return n_pix >= 4.0 * n_samples && n_pix * n_pri * n_samples >= (band ? 5e8 : TDC_PROFILE_MIN_WORK);
 }
 
 // Smooth motion through range profiles: largest bend of the phase at a row's ends [rad].
@@ -1220,7 +1226,7 @@ int profile_group(tdc_processor *p, int path, ProfileBuild &b)
     const bool band = std::isfinite(half_bw);
     if (!band && (!p->rec_finite || !(half_bw > 0.0f))) return 0;
     const long long P = std::max(p->P, p->plan_pixels);
-    if (!profile_pays((double)P, p->C, p->S)) return 0;
+    if (!profile_pays((double)P, p->C, p->S, band)) return 0;
     const double g1 = 2.0 * p->F1 / kC0, gc = 2.0 * p->F0 / kC0 + g1 * (p->S / 2);
     b.cells_per_m = 4.0 * p->S * g1;
     double diag2 = 0.0;

@@ -140,7 +140,8 @@ double pair_work(const FocusPlan &pl, int n_samples)
 // The same before the job is planned (its size decides, barring inputs that rule profiles out).
 double pair_work_estimate(const tdc_job_desc &d)
 {
-    const bool profile = profile_pays((double)d.n_pix, d.n_pri, d.n_samples);
+    const bool profile =
+        profile_pays((double)d.n_pix, d.n_pri, d.n_samples, std::isfinite(d.doppler_bandwidth / 2.0f));
     return profile ? kProfilePairCost : d.n_samples;
 }
 
@@ -157,7 +158,7 @@ size_t device_footprint(const tdc_job_desc &d, int n_sm, size_t &table)
     if (cpg > cpg_cap) groups = (d.n_pri + cpg_cap - 1) / cpg_cap;
     const size_t n_tiles = (P + kFocusTile - 1) / kFocusTile;
     size_t b = 0;
-    if (profile_pays((double)P, (double)C, (double)S)) {
+    if (profile_pays((double)P, (double)C, (double)S, std::isfinite(d.doppler_bandwidth / 2.0f))) {
         // range profiles: the table, bounded by its ratio to the samples whatever the grid, and
         // this plan's groups where they are more
         auto g = [&](long long i, int k) { return d.grid_f64 ? d.grid_f64[3 * i + k] : (double)d.grid[3 * i + k]; };
