@@ -190,9 +190,12 @@ int tdc_processor_set_plan_pixels(tdc_processor *proc, int64_t n_pix);
  * next focus. */
 int tdc_processor_set_motion_path(tdc_processor *proc, int enable);
 
-/* Large focuses on the FP32-bulk path (at least 3e8 correlations and 4 pixels a sample) read each (pixel, chirp) sum from a table of the chirp's spectrum
- * over the grid's ranges instead of adding up its samples (range profiles): the same sums to
- * FP32 rounding, at a cost that does not grow with the row's length.
+/* Large focuses (at least 4 pixels a sample and 3e8 correlations, 5e8 under a finite Doppler band)
+ * read each (pixel, chirp) sum from a table of the chirp's spectrum over the grid's ranges
+ * instead of adding up its samples (range profiles): the same sums to FP32 rounding, at a cost that
+ * does not grow with the row's length. They serve the FP32-bulk path, and under an unbounded band
+ * the smooth-motion path and, on the FP32 general path, antennas that move at a constant velocity
+ * within each chirp but for vibrations of at most 0.1 rad of carrier phase.
  *
  * Anchored ranges in the FP32-bulk kernel on (1, default) or off (0). With an unbounded Doppler
  * band, finite velocities, no kept per-chirp sums and rows of 3-16 chirps per pipeline stage

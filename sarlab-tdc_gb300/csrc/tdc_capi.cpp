@@ -408,6 +408,7 @@ int prepare(tdc_processor *p, const StartOpts &o, int &launches)
     // of the input (up to half an ulp per sample, spread a little further by the fit).
     std::vector<MotionRec> mrecs;
     std::vector<MoveRec> vrecs;  // the same fits about the middle sample (range profiles)
+    p->vib_known = false;
     p->motion_fit_ok = false;
     p->motion_v1max = p->motion_v2max = 0.0;
     if (p->traj_varies && !p->win_varies && S >= 3) {
@@ -628,6 +629,9 @@ int prepare(tdc_processor *p, const StartOpts &o, int &launches)
     p->offsets_applied = false;
     ++p->state_epoch;
     p->plan_path = -1;  // job parameters changed
+    if (p->P > 0 && p->traj_varies && !p->win_varies && !std::isfinite(o.bw) &&
+        profile_pays((double)std::max(p->P, p->plan_pixels), C, S, false) && choose_path(p) == TDC_PATH_GENERAL)
+        return measure_vibration(p);
     return TDC_OK;
 }
 
@@ -650,6 +654,32 @@ int measure_group_reach(tdc_processor *p)
     TDC_CK(cudaMemcpyAsync(bits, reach, sizeof(bits), cudaMemcpyDeviceToHost, p->stream), "read reach");
     TDC_CK(cudaStreamSynchronize(p->stream), "reach sync");
     set_group_reach(p, bits);
+    return TDC_OK;
+}
+
+// Fits of the resident acquisition's per-sample positions (profile_group), measured once per
+// prepared acquisition: by prepare where the grid is known to ask for it, else when a plan does.
+int measure_vibration(tdc_processor *p)
+{
+    const double g1 = 2.0 * p->F1 / kC0, gc = 2.0 * p->F0 / kC0 + g1 * (p->S / 2);
+    const double phase_per_m = 2.0 * M_PI * (std::fabs(gc) + std::fabs(g1) * 0.5 * p->S);
+    int bits[3];
+    TDC_CK(p->vib_rec.ensure((size_t)p->C * sizeof(VibRec) + 16), "alloc vibration records");
+    VibRec *recs = p->vib_rec.as<VibRec>();
+    int *maxima = reinterpret_cast<int *>(recs + p->C);
+    TDC_CK(cudaMemsetAsync(maxima, 0, sizeof(bits), p->stream), "reset maxima");
+    TDC_CK(launch_vib_fit(p->traj.as<const float4>(), p->gen_rec.as<const ChirpRec>(), p->C, p->S, p->s_pad,
+                          (float)phase_per_m, recs,
+                          maxima, p->stream),
+           "vibration fit kernel");
+    TDC_CK(cudaMemcpyAsync(bits, maxima, sizeof(bits), cudaMemcpyDeviceToHost, p->stream), "read maxima");
+    TDC_CK(cudaStreamSynchronize(p->stream), "vibration sync");
+    for (int k = 0; k < 3; ++k) {
+        float v;
+        std::memcpy(&v, &bits[k], 4);
+        p->vib_max[k] = v;
+    }
+    p->vib_known = true;
     return TDC_OK;
 }
 
@@ -1199,10 +1229,18 @@ bool profile_pays(double n_pix, double n_pri, double n_samples, bool band)
     return n_pix >= 4.0 * n_samples && n_pix * n_pri * n_samples >= (band ? 5e8 : TDC_PROFILE_MIN_WORK);
 }
 
+// Vibration through range profiles [rad]: largest carrier phase of the deviations from constant
+// velocity (their series leaves 5e-7 at 0.1), of their part off the chirp's principal direction
+// (kept to first order), of the range's second order (kept at the middle carrier), and of the
+// deviations' change over a group of pixels (half its square is left out).
+constexpr double kVibMaxPhase = 0.1, kVibMaxSide = 5e-4, kVibMaxBow = 3e-5, kVibMaxTurn = 3e-3;
+
 // Smooth motion through range profiles: largest bend of the phase at a row's ends [rad].
 constexpr double kMoveMaxBend = 0.1;
-// ... and of its difference within a group [rad] (the neglected second order is half its square).
-constexpr double kMoveMaxTurn = 4e-3;
+// ... of the phase's third order there (left out, weighted by s~^3) [rad],
+constexpr double kMoveMaxThird = 8e-6;
+// ... and of the bend's difference within a group [rad] (the neglected second order is half its square).
+constexpr double kMoveMaxTurn = 2e-3;
 
 bool profile_table_fits(int n_cells, int n_samples, double table_ratio)
 {
@@ -1240,19 +1278,42 @@ int profile_group(tdc_processor *p, int path, ProfileBuild &b)
     b.n_cells = profile_cells(b.cells_per_m, std::sqrt(diag2));
     b.margin = 0;
     b.chirp_words = 3;
-    const bool motion = path == TDC_PATH_FP32_MOTION;
+    const bool vibration = path == TDC_PATH_GENERAL;
+    const bool motion = path == TDC_PATH_FP32_MOTION || vibration;
+    b.traj = nullptr;
     double slack = 0.0, max_bend = 0.0;  // largest shift of a pixel's cell [cells], bend [rad]
     const double rmin = min_range(p->ant_min, p->ant_max, p->grid_min, p->grid_max);
-    const double w1 = p->motion_v1max + 2.0 * p->motion_v2max * p->S, h = 0.5 * p->S;
+    const double h = 0.5 * p->S, g_max = std::fabs(gc) + std::fabs(g1) * h;
+    double w1 = p->motion_v1max + 2.0 * p->motion_v2max * p->S, v2 = p->motion_v2max, amp = 0.0;
+    if (vibration) {
+        // per-sample positions only, uniform sampling, an antenna clear of the grid
+        const double rmax_phase = 2.0 * M_PI * 2.0 * p->resid_hz * rmax / kC0;
+        if (!p->traj_varies || p->win_varies || !p->motion_enabled || band || !(rmin > 0.0) ||
+            rmax_phase > kUniformPhaseTolRad || (!p->vib_known && measure_vibration(p)))
+            return 0;
+        w1 = p->vib_max[2];
+        v2 = 0.0;
+        amp = 2.0 * M_PI * g_max * p->vib_max[0];
+        if (!(amp <= kVibMaxPhase && 2.0 * M_PI * g_max * p->vib_max[1] <= kVibMaxSide &&
+              M_PI * g_max * p->vib_max[0] * p->vib_max[0] / rmin <= kVibMaxBow))
+            return 0;
+    }
     if (motion) {
-        // (motion_segment has bounded the motion: rmin > 0)
+        // (motion_segment has bounded the smooth motion: rmin > 0)
         const double bend = 2.0 * M_PI * h * h *
-                            (std::fabs(g1) * w1 + std::fabs(gc) * (w1 * w1 / (2.0 * rmin) + p->motion_v2max));
+                            (std::fabs(g1) * w1 + std::fabs(gc) * (w1 * w1 / (2.0 * rmin) + v2));
         const double shift = 4.0 * p->S * std::fabs(gc) * w1;
-        if (band || !(bend <= kMoveMaxBend) || !(shift <= 64.0)) return 0;
+        // third order of the range change, (e.W |W x e|^2 / 2 R^2 + W.V2 / R) s~^3
+        const double third = 2.0 * M_PI * std::fabs(gc) * h * h * h * w1 / rmin * (0.2 * w1 * w1 / rmin + v2);
+        if (band || !(bend <= kMoveMaxBend) || !(shift <= 64.0) || !(third <= kMoveMaxThird)) return 0;
         b.margin = 2 * (int)std::ceil(0.5 * shift) + 2;
         b.n_cells += 2 * b.margin;
-        b.chirp_words = 4;
+        b.chirp_words = vibration ? 6 : 4;
+        if (vibration) {
+            b.traj = p->traj.as<const float4>();
+            b.phase_g = (float)(2.0 * M_PI * gc);
+            b.phase_g1 = (float)(2.0 * M_PI * g1);
+        }
         slack = shift;
         max_bend = bend;
     }
@@ -1260,7 +1321,7 @@ int profile_group(tdc_processor *p, int path, ProfileBuild &b)
     b.C = p->C;
     b.S = p->S;
     b.s_pad = p->s_pad;
-    const size_t bytes = (size_t)p->C * b.n_cells * kProfileCoefs * 8;
+    const size_t bytes = (size_t)p->C * b.n_cells * kProfileCoefs * 8 * (vibration ? kVibTables : 1);
     if (bytes > p->cells.cap) {
         size_t free_b = 0, total_b = 0;
         if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || bytes > free_b / 2) return 0;
@@ -1271,11 +1332,11 @@ int profile_group(tdc_processor *p, int path, ProfileBuild &b)
     // |t| <= 1/2 (the anchor's place in its cell) + the group's reach
     for (int k = 0; k < 3; ++k)
     {
-        const double reach = p->group_reach[k], turn = motion ? 2.0 * reach / rmin : 0.0;
+        const double reach = p->group_reach[k], turn = motion ? reach / rmin : 0.0;
         // moving antennas: the group's spread of directions (turn) changes its pixels' shifts, their
         // bends (kept to first order) and the part of the bend from V2 (taken as the anchor's)
         if (motion && !(turn * max_bend <= kMoveMaxTurn &&
-                        2.0 * M_PI * h * h * std::fabs(gc) * p->motion_v2max * turn <= 2e-6))
+                        2.0 * M_PI * h * h * std::fabs(gc) * v2 * turn <= 1e-6 && turn * amp <= kVibMaxTurn))
             continue;
         if (std::fabs(b.cells_per_m) * reach + slack * turn <= kProfileReach - 0.52) return 8 >> k;
     }
@@ -1334,7 +1395,9 @@ int focus_plan(tdc_processor *p, FocusPlan &plan, double max_unit_work)
     int slots;
     bool anchored = false;
     ProfileBuild build{};
-    const int profile = path == TDC_PATH_FP32_BULK || path == TDC_PATH_FP32_MOTION ? profile_group(p, path, build) : 0;
+    const int profile = path == TDC_PATH_FP32_BULK || path == TDC_PATH_FP32_MOTION || path == TDC_PATH_GENERAL
+                            ? profile_group(p, path, build)
+                            : 0;
     if (profile) {
         slots = p->n_sm * kProfileCtasPerSm;
     } else if (path == TDC_PATH_FP32_MOTION) {
@@ -1420,7 +1483,8 @@ int focus_plan(tdc_processor *p, FocusPlan &plan, double max_unit_work)
         p->plan_uploaded = false;
     }
     if (profile) {
-        TDC_CK(p->cells.ensure((size_t)p->C * build.n_cells * kProfileCoefs * 8), "alloc range profiles");
+        TDC_CK(p->cells.ensure((size_t)p->C * build.n_cells * kProfileCoefs * 8 * (build.traj ? kVibTables : 1)),
+               "alloc range profiles");
         TDC_CK(p->cell_base.ensure(sizeof(ProfileJob) + (size_t)p->C * 4), "alloc range profile bases");
         const size_t tw_bytes = (size_t)p->S * (kProfileNodes * 8 + 4);
         if (tw_bytes > p->twiddle.cap) p->twiddle_S = 0;
@@ -1454,6 +1518,7 @@ int focus_plan(tdc_processor *p, FocusPlan &plan, double max_unit_work)
     if (profile) {
         build.rows = p->xw.as<const float2>();
         if (path == TDC_PATH_FP32_MOTION) plan.job.chirps = reinterpret_cast<const ChirpRec *>(p->move_rec.p);
+        if (build.traj) plan.job.chirps = reinterpret_cast<const ChirpRec *>(p->vib_rec.p);
         build.chirps = reinterpret_cast<const float4 *>(plan.job.chirps);
         build.twiddle = p->twiddle.as<const float2>();
         build.factor = reinterpret_cast<const float *>(build.twiddle + (size_t)p->S * kProfileNodes);
@@ -1513,6 +1578,7 @@ void processor_release_memory(tdc_processor *p)
     p->grid_lo_valid = false;
     p->twiddle_S = 0;
     p->table_epoch = 0;
+    p->vib_known = false;
 }
 
 size_t processor_device_bytes(tdc_processor *p)
@@ -1566,7 +1632,7 @@ int focus_resident(tdc_processor *p, float2 *image_dev, cudaStream_t st, int &la
         if (int rc = profile_build(p, plan, st, launches)) return rc;
         p->table_epoch = p->state_epoch;
         const bool band = std::isfinite(job.half_bw);
-        const bool motion = path == TDC_PATH_FP32_MOTION;
+        const int motion = plan.build.traj ? 2 : path == TDC_PATH_FP32_MOTION ? 1 : 0;
         const int grid = std::min(n_units, p->n_sm * focus_profile_blocks_per_sm(plan.profile, band, false, motion));
         TDC_CK(launch_focus_profile(plan.profile, band, motion, jobs_dev, units_dev, n_units, counter, grid, st),
                "focus kernel (range profiles)");
@@ -1605,7 +1671,7 @@ int focus_resident(tdc_processor *p, float2 *image_dev, cudaStream_t st, int &la
     const int row = path == TDC_PATH_GENERAL ? job.seg_len : plan.seg ? kSegmentSamples : p->s_pad;
     p->stats.stage_samples = staged ? std::min(row, p->s_pad) : 0;
     p->stats.stage_chirps = staged ? (row < p->s_pad ? 1 : plan.cb) : 0;
-    p->stats.general_variant = path == TDC_PATH_GENERAL ? plan.variant : 0;
+    p->stats.general_variant = path == TDC_PATH_GENERAL && !plan.profile ? plan.variant : 0;
     p->stats.tile_cols = job.tile_cols;
     p->stats.motion_segment = path == TDC_PATH_FP32_MOTION && !plan.profile ? job.seg_len : 0;
     p->stats.span_permille = path == TDC_PATH_FP32_BULK && !plan.seg && !store ? p->span_permille : 1000;

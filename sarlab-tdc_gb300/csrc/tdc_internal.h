@@ -94,6 +94,18 @@ struct __align__(16) MoveRec {
 };
 static_assert(sizeof(MoveRec) == 64, "MoveRec must be 64 bytes");
 
+// One chirp's record for vibration about a constant velocity, 96 bytes: the smooth part as above (V2
+// zero), and
+//   f0.xyz  P(sc) - P[c, 0], so that the deviation of sample s is D_s - f0 - W1 (s - sc)
+//   n.xyz   its principal direction (unit); n.w = its largest carrier phase squared [rad^2]
+struct __align__(16) VibRec {
+    MoveRec m;
+    float4 f0;
+    float4 n;
+};
+static_assert(sizeof(VibRec) == 96, "VibRec must be 96 bytes");
+constexpr int kVibTables = 6;  // range-profile tables of a vibrating acquisition (tdc_profile.cu)
+
 // One sample point of the reference's chunk skip test (tdcprocessor.cpp:355-378).
 struct __align__(16) SkipPoint {
     float4 pos_fdc;  // position xyz, window centre
@@ -224,6 +236,8 @@ struct ProfileBuild {
     int C, S, s_pad, n_cells;
     int chirp_words;
     int margin;              // cells the table starts early (even; smooth motion)
+    const float4 *traj;      // vibration: [C][s_pad] D_s = P[c, s] - P[c, 0] (else null)
+    float phase_g, phase_g1; // 2 pi gc and 2 pi g1 [rad / m]
 };
 
 // Tiles of a P-pixel grid whose runs are `run` pixels long: groups of kProfilePixels
@@ -317,15 +331,21 @@ cudaError_t launch_profile_build(const ProfileBuild &b, cudaStream_t st);
 // The same with its inputs in device memory, of at most max_cells cells; nothing where *enabled is 0.
 cudaError_t launch_profile_build_indirect(const ProfileBuild *dev, const int *enabled, int C, int max_cells,
                                           cudaStream_t st);
-// motion: the records are MoveRec, every sample of a chirp at a range of its own.
-cudaError_t launch_focus_profile(int group, bool band, bool motion, const FocusJob *jobs_dev, const FocusUnit *units_dev, int n_units,
+// motion: 1, the records are MoveRec, every sample of a chirp at a range of its own; 2, they are
+// VibRec and there are kVibTables tables.
+cudaError_t launch_focus_profile(int group, bool band, int motion, const FocusJob *jobs_dev, const FocusUnit *units_dev, int n_units,
                                  int *counter_dev, int grid_ctas, cudaStream_t st);
 // Its adjoint: gpart[tile][C] = (d/dx, d/dy, d/dz) of each chirp over the tile's pixels (sums of
 // Re(conj(G) dI/dR) (P - T) / R; .w is not written).
 cudaError_t launch_adjoint_profile(int group, bool band, const FocusJob *jobs_dev, const FocusUnit *units_dev,
                                    int n_units, int *counter_dev, int grid_ctas, const float2 *gimg, float4 *gpart,
                                    cudaStream_t st);
-int focus_profile_blocks_per_sm(int group, bool band, bool adjoint, bool motion);
+int focus_profile_blocks_per_sm(int group, bool band, bool adjoint, int motion);
+// Straight-line fit of every chirp's offsets traj ([C][s_pad], chirps with sample-0 positions) and the
+// principal direction of what it leaves, as VibRec; maxima[0..2] = max(maxima, largest deviation,
+// deviation off that direction, |W1|) as float bits (starting at 0; NaN above all).
+cudaError_t launch_vib_fit(const float4 *traj, const ChirpRec *chirps, int C, int S, int s_pad, float phase_per_m,
+                           VibRec *recs, int *maxima, cudaStream_t st);
 // out[0..2] = max(out, largest distance of a pixel from the anchor of its group of 8 / 4 / 2
 // consecutive pixels of a run) as float bits (out starts at 0; a NaN compares above any distance).
 cudaError_t launch_group_reach(const float4 *hi, long long P, int run, int *out, cudaStream_t st);

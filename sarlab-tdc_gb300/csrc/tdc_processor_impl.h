@@ -171,6 +171,11 @@ struct tdc_processor {
     tdc::impl::DevBuf gen_rec, traj, wins, wdot, gres;
     // Smooth-motion kernel: one MotionRec per chirp.
     tdc::impl::DevBuf motion_rec, move_rec;
+    // Vibration about a smooth motion (range profiles): VibRec per chirp and maxima over the chirps
+    // (deviation, deviation off its principal direction, |W1|), measured when a plan asks.
+    tdc::impl::DevBuf vib_rec;
+    bool vib_known = false;
+    double vib_max[3] = {0, 0, 0};
     // Autofocus: the forward's per-(chirp, pixel) sums and the rows pre-scaled by the sample
     // index, so the adjoint computes only the index-weighted sums (keep_sums on).
     tdc::impl::DevBuf chirp_sums, xs_scaled;
@@ -243,7 +248,7 @@ struct tdc_processor {
     {
         return {&xw,      &chirps,     &skip,    &gs,      &pos_base, &wr,      &offsets,     &flag,     &gen_rec,
                 &traj,    &wins,       &wdot,    &gres,    &grid_stage, &grid_hi, &grid_lo, &scratch, &adj_scratch,
-                &chirp_sums, &xs_scaled, &motion_rec, &move_rec, &cells, &cell_base, &twiddle, &tile_radius,
+                &chirp_sums, &xs_scaled, &motion_rec, &move_rec, &vib_rec, &cells, &cell_base, &twiddle, &tile_radius,
                 &image_dev};
     }
 };
@@ -290,6 +295,7 @@ int general_variant(const tdc_processor *p);
 // Segment length (samples, a power of two) of the smooth-motion kernel for the resident
 // acquisition and grid, or 0 when that kernel does not take them.
 int motion_segment(const tdc_processor *p);
+int measure_vibration(tdc_processor *p);
 int motion_stage_bytes_for(int s_pad, int &cb);
 FocusJob make_job(const tdc_processor *p, float4 *partial, int cb, int path);
 // Plan units (p->units_host) and make sure the processor's scratch holds them and the partials.

@@ -158,7 +158,7 @@ __global__ void __launch_bounds__(kBuildThreads)
     const int c0 = blockIdx.x * kBuildChirps;
     const unsigned int nn = 2u * (unsigned)b.S;
 
-    if (blockIdx.x == 0 && blockIdx.y == 0 && tid == 0) *b.job_out = b.job;
+    if (blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && tid == 0) *b.job_out = b.job;
     if (tid < kBuildChirps) {
         // first cell: the smallest cell coordinate of any point in the grid's bounding box
         const int c = min(c0 + tid, b.C - 1);
@@ -174,7 +174,7 @@ __global__ void __launch_bounds__(kBuildThreads)
         const double u = fmin(b.cells_per_m * sqrt(near2), b.cells_per_m * sqrt(far2));
         // (positions far outside what the table can index: any base will do, reads are clamped)
         const int base = fabs(u) < 1e9 ? 2 * (int)floor(0.5 * u) - 2 - b.margin : 0;
-        if (blockIdx.y == 0 && c0 + tid < b.C) b.cell_base[c0 + tid] = base;
+        if (blockIdx.y == 0 && blockIdx.z == 0 && c0 + tid < b.C) b.cell_base[c0 + tid] = base;
         const int node = base >> 1;
         const int block = (node >= 0 ? node / kOwn : -((kOwn - 1 - node) / kOwn)) + (int)blockIdx.y;
         s_cell[tid] = 2 * (block * kOwn - node);
@@ -228,6 +228,22 @@ __global__ void __launch_bounds__(kBuildThreads)
         }
     }
     const float fnn = (float)nn, inv_nn = 1.0f / fnn;
+    // Vibration: table blockIdx.z is of the samples times 1, phi_x, phi_y, phi_z, chi^2, chi^3 (phi the
+    // deviation from the smooth motion in radians of carrier phase, chi its principal component).
+    const int family = blockIdx.z;
+    auto family_weight = [&](int q, int s) {
+        const int c = c0 + q;
+        if (s >= b.S || c >= b.C) return 0.f;
+        const float4 *rec = b.chirps + (size_t)c * b.chirp_words;
+        const float4 w1 = rec[2], f0 = rec[4], n = rec[5];
+        const float4 d = b.traj[(size_t)c * b.s_pad + s];
+        const float t = (float)(s - b.S / 2);
+        const float g = fmaf(b.phase_g1, t, b.phase_g);
+        const float x = g * fmaf(-w1.x, t, d.x - f0.x), y = g * fmaf(-w1.y, t, d.y - f0.y),
+                    z = g * fmaf(-w1.z, t, d.z - f0.z);
+        const float chi = fmaf(n.x, x, fmaf(n.y, y, n.z * z));
+        return family == 1 ? x : family == 2 ? y : family == 3 ? z : family == 4 ? chi * chi : chi * chi * chi;
+    };
     load_ahead(0);
 
     for (int s0 = 0, tile = 0; s0 < b.S; s0 += kBuildStep, ++tile) {
@@ -243,7 +259,11 @@ __global__ void __launch_bounds__(kBuildThreads)
             ratio = fmaf(fmaf(-ratio, fnn, fr), inv_nn, ratio);
             float sn, cs;
             sincospif(2.0f * ratio, &sn, &cs);
-            const float2 x = ahead_x[i];
+            float2 x = ahead_x[i];
+            if (family) {
+                const float w = family_weight((warp >> 1) + 4 * i, s0 + si_mine);
+                x = make_float2(w * x.x, w * x.y);
+            }
             sx[si_mine][(warp >> 1) + 4 * i] =
                 make_float2(ahead_f * fmaf(x.x, cs, -x.y * sn), ahead_f * fmaf(x.x, sn, x.y * cs));
         }
@@ -303,7 +323,8 @@ __global__ void __launch_bounds__(kBuildThreads)
         float2 v[kTaps];
 #pragma unroll
         for (int k = 0; k < kTaps; ++k) v[k] = sv[q * kNodes + j + k];
-        float4 *__restrict__ out = b.cells + ((size_t)c * b.n_cells + l) * (kProfileCoefs / 2);
+        float4 *__restrict__ out =
+            b.cells + (((size_t)family * b.C + c) * b.n_cells + l) * (kProfileCoefs / 2);
 #pragma unroll
         for (int par = 0; par < 2; ++par)
 #pragma unroll
@@ -319,6 +340,107 @@ __global__ void __launch_bounds__(kBuildThreads)
                 out[par * (kProfileCoefs / 2) + m / 2] = make_float4(a0.x, a0.y, a1.x, a1.y);
             }
     }
+}
+
+// One warp a chirp: least squares of D_s by a line in s (FP64), re-centred on the middle sample; then
+// the covariance of the deviations, its principal direction by power iteration, and the largest
+// deviation off it. (A quadratic would take part of the vibration's bow into the smooth
+// motion, whose bend a group of pixels then shares.)
+__global__ void __launch_bounds__(128)
+    vib_fit_kernel(const float4 *__restrict__ traj, const ChirpRec *__restrict__ chirps, int C, int S, int s_pad,
+                   float phase_per_m, VibRec *__restrict__ recs, int *__restrict__ maxima)
+{
+    const int c = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (c >= C) return;
+    const float4 *row = traj + (size_t)c * s_pad;
+    const double hs = 0.5 * (S - 1);
+    double a[6] = {0, 0, 0, 0, 0, 0}, sxx = 0.0;
+    for (int s = lane; s < S; s += 32) {
+        const float4 d = row[s];
+        const double x = s - hs, v[3] = {d.x, d.y, d.z};
+        sxx += x * x;
+        for (int k = 0; k < 3; ++k) {
+            a[k] += v[k];
+            a[3 + k] += v[k] * x;
+        }
+    }
+    for (int off = 16; off > 0; off >>= 1) {
+        sxx += __shfl_xor_sync(0xffffffffu, sxx, off);
+        for (int k = 0; k < 6; ++k) a[k] += __shfl_xor_sync(0xffffffffu, a[k], off);
+    }
+    const double xc = (double)(S / 2) - hs;
+    double f0[3], w1[3], n1 = 0.0;
+    for (int k = 0; k < 3; ++k) {
+        w1[k] = sxx > 0.0 ? a[3 + k] / sxx : 0.0;
+        f0[k] = a[k] / S + w1[k] * xc;
+        n1 += w1[k] * w1[k];
+    }
+    const float ff[3] = {(float)f0[0], (float)f0[1], (float)f0[2]}, fw[3] = {(float)w1[0], (float)w1[1], (float)w1[2]};
+    auto deviation = [&](int s, float &x, float &y, float &z) {
+        const float4 d = row[s];
+        const float t = (float)(s - S / 2);
+        x = fmaf(-fw[0], t, d.x - ff[0]);
+        y = fmaf(-fw[1], t, d.y - ff[1]);
+        z = fmaf(-fw[2], t, d.z - ff[2]);
+    };
+    float cov[6] = {0, 0, 0, 0, 0, 0}, most = 0.f;
+    for (int s = lane; s < S; s += 32) {
+        float x, y, z;
+        deviation(s, x, y, z);
+        cov[0] += x * x;
+        cov[1] += y * y;
+        cov[2] += z * z;
+        cov[3] += x * y;
+        cov[4] += x * z;
+        cov[5] += y * z;
+        const float m = sqrtf(x * x + y * y + z * z);
+        most = m > most || m != m ? m : most;
+    }
+    for (int off = 16; off > 0; off >>= 1)
+        for (int k = 0; k < 6; ++k) cov[k] += __shfl_xor_sync(0xffffffffu, cov[k], off);
+    // power iteration from the axis of largest variance (scaled to its trace)
+    float n[3] = {0.f, 0.f, 0.f};
+    const int axis = cov[0] >= cov[1] && cov[0] >= cov[2] ? 0 : cov[1] >= cov[2] ? 1 : 2;
+    n[axis] = 1.f;
+    const float tr = cov[0] + cov[1] + cov[2];
+    if (tr > 0.f)
+        for (int it = 0; it < 24; ++it) {
+            const float x = (cov[0] * n[0] + cov[3] * n[1] + cov[4] * n[2]) / tr,
+                        y = (cov[3] * n[0] + cov[1] * n[1] + cov[5] * n[2]) / tr,
+                        z = (cov[4] * n[0] + cov[5] * n[1] + cov[2] * n[2]) / tr;
+            const float r = rsqrtf(x * x + y * y + z * z);
+            n[0] = x * r;
+            n[1] = y * r;
+            n[2] = z * r;
+        }
+    float side = 0.f;
+    for (int s = lane; s < S; s += 32) {
+        float x, y, z;
+        deviation(s, x, y, z);
+        const float r = n[0] * x + n[1] * y + n[2] * z;
+        const float px = x - r * n[0], py = y - r * n[1], pz = z - r * n[2];
+        const float m = sqrtf(px * px + py * py + pz * pz);
+        side = m > side || m != m ? m : side;
+    }
+    const int im = __reduce_max_sync(0xffffffffu, __float_as_int(fabsf(most)));
+    const int is = __reduce_max_sync(0xffffffffu, __float_as_int(fabsf(side)));
+    if (lane) return;
+    VibRec r;
+    const ChirpRec base = chirps[c];
+    // (what is kept of f0 and W1 in FP32 is what the deviations were taken from)
+    const double p[3] = {(double)base.p_hi.x + base.p_lo.x + ff[0], (double)base.p_hi.y + base.p_lo.y + ff[1],
+                         (double)base.p_hi.z + base.p_lo.z + ff[2]};
+    r.m.p_hi = make_float4((float)p[0], (float)p[1], (float)p[2], 0.f);
+    r.m.p_lo = make_float4((float)(p[0] - r.m.p_hi.x), (float)(p[1] - r.m.p_hi.y), (float)(p[2] - r.m.p_hi.z), 0.f);
+    r.m.w1 = make_float4(fw[0], fw[1], fw[2], (float)n1);
+    r.m.v2 = make_float4(0.f, 0.f, 0.f, 0.f);
+    r.f0 = make_float4(ff[0], ff[1], ff[2], 0.f);
+    const float amp = phase_per_m * __int_as_float(im);
+    r.n = make_float4(n[0], n[1], n[2], amp * amp);
+    recs[c] = r;
+    atomicMax(&maxima[0], im);
+    atomicMax(&maxima[1], is);
+    atomicMax(&maxima[2], __float_as_int((float)sqrt(n1)) & 0x7fffffff);
 }
 
 // ---- focus ------------------------------------------------------------------
@@ -424,6 +546,7 @@ __device__ __forceinline__ float2 fresh2(const float2 *p)
 // and the anchor's cell and place in it.
 struct Anchor {
     float ex, ey, ez, rh, h, turn, t0;
+    const float4 *cell;  // its first table's cell (MOVE == 2)
     float w;  // Doppler window (BAND with every pixel its own anchor); cell shift of its motion (MOVE)
     float2 a[kProfileCoefs];
 };
@@ -499,10 +622,112 @@ __device__ __forceinline__ float move_coefs(const Anchor &n, float4 w1, float4 v
     return eps;
 }
 
+__device__ __forceinline__ float2 neg(float2 v) { return make_float2(-v.x, -v.y); }
+// a + j s b
+__device__ __forceinline__ float2 plus_j(float2 a, float s, float2 b)
+{
+    return make_float2(fmaf(-s, b.y, a.x), fmaf(s, b.x, a.y));
+}
+
+// Vibration: a (the first table's cell) := the combined cell polynomial for the anchor's direction;
+// turn_k := its gradient in the direction, coefficients of degree < kVibCoefs (it is multiplied
+// by changes of direction of a few per cent; the terms left out are below 1e-3 of it).
+constexpr int kVibCoefs = 6;
+template <bool TURN>
+__device__ __forceinline__ void vib_coefs(const Anchor &n, float4 w1, float4 axis, size_t table, int samples,
+                                          const ProfileJob &job, float2 (&a)[kProfileCoefs],
+                                          float2 (&tx)[kVibCoefs], float2 (&ty)[kVibCoefs], float2 (&tz)[kVibCoefs])
+{
+    const float ri = n.rh > 0.0f ? 2.0f * n.h * job.inv_gc : 0.0f;
+    const float u[3] = {n.ex * ri, n.ey * ri, n.ez * ri};
+    const float rate = fmaf(u[0], w1.x, fmaf(u[1], w1.y, u[2] * w1.z));
+    const float un = fmaf(u[0], axis.x, fmaf(u[1], axis.y, u[2] * axis.z));
+    // direction's turn along the chirp, times s~ = -j (2 S / pi) d/dt of j phi_k: (2 S / pi) w_k a_k'
+    const float scale = (float)samples * (2.0f / kPiF) * ri;
+    const float w[3] = {scale * fmaf(-rate, u[0], w1.x), scale * fmaf(-rate, u[1], w1.y),
+                        scale * fmaf(-rate, u[2], w1.z)};
+    // cosine to fourth order, economised over |(u.n) chi| <= A: 1 - x^2 / 2 + x^4 / 24 = 1 - A^4 / 192
+    // - x^2 (1 / 2 - A^2 / 24) within A^4 / 192; and the range's second order, chi^2 (1 - (u.n)^2) / (2 2 pi gc R)
+    const float u2 = un * un, ua = u2 * axis.w;
+    const float c4 = u2 * fmaf(ua, 1.0f / 24.0f, -0.5f), d4 = un * fmaf(ua, 1.0f / 6.0f, -1.0f);
+    const float c5 = -u2 * un * (1.0f / 6.0f), d5 = -0.5f * u2;
+    const float bow = (1.0f - u2) * n.h * (job.inv_gc * job.inv_gc) * (0.5f / kPiF);
+    const float one = fmaf(ua * ua, -1.0f / 192.0f, 1.0f);
+#pragma unroll
+    for (int m = 0; m < kProfileCoefs; ++m) a[m] = __fmul2_rn(a[m], both(one));
+    const float4 *p = n.cell;
+    if (!TURN) {  // (one table at a time: all five at once do not fit the registers)
+#pragma unroll 1
+        for (int f = 1; f < kVibTables; ++f) {
+            p += table;
+            const float im = f == 1 ? u[0] : f == 2 ? u[1] : f == 3 ? u[2] : f == 4 ? bow : c5;
+            const float re = f == 4 ? c4 : 0.f;
+            const float wf = f == 1 ? w[0] : f == 2 ? w[1] : f == 3 ? w[2] : 0.f;
+#pragma unroll
+            for (int m = 0; m < kProfileCoefs / 2; ++m) {
+                const float4 q = __ldg(p + m);
+                const float2 v0 = make_float2(q.x, q.y), v1 = make_float2(q.z, q.w);
+                if (m) a[2 * m - 1] = __ffma2_rn(v0, both(wf * (float)(2 * m)), a[2 * m - 1]);
+                a[2 * m] = __ffma2_rn(v1, both(wf * (float)(2 * m + 1)), __ffma2_rn(v0, both(re), plus_j(a[2 * m], im, v0)));
+                a[2 * m + 1] = __ffma2_rn(v1, both(re), plus_j(a[2 * m + 1], im, v1));
+            }
+        }
+        return;
+    }
+#pragma unroll
+    for (int f = 1; f < kVibTables; ++f) {
+        p += table;
+        float2 v[kProfileCoefs];
+#pragma unroll
+        for (int m = 0; m < kProfileCoefs / 2; ++m) {
+            const float4 q = __ldg(p + m);
+            v[2 * m] = make_float2(q.x, q.y);
+            v[2 * m + 1] = make_float2(q.z, q.w);
+        }
+        if (f < 4) {
+            float2(&t)[kVibCoefs] = f == 1 ? tx : f == 2 ? ty : tz;
+#pragma unroll
+            for (int m = 0; m < kProfileCoefs; ++m) {
+                a[m] = plus_j(a[m], u[f - 1], v[m]);
+                if (m + 1 < kProfileCoefs) a[m] = __ffma2_rn(v[m + 1], both(w[f - 1] * (float)(m + 1)), a[m]);
+                if (m < kVibCoefs) t[m] = make_float2(-v[m].y, v[m].x);
+            }
+        } else {
+            // - (u.n)^2 / 2 v4, - j (u.n)^3 / 6 v5, and their gradients along n
+            const float c = f == 4 ? c4 : c5, d = f == 4 ? d4 : d5;
+#pragma unroll
+            for (int m = 0; m < kProfileCoefs; ++m) {
+                const float2 x = f == 4 ? v[m] : make_float2(-v[m].y, v[m].x);
+                a[m] = __ffma2_rn(x, both(c), a[m]);
+                if (f == 4) a[m] = plus_j(a[m], bow, v[m]);
+                if (m < kVibCoefs) {
+                    tx[m] = __ffma2_rn(x, both(d * axis.x), tx[m]);
+                    ty[m] = __ffma2_rn(x, both(d * axis.y), ty[m]);
+                    tz[m] = __ffma2_rn(x, both(d * axis.z), tz[m]);
+                }
+            }
+        }
+    }
+}
+
+// The gradient's change for a change (x, y, z) of direction, at place t of the cell.
+__device__ __forceinline__ float2 turn_value(const float2 (&tx)[kVibCoefs], const float2 (&ty)[kVibCoefs],
+                                             const float2 (&tz)[kVibCoefs], float x, float y, float z, float t)
+{
+    float2 h = both(0.f);
+#pragma unroll
+    for (int m = kVibCoefs - 1; m >= 0; --m) {
+        const float2 c = __ffma2_rn(tx[m], both(x), __ffma2_rn(ty[m], both(y), __fmul2_rn(tz[m], both(z))));
+        h = m == kVibCoefs - 1 ? c : __ffma2_rn(h, both(t), c);
+    }
+    return h;
+}
+
 // add_pair with the pixels' places t in the cell and bends eps beside the anchor's.
 __device__ __forceinline__ void add_moving_pair(float2 psi, float turn, float2 t, float2 eps,
                                                 const float2 (&a)[kProfileCoefs],
-                                                const float2 (&bend)[kProfileCoefs - 2], float2 &c0, float2 &s0,
+                                                const float2 (&bend)[kProfileCoefs - 2], float2 more0, float2 more1,
+                                                float2 &c0, float2 &s0,
                                                 float2 &c1, float2 &s1)
 {
     const float2 n = __fadd2_rn(__fadd2_rn(psi, both(12582912.0f)), both(-12582912.0f));  // nearest integer
@@ -522,6 +747,8 @@ __device__ __forceinline__ void add_moving_pair(float2 psi, float turn, float2 t
         b0 = __ffma2_rn(b0, ta, bend[m]);
         b1 = __ffma2_rn(b1, tb, bend[m]);
     }
+    h0 = __fadd2_rn(h0, more0);
+    h1 = __fadd2_rn(h1, more1);
     h0 = make_float2(fmaf(-eps.x, b0.y, h0.x), fmaf(eps.x, b0.x, h0.y));  // + j eps b
     h1 = make_float2(fmaf(-eps.y, b1.y, h1.x), fmaf(eps.y, b1.x, h1.y));
     c0 = __ffma2_rn(h0, both(cs0), c0);
@@ -612,16 +839,27 @@ __device__ __forceinline__ void adjoint_pair(float2 psi, float turn, float t0, f
 // - j eps^3 / 6 E, all polynomials of the cell formed once an anchor; the pixel's difference in
 // eps from its anchor, at most a few per cent of it, enters to first order. 64 x 512 pixels x 512
 // chirps x 1024 samples: 2.64 ms in the per-segment kernel of tdc_motion.cu, 0.21 ms here.
-template <int G, bool BAND, bool ADJ, bool MOVE>
-__global__ void __launch_bounds__(kThreads, G == 1 ? (BAND || ADJ ? 4 : 6) : BAND || MOVE || (ADJ && G == 2) ? 6 : TDC_PROFILE_MINB)
+//
+// MOVE = 2: vibration about a constant velocity, rho_s = P[c, s] minus the chirp's line. Its phase is
+// psi_s = u.phi_s (u = e / R the direction of the antenna, phi = 2 pi g_s rho, at most 0.1 rad), so
+//   e^{j psi} = 1 + j u.phi - (u.n)^2 chi^2 / 2 - j (u.n)^3 chi^3 / 6,
+// six tables of the same samples times 1, phi_x, phi_y, phi_z, chi^2 and chi^3 (chi = n.phi, n the
+// principal direction of the chirp's deviations: what lies off it, the rounding of the FP32
+// positions, is kept to first order). An anchor combines them for its own u into one cell
+// polynomial; the direction turning along the chirp (W1 / R) enters through the derivative of
+// the phi tables, a pixel's own direction as the polynomial's gradient in u, to first order.
+// 151 x 97 pixels x 333 chirps x 500 samples: 1930 us in the general kernel of tdc_general.cu, which
+// corrects every sample, 120 us here (57 the six tables, 57 this kernel).
+template <int G, bool BAND, bool ADJ, int MOVE>
+__global__ void __launch_bounds__(kThreads, MOVE == 2 ? 4 : G == 1 ? (BAND || ADJ ? 4 : 6) : BAND || MOVE || (ADJ && G == 2) ? 6 : TDC_PROFILE_MINB)
     profile_focus_kernel(const FocusJob *__restrict__ jobs, const FocusUnit *__restrict__ units, int n_units,
                          int *__restrict__ counter, const float2 *__restrict__ gimg, float4 *__restrict__ gpart)
 {
     constexpr int kSub = kPT / G;  // anchors per thread
     __shared__ SharedSums sums;
     static_assert(!MOVE || (!BAND && !ADJ), "smooth motion: unbounded band, forward only");
-    constexpr int kWords = MOVE ? 4 : BAND ? 3 : 2;  // float4 staged per record
-    constexpr int kStride = MOVE ? 4 : 3;            // float4 per record in memory
+    constexpr int kWords = MOVE == 2 ? 6 : MOVE ? 4 : BAND ? 3 : 2;  // float4 staged per record
+    constexpr int kStride = MOVE ? kWords : 3;                      // float4 per record in memory
     __shared__ __align__(16) SharedChirps<kWords> recs[2];
     __shared__ float red[ADJ ? kFlush : 1][3][kThreads / 4];  // (ADJ) 8 partial sums a warp
     __shared__ int s_unit;
@@ -732,7 +970,7 @@ __global__ void __launch_bounds__(kThreads, G == 1 ? (BAND || ADJ ? 4 : 6) : BAN
             // its cell, and its place in it
             float shift = 0.f;
             if (MOVE) {
-                const float4 w1 = recs[buf].p[k][kWords - 2];
+                const float4 w1 = recs[buf].p[k][MOVE ? 2 : 0];
                 shift = sP.rate_cells * (fmaf(n.ex, w1.x, fmaf(n.ey, w1.y, n.ez * w1.z)) * rinv);
                 if (!(n.rh > 0.0f)) shift = 0.f;
             }
@@ -743,6 +981,7 @@ __global__ void __launch_bounds__(kThreads, G == 1 ? (BAND || ADJ ? 4 : 6) : BAN
             if (MOVE) n.t0 += shift;
             const int cell = min(max((int)kf - base, 0), n_cells - 1);
             const float4 *__restrict__ pc = cells + ((size_t)(b0 + k) * n_cells + cell) * (kProfileCoefs / 2);
+            if (MOVE == 2) n.cell = pc;
 #pragma unroll
             for (int m = 0; m < kProfileCoefs / 2; ++m) {
                 const float4 v = __ldg(pc + m);
@@ -864,7 +1103,13 @@ __global__ void __launch_bounds__(kThreads, G == 1 ? (BAND || ADJ ? 4 : 6) : BAN
                         for (int m = 0; m < kProfileCoefs; ++m) a[m] = cur.a[m];
                         if constexpr (MOVE) {
                             float2 bend[kProfileCoefs - 2];
-                            move_coefs(cur, recs[buf].p[k][kWords - 2], recs[buf].p[k][kWords - 1], sP, a, bend);
+                            if constexpr (MOVE == 2) {
+                                float2 turn_x[kVibCoefs], turn_y[kVibCoefs], turn_z[kVibCoefs];
+                                vib_coefs<false>(cur, recs[buf].p[k][2], recs[buf].p[k][kWords - 1],
+                                          (size_t)sJ.C * sP.n_cells * (kProfileCoefs / 2), sJ.S, sP, a, turn_x, turn_y,
+                                          turn_z);
+                            }
+                            move_coefs(cur, recs[buf].p[k][2], recs[buf].p[k][3 % kWords], sP, a, bend);
                         }
                         float2 h = a[kProfileCoefs - 1];
 #pragma unroll
@@ -996,10 +1241,17 @@ __global__ void __launch_bounds__(kThreads, G == 1 ? (BAND || ADJ ? 4 : 6) : BAN
                             continue;
                         }
                         if constexpr (MOVE) {
-                            const float4 w1 = recs[buf].p[k][kWords - 2], v2 = recs[buf].p[k][kWords - 1];
+                            const float4 w1 = recs[buf].p[k][2], v2 = recs[buf].p[k][3 % kWords];
                             float2 a[kProfileCoefs], bend[kProfileCoefs - 2];
 #pragma unroll
                             for (int m = 0; m < kProfileCoefs; ++m) a[m] = cur.a[m];
+                            constexpr int kTurn = MOVE == 2 ? kVibCoefs : 1;
+                            float2 turn_x[kTurn], turn_y[kTurn], turn_z[kTurn];
+                            if constexpr (MOVE == 2)
+                                vib_coefs<true>(cur, w1, recs[buf].p[k][kWords - 1],
+                                          (size_t)sJ.C * sP.n_cells * (kProfileCoefs / 2), sJ.S, sP, a, turn_x, turn_y,
+                                          turn_z);
+                            const float ri0 = 2.0f * cur.h * sP.inv_gc;
                             const float eps0 = move_coefs(cur, w1, v2, sP, a, bend);
                             const float ew = fmaf(cur.ex, w1.x, fmaf(cur.ey, w1.y, cur.ez * w1.z));
                             const float bend_v = 2.0f * sP.bend2 * fmaf(cur.ex, v2.x, fmaf(cur.ey, v2.y, cur.ez * v2.z));
@@ -1025,8 +1277,18 @@ __global__ void __launch_bounds__(kThreads, G == 1 ? (BAND || ADJ ? 4 : 6) : BAN
                                                both(bend_v)),
                                     ri);
                                 const float2 eps = __ffma2_rn(both(sP.bend1), rate, bow);
-                                add_moving_pair(psi[i / 2], cur.turn, t, __fadd2_rn(eps, both(-eps0)), a, bend, hc[s],
-                                                hs[s], hc[s + 1], hs[s + 1]);
+                                float2 h0 = both(0.f), h1 = h0;
+                                if constexpr (MOVE == 2) {
+                                    // the pixels' directions less the anchor's
+                                    const float2 ux = __ffma2_rn(__fadd2_rn(both(cur.ex), neg(dx[q])), ri, both(-cur.ex * ri0)),
+                                                 uy = __ffma2_rn(__fadd2_rn(both(cur.ey), neg(dy[q])), ri, both(-cur.ey * ri0)),
+                                                 uz = __ffma2_rn(__fadd2_rn(both(cur.ez), neg(fresh2(&sums.dz[q][tid]))), ri,
+                                                                 both(-cur.ez * ri0));
+                                    h0 = turn_value(turn_x, turn_y, turn_z, ux.x, uy.x, uz.x, t.x);
+                                    h1 = turn_value(turn_x, turn_y, turn_z, ux.y, uy.y, uz.y, t.y);
+                                }
+                                add_moving_pair(psi[i / 2], cur.turn, t, __fadd2_rn(eps, both(-eps0)), a, bend, h0, h1,
+                                                hc[s], hs[s], hc[s + 1], hs[s + 1]);
                             }
                             if (zero) {
 #pragma unroll
@@ -1103,7 +1365,7 @@ cudaError_t launch_profile_build(const ProfileBuild &b, cudaStream_t st)
     static const ProfileStencil stencil = make_stencil();
     // nodes of n_cells / 2 from an even cell on, wherever the first block starts
     const int blocks = (b.n_cells / 2 + kOwn - 2) / kOwn + 1;
-    const dim3 grid((b.C + kBuildChirps - 1) / kBuildChirps, blocks);
+    const dim3 grid((b.C + kBuildChirps - 1) / kBuildChirps, blocks, b.traj ? kVibTables : 1);
     profile_build_kernel<false><<<grid, kBuildThreads, 0, st>>>(b, stencil, nullptr, nullptr);
     return cudaGetLastError();
 }
@@ -1119,7 +1381,7 @@ cudaError_t launch_profile_build_indirect(const ProfileBuild *dev, const int *en
 
 using ProfileFn = void (*)(const FocusJob *, const FocusUnit *, int, int *, const float2 *, float4 *);
 
-template <bool BAND, bool ADJ, bool MOVE>
+template <bool BAND, bool ADJ, int MOVE>
 static ProfileFn profile_fn(int group)
 {
     switch (group) {
@@ -1130,14 +1392,22 @@ static ProfileFn profile_fn(int group)
     }
 }
 
-static ProfileFn profile_fn(int group, bool band, bool adjoint, bool motion)
+static ProfileFn profile_fn(int group, bool band, bool adjoint, int motion)
 {
-    if (motion) return profile_fn<false, false, true>(group);
-    if (adjoint) return band ? profile_fn<true, true, false>(group) : profile_fn<false, true, false>(group);
-    return band ? profile_fn<true, false, false>(group) : profile_fn<false, false, false>(group);
+    if (motion == 2) return profile_fn<false, false, 2>(group);
+    if (motion) return profile_fn<false, false, 1>(group);
+    if (adjoint) return band ? profile_fn<true, true, 0>(group) : profile_fn<false, true, 0>(group);
+    return band ? profile_fn<true, false, 0>(group) : profile_fn<false, false, 0>(group);
 }
 
-cudaError_t launch_focus_profile(int group, bool band, bool motion, const FocusJob *jobs_dev,
+cudaError_t launch_vib_fit(const float4 *traj, const ChirpRec *chirps, int C, int S, int s_pad, float phase_per_m,
+                           VibRec *recs, int *maxima, cudaStream_t st)
+{
+    vib_fit_kernel<<<(C + 3) / 4, 128, 0, st>>>(traj, chirps, C, S, s_pad, phase_per_m, recs, maxima);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_focus_profile(int group, bool band, int motion, const FocusJob *jobs_dev,
                                  const FocusUnit *units_dev, int n_units, int *counter_dev, int grid_ctas,
                                  cudaStream_t st)
 {
@@ -1151,12 +1421,12 @@ cudaError_t launch_adjoint_profile(int group, bool band, const FocusJob *jobs_de
                                    int n_units, int *counter_dev, int grid_ctas, const float2 *gimg, float4 *gpart,
                                    cudaStream_t st)
 {
-    profile_fn(group, band, true, false)<<<grid_ctas, kThreads, 0, st>>>(jobs_dev, units_dev, n_units, counter_dev,
+    profile_fn(group, band, true, 0)<<<grid_ctas, kThreads, 0, st>>>(jobs_dev, units_dev, n_units, counter_dev,
                                                                          gimg, gpart);
     return cudaGetLastError();
 }
 
-int focus_profile_blocks_per_sm(int group, bool band, bool adjoint, bool motion)
+int focus_profile_blocks_per_sm(int group, bool band, bool adjoint, int motion)
 {
     int blocks = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, profile_fn(group, band, adjoint, motion), kThreads, 0) !=
