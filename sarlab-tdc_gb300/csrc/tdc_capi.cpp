@@ -349,6 +349,14 @@ int prepare(tdc_processor *p, const StartOpts &o, int &launches)
         gres[2 * (size_t)s_pad + s] = (float)(2.0 * M_PI * gsv);
     }
     std::vector<float4> traj, wins;
+    // two samples side by side (FocusJob::traj)
+    auto put_sample = [s_pad](std::vector<float4> &t, int c, int s, float x, float y, float z, float w) {
+        float *f = &t[(size_t)c * s_pad + (s & ~1)].x + (s & 1);
+        f[0] = x;
+        f[2] = y;
+        f[4] = z;
+        f[6] = w;
+    };
     std::vector<float> wdot;
     p->traj_varies = pos_differ;
     p->delta_max = 0.0;
@@ -371,8 +379,7 @@ int prepare(tdc_processor *p, const StartOpts &o, int &launches)
                     const float *ps = p->pos + 3 * ti(c, s);
                     const double dx = (double)ps[0] - p0[0], dy = (double)ps[1] - p0[1], dz = (double)ps[2] - p0[2];
                     m = std::max(m, dx * dx + dy * dy + dz * dz);
-                    traj[(size_t)c * s_pad + s] =
-                        make_float4((float)dx, (float)dy, (float)dz, (float)(dx * dx + dy * dy + dz * dz));
+                    put_sample(traj, c, s, (float)dx, (float)dy, (float)dz, (float)(dx * dx + dy * dy + dz * dz));
                 }
             }
             d2[t] = m;
@@ -380,23 +387,25 @@ int prepare(tdc_processor *p, const StartOpts &o, int &launches)
         p->delta_max = std::sqrt(*std::max_element(d2.begin(), d2.begin() + nt));
     }
     if (p->win_varies) {
-        // In band units: velocity x (-2 / lambda) / B and window centre / B, so the kernel forms
-        // (fDop - centre) / B with one dot product and one fused multiply-add. With positions
-        // moving within chirps the kernel dots the velocity with 2 (P0 - T) and adds the
-        // pixel-independent part u . D_s from its own table, so u is stored halved.
+        // As angles: velocity x (-2 / lambda) and window centre x 2 pi / B, so the kernel forms
+        // 2 pi (fDop - centre) / B with one dot product and one fused multiply-add (the band's edge at
+        // pi rounded to FP32, exactly as the kernel compares). With positions moving within
+        // chirps the pixel-independent part u . D_s comes from its own table.
         const bool with_traj = p->traj_varies;
-        wins.assign((size_t)C * s_pad, make_float4(0.f, 0.f, 0.f, 0.f));
+        wins.assign((size_t)C * s_pad + 2 * (size_t)C, make_float4(0.f, 0.f, 0.f, 0.f));
         if (with_traj) wdot.assign((size_t)C * s_pad, 0.f);
-        const double vs = -2.0 / (double)p->lambda / (double)o.bw, cs = 1.0 / (double)o.bw;
-        const double us = with_traj ? 0.5 : 1.0;
+        const double cs = 2.0 * (double)3.14159265358979323846f / (double)o.bw, vs = -2.0 / (double)p->lambda * cs;
         parallel_chirps(C, S, [&](int, int cb, int ce) {
             for (int c = cb; c < ce; ++c)
                 for (int s = 0; s < S; ++s) {
                     const size_t i = (size_t)c * s_pad + s;
                     const ChirpRec r = make_record(p, c, s, o.centroid != 0, o.center);
                     const double ux = r.vel.x * vs, uy = r.vel.y * vs, uz = r.vel.z * vs;
-                    wins[i] = make_float4((float)(us * ux), (float)(us * uy), (float)(us * uz), (float)(r.p_hi.w * cs));
-                    if (with_traj) wdot[i] = (float)(ux * traj[i].x + uy * traj[i].y + uz * traj[i].z);
+                    put_sample(wins, c, s, (float)ux, (float)uy, (float)uz, (float)(r.p_hi.w * cs));
+                    if (with_traj) {
+                        const float *d = &traj[i - (s & 1)].x + (s & 1);
+                        wdot[i] = (float)(ux * d[0] + uy * d[2] + uz * d[4]);
+                    }
                 }
         });
     }
@@ -619,6 +628,12 @@ int prepare(tdc_processor *p, const StartOpts &o, int &launches)
         TDC_CK(launch_range_window(p->wr.as<float>(), S, o.range_win, st), "range window kernel");
         TDC_CK(launch_prewindow(p->xw.as<float2>(), p->wr.as<float>(), C, S, s_pad, st), "prewindow kernel");
         launches += 2;
+    }
+    if (!wins.empty()) {
+        TDC_CK(launch_window_bounds(p->wins.as<float4>(), traj.empty() ? nullptr : p->traj.as<const float4>(),
+                                    p->xw.as<const float2>(), C, S, s_pad, st),
+               "window bounds kernel");
+        ++launches;
     }
     // The host vectors above are read by the async copies: wait before they go out of scope.
     TDC_CK(cudaStreamSynchronize(st), "prepare sync");

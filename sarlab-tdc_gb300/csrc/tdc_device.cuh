@@ -29,6 +29,14 @@ __device__ __forceinline__ long long tile_pixel(int tile_cols, int grid_cols, lo
     return col < grid_cols && p < P ? p : -1;
 }
 
+// Entry s of a row of the general kernels' per-sample tables, which keep two samples side by side: (x0, x1,
+// y0, y1)(z0, z1, w0, w1) (FocusJob::traj).
+__device__ __forceinline__ float4 sample_table(const float4 *row, int s)
+{
+    const float4 a = row[s & ~1], b = row[s | 1];
+    return s & 1 ? make_float4(a.y, a.w, b.y, b.w) : make_float4(a.x, a.z, b.x, b.z);
+}
+
 // ---------------------------------------------------------------------------
 // Error-free transformations (Knuth two-sum, FMA two-product).
 

@@ -12,24 +12,35 @@
 // Split about sample 0 (R0 = |P[c,0] - T| in double-float, as in the bulk kernel)
 // and the affine fit g_s = g0 + g1 s + r_s:
 //   g_s R_s = (g0 + g1 s) R0  +  r_s R0  +  g_s d_s,   d_s = R_s - R0.
-// The first term is the bulk kernel's alpha + beta s, evaluated with the same
-// blocked Horner recurrence (H <- H QL + sum_k x'_k p_k). The rest, psi_s, is a
-// per-(pixel, sample) correction folded into the sample: x'_s = x_s w_s e^{j 2 pi psi_s}.
+// The first term is alpha + beta s; the rest, psi_s, is a phase of every (pixel, sample). Where
+// there is one (all variants but per-sample windows alone) each sample takes one sincos of
+// 2 pi (beta s + psi_s): beta s is the block of 8's turn, a 32-bit fraction of a cycle stepped by
+// 8 beta, plus a table of k beta. (Correcting the sample by psi_s first and feeding it to the
+// bulk kernel's Horner recurrence took 4 more operations and as much state.) With per-sample
+// windows alone the recurrence runs on the weighted samples.
 // d_s comes without cancellation from the per-sample offset D_s = P[c,s] - P[c,0]
 // (host table: D_s and |D_s|^2 per (chirp, sample)):
-//   N = 2 (P0 - T).D + |D|^2 = R_s^2 - R0^2,   d_s = N / (R0 + R_s) = (N / 2R0) f(N / R0^2),
+//   m = n0.D + |D|^2 / 2R0 = (R_s^2 - R0^2) / 2R0,   d_s = m f(e),   e = 2 m / R0,
 //   f(e) = 2 / (1 + sqrt(1 + e)) = 1 - e/4 + e^2/8 - 5e^3/64 + 7e^4/128 - ...,
 // the series taken to e^2 when the host bounds |e| <= 0.02 and |psi| <= 4 cycles (then
-// the sincos takes psi unreduced: its argument scaling adds < 2e-6 rad), else to e^4 with
-// psi reduced modulo one cycle ("wide" variants, which also carry the non-uniform
+// the sincos takes the phase unreduced: its argument scaling adds < 2e-6 rad), else to e^4 with
+// the phase reduced modulo one cycle ("wide" variants, which also carry the non-uniform
 // sampling residual; the host routes |e| > 0.1 to the FP64 kernel; at 0.1 the
 // truncation is 4e-7 of d_s).
 //
+// Bound: the FMA pipe (63% busy, 63% of the issue slots). Two samples stand side by side in the
+// two halves of FFMA2, which halves the issue slots (the tables are laid out for it; what is a
+// pixel's own sits in both halves). 128^2 pixels x 512 chirps x 512 samples, 256 threads x 2 CTAs an SM
+// throughout: positions and windows per sample 5.19 ms as scalar code with a Horner recurrence,
+// 4.54 with pairs and dead chirps left out (23% of them there), 3.70 with one sincos for the whole
+// phase and the reciprocal by the special-function unit, 3.50 in units half as long. 128^2 x
+// 256 x 512: positions alone 1.62 -> 1.37 ms, windows alone 1.49 -> 1.16, non-uniform times 1.26
+// -> 1.17, windows and times 3.03 -> 1.72, all three 3.53 -> 2.52.
+//
 // Same unit decomposition, staging (cp.async.bulk + mbarrier pipeline), skip test,
-// Kahan accumulation and FP64 group reduction as the bulk kernel; a chirp whose
-// chirp-level weight is zero for every pixel of a warp skips the Horner loop. The
-// per-sample window works in band units, q = (fDop - centre) / B, from a table of
-// velocities pre-scaled by -2 / (lambda B) and centres by 1 / B.
+// Kahan accumulation and group reduction as the bulk kernel. A chirp skips its samples where its
+// chirp-level weight is zero, or every sample provably out of band, for every pixel of a warp (see
+// window_bounds_kernel).
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -52,6 +63,17 @@ constexpr int kTile = kT * kPT;
 // longer than its copy, and the smaller footprint keeps two CTAs resident per SM.
 constexpr int kStages = 2;
 static_assert(kTile == kFocusTile, "work units tile the grid like the FP32-bulk kernel");
+
+// 1 / v to an ulp, by the special-function unit.
+__device__ __forceinline__ float rcp(float v)
+{
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
+    return r;
+}
+
+__device__ __forceinline__ float2 both(float v) { return make_float2(v, v); }
+__device__ __forceinline__ float2 neg(float2 v) { return make_float2(-v.x, -v.y); }
 
 struct GenShared {
     float t[kPT * 6][kT];  // (x_hi, y_hi, z_hi, x_lo, y_lo, z_lo) per pixel slot
@@ -90,6 +112,7 @@ __global__ void __launch_bounds__(kT, (!TRAJ && WIN && WIDE) ? 1 : TDC_GENERAL_M
     GenShared &sp = *reinterpret_cast<GenShared *>(smem + kStages * stage_bytes);
 
     constexpr bool TW = TRAJ && WIN;  // per-sample positions and windows: window-offset rows staged
+    constexpr bool PHASE = TRAJ || WIDE;  // a phase of its own for every sample
     const int tid = threadIdx.x;
     if (tid == 0) {
         for (int i = 0; i < kStages; ++i) mbar_init(&full_bar[i], 1);
@@ -129,6 +152,7 @@ __global__ void __launch_bounds__(kT, (!TRAJ && WIN && WIDE) ? 1 : TDC_GENERAL_M
         const float4 *__restrict__ xw = sJ.xw;
         const float4 *__restrict__ traj = sJ.traj;
         const float4 *__restrict__ wins = sJ.wins;
+        const float4 *__restrict__ bounds = wins + (size_t)C * s_pad;  // see window_bounds_kernel
         const float *__restrict__ wdot = sJ.wdot;
         const float *__restrict__ gres = sJ.gres;
         const float *__restrict__ gsam = sJ.gsam;
@@ -205,6 +229,7 @@ __global__ void __launch_bounds__(kT, (!TRAJ && WIN && WIDE) ? 1 : TDC_GENERAL_M
         const float tol = sJ.two_over_lambda, half_bw = sJ.half_bw, inv_bw = sJ.inv_bw, az_a = sJ.az_a;
         const bool taper = (sJ.flags & kFlagTaper) != 0;
         const bool skip_test = (sJ.flags & kFlagSkipTest) != 0;
+        const float taper_a = taper ? az_a : 1.0f, taper_b = taper ? 1.0f - az_a : 0.0f;
         const int chunk = sJ.chunk;
         const SkipPoint *__restrict__ skip = sJ.skip;
 
@@ -216,12 +241,17 @@ __global__ void __launch_bounds__(kT, (!TRAJ && WIN && WIDE) ? 1 : TDC_GENERAL_M
             comp[i] = make_float2(0.f, 0.f);
             wskip[i] = 1.0f;
         }
-        // per-(pixel, chirp) state, carried across the segments of a chirp
-        float2 p[kPT][kL - 1];
-        float2 ql[kPT], q0[kPT], h[kPT];
-        float t2x[kPT], t2y[kPT], t2z[kPT];
-        float r0[kPT], a2[kPT], b2[kPT];  // R0, 1/2R0, 1/R0^2
-        float r0sq[kPT];                   // R0^2 (per-sample positions and windows)
+        // per-(pixel, chirp) state, carried across the segments of a chirp; what two samples side by
+        // side share is kept in both halves
+        constexpr int kTab = kL / 2, kRot = PHASE ? 1 : kTab, kTurns = PHASE ? kTab : 1;
+        float2 px[kPT][kRot], py[kPT][kRot], ql[kPT], h[kPT];  // in-block phasors, block step, Horner state
+        float2 turns[kPT][kTurns];                             // (PHASE) k beta of the block's samples
+        unsigned int step[kPT];                                // (PHASE) 8 beta [2^-32 cycles]
+        float2 accx[kPT], accy[kPT];                           // (PHASE) sums of the even and the odd samples
+        float2 q0[kPT];
+        float2 nx[kPT], ny[kPT], nz[kPT];   // (P0 - T) / R0
+        float2 r0[kPT], rs1[kPT];           // R0, 1 / R0
+        float2 a2[kPT], k2[kPT];            // 1 / 2R0, 1 / 2R0^2
         bool live = true;
         int cur_chunk = -1;
         bool timed_out = false;
@@ -273,42 +303,68 @@ __global__ void __launch_bounds__(kT, (!TRAJ && WIN && WIDE) ? 1 : TDC_GENERAL_M
                         dd_sub(r.p_hi.z, r.p_lo.z, sp.t[i * 6 + 2][tid], sp.t[i * 6 + 5][tid], dzh, dzl);
                         float rh, rl, rs, dh;
                         dd_range(dxh, dxl, dyh, dyl, dzh, dzl, rh, rl, rs, dh);
+                        // 1 / R0 to FP32 rounding (rsqrt is not)
+                        const float rinv = fmaf(rs, fmaf(-rl, rs, fmaf(-rh, rs, 1.0f)), rs);
                         const float alpha = dd_frac_mul(g0h, g0l, rh, rl);
                         float bh = g1 * rh;
                         float bl = fmaf(g1, rh, -bh);
                         bl = fmaf(g1, rl, bl);
                         bl = fmaf(g1l, rh, bl);
                         bh -= rintf(bh);
-                        float s1, c1s;
-                        __sincosf(kTwoPiF * (bh + bl), &s1, &c1s);
-                        p[i][0] = make_float2(c1s, s1);
-#pragma unroll
-                        for (int k = 1; k < kL - 1; ++k) p[i][k] = cmul(p[i][k - 1], p[i][0]);
                         const float lbh = (float)kL * bh;
-                        const float lfr = (lbh - rintf(lbh)) + (float)kL * bl;
-                        float sl, cl;
-                        sincospif(2.0f * lfr, &sl, &cl);
-                        ql[i] = make_float2(cl, sl);
+                        if constexpr (PHASE) {
+#pragma unroll
+                            for (int k = 0; k < kL; k += 2) {
+                                const float e = (float)k * bh, o = (float)(k + 1) * bh;
+                                const float2 v = make_float2(fmaf((float)k, bh, -rintf(e)) + (float)k * bl,
+                                                             fmaf((float)(k + 1), bh, -rintf(o)) + (float)(k + 1) * bl);
+                                turns[i][k / 2] = WIDE ? v : __fmul2_rn(v, both(kTwoPiF));
+                            }
+                            step[i] = (unsigned)__float2int_rn((lbh - rintf(lbh)) * 4294967296.0f) +
+                                      (unsigned)__float2int_rn(((float)kL * bl) * 4294967296.0f);
+                            accx[i] = accy[i] = both(0.f);
+                        } else {
+                            float s1, c1s;
+                            __sincosf(kTwoPiF * (bh + bl), &s1, &c1s);
+                            const float2 p1 = make_float2(c1s, s1);
+                            float2 pe = make_float2(1.f, 0.f);
+#pragma unroll
+                            for (int k = 0; k < kL; k += 2) {
+                                const float2 po = cmul(pe, p1);
+                                px[i][k / 2] = make_float2(pe.x, po.x);
+                                py[i][k / 2] = make_float2(pe.y, po.y);
+                                pe = cmul(po, p1);
+                            }
+                            const float lfr = (lbh - rintf(lbh)) + (float)kL * bl;
+                            float sl, cl;
+                            sincospif(2.0f * lfr, &sl, &cl);
+                            ql[i] = make_float2(cl, sl);
+                            h[i] = make_float2(0.f, 0.f);
+                        }
                         float w = wskip[i];
                         if (!WIN) {
                             const float fd = doppler_freq(tol, r.vel.x, r.vel.y, r.vel.z, dxh, dyh, dzh, rs);
                             w *= doppler_window(fd, r.p_hi.w, half_bw, inv_bw, taper, az_a);
                         }
-                        any |= w != 0.0f;
+                        bool out = false;
+                        if (WIN) {
+                            // every sample's window angle lies within `span` of this one
+                            const float4 wr = __ldg(&bounds[2 * c]), wb = __ldg(&bounds[2 * c + 1]);
+                            const float q = fmaf(rs, fmaf(wr.x, dxh, fmaf(wr.y, dyh, wr.z * dzh)), -wr.w);
+                            const float span = TRAJ ? fmaf(wb.y, __fdividef(wb.z, fmaxf(rh - wb.z, 0.0f)), wb.x) : wb.x;
+                            out = fabsf(q) > kPiF + span;
+                        }
+                        any |= w != 0.0f && !out;
                         float sa, ca;
                         __sincosf(kTwoPiF * alpha, &sa, &ca);
                         q0[i] = make_float2(w * ca, w * sa);
-                        h[i] = make_float2(0.f, 0.f);
-                        // TRAJ: 2 (P0 - T) for the range change; else the unit vector (P0 - T) / R0
-                        // of the per-sample window
-                        const float sc = TRAJ ? 2.0f : rs;
-                        t2x[i] = sc * dxh;
-                        t2y[i] = sc * dyh;
-                        t2z[i] = sc * dzh;
-                        r0[i] = rh;
-                        a2[i] = 0.5f * rs;  // 1 / 2R0
-                        b2[i] = rs * rs;    // 1 / R0^2
-                        if (TW) r0sq[i] = rh * rh;
+                        nx[i] = both(rinv * dxh);
+                        ny[i] = both(rinv * dyh);
+                        nz[i] = both(rinv * dzh);
+                        r0[i] = both(rh);
+                        rs1[i] = both(rinv);
+                        a2[i] = both(0.5f * rinv);
+                        k2[i] = both(0.5f * rinv * rinv);
                     }
                     // a chirp whose chirp-level weight (skip test, and the window unless it is
                     // per sample) is zero for every pixel of the warp contributes nothing
@@ -316,91 +372,121 @@ __global__ void __launch_bounds__(kT, (!TRAJ && WIN && WIDE) ? 1 : TDC_GENERAL_M
                 }
                 if (!live) continue;
 
-                // Horner over this segment's blocks, last block first; each sample corrected per pixel.
+                // This segment's blocks; each sample corrected per pixel.
                 for (int b = len / kL - 1; b >= 0; --b) {
-                    float2 acc[kPT];
+                    float2 base[kPT];  // (PHASE) turn of the block's first sample, beta s
+                    float2 bx[kPT], by[kPT];
 #pragma unroll
-                    for (int i = 0; i < kPT; ++i) acc[i] = cmul(h[i], ql[i]);
-#pragma unroll
-                    for (int k = 0; k < kL; ++k) {
-                        const int s = b * kL + k;  // sample within the segment
-                        const float4 xv = xs[s >> 1];
-                        const float xr = (k & 1) ? xv.z : xv.x;
-                        const float xi = (k & 1) ? xv.w : xv.y;
-                        float4 av = make_float4(0.f, 0.f, 0.f, 0.f), bv = av;
-                        if (TRAJ) av = as[s];
-                        if (WIN) bv = bs[s];
-                        const float uD = TW ? us[s] : 0.0f;
-                        const float res = WIDE ? sgr[s] : 0.0f;
-                        const float gsv = TRAJ ? sgg[s] : 0.0f;
-#pragma unroll
-                        for (int i = 0; i < kPT; ++i) {
-                            float yr = xr, yi = xi;
-                            float n = 0.0f;  // N = 2 (P0 - T).D + |D|^2 = |P0 - T + D|^2 - R0^2
-                            if (TRAJ || WIDE) {
-                                float psi = 0.0f;
-                                if (TRAJ) {
-                                    // |D|^2 from the table
-                                    n = fmaf(t2x[i], av.x, fmaf(t2y[i], av.y, fmaf(t2z[i], av.z, av.w)));
-                                    const float e = n * b2[i];
-                                    float f;
-                                    if (WIDE) {
-                                        f = fmaf(e, 7.0f / 128.0f, -5.0f / 64.0f);
-                                        f = fmaf(f, e, 0.125f);
-                                        f = fmaf(f, e, -0.25f);
-                                    } else {
-                                        f = fmaf(e, 0.125f, -0.25f);
-                                    }
-                                    f = fmaf(f, e, 1.0f);
-                                    psi = (gsv * a2[i]) * (n * f);  // g_s d_s (radians when narrow)
-                                }
-                                if (WIDE) {
-                                    psi = fmaf(res, r0[i], psi);
-                                    psi -= round_small(psi);
-                                    psi *= kTwoPiF;
-                                }
-                                float sn, cs;
-                                __sincosf(psi, &sn, &cs);
-                                yr = fmaf(xr, cs, -xi * sn);
-                                yi = fmaf(xr, sn, xi * cs);
-                            }
-                            if (WIN) {
-                                // per-sample window at P[c,s] (d = P0 - T + D_s) in band units:
-                                // q = (fDop - centre) / B from the table's velocity scaled by
-                                // -2/(lambda B) and centre / B; in band for |q| <= 1/2, taper
-                                // a - (1-a) cos(2 pi q - pi) = a + (1-a) cos(2 pi q)
-                                // (with moving positions: u.d = (u/2).2(P0 - T) + u.D, the second
-                                // term from the table, and |d|^2 = R0^2 + N)
-                                float q;
-                                if (TRAJ) {
-                                    const float ud = fmaf(bv.x, t2x[i], fmaf(bv.y, t2y[i], fmaf(bv.z, t2z[i], uD)));
-                                    q = fmaf(ud, rsqrtf(r0sq[i] + n), -bv.w);
-                                } else {
-                                    q = fmaf(bv.x, t2x[i], fmaf(bv.y, t2y[i], fmaf(bv.z, t2z[i], -bv.w)));
-                                }
-                                float w = taper ? fmaf(1.0f - az_a, __cosf(kTwoPiF * q), az_a) : 1.0f;
-                                w = fabsf(q) <= 0.5f ? w : 0.0f;
-                                yr *= w;
-                                yi *= w;
-                            }
-                            if (k == 0) {
-                                acc[i].x += yr;
-                                acc[i].y += yi;
-                            } else {
-                                acc[i].x = fmaf(yr, p[i][k - 1].x, acc[i].x);
-                                acc[i].x = fmaf(-yi, p[i][k - 1].y, acc[i].x);
-                                acc[i].y = fmaf(yr, p[i][k - 1].y, acc[i].y);
-                                acc[i].y = fmaf(yi, p[i][k - 1].x, acc[i].y);
-                            }
+                    for (int i = 0; i < kPT; ++i) {
+                        if constexpr (PHASE) {
+                            const int turn = (int)((unsigned)(off / kL + b) * step[i]);
+                            base[i] = both((float)turn * (WIDE ? 1.0f / 4294967296.0f : kTwoPiF / 4294967296.0f));
+                        } else {
+                            const float2 v = cmul(h[i], ql[i]);
+                            bx[i] = make_float2(v.x, 0.f);
+                            by[i] = make_float2(v.y, 0.f);
                         }
                     }
 #pragma unroll
-                    for (int i = 0; i < kPT; ++i) h[i] = acc[i];
+                    for (int k = 0; k < kL; k += 2) {
+                        const int s = b * kL + k;  // samples s and s + 1 within the segment
+                        const float4 xv = xs[s >> 1];
+                        const float2 xr = make_float2(xv.x, xv.z), xi = make_float2(xv.y, xv.w);
+                        float4 a01 = make_float4(0.f, 0.f, 0.f, 0.f), a23 = a01, b01 = a01, b23 = a01;
+                        if (TRAJ) {
+                            a01 = as[s];
+                            a23 = as[s + 1];
+                        }
+                        if (WIN) {
+                            b01 = bs[s];
+                            b23 = bs[s + 1];
+                        }
+                        const float2 uD = TW ? *reinterpret_cast<const float2 *>(us + s) : both(0.f);
+                        const float2 res = WIDE ? *reinterpret_cast<const float2 *>(sgr + s) : both(0.f);
+                        const float2 gsv = TRAJ ? *reinterpret_cast<const float2 *>(sgg + s) : both(0.f);
+#pragma unroll
+                        for (int i = 0; i < kPT; ++i) {
+                            float2 d = both(0.f);  // R_s - R0
+                            if (TRAJ) {
+                                // m = (R_s^2 - R0^2) / 2R0, d = m f(e), e = 2 m / R0
+                                const float2 m = __ffma2_rn(
+                                    nx[i], make_float2(a01.x, a01.y),
+                                    __ffma2_rn(ny[i], make_float2(a01.z, a01.w),
+                                               __ffma2_rn(nz[i], make_float2(a23.x, a23.y),
+                                                          __fmul2_rn(a2[i], make_float2(a23.z, a23.w)))));
+                                if (WIDE) {
+                                    const float2 e = __fmul2_rn(m, __fadd2_rn(rs1[i], rs1[i]));
+                                    float2 f = __ffma2_rn(e, both(7.0f / 128.0f), both(-5.0f / 64.0f));
+                                    f = __ffma2_rn(f, e, both(0.125f));
+                                    f = __ffma2_rn(f, e, both(-0.25f));
+                                    f = __ffma2_rn(f, e, both(1.0f));
+                                    d = __fmul2_rn(m, f);
+                                } else {
+                                    d = __ffma2_rn(__fmul2_rn(m, m), __ffma2_rn(m, k2[i], neg(a2[i])), m);
+                                }
+                            }
+                            float2 cs = both(1.f), sn = both(0.f);
+                            if constexpr (PHASE) {
+                                float2 th = __fadd2_rn(base[i], turns[i][k / 2]);
+                                if (TRAJ) th = __ffma2_rn(gsv, d, th);  // g_s d_s (radians when narrow)
+                                if (WIDE) {
+                                    th = __ffma2_rn(res, r0[i], th);
+                                    th = make_float2(th.x - round_small(th.x), th.y - round_small(th.y));
+                                    th = __fmul2_rn(th, both(kTwoPiF));
+                                }
+                                __sincosf(th.x, &sn.x, &cs.x);
+                                __sincosf(th.y, &sn.y, &cs.y);
+                            }
+                            float2 w = both(1.f);
+                            if (WIN) {
+                                // per-sample window at P[c,s] (d = P0 - T + D_s), as an angle:
+                                // q = 2 pi (fDop - centre) / B, the table's velocity scaled by
+                                // -4 pi / (lambda B) and centre by 2 pi / B; in band for |q| <= pi, taper
+                                // a - (1-a) cos(q - pi) = a + (1-a) cos(q) (with moving positions
+                                // u.d / R_s = (u.n0 + u.D / R0) / (1 + d_s / R0), u.D from the table)
+                                float2 q = __ffma2_rn(make_float2(b01.x, b01.y), nx[i],
+                                                      __ffma2_rn(make_float2(b01.z, b01.w), ny[i],
+                                                                 __fmul2_rn(make_float2(b23.x, b23.y), nz[i])));
+                                if (TRAJ) {
+                                    q = __ffma2_rn(uD, rs1[i], q);
+                                    const float2 y = __ffma2_rn(d, rs1[i], both(1.0f));
+                                    q = __ffma2_rn(q, make_float2(rcp(y.x), rcp(y.y)),
+                                                   make_float2(-b23.z, -b23.w));
+                                } else {
+                                    q = __fadd2_rn(q, make_float2(-b23.z, -b23.w));
+                                }
+                                w = __ffma2_rn(make_float2(__cosf(q.x), __cosf(q.y)), both(taper_b), both(taper_a));
+                                w.x = fabsf(q.x) <= kPiF ? w.x : 0.0f;
+                                w.y = fabsf(q.y) <= kPiF ? w.y : 0.0f;
+                            }
+                            if constexpr (PHASE) {
+                                if (WIN) {
+                                    cs = __fmul2_rn(cs, w);
+                                    sn = __fmul2_rn(sn, w);
+                                }
+                                accx[i] = __ffma2_rn(xr, cs, accx[i]);
+                                accx[i] = __ffma2_rn(neg(xi), sn, accx[i]);
+                                accy[i] = __ffma2_rn(xr, sn, accy[i]);
+                                accy[i] = __ffma2_rn(xi, cs, accy[i]);
+                            } else {
+                                const float2 yr = __fmul2_rn(xr, w), yi = __fmul2_rn(xi, w);
+                                bx[i] = __ffma2_rn(yr, px[i][k / 2], bx[i]);
+                                bx[i] = __ffma2_rn(neg(yi), py[i][k / 2], bx[i]);
+                                by[i] = __ffma2_rn(yr, py[i][k / 2], by[i]);
+                                by[i] = __ffma2_rn(yi, px[i][k / 2], by[i]);
+                            }
+                        }
+                    }
+                    if constexpr (!PHASE) {
+#pragma unroll
+                        for (int i = 0; i < kPT; ++i) h[i] = make_float2(bx[i].x + bx[i].y, by[i].x + by[i].y);
+                    }
                 }
 
                 if (sg == 0) {
 #pragma unroll
                     for (int i = 0; i < kPT; ++i) {
+                        if constexpr (PHASE) h[i] = make_float2(accx[i].x + accx[i].y, accy[i].x + accy[i].y);
                         const float2 v = cmul(q0[i], h[i]);
                         const float yr = v.x - comp[i].x, yi = v.y - comp[i].y;
                         const float tr = sum[i].x + yr, ti = sum[i].y + yi;
@@ -440,6 +526,55 @@ __global__ void __launch_bounds__(kT, (!TRAJ && WIN && WIDE) ? 1 : TDC_GENERAL_M
     }
 }
 
+// Per chirp, how far the per-sample windows stray from one: with u_s the scaled velocity, c_s the
+// scaled window centre, and n_s the unit vector from the pixel, q_s = u_s.n_s - c_s. About the
+// mean (u, c) and the direction n_0 from sample 0, |q_s - (u.n_0 - c)| <= max|u_s - u| + max|c_s - c|
+// + max|u_s| |n_s - n_0|, and |n_s - n_0| <= max|D_s| / (R0 - max|D_s|). Writes (u, c) and (the first two
+// terms plus FP32 rounding, max|u_s|, max|D_s|) behind the windows. A row with a sample that
+// is not finite is never skipped (its product with a zero window is NaN). One warp a chirp.
+__global__ void __launch_bounds__(128)
+    window_bounds_kernel(float4 *__restrict__ wins, const float4 *__restrict__ traj, const float2 *__restrict__ xw,
+                         int C, int S, int s_pad)
+{
+    const int c = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (c >= C) return;
+    const size_t row = (size_t)c * s_pad;
+    auto window = [&](int s) { return sample_table(wins + row, s); };
+    float4 m = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int s = lane; s < S; s += 32) {
+        const float4 w = window(s);
+        m = make_float4(m.x + w.x, m.y + w.y, m.z + w.z, m.w + w.w);
+    }
+    const float inv = 1.0f / (float)S;
+    for (int off = 16; off > 0; off >>= 1)
+        m = make_float4(m.x + __shfl_xor_sync(0xffffffffu, m.x, off), m.y + __shfl_xor_sync(0xffffffffu, m.y, off),
+                        m.z + __shfl_xor_sync(0xffffffffu, m.z, off), m.w + __shfl_xor_sync(0xffffffffu, m.w, off));
+    m = make_float4(m.x * inv, m.y * inv, m.z * inv, m.w * inv);
+    float du = 0.f, dc = 0.f, dd = 0.f;
+    bool bad = false;
+    for (int s = lane; s < S; s += 32) {
+        const float4 w = window(s);
+        const float x = w.x - m.x, y = w.y - m.y, z = w.z - m.z;
+        du = fmaxf(du, sqrtf(x * x + y * y + z * z));
+        dc = fmaxf(dc, fabsf(w.w - m.w));
+        if (traj) dd = fmaxf(dd, sqrtf(sample_table(traj + row, s).w));
+        const float2 v = xw[row + s];
+        bad |= !isfinite(v.x) || !isfinite(v.y) || !isfinite(x + y + z + w.w + dd);
+    }
+    for (int off = 16; off > 0; off >>= 1) {
+        du = fmaxf(du, __shfl_xor_sync(0xffffffffu, du, off));
+        dc = fmaxf(dc, __shfl_xor_sync(0xffffffffu, dc, off));
+        dd = fmaxf(dd, __shfl_xor_sync(0xffffffffu, dd, off));
+    }
+    bad = __any_sync(0xffffffffu, bad);
+    if (lane) return;
+    const float u = sqrtf(m.x * m.x + m.y * m.y + m.z * m.z) + du;
+    const float slack = 1.01f * (du + dc) + 1e-5f * (1.0f + u + fabsf(m.w));
+    float4 *out = wins + (size_t)C * s_pad + 2 * (size_t)c;
+    out[0] = m;
+    out[1] = make_float4(bad ? INFINITY : slack, 1.01f * u, 1.001f * dd, 0.f);
+}
+
 template <bool TRAJ, bool WIN, bool WIDE>
 struct GeneralKernel {
     static constexpr auto fn = focus_general_kernel<TRAJ, WIN, WIDE>;
@@ -462,6 +597,13 @@ KernelFn select_kernel(int variant)
 }
 
 }  // namespace
+
+cudaError_t launch_window_bounds(float4 *wins, const float4 *traj, const float2 *xw, int C, int S, int s_pad,
+                                 cudaStream_t st)
+{
+    window_bounds_kernel<<<(C + 3) / 4, 128, 0, st>>>(wins, traj, xw, C, S, s_pad);
+    return cudaGetLastError();
+}
 
 int focus_general_smem_bytes(int stage_bytes)
 {

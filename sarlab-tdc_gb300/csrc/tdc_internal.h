@@ -39,9 +39,10 @@ constexpr double kAnchorMaxDistance = 0.05;  // metres
 // it. CTAs that share an SM need not progress at the same rate, so with a few long
 // units per slot the last units end far apart (measured on 256^2 pixels x 256 chirps
 // x 1024 samples, general kernel: SMs busy 72-100% of the launch at 3 units per slot,
-// +14% throughput at 4 or more).
+// +14% throughput at 4 or more; with dead chirps skipped, 128^2 x 512 x 512, 4.08 ms at 2 units a
+// slot, 3.70 at 4, 3.50 at 8, 3.47 at 16).
 #ifndef TDC_GENERAL_MIN_UNITS
-#define TDC_GENERAL_MIN_UNITS 4
+#define TDC_GENERAL_MIN_UNITS 8
 #endif
 #ifndef TDC_FOCUS_MIN_UNITS
 #define TDC_FOCUS_MIN_UNITS 8
@@ -127,11 +128,11 @@ struct FocusJob {
     const float4 *grid_lo;   // [P] or nullptr
     const SkipPoint *skip;   // [n_chunks][9]
     const double *gs;        // [S] 2 f_s / c0 (FP64 kernels only)
-    const float4 *traj;      // [C][s_pad] (P[c,s] - P[c,0], |P[c,s] - P[c,0]|^2) (FP32 general kernel, per-sample positions)
-    const float4 *wins;      // [C][s_pad] (velocity x -2/(lambda B), window centre / B) per sample (FP32 general
-                             // kernel, per-sample windows); the velocity term halved when positions also
-                             // move within chirps
-    const float *wdot;       // [C][s_pad] velocity x -2/(lambda B) . (P[c,s] - P[c,0]) (per-sample positions
+    const float4 *traj;      // [C][s_pad] (P[c,s] - P[c,0], |P[c,s] - P[c,0]|^2) (FP32 general kernel, per-sample
+                             // positions), two samples side by side: (x0, x1, y0, y1)(z0, z1, w0, w1)
+    const float4 *wins;      // [C][s_pad] 2 pi / B (velocity x -2 / lambda, window centre) per sample, likewise (FP32
+                             // general kernel, per-sample windows); then [C][2] bounds (launch_window_bounds)
+    const float *wdot;       // [C][s_pad] 2 pi / B velocity x -2 / lambda . (P[c,s] - P[c,0]) (per-sample positions
                              // and windows)
     const float *gres;       // [s_pad] 2 f_s / c0 - (g0 + g1 s) (FP32 general kernel, non-uniform sampling)
     const float *gsam;       // [s_pad] 2 f_s / c0 [cycles / m] (wide variants) or 2 pi x that [rad / m]
@@ -236,7 +237,7 @@ struct ProfileBuild {
     int C, S, s_pad, n_cells;
     int chirp_words;
     int margin;              // cells the table starts early (even; smooth motion)
-    const float4 *traj;      // vibration: [C][s_pad] D_s = P[c, s] - P[c, 0] (else null)
+    const float4 *traj;      // vibration: FocusJob::traj (else null)
     float phase_g, phase_g1; // 2 pi gc and 2 pi g1 [rad / m]
 };
 
@@ -318,6 +319,9 @@ cudaError_t launch_focus_reduce(const float4 *partial, int n_groups, long long P
 // samples at a time: whole rows (seg_len = s_pad, job.stage_chirps chirps a stage) or
 // segments of one chirp; stage_bytes = chirps x (seg_len x row bytes per sample + one
 // record) + seg_len x table bytes per sample (see general_stage_bytes_for).
+// Bounds on each chirp's windows over its samples, behind the table wins [C][s_pad].
+cudaError_t launch_window_bounds(float4 *wins, const float4 *traj, const float2 *xw, int C, int S, int s_pad,
+                                 cudaStream_t st);
 cudaError_t launch_focus_general(int variant, const FocusJob *jobs_dev, const FocusUnit *units_dev, int n_units,
                                  int *counter_dev, int *status_dev, int stage_bytes, int grid_ctas, cudaStream_t st);
 int focus_general_blocks_per_sm(int variant, int stage_bytes);
@@ -341,7 +345,7 @@ cudaError_t launch_adjoint_profile(int group, bool band, const FocusJob *jobs_de
                                    int n_units, int *counter_dev, int grid_ctas, const float2 *gimg, float4 *gpart,
                                    cudaStream_t st);
 int focus_profile_blocks_per_sm(int group, bool band, bool adjoint, int motion);
-// Straight-line fit of every chirp's offsets traj ([C][s_pad], chirps with sample-0 positions) and the
+// Straight-line fit of every chirp's offsets (FocusJob::traj, chirps with sample-0 positions) and the
 // principal direction of what it leaves, as VibRec; maxima[0..2] = max(maxima, largest deviation,
 // deviation off that direction, |W1|) as float bits (starting at 0; NaN above all).
 cudaError_t launch_vib_fit(const float4 *traj, const ChirpRec *chirps, int C, int S, int s_pad, float phase_per_m,

@@ -236,7 +236,7 @@ __global__ void __launch_bounds__(kBuildThreads)
         if (s >= b.S || c >= b.C) return 0.f;
         const float4 *rec = b.chirps + (size_t)c * b.chirp_words;
         const float4 w1 = rec[2], f0 = rec[4], n = rec[5];
-        const float4 d = b.traj[(size_t)c * b.s_pad + s];
+        const float4 d = sample_table(b.traj + (size_t)c * b.s_pad, s);
         const float t = (float)(s - b.S / 2);
         const float g = fmaf(b.phase_g1, t, b.phase_g);
         const float x = g * fmaf(-w1.x, t, d.x - f0.x), y = g * fmaf(-w1.y, t, d.y - f0.y),
@@ -356,7 +356,7 @@ __global__ void __launch_bounds__(128)
     const double hs = 0.5 * (S - 1);
     double a[6] = {0, 0, 0, 0, 0, 0}, sxx = 0.0;
     for (int s = lane; s < S; s += 32) {
-        const float4 d = row[s];
+        const float4 d = sample_table(row, s);
         const double x = s - hs, v[3] = {d.x, d.y, d.z};
         sxx += x * x;
         for (int k = 0; k < 3; ++k) {
@@ -377,7 +377,7 @@ __global__ void __launch_bounds__(128)
     }
     const float ff[3] = {(float)f0[0], (float)f0[1], (float)f0[2]}, fw[3] = {(float)w1[0], (float)w1[1], (float)w1[2]};
     auto deviation = [&](int s, float &x, float &y, float &z) {
-        const float4 d = row[s];
+        const float4 d = sample_table(row, s);
         const float t = (float)(s - S / 2);
         x = fmaf(-fw[0], t, d.x - ff[0]);
         y = fmaf(-fw[1], t, d.y - ff[1]);
