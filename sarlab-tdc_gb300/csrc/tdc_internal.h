@@ -333,7 +333,7 @@ int focus_general_smem_bytes(int stage_bytes);
 cudaError_t launch_profile_twiddle(float2 *twiddle, float *factor, int S, cudaStream_t st);
 cudaError_t launch_profile_build(const ProfileBuild &b, cudaStream_t st);
 // The same with its inputs in device memory, of at most max_cells cells; nothing where *enabled is 0.
-cudaError_t launch_profile_build_indirect(const ProfileBuild *dev, const int *enabled, int C, int max_cells,
+cudaError_t launch_profile_build_indirect(const ProfileBuild *dev, const int *enabled, int C, int S, int max_cells,
                                           cudaStream_t st);
 // motion: 1, the records are MoveRec, every sample of a chirp at a range of its own; 2, they are
 // VibRec and there are kVibTables tables.

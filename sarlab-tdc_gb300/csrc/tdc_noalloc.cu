@@ -369,7 +369,7 @@ int enqueue(const tdc_noalloc_focus_args *a, float *image_dev, cudaStream_t st, 
         if (e == cudaSuccess)
             e = launch_profile_twiddle(const_cast<float2 *>(pp.build.twiddle), const_cast<float *>(pp.build.factor), S, st);
         if (e == cudaSuccess)
-            e = launch_profile_build_indirect(pp.build_out, words + kWordProfile, C, pp.max_cells, st);
+            e = launch_profile_build_indirect(pp.build_out, words + kWordProfile, C, S, pp.max_cells, st);
         const int n = pp.n_tiles * pp.n_groups;
         const int ctas = std::min(n, n_sm * focus_profile_blocks_per_sm(1, band, false, false));
         if (e == cudaSuccess)

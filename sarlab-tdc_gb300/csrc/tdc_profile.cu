@@ -26,8 +26,12 @@
 
 #include <cmath>
 
+#include <cooperative_groups.h>
+
 #include "tdc_device.cuh"
 #include "tdc_internal.h"
+
+namespace cg = cooperative_groups;
 
 namespace tdc {
 
@@ -133,12 +137,13 @@ __global__ void profile_twiddle_kernel(float2 *__restrict__ tw, float *__restric
 // not grow with the row, and the cells' coefficients are formed from the nodes in shared memory.
 // Bound: FP32 FMA; C x S x (nodes the grid spans + up to one block) complex MACs, a few per cent
 // of the focus it serves.
+// A cluster of `split` CTAs shares a row's samples (launch_build).
 // INDIRECT: the inputs come from device memory (`dev`, written by an earlier kernel of the stream)
 // and the CTAs return at once where *enabled is 0.
 template <bool INDIRECT>
 __global__ void __launch_bounds__(kBuildThreads)
     profile_build_kernel(const __grid_constant__ ProfileBuild direct, const __grid_constant__ ProfileStencil stencil,
-                         const ProfileBuild *__restrict__ dev, const int *__restrict__ enabled)
+                         const ProfileBuild *__restrict__ dev, const int *__restrict__ enabled, int split)
 {
     __shared__ ProfileBuild sb;
     if (INDIRECT) {
@@ -155,7 +160,8 @@ __global__ void __launch_bounds__(kBuildThreads)
     __shared__ unsigned int s_shift[kBuildChirps];  // first node of the block modulo 2 S
     static_assert(kBuildStep >= 2 * kBuildChirps, "node values reuse the phasor tile");
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int c0 = blockIdx.x * kBuildChirps;
+    const int rank = (int)blockIdx.x % split;  // in the cluster: this CTA's part of the samples
+    const int c0 = (int)blockIdx.x / split * kBuildChirps;
     const unsigned int nn = 2u * (unsigned)b.S;
 
     if (blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && tid == 0) *b.job_out = b.job;
@@ -174,12 +180,13 @@ __global__ void __launch_bounds__(kBuildThreads)
         const double u = fmin(b.cells_per_m * sqrt(near2), b.cells_per_m * sqrt(far2));
         // (positions far outside what the table can index: any base will do, reads are clamped)
         const int base = fabs(u) < 1e9 ? 2 * (int)floor(0.5 * u) - 2 - b.margin : 0;
-        if (blockIdx.y == 0 && blockIdx.z == 0 && c0 + tid < b.C) b.cell_base[c0 + tid] = base;
+        if (rank == 0 && blockIdx.y == 0 && blockIdx.z == 0 && c0 + tid < b.C) b.cell_base[c0 + tid] = base;
         const int node = base >> 1;
         const int block = (node >= 0 ? node / kOwn : -((kOwn - 1 - node) / kOwn)) + (int)blockIdx.y;
         s_cell[tid] = 2 * (block * kOwn - node);
-        long long n0 = ((long long)block * kOwn - kTaps / 2) % (long long)nn;
-        s_shift[tid] = (unsigned)(n0 < 0 ? n0 + nn : n0);
+        // (cell indices stay below 2^22)
+        const int n0 = (block * kOwn - kTaps / 2) % (int)nn;
+        s_shift[tid] = (unsigned)(n0 < 0 ? n0 + (int)nn : n0);
     }
     __syncthreads();
     if (!__syncthreads_or(tid < kBuildChirps && s_cell[tid & (kBuildChirps - 1)] < b.n_cells)) return;
@@ -215,16 +222,23 @@ __global__ void __launch_bounds__(kBuildThreads)
             ahead_z[i] = e < ns * kNodes / 2 ? __ldg(&src[e]) : make_float4(0.f, 0.f, 0.f, 0.f);
         }
     };
+    // this CTA's tiles, in whole pairs (the sums are carried over two)
+    const int tiles = (b.S + kBuildStep - 1) / kBuildStep, each = ((tiles + split - 1) / split + 1) & ~1;
+    const int s_begin = rank * each * kBuildStep, s_end = min(b.S, s_begin + each * kBuildStep);
     // shift's turns at this thread's sample, modulo 2 S: (first node) x (s - sc), advanced a tile at a time
     unsigned int turn[kRowsEach], turn_step[kRowsEach];
     {
-        const int d = si_mine - b.S / 2;
-        const long long dm = d < 0 ? d + (long long)nn : d;
+        const int d = s_begin + si_mine - b.S / 2;
+        const unsigned int dm = d < 0 ? (unsigned)(d + (int)nn) : (unsigned)d;
+        // (64-bit remainders cost about 100 instructions each)
+        auto mul_mod = [nn](unsigned int a, unsigned int m) {
+            return nn <= 65536 ? a * m % nn : (unsigned)((unsigned long long)a * m % nn);
+        };
 #pragma unroll
         for (int i = 0; i < kRowsEach; ++i) {
-            const unsigned long long sh = s_shift[(warp >> 1) + 4 * i];
-            turn[i] = (unsigned)((sh * (unsigned long long)(dm % nn)) % nn);
-            turn_step[i] = (unsigned)((sh * kBuildStep) % nn);
+            const unsigned int sh = s_shift[(warp >> 1) + 4 * i];
+            turn[i] = mul_mod(sh, dm % nn);
+            turn_step[i] = mul_mod(sh, (unsigned)kBuildStep % nn);
         }
     }
     const float fnn = (float)nn, inv_nn = 1.0f / fnn;
@@ -244,9 +258,9 @@ __global__ void __launch_bounds__(kBuildThreads)
         const float chi = fmaf(n.x, x, fmaf(n.y, y, n.z * z));
         return family == 1 ? x : family == 2 ? y : family == 3 ? z : family == 4 ? chi * chi : chi * chi * chi;
     };
-    load_ahead(0);
+    load_ahead(s_begin);
 
-    for (int s0 = 0, tile = 0; s0 < b.S; s0 += kBuildStep, ++tile) {
+    for (int s0 = s_begin, tile = 0; s0 < s_end; s0 += kBuildStep, ++tile) {
         // rows: shifted by the block's first node, scaled, zero past the row's end
 #pragma unroll
         for (int i = 0; i < kRowsEach; ++i) {
@@ -270,7 +284,7 @@ __global__ void __launch_bounds__(kBuildThreads)
 #pragma unroll
         for (int i = 0; i < kPhasorsEach; ++i) reinterpret_cast<float4 *>(sv)[tid + i * kBuildThreads] = ahead_z[i];
         __syncthreads();
-        if (s0 + kBuildStep < b.S) load_ahead(s0 + kBuildStep);
+        if (s0 + kBuildStep < s_end) load_ahead(s0 + kBuildStep);
 #pragma unroll 8
         for (int si = 0; si < kBuildStep / 2; ++si) {
             const int s = half * (kBuildStep / 2) + si;
@@ -290,7 +304,7 @@ __global__ void __launch_bounds__(kBuildThreads)
                 }
             }
         }
-        if ((tile & 1) || s0 + kBuildStep >= b.S) {
+        if ((tile & 1) || s0 + kBuildStep >= s_end) {
 #pragma unroll
             for (int i = 0; i < 4; ++i)
 #pragma unroll
@@ -312,17 +326,36 @@ __global__ void __launch_bounds__(kBuildThreads)
         const float2 a = sv[i], z = sv[kBuildChirps * kNodes + i];
         sv[i] = make_float2(a.x + z.x, a.y + z.y);
     }
-    __syncthreads();
+    // the cluster's sums, each CTA for its share of the chirps, in order of the samples
+    const int share = kBuildChirps / split;
+    float2 *nodes = sv;
+    if (split > 1) {
+        cg::cluster_group cluster = cg::this_cluster();
+        cluster.sync();
+        nodes = &sx[0][0];
+        for (int i = tid; i < share * kNodes; i += kBuildThreads) {
+            float2 v = make_float2(0.f, 0.f);
+            for (int r = 0; r < split; ++r) {
+                const float2 x = cluster.map_shared_rank(sv, r)[rank * share * kNodes + i];
+                v.x += x.x;
+                v.y += x.y;
+            }
+            nodes[i] = v;
+        }
+        cluster.sync();
+    } else {
+        __syncthreads();
+    }
 
-    for (int i = tid; i < kBuildChirps * kOwn; i += kBuildThreads) {
-        const int q = i / kOwn, j = i - q * kOwn;
+    for (int i = tid; i < share * kOwn; i += kBuildThreads) {
+        const int q = rank * share + i / kOwn, j = i % kOwn;
         const int c = c0 + q;
         if (c >= b.C) break;
         const int l = s_cell[q] + 2 * j;  // cell within the chirp's table
         if (l < 0 || l >= b.n_cells) continue;
         float2 v[kTaps];
 #pragma unroll
-        for (int k = 0; k < kTaps; ++k) v[k] = sv[q * kNodes + j + k];
+        for (int k = 0; k < kTaps; ++k) v[k] = nodes[(q - rank * share) * kNodes + j + k];
         float4 *__restrict__ out =
             b.cells + (((size_t)family * b.C + c) * b.n_cells + l) * (kProfileCoefs / 2);
 #pragma unroll
@@ -1360,23 +1393,47 @@ cudaError_t launch_profile_twiddle(float2 *twiddle, float *factor, int S, cudaSt
     return cudaGetLastError();
 }
 
+// A row's samples are split over the CTAs of a cluster (their sums meet in its shared memory) while
+// the chirps alone leave SMs idle: up to 8 ways, at least two tiles a CTA, at most 5/3 CTAs an SM. By
+// chirps and samples only: the sums must not depend on where a row block of a grid lies. Whole
+// focus, split or not: 256^2 pixels x 64 chirps x 12345 samples 103 / 511 us, 64 x 512 x 512 x 1024
+// (moving) 117 / 148, 128^2 x 256 x 256 50 / 54, vibration (151 x 97 x 333 x 500) 107 / 126; up to 2
+// CTAs an SM, 256^2 x 1024 x 512 179 / 175.
+constexpr int kBuildMaxSplit = 8, kBuildMaxCtas = 152 * 5 / 3;
+
+template <bool INDIRECT>
+static cudaError_t launch_build(const ProfileBuild &b, const ProfileStencil &stencil, const ProfileBuild *dev,
+                                const int *enabled, int C, int S, int blocks, int tables, cudaStream_t st)
+{
+    const int chirp_blocks = (C + kBuildChirps - 1) / kBuildChirps, tiles = (S + kBuildStep - 1) / kBuildStep;
+    int split = 1;
+    while (split < kBuildMaxSplit && 2LL * split * chirp_blocks * tables <= kBuildMaxCtas && tiles >= 4 * split) split *= 2;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(chirp_blocks * split, blocks, tables);
+    cfg.blockDim = dim3(kBuildThreads);
+    cfg.stream = st;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = split;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = split > 1;
+    return cudaLaunchKernelEx(&cfg, profile_build_kernel<INDIRECT>, b, stencil, dev, enabled, split);
+}
+
 cudaError_t launch_profile_build(const ProfileBuild &b, cudaStream_t st)
 {
     static const ProfileStencil stencil = make_stencil();
     // nodes of n_cells / 2 from an even cell on, wherever the first block starts
     const int blocks = (b.n_cells / 2 + kOwn - 2) / kOwn + 1;
-    const dim3 grid((b.C + kBuildChirps - 1) / kBuildChirps, blocks, b.traj ? kVibTables : 1);
-    profile_build_kernel<false><<<grid, kBuildThreads, 0, st>>>(b, stencil, nullptr, nullptr);
-    return cudaGetLastError();
+    return launch_build<false>(b, stencil, nullptr, nullptr, b.C, b.S, blocks, b.traj ? kVibTables : 1, st);
 }
 
-cudaError_t launch_profile_build_indirect(const ProfileBuild *dev, const int *enabled, int C, int max_cells,
+cudaError_t launch_profile_build_indirect(const ProfileBuild *dev, const int *enabled, int C, int S, int max_cells,
                                           cudaStream_t st)
 {
     static const ProfileStencil stencil = make_stencil();
-    const dim3 grid((C + kBuildChirps - 1) / kBuildChirps, (max_cells / 2 + kOwn - 2) / kOwn + 1);
-    profile_build_kernel<true><<<grid, kBuildThreads, 0, st>>>(ProfileBuild{}, stencil, dev, enabled);
-    return cudaGetLastError();
+    return launch_build<true>(ProfileBuild{}, stencil, dev, enabled, C, S, (max_cells / 2 + kOwn - 2) / kOwn + 1, 1, st);
 }
 
 using ProfileFn = void (*)(const FocusJob *, const FocusUnit *, int, int *, const float2 *, float4 *);
