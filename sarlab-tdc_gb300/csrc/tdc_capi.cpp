@@ -261,9 +261,12 @@ int prepare(tdc_processor *p, const StartOpts &o, int &launches)
         TDC_CK(p->flag.ensure(64), "alloc flag");
         int *flag = p->flag.as<int>();
         TDC_CK(cudaMemsetAsync(flag, 0, 8, p->stream), "reset flag");
-        if (!p->pos64) TDC_CK(launch_rows_differ(p->pos, C, S, 3, flag, p->stream), "scan kernel");
-        if (p->vel) TDC_CK(launch_rows_differ(p->vel, C, S, 3, flag + 1, p->stream), "scan kernel");
-        if (p->att) TDC_CK(launch_rows_differ(p->att, C, S, 4, flag + 1, p->stream), "scan kernel");
+        RowScan scans[3];
+        int n_scans = 0;
+        if (!p->pos64) scans[n_scans++] = {p->pos, 3, 0};
+        if (p->vel) scans[n_scans++] = {p->vel, 3, 1};
+        if (p->att) scans[n_scans++] = {p->att, 4, 1};
+        TDC_CK(launch_rows_differ(scans, n_scans, C, S, flag, p->stream), "scan kernel");
         int differ[2] = {0, 0};
         TDC_CK(cudaMemcpyAsync(differ, flag, 8, cudaMemcpyDeviceToHost, p->stream), "read flag");
         TDC_CK(cudaEventRecord(p->ev[5], p->stream), "event");
@@ -272,7 +275,7 @@ int prepare(tdc_processor *p, const StartOpts &o, int &launches)
         TDC_CK(cudaEventSynchronize(p->ev[5]), "scan sync");
         pos_differ = differ[0] != 0;
         motion_differ = differ[1] != 0;
-        launches += (!p->pos64) + (p->vel != nullptr) + (p->att != nullptr);
+        ++launches;
     } else {
         pos_differ = !p->pos64 && !rows_constant(p->pos, C, S, 3);
         motion_differ = !rows_constant(p->vel, C, S, 3) || !rows_constant(p->att, C, S, 4);

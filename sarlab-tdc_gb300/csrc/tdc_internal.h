@@ -278,7 +278,12 @@ cudaError_t launch_chirp_positions(ChirpRec *recs, const double *base, const dou
 // Direct-read ingest (source may be pageable host memory where the device reads it coherently).
 cudaError_t launch_prewindow_from(const float2 *src, const float *w, int C, int S, int s_pad, float2 *xw,
                                   cudaStream_t st);
-cudaError_t launch_rows_differ(const float *a, int C, int S, int k, int *flag, cudaStream_t st);
+// flags[flag] |= 1 when a sample of any chirp differs (bitwise) from the chirp's first; a is [C][S][k].
+struct RowScan {
+    const float *a;
+    int k, flag;
+};
+cudaError_t launch_rows_differ(const RowScan *scans, int n, int C, int S, int *flags, cudaStream_t st);
 cudaError_t launch_tile_radius(const float4 *hi, long long P, int rows, int cols, int tile_cols, int n_tiles,
                                float *radius, cudaStream_t st);
 cudaError_t launch_grid_bbox(const float4 *hi, long long P, int *out, cudaStream_t st);

@@ -5,6 +5,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <algorithm>
+
 #include "tdc_device.cuh"
 #include "tdc_internal.h"
 
@@ -73,31 +75,60 @@ __global__ void rows_differ_kernel(const unsigned int *__restrict__ a, int C, in
     if (__syncthreads_or(differ) && threadIdx.x == 0) atomicOr(flag, 1);
 }
 
-// The same test reading 16 bytes per load (a 16-byte aligned, C x S x k < 2^31 elements):
-// the arrays usually sit in the caller's host memory, where wide loads move them faster.
-__global__ void rows_differ_vec_kernel(const uint4 *__restrict__ a4, unsigned int total, unsigned int per,
-                                       unsigned int k, int *__restrict__ flag)
+// The same test of up to three arrays (blockIdx.y) reading 16 bytes per load (16-byte aligned, C x S x k
+// < 2^31 elements, S >= 2, k of 3 or 4): all samples of a chirp equal its first exactly when
+// each equals the one before, k elements back, which lies in this lane's vector or the previous
+// lane's. A warp's first lane repeats the last vector of the warp before it instead of
+// fetching it separately. The arrays usually sit in the caller's host memory: what counts
+// is loads in flight, kScanLoads a thread.
+constexpr int kScanLoads = 4;
+struct RowScans {
+    const uint4 *a[3];
+    unsigned int total[3], per[3], k[3];
+    int flag[3];
+};
+
+__global__ void __launch_bounds__(256) rows_differ_vec_kernel(const __grid_constant__ RowScans scans, int *__restrict__ flags)
 {
-    const unsigned int *a = reinterpret_cast<const unsigned int *>(a4);
+    const int y = blockIdx.y, lane = threadIdx.x & 31;
+    const uint4 *__restrict__ a4 = scans.a[y];
+    const unsigned int total = scans.total[y], per = scans.per[y], k = scans.k[y];
     const unsigned int n4 = total / 4;
+    const unsigned int warp = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32, warps = gridDim.x * (blockDim.x / 32);
     bool differ = false;
-    for (unsigned int i = blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += gridDim.x * blockDim.x) {
-        const uint4 v = a4[i];
-        const unsigned int w[4] = {v.x, v.y, v.z, v.w};
+    // 31 new vectors a warp and load
+    for (unsigned int w0 = warp; w0 * 31u < n4; w0 += warps * kScanLoads) {
+        uint4 v[kScanLoads];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const unsigned int e = 4 * i + q;
-            const unsigned int c = e / per;
-            const unsigned int r = e - c * per;
-            differ |= w[q] != a[c * per + r % k];
+        for (int u = 0; u < kScanLoads; ++u) {
+            const unsigned int i = (w0 + u * warps) * 31u + lane;
+            v[u] = i < n4 ? __ldg(&a4[i]) : make_uint4(0u, 0u, 0u, 0u);
+        }
+#pragma unroll
+        for (int u = 0; u < kScanLoads; ++u) {
+            const unsigned int i = (w0 + u * warps) * 31u + lane;
+            const uint4 b = make_uint4(__shfl_up_sync(0xffffffffu, v[u].x, 1), __shfl_up_sync(0xffffffffu, v[u].y, 1),
+                                       __shfl_up_sync(0xffffffffu, v[u].z, 1), __shfl_up_sync(0xffffffffu, v[u].w, 1));
+            if (i >= n4) continue;
+            const unsigned int cur[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
+            // element k back of each; of a warp's first vector only what lies in it
+            const unsigned int back[4] = {k == 3 ? b.y : b.x, k == 3 ? b.z : b.y, k == 3 ? b.w : b.z,
+                                          k == 3 ? v[u].x : b.w};
+            unsigned int r = 4u * i % per;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const bool known = lane > 0 || (k == 3 && q == 3);
+                differ |= known && r >= k && cur[q] != back[q];
+                if (++r == per) r = 0;
+            }
         }
     }
-    for (unsigned int e = 4 * n4 + blockIdx.x * blockDim.x + threadIdx.x; e < total; e += gridDim.x * blockDim.x) {
-        const unsigned int c = e / per;
-        const unsigned int r = e - c * per;
-        differ |= a[e] != a[c * per + r % k];
+    if (blockIdx.x == 0 && threadIdx.x < total - 4 * n4) {
+        const unsigned int *a = reinterpret_cast<const unsigned int *>(a4);
+        const unsigned int el = 4 * n4 + threadIdx.x;
+        differ |= el % per >= k && a[el] != a[el - k];
     }
-    if (__syncthreads_or(differ) && threadIdx.x == 0) atomicOr(flag, 1);
+    if (__syncthreads_or(differ) && threadIdx.x == 0) atomicOr(&flags[scans.flag[y]], 1);
 }
 
 // out[c][s] = s * rows[c][s]: rows pre-scaled by the sample index (the adjoint's B = sum_s s x_s z^s).
@@ -296,22 +327,32 @@ cudaError_t launch_prewindow_from(const float2 *src, const float *w, int C, int 
     return cudaGetLastError();
 }
 
-cudaError_t launch_rows_differ(const float *a, int C, int S, int k, int *flag, cudaStream_t st)
+cudaError_t launch_rows_differ(const RowScan *scans, int n, int C, int S, int *flags, cudaStream_t st)
 {
-    const long long total = (long long)C * S * k;
-    if (total <= 0) return cudaSuccess;
-    if ((reinterpret_cast<uintptr_t>(a) & 15u) == 0 && total < (1LL << 31)) {
-        long long blocks = (total / 4 + 255) / 256;
-        if (blocks > 152 * 16) blocks = 152 * 16;
-        if (blocks < 1) blocks = 1;
-        rows_differ_vec_kernel<<<(unsigned)blocks, 256, 0, st>>>(reinterpret_cast<const uint4 *>(a),
-                                                                (unsigned)total, (unsigned)((long long)S * k),
-                                                                (unsigned)k, flag);
-        return cudaGetLastError();
+    RowScans vec{};
+    int n_vec = 0;
+    long long blocks = 1;
+    for (int i = 0; i < n; ++i) {
+        const RowScan &r = scans[i];
+        const long long total = (long long)C * S * r.k;
+        if (total <= 0 || S < 2) continue;
+        if ((reinterpret_cast<uintptr_t>(r.a) & 15u) == 0 && total < (1LL << 31) && (r.k == 3 || r.k == 4) && n_vec < 3) {
+            vec.a[n_vec] = reinterpret_cast<const uint4 *>(r.a);
+            vec.total[n_vec] = (unsigned)total;
+            vec.per[n_vec] = (unsigned)((long long)S * r.k);
+            vec.k[n_vec] = (unsigned)r.k;
+            vec.flag[n_vec] = r.flag;
+            blocks = std::max(blocks, (total / 4 + 256 * kScanLoads - 1) / (256 * kScanLoads));
+            ++n_vec;
+            continue;
+        }
+        const long long b = std::min<long long>((total + 255) / 256, 152 * 16);
+        rows_differ_kernel<<<(unsigned)b, 256, 0, st>>>(reinterpret_cast<const unsigned int *>(r.a), C, S, r.k,
+                                                         flags + r.flag);
+        if (const cudaError_t e = cudaGetLastError()) return e;
     }
-    long long blocks = (total + 255) / 256;
-    if (blocks > 152 * 16) blocks = 152 * 16;
-    rows_differ_kernel<<<(unsigned)blocks, 256, 0, st>>>(reinterpret_cast<const unsigned int *>(a), C, S, k, flag);
+    if (n_vec == 0) return cudaSuccess;
+    rows_differ_vec_kernel<<<dim3((unsigned)std::min<long long>(blocks, 152 * 4), n_vec), 256, 0, st>>>(vec, flags);
     return cudaGetLastError();
 }
 
