@@ -258,7 +258,7 @@ int prepare(tdc_processor *p, const StartOpts &o, int &launches)
         // The device reads the caller's per-sample arrays in place (coherent host access)
         // and reports whether any chirp's samples differ: flag[0] positions, flag[1] velocity
         // or attitude.
-        TDC_CK(p->flag.ensure(64), "alloc flag");
+        TDC_CK(p->flag.ensure(128), "alloc flag");
         int *flag = p->flag.as<int>();
         TDC_CK(cudaMemsetAsync(flag, 0, 8, p->stream), "reset flag");
         RowScan scans[3];
@@ -660,15 +660,19 @@ void set_group_reach(tdc_processor *p, const int *bits)
         std::memcpy(&f, &bits[k], 4);
         p->group_reach[k] = f;
     }
+    // runs parallel to an axis: no offset along the other two in any group (a NaN is one)
+    p->run_axis = -1;
+    for (int k = 0; k < 3; ++k)
+        if (bits[4 + (k + 1) % 3] == 0 && bits[4 + (k + 2) % 3] == 0) p->run_axis = k;
     p->reach_known = true;
 }
 
 // Reach of the anchored pixel groups of the resident grid (range profiles), measured now.
 int measure_group_reach(tdc_processor *p)
 {
-    int bits[3], *reach = p->flag.as<int>() + 10;
+    int bits[7], *reach = p->flag.as<int>() + 10;
     TDC_CK(cudaMemsetAsync(reach, 0, sizeof(bits), p->stream), "reset reach");
-    TDC_CK(launch_group_reach(p->grid_hi.as<float4>(), p->P, p->grid_run, reach, p->stream), "reach kernel");
+    TDC_CK(launch_group_reach(p->grid_hi.as<float4>(), p->grid_lo_valid ? p->grid_lo.as<float4>() : nullptr, p->P, p->grid_run, reach, p->stream), "reach kernel");
     TDC_CK(cudaMemcpyAsync(bits, reach, sizeof(bits), cudaMemcpyDeviceToHost, p->stream), "read reach");
     TDC_CK(cudaStreamSynchronize(p->stream), "reach sync");
     set_group_reach(p, bits);
@@ -782,7 +786,7 @@ int upload_grid(tdc_processor *p, int &launches)
         p->grid_lo_valid = false;
     }
     launches += 1;
-    TDC_CK(p->flag.ensure(64), "alloc flag");
+    TDC_CK(p->flag.ensure(128), "alloc flag");
     p->grid_run = detect_run(
         P, [&](long long i, int k) { return p->grid64 ? p->grid64[3 * i + k] : (double)p->grid[3 * i + k]; });
     // (small focuses do not ask for the reach: measured when a plan first does)
@@ -790,13 +794,15 @@ int upload_grid(tdc_processor *p, int &launches)
     if (P > 0) {
         // bounding box, reach and anchor span of the grid, measured on the device (the box as
         // order-preserving integer keys of the floats)
-        const int init[10] = {0x7fffffff, 0x7fffffff, 0x7fffffff, (int)0x80000000, (int)0x80000000,
-                              (int)0x80000000, 0, 0, 0, 0};
-        int keys[10];
+        const int init[13] = {0x7fffffff, 0x7fffffff, 0x7fffffff, (int)0x80000000, (int)0x80000000,
+                              (int)0x80000000, 0, 0, 0, 0, 0, 0, 0};
+        int keys[13];
         int *box = p->flag.as<int>() + 4;
         TDC_CK(cudaMemcpyAsync(box, init, sizeof(init), cudaMemcpyHostToDevice, st), "init bbox");
         if (p->reach_known)
-            TDC_CK(launch_group_reach(p->grid_hi.as<float4>(), P, p->grid_run, box + 6, st), "reach kernel");
+            TDC_CK(launch_group_reach(p->grid_hi.as<float4>(), p->grid_lo_valid ? p->grid_lo.as<float4>() : nullptr, P,
+                                      p->grid_run, box + 6, st),
+                   "reach kernel");
         TDC_CK(launch_grid_bbox(p->grid_hi.as<float4>(), P, box, st), "bbox kernel");
         TDC_CK(cudaMemcpyAsync(keys, box, sizeof(keys), cudaMemcpyDeviceToHost, st), "read bbox");
         TDC_CK(cudaStreamSynchronize(st), "grid sync");
@@ -1361,6 +1367,14 @@ int profile_group(tdc_processor *p, int path, ProfileBuild &b)
     return 1;
 }
 
+// Runs parallel to an axis whose groups span few carrier cycles (kernels with LINE).
+bool profile_line(const tdc_processor *p, int group, int path)
+{
+    const double gc = 2.0 * p->F0 / kC0 + 2.0 * p->F1 / kC0 * (p->S / 2);
+    return path == TDC_PATH_FP32_BULK && group == 8 && p->run_axis >= 0 &&
+           std::fabs(gc) * p->group_reach[0] <= kLineMaxCycles;
+}
+
 int profile_build(tdc_processor *p, const FocusPlan &plan, cudaStream_t st, int &launches)
 {
     const int S = p->S;
@@ -1516,6 +1530,7 @@ int focus_plan(tdc_processor *p, FocusPlan &plan, double max_unit_work)
     }
     unsigned char *scr = p->scratch.as<unsigned char>();
     plan.path = path;
+    plan.line = profile && profile_line(p, profile, path);
     plan.variant = variant;
     plan.seg = seg;
     plan.cb = cb;
@@ -1565,6 +1580,7 @@ int focus_plan(tdc_processor *p, FocusPlan &plan, double max_unit_work)
         job.bend2 = (float)(M_PI * h * h * gc);
         job.bend3 = (float)(2.0 * M_PI * h * h * h * g1);
         job.reach = (float)reach;
+        job.axis = std::max(0, p->run_axis);
         job.r_safe = (float)(reach / 0.03);
         plan.build = build;
     }
@@ -1651,8 +1667,8 @@ int focus_resident(tdc_processor *p, float2 *image_dev, cudaStream_t st, int &la
         p->table_epoch = p->state_epoch;
         const bool band = std::isfinite(job.half_bw);
         const int motion = plan.build.traj ? 2 : path == TDC_PATH_FP32_MOTION ? 1 : 0;
-        const int grid = std::min(n_units, p->n_sm * focus_profile_blocks_per_sm(plan.profile, band, false, motion));
-        TDC_CK(launch_focus_profile(plan.profile, band, motion, jobs_dev, units_dev, n_units, counter, grid, st),
+        const int grid = std::min(n_units, p->n_sm * focus_profile_blocks_per_sm(plan.profile, band, false, motion, plan.line));
+        TDC_CK(launch_focus_profile(plan.profile, band, motion, plan.line, jobs_dev, units_dev, n_units, counter, grid, st),
                "focus kernel (range profiles)");
     } else if (path == TDC_PATH_FP32_BULK) {
         const int grid = std::min(n_units, slots);
@@ -1723,8 +1739,8 @@ int adjoint_profile(tdc_processor *p, const FocusPlan &plan, const float2 *gimg,
     TDC_CK(cudaMemsetAsync(scr, 0, 8, st), "reset counter");
     float4 *gpart = reinterpret_cast<float4 *>(scr + off_gpart);
     const bool band = std::isfinite(plan.job.half_bw);
-    const int grid = std::min(n_units, p->n_sm * focus_profile_blocks_per_sm(plan.profile, band, true, false));
-    TDC_CK(launch_adjoint_profile(plan.profile, band, reinterpret_cast<const FocusJob *>(scr + off_job),
+    const int grid = std::min(n_units, p->n_sm * focus_profile_blocks_per_sm(plan.profile, band, true, 0, plan.line));
+    TDC_CK(launch_adjoint_profile(plan.profile, band, plan.line, reinterpret_cast<const FocusJob *>(scr + off_job),
                                   reinterpret_cast<const FocusUnit *>(scr + off_units), n_units,
                                   reinterpret_cast<int *>(scr), grid, gimg, gpart, st),
            "adjoint kernel (range profiles)");

@@ -29,6 +29,14 @@ __device__ __forceinline__ long long tile_pixel(int tile_cols, int grid_cols, lo
     return col < grid_cols && p < P ? p : -1;
 }
 
+// 1 / v to an ulp, by the special-function unit.
+__device__ __forceinline__ float rcp(float v)
+{
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
+    return r;
+}
+
 // Entry s of a row of the general kernels' per-sample tables, which keep two samples side by side: (x0, x1,
 // y0, y1)(z0, z1, w0, w1) (FocusJob::traj).
 __device__ __forceinline__ float4 sample_table(const float4 *row, int s)

@@ -64,14 +64,6 @@ constexpr int kTile = kT * kPT;
 constexpr int kStages = 2;
 static_assert(kTile == kFocusTile, "work units tile the grid like the FP32-bulk kernel");
 
-// 1 / v to an ulp, by the special-function unit.
-__device__ __forceinline__ float rcp(float v)
-{
-    float r;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
-    return r;
-}
-
 __device__ __forceinline__ float2 both(float v) { return make_float2(v, v); }
 __device__ __forceinline__ float2 neg(float2 v) { return make_float2(-v.x, -v.y); }
 

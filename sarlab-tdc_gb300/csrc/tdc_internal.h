@@ -180,7 +180,8 @@ struct __align__(16) ProfileJob {
     const int *cell_base;      // [C] absolute index of each chirp's first cell
     float inv_gc;              // 1 / gc
     float reach;               // largest distance of a pixel from its anchor [m]
-    float pad_[2];
+    int axis;                  // axis the runs are parallel to (kernels with LINE)
+    float pad_;
     // smooth motion: cells per (m / sample) of range rate, 4 S gc; with h = S / 2, the bend of the
     // phase at the row's ends is bend1 a + bend2 (|W1|^2 - a^2) / R + 2 bend2 e.V2 / R radians
     // (a = e.W1 / R), and its cubic part bend3 d2R/ds2 / 2
@@ -221,6 +222,9 @@ constexpr int kProfileCtasPerSm = TDC_PROFILE_CTAS;
 #endif
 constexpr int kProfileMinUnitsPerSlot = TDC_PROFILE_MIN_UNITS;
 constexpr int kProfileBandMinUnitsPerSlot = 8;  // (units differ in their live chirps)
+
+// Groups of at most this many carrier cycles take their phase unreduced (kernels with LINE).
+constexpr double kLineMaxCycles = 4.5;
 
 // Inputs and outputs of profile_build_kernel.
 struct ProfileBuild {
@@ -342,14 +346,14 @@ cudaError_t launch_profile_build_indirect(const ProfileBuild *dev, const int *en
                                           cudaStream_t st);
 // motion: 1, the records are MoveRec, every sample of a chirp at a range of its own; 2, they are
 // VibRec and there are kVibTables tables.
-cudaError_t launch_focus_profile(int group, bool band, int motion, const FocusJob *jobs_dev, const FocusUnit *units_dev, int n_units,
+cudaError_t launch_focus_profile(int group, bool band, int motion, bool line, const FocusJob *jobs_dev, const FocusUnit *units_dev, int n_units,
                                  int *counter_dev, int grid_ctas, cudaStream_t st);
 // Its adjoint: gpart[tile][C] = (d/dx, d/dy, d/dz) of each chirp over the tile's pixels (sums of
 // Re(conj(G) dI/dR) (P - T) / R; .w is not written).
-cudaError_t launch_adjoint_profile(int group, bool band, const FocusJob *jobs_dev, const FocusUnit *units_dev,
+cudaError_t launch_adjoint_profile(int group, bool band, bool line, const FocusJob *jobs_dev, const FocusUnit *units_dev,
                                    int n_units, int *counter_dev, int grid_ctas, const float2 *gimg, float4 *gpart,
                                    cudaStream_t st);
-int focus_profile_blocks_per_sm(int group, bool band, bool adjoint, int motion);
+int focus_profile_blocks_per_sm(int group, bool band, bool adjoint, int motion, bool line);
 // Straight-line fit of every chirp's offsets (FocusJob::traj, chirps with sample-0 positions) and the
 // principal direction of what it leaves, as VibRec; maxima[0..2] = max(maxima, largest deviation,
 // deviation off that direction, |W1|) as float bits (starting at 0; NaN above all).
@@ -357,7 +361,7 @@ cudaError_t launch_vib_fit(const float4 *traj, const ChirpRec *chirps, int C, in
                            VibRec *recs, int *maxima, cudaStream_t st);
 // out[0..2] = max(out, largest distance of a pixel from the anchor of its group of 8 / 4 / 2
 // consecutive pixels of a run) as float bits (out starts at 0; a NaN compares above any distance).
-cudaError_t launch_group_reach(const float4 *hi, long long P, int run, int *out, cudaStream_t st);
+cudaError_t launch_group_reach(const float4 *hi, const float4 *lo, long long P, int run, int *out, cudaStream_t st);
 
 // Adjoint of the FP32-bulk focus w.r.t. per-chirp position offsets: per-(tile, chirp)
 // float4 partials, then an FP64 sum over tiles into grad[C][3]. stored: job.xw holds the

@@ -307,7 +307,7 @@ int enqueue(const tdc_noalloc_focus_args *a, float *image_dev, cudaStream_t st, 
         const double gc = a->g0 + a->g1 * (S / 2), cells_per_m = 4.0 * S * a->g1;
         const int tiles = (int)profile_tiles(P, (int)std::min<long long>(P, 1 << 30));
         // two units per CTA, partials in at most a third of the array
-        const int pslots = n_sm * focus_profile_blocks_per_sm(1, band, false, false);
+        const int pslots = n_sm * focus_profile_blocks_per_sm(1, band, false, 0, false);
         const long long fit = (long long)(TDC_NOALLOC_SCRATCH_BYTES / 3) / (P * 16);
         int pg = (int)std::max<long long>(1, std::min<long long>({(long long)C, fit, (2LL * pslots + tiles - 1) / tiles}));
         const int pcpg = (C + pg - 1) / pg;
@@ -371,9 +371,9 @@ int enqueue(const tdc_noalloc_focus_args *a, float *image_dev, cudaStream_t st, 
         if (e == cudaSuccess)
             e = launch_profile_build_indirect(pp.build_out, words + kWordProfile, C, S, pp.max_cells, st);
         const int n = pp.n_tiles * pp.n_groups;
-        const int ctas = std::min(n, n_sm * focus_profile_blocks_per_sm(1, band, false, false));
+        const int ctas = std::min(n, n_sm * focus_profile_blocks_per_sm(1, band, false, 0, false));
         if (e == cudaSuccess)
-            e = launch_focus_profile(1, band, false, pp.job_out, pp.units, n, words + kWordProfileCounter, ctas, st);
+            e = launch_focus_profile(1, band, 0, false, pp.job_out, pp.units, n, words + kWordProfileCounter, ctas, st);
         if (e == cudaSuccess)
             e = launch_focus_reduce(pp.job.partial, pp.n_groups, P, reinterpret_cast<float2 *>(image_dev), st,
                                     words + kWordProfile, 1);

@@ -225,9 +225,12 @@ __global__ void tile_radius_kernel(const float4 *__restrict__ hi, long long P, i
 
 // Reach of the anchored pixel groups of the range-profile focus: the largest distance from a
 // group's anchor (its middle pixel) to its other pixels, for groups of 8, 4 and 2 consecutive
-// pixels of a run; one thread per 8 pixels of a run.
-__global__ void group_reach_kernel(const float4 *__restrict__ hi, long long P, int run, int *__restrict__ out)
+// pixels of a run (out[0..2]), and the largest offset along each axis in the groups of 8 (out[4..6]);
+// one thread per 8 pixels of a run.
+__global__ void group_reach_kernel(const float4 *__restrict__ hi, const float4 *__restrict__ lo, long long P, int run,
+                                   int *__restrict__ out)
 {
+    float spread[3] = {0.f, 0.f, 0.f};
     const int per = (run + 7) / 8;
     const long long n = (P / run) * per + (P % run + 7) / 8;
     float reach[3] = {0.f, 0.f, 0.f};
@@ -241,11 +244,16 @@ __global__ void group_reach_kernel(const float4 *__restrict__ hi, long long P, i
             for (int s = 0; s < valid; s += g) {
                 const int m = min(g, valid - s);
                 const float4 a = hi[p0 + s + m / 2];
+                const float4 b = lo ? lo[p0 + s + m / 2] : make_float4(0.f, 0.f, 0.f, 0.f);
                 for (int i = 0; i < m; ++i) {
                     const float4 v = hi[p0 + s + i];
                     const float dx = v.x - a.x, dy = v.y - a.y, dz = v.z - a.z;
                     const float d = sqrtf(dx * dx + dy * dy + dz * dz);
                     reach[k] = d > reach[k] || d != d ? d : reach[k];
+                    if (k) continue;
+                    const float4 l = lo ? lo[p0 + s + i] : b;
+                    const float o[3] = {fabsf(dx + (l.x - b.x)), fabsf(dy + (l.y - b.y)), fabsf(dz + (l.z - b.z))};
+                    for (int x = 0; x < 3; ++x) spread[x] = o[x] > spread[x] || o[x] != o[x] ? o[x] : spread[x];
                 }
             }
         }
@@ -253,6 +261,8 @@ __global__ void group_reach_kernel(const float4 *__restrict__ hi, long long P, i
     for (int k = 0; k < 3; ++k) {
         const int v = __reduce_max_sync(0xffffffffu, __float_as_int(fabsf(reach[k])));
         if ((threadIdx.x & 31) == 0 && v > 0) atomicMax(&out[k], v);
+        const int w = __reduce_max_sync(0xffffffffu, __float_as_int(fabsf(spread[k])));
+        if ((threadIdx.x & 31) == 0 && w > 0) atomicMax(&out[4 + k], w);
     }
 }
 
@@ -384,13 +394,13 @@ cudaError_t launch_tile_radius(const float4 *hi, long long P, int rows, int cols
     return cudaGetLastError();
 }
 
-cudaError_t launch_group_reach(const float4 *hi, long long P, int run, int *out, cudaStream_t st)
+cudaError_t launch_group_reach(const float4 *hi, const float4 *lo, long long P, int run, int *out, cudaStream_t st)
 {
     if (P <= 0 || run <= 0) return cudaSuccess;
     long long blocks = (P / 8 + 255) / 256;
     if (blocks > 152 * 8) blocks = 152 * 8;
     if (blocks < 1) blocks = 1;
-    group_reach_kernel<<<(unsigned)blocks, 256, 0, st>>>(hi, P, run, out);
+    group_reach_kernel<<<(unsigned)blocks, 256, 0, st>>>(hi, lo, P, run, out);
     return cudaGetLastError();
 }
 

@@ -198,7 +198,8 @@ struct tdc_processor {
     // the groups of 8 / 4 / 2 pixels sharing an anchor, the table and the per-length constants.
     int grid_run = 1;
     double group_reach[3] = {0, 0, 0};
-    bool reach_known = false;  // group_reach is the resident grid's
+    int run_axis = -1;         // axis the runs are parallel to, or -1
+    bool reach_known = false;  // group_reach and run_axis are the resident grid's
     tdc::impl::DevBuf cells, cell_base, twiddle;
     double table_ratio = 0.0;  // largest table taken, in bytes per byte of samples (0: no limit)
     uint64_t table_epoch = 0;  // state_epoch the table was built at by a focus (0: none)
@@ -267,6 +268,7 @@ struct FocusPlan {
     bool anchored = false;  // FP32-bulk kernel with anchored ranges
     int profile = 0;      // FP32-bulk focus through range profiles: pixels sharing an anchor (8, 4, 2, 1); else 0
     ProfileBuild build{};  // its table (profile > 0)
+    bool line = false;     // ... through the kernels for runs parallel to an axis
     size_t off_job = 0;   // job record and unit table offsets in the processor's scratch
     size_t off_units = 0;
     FocusJob job{};       // partial -> the processor's scratch

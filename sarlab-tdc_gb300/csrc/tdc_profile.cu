@@ -584,17 +584,26 @@ struct Anchor {
     float2 a[kProfileCoefs];
 };
 
+// turn + 2 pi psi [rad], psi modulo one cycle unless SMALL (the sincos's argument is then rounded at up
+// to 2 pi kLineMaxCycles + pi: 1e-6 rad rms at a group's edge, 5e-7 over it).
+template <bool SMALL>
+__device__ __forceinline__ float2 phase_of(float2 psi, float turn)
+{
+    if (SMALL) return __ffma2_rn(psi, both(kTwoPiF), both(turn));
+    const float2 n = __fadd2_rn(__fadd2_rn(psi, both(12582912.0f)), both(-12582912.0f));  // nearest integer
+    return __ffma2_rn(__fadd2_rn(psi, make_float2(-n.x, -n.y)), both(kTwoPiF), both(turn));
+}
+
 // One chirp's contributions to two pixels with phase differences psi (cycles) from their
 // anchor: e^{j (turn + 2 pi psi)} A(t0 + psi cells_per_cycle), A the cell's polynomial with
 // coefficients a, times its window (WEIGHTED). Real and imaginary part of the value h advance together; the product with
 // the phasor is kept as h cos and h sin (c_i, s_i) and combined when the sums are flushed.
-template <bool WEIGHTED>
+template <bool WEIGHTED, bool LINE>
 __device__ __forceinline__ void add_pair(float2 psi, float turn, float t0, float cells_per_cycle,
                                          const float2 (&a)[kProfileCoefs], float w0, float w1, float2 &c0, float2 &s0, float2 &c1,
                                          float2 &s1)
 {
-    const float2 n = __fadd2_rn(__fadd2_rn(psi, both(12582912.0f)), both(-12582912.0f));  // nearest integer
-    const float2 x = __ffma2_rn(__fadd2_rn(psi, make_float2(-n.x, -n.y)), both(kTwoPiF), both(turn));
+    const float2 x = phase_of<LINE>(psi, turn);
     const float2 t = __ffma2_rn(psi, both(cells_per_cycle), both(t0));
     float sn0, cs0, sn1, cs1;
     __sincosf(x.x, &sn0, &cs0);
@@ -805,13 +814,13 @@ __device__ __forceinline__ void adjoint_coefs(const float2 (&a)[kProfileCoefs], 
 // One chirp's terms of the adjoint for two pixels: with D = (dF/dR) / (j 2 pi gc e^{j phase}) given
 // by the coefficients d, gi the image gradient (re, im) and range = R, adds
 // dl = Im(conj(gi) e^{j phase} D) / R and dl x offset to the sums.
+template <bool LINE>
 __device__ __forceinline__ void adjoint_pair(float2 psi, float turn, float t0, float cells_per_cycle,
                                              const float2 (&d)[kProfileCoefs - 1], float w0, float w1, float2 g0,
                                              float2 g1, float2 range, float2 dx, float2 dy, float2 dz, float2 &s,
                                              float2 &sx, float2 &sy, float2 &sz)
 {
-    const float2 n = __fadd2_rn(__fadd2_rn(psi, both(12582912.0f)), both(-12582912.0f));
-    const float2 x = __ffma2_rn(__fadd2_rn(psi, make_float2(-n.x, -n.y)), both(kTwoPiF), both(turn));
+    const float2 x = phase_of<LINE>(psi, turn);
     const float2 t = __ffma2_rn(psi, both(cells_per_cycle), both(t0));
     float sn0, cs0, sn1, cs1;
     __sincosf(x.x, &sn0, &cs0);
@@ -831,6 +840,7 @@ __device__ __forceinline__ void adjoint_pair(float2 psi, float turn, float t0, f
                                   w1 * __fdividef(p1 * h1.x - q1 * h1.y, range.y));
     s = __fadd2_rn(s, dl);
     sx = __ffma2_rn(dl, dx, sx);
+    if (LINE) return;  // (offsets along one axis only)
     sy = __ffma2_rn(dl, dy, sy);
     sz = __ffma2_rn(dl, dz, sz);
 }
@@ -883,7 +893,13 @@ __device__ __forceinline__ void adjoint_pair(float2 psi, float turn, float t0, f
 // the phi tables, a pixel's own direction as the polynomial's gradient in u, to first order.
 // 151 x 97 pixels x 333 chirps x 500 samples: 1930 us in the general kernel of tdc_general.cu, which
 // corrects every sample, 120 us here (57 the six tables, 57 this kernel).
-template <int G, bool BAND, bool ADJ, int MOVE>
+//
+// LINE: every group's pixels lie on a line parallel to one axis (sP.axis; checked when the grid is
+// measured: the offsets along the others are exactly zero) and span at most kLineMaxCycles carrier
+// cycles. The offsets are one number a pixel, in registers: Q = d (e' + d h) in 2 operations, and
+// the phase needs no reduction: 5 operations of 45 a pixel and chirp less (1024^2 x 4096 x 1024: 6.52 ->
+// 6.06 ms; adjoint and finite band likewise 7-10%).
+template <int G, bool BAND, bool ADJ, int MOVE, bool LINE>
 __global__ void __launch_bounds__(kThreads, MOVE == 2 ? 4 : G == 1 ? (BAND || ADJ ? 4 : 6) : BAND || MOVE || (ADJ && G == 2) ? 6 : TDC_PROFILE_MINB)
     profile_focus_kernel(const FocusJob *__restrict__ jobs, const FocusUnit *__restrict__ units, int n_units,
                          int *__restrict__ counter, const float2 *__restrict__ gimg, float4 *__restrict__ gpart)
@@ -891,6 +907,7 @@ __global__ void __launch_bounds__(kThreads, MOVE == 2 ? 4 : G == 1 ? (BAND || AD
     constexpr int kSub = kPT / G;  // anchors per thread
     __shared__ SharedSums sums;
     static_assert(!MOVE || (!BAND && !ADJ), "smooth motion: unbounded band, forward only");
+    static_assert(!LINE || (G > 1 && !MOVE), "runs along an axis: still antennas, shared anchors");
     constexpr int kWords = MOVE == 2 ? 6 : MOVE ? 4 : BAND ? 3 : 2;  // float4 staged per record
     constexpr int kStride = MOVE ? kWords : 3;                      // float4 per record in memory
     __shared__ __align__(16) SharedChirps<kWords> recs[2];
@@ -917,6 +934,8 @@ __global__ void __launch_bounds__(kThreads, MOVE == 2 ? 4 : G == 1 ? (BAND || AD
 
         const int c0 = un.group * sJ.chirps_per_group;
         const int c1 = min(sJ.C, c0 + sJ.chirps_per_group);
+        const int axis = LINE ? sP.axis : 0;
+        auto along = [&](float x, float y, float z) { return axis == 0 ? x : axis == 1 ? y : z; };
 
         // anchors (the middle pixel of each group) and the pixels' offsets from them, in pairs
         float ax[kSub][6];
@@ -955,6 +974,10 @@ __global__ void __launch_bounds__(kThreads, MOVE == 2 ? 4 : G == 1 ? (BAND || AD
 #pragma unroll
                 for (int i = 0; i + 1 < G; i += 2) {
                     const int q = (g * G + i) / 2;
+                    if (LINE) {
+                        dx[q] = make_float2(along(ox[i], oy[i], oz[i]), along(ox[i + 1], oy[i + 1], oz[i + 1]));
+                        continue;
+                    }
                     dx[q] = make_float2(ox[i], ox[i + 1]);
                     dy[q] = make_float2(oy[i], oy[i + 1]);
                     const float2 dz = make_float2(oz[i], oz[i + 1]);
@@ -1163,9 +1186,11 @@ __global__ void __launch_bounds__(kThreads, MOVE == 2 ? 4 : G == 1 ? (BAND || AD
                             for (int i = 0; i < G / 2; ++i) {
                                 const int s = g * (G / 2) + i;
                                 const float2 q =
-                                    __ffma2_rn(dx[s], both(e2x),
-                                               __ffma2_rn(dy[s], both(e2y),
-                                                          __ffma2_rn(fresh2(&sums.dz[s][tid]), both(e2z), __fmul2_rn(fresh2(&sums.dd[s][tid]), both(h)))));
+                                    LINE ? __fmul2_rn(dx[s], __ffma2_rn(dx[s], both(h), both(along(e2x, e2y, e2z))))
+                                         : __ffma2_rn(dx[s], both(e2x),
+                                                      __ffma2_rn(dy[s], both(e2y),
+                                                                 __ffma2_rn(fresh2(&sums.dz[s][tid]), both(e2z),
+                                                                            __fmul2_rn(fresh2(&sums.dd[s][tid]), both(h)))));
                                 float2 f = __ffma2_rn(q, both(b3), both(b2));
                                 f = __ffma2_rn(q, f, both(b1));
                                 psi[i] = __ffma2_rn(__fmul2_rn(q, q), f, q);
@@ -1175,8 +1200,15 @@ __global__ void __launch_bounds__(kThreads, MOVE == 2 ? 4 : G == 1 ? (BAND || AD
 #pragma unroll
                             for (int i = 0; i < G; ++i) {
                                 const int s = (g * G + i) / 2;
-                                const float x = i & 1 ? dx[s].y : dx[s].x, y = i & 1 ? dy[s].y : dy[s].x,
-                                            z = i & 1 ? sums.dz[s][tid].y : sums.dz[s][tid].x;
+                                float x = i & 1 ? dx[s].y : dx[s].x, y, z;
+                                if (LINE) {
+                                    y = axis == 1 ? x : 0.f;
+                                    z = axis == 2 ? x : 0.f;
+                                    x = axis == 0 ? x : 0.f;
+                                } else {
+                                    y = i & 1 ? dy[s].y : dy[s].x;
+                                    z = i & 1 ? sums.dz[s][tid].y : sums.dz[s][tid].x;
+                                }
                                 const float vx = cur.ex - x, vy = cur.ey - y, vz = cur.ez - z;
                                 const float num = fmaf(x, fmaf(-2.0f, cur.ex, x),
                                                        fmaf(y, fmaf(-2.0f, cur.ey, y), z * fmaf(-2.0f, cur.ez, z)));
@@ -1211,9 +1243,10 @@ __global__ void __launch_bounds__(kThreads, MOVE == 2 ? 4 : G == 1 ? (BAND || AD
                             for (int i = 0; i < G; i += 2) {
                                 const int s = (g * G + i) / 2;
                                 const float2 dot =
-                                    __ffma2_rn(dx[s], both(tx),
-                                               __ffma2_rn(dy[s], both(ty),
-                                                          __ffma2_rn(fresh2(&sums.dz[s][tid]), both(tz), both(te))));
+                                    LINE ? __ffma2_rn(dx[s], both(along(tx, ty, tz)), both(te))
+                                         : __ffma2_rn(dx[s], both(tx),
+                                                      __ffma2_rn(dy[s], both(ty),
+                                                                 __ffma2_rn(fresh2(&sums.dz[s][tid]), both(tz), both(te))));
                                 const float2 r = __ffma2_rn(psi[i / 2], both(sP.inv_gc), both(cur.rh));
 #pragma unroll
                                 for (int q = 0; q < 2; ++q) {
@@ -1262,15 +1295,25 @@ __global__ void __launch_bounds__(kThreads, MOVE == 2 ? 4 : G == 1 ? (BAND || AD
                                 float2 r = __ffma2_rn(psi[i / 2], both(sP.inv_gc), both(cur.rh));
                                 if (zero >> i & 1u) r.x = 1.0f;
                                 if (zero >> (i + 1) & 1u) r.y = 1.0f;
-                                adjoint_pair(psi[i / 2], cur.turn, cur.t0, jc.y, d, w[i], w[i + 1], gi[g * G + i],
-                                             gi[g * G + i + 1], r, dx[s], dy[s], fresh2(&sums.dz[s][tid]), sum, sx, sy,
-                                             sz);
+                                float2 oy = both(0.f), oz = oy;
+                                if (!LINE) {
+                                    oy = dy[s];
+                                    oz = fresh2(&sums.dz[s][tid]);
+                                }
+                                adjoint_pair<LINE>(psi[i / 2], cur.turn, cur.t0, jc.y, d, w[i], w[i + 1], gi[g * G + i],
+                                                   gi[g * G + i + 1], r, dx[s], oy, oz, sum, sx, sy, sz);
                             }
                             // sum over the pixels of dl (e - d)
                             const float all = sum.x + sum.y;
-                            grad[0] += fmaf(all, cur.ex, -(sx.x + sx.y));
-                            grad[1] += fmaf(all, cur.ey, -(sy.x + sy.y));
-                            grad[2] += fmaf(all, cur.ez, -(sz.x + sz.y));
+                            float bx = sx.x + sx.y, by = sy.x + sy.y, bz = sz.x + sz.y;
+                            if (LINE) {
+                                by = axis == 1 ? bx : 0.f;
+                                bz = axis == 2 ? bx : 0.f;
+                                bx = axis == 0 ? bx : 0.f;
+                            }
+                            grad[0] += fmaf(all, cur.ex, -bx);
+                            grad[1] += fmaf(all, cur.ey, -by);
+                            grad[2] += fmaf(all, cur.ez, -bz);
                             continue;
                         }
                         if constexpr (MOVE) {
@@ -1296,7 +1339,7 @@ __global__ void __launch_bounds__(kThreads, MOVE == 2 ? 4 : G == 1 ? (BAND || AD
                                                                          __ffma2_rn(fresh2(&sums.dz[q][tid]),
                                                                                     both(-w1.z), both(ew))));
                                 const float2 r = __ffma2_rn(psi[i / 2], both(sP.inv_gc), both(cur.rh));
-                                float2 ri = make_float2(__frcp_rn(r.x), __frcp_rn(r.y));
+                                float2 ri = make_float2(rcp(r.x), rcp(r.y));
                                 if (zero) {
                                     if (zero >> i & 1u) ri.x = 0.f;
                                     if (zero >> (i + 1) & 1u) ri.y = 0.f;
@@ -1333,7 +1376,7 @@ __global__ void __launch_bounds__(kThreads, MOVE == 2 ? 4 : G == 1 ? (BAND || AD
 #pragma unroll
                         for (int i = 0; i < G; i += 2) {
                             const int s = g * G + i;
-                            add_pair<BAND>(psi[i / 2], cur.turn, cur.t0, jc.y, cur.a, w[i], w[i + 1], hc[s], hs[s], hc[s + 1],
+                            add_pair<BAND, LINE>(psi[i / 2], cur.turn, cur.t0, jc.y, cur.a, w[i], w[i + 1], hc[s], hs[s], hc[s + 1],
                                            hs[s + 1]);
                         }
                         if (!BAND && !ADJ && zero) {
@@ -1442,15 +1485,17 @@ template <bool BAND, bool ADJ, int MOVE>
 static ProfileFn profile_fn(int group)
 {
     switch (group) {
-    case 8: return profile_focus_kernel<8, BAND, ADJ, MOVE>;
-    case 4: return profile_focus_kernel<4, BAND, ADJ, MOVE>;
-    case 2: return profile_focus_kernel<2, BAND, ADJ, MOVE>;
-    default: return profile_focus_kernel<1, BAND, ADJ, MOVE>;
+    case 8: return profile_focus_kernel<8, BAND, ADJ, MOVE, false>;
+    case 4: return profile_focus_kernel<4, BAND, ADJ, MOVE, false>;
+    case 2: return profile_focus_kernel<2, BAND, ADJ, MOVE, false>;
+    default: return profile_focus_kernel<1, BAND, ADJ, MOVE, false>;
     }
 }
 
-static ProfileFn profile_fn(int group, bool band, bool adjoint, int motion)
+static ProfileFn profile_fn(int group, bool band, bool adjoint, int motion, bool line)
 {
+    if (line && adjoint) return band ? profile_focus_kernel<8, true, true, 0, true> : profile_focus_kernel<8, false, true, 0, true>;
+    if (line) return band ? profile_focus_kernel<8, true, false, 0, true> : profile_focus_kernel<8, false, false, 0, true>;
     if (motion == 2) return profile_fn<false, false, 2>(group);
     if (motion) return profile_fn<false, false, 1>(group);
     if (adjoint) return band ? profile_fn<true, true, 0>(group) : profile_fn<false, true, 0>(group);
@@ -1464,29 +1509,29 @@ cudaError_t launch_vib_fit(const float4 *traj, const ChirpRec *chirps, int C, in
     return cudaGetLastError();
 }
 
-cudaError_t launch_focus_profile(int group, bool band, int motion, const FocusJob *jobs_dev,
+cudaError_t launch_focus_profile(int group, bool band, int motion, bool line, const FocusJob *jobs_dev,
                                  const FocusUnit *units_dev, int n_units, int *counter_dev, int grid_ctas,
                                  cudaStream_t st)
 {
     if (band && motion) return cudaErrorInvalidValue;
-    profile_fn(group, band, false, motion)<<<grid_ctas, kThreads, 0, st>>>(jobs_dev, units_dev, n_units, counter_dev,
+    profile_fn(group, band, false, motion, line)<<<grid_ctas, kThreads, 0, st>>>(jobs_dev, units_dev, n_units, counter_dev,
                                                                            nullptr, nullptr);
     return cudaGetLastError();
 }
 
-cudaError_t launch_adjoint_profile(int group, bool band, const FocusJob *jobs_dev, const FocusUnit *units_dev,
+cudaError_t launch_adjoint_profile(int group, bool band, bool line, const FocusJob *jobs_dev, const FocusUnit *units_dev,
                                    int n_units, int *counter_dev, int grid_ctas, const float2 *gimg, float4 *gpart,
                                    cudaStream_t st)
 {
-    profile_fn(group, band, true, 0)<<<grid_ctas, kThreads, 0, st>>>(jobs_dev, units_dev, n_units, counter_dev,
+    profile_fn(group, band, true, 0, line)<<<grid_ctas, kThreads, 0, st>>>(jobs_dev, units_dev, n_units, counter_dev,
                                                                          gimg, gpart);
     return cudaGetLastError();
 }
 
-int focus_profile_blocks_per_sm(int group, bool band, bool adjoint, int motion)
+int focus_profile_blocks_per_sm(int group, bool band, bool adjoint, int motion, bool line)
 {
     int blocks = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, profile_fn(group, band, adjoint, motion), kThreads, 0) !=
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, profile_fn(group, band, adjoint, motion, line), kThreads, 0) !=
         cudaSuccess)
         return 0;
     return blocks;

@@ -116,6 +116,7 @@ constexpr double kAging = TDC_SERVER_AGING;
 // batched (the FP64 general path: focused alone on the side stream).
 int job_kind(const FocusPlan &pl)
 {
+    if (pl.line) return std::isfinite(pl.job.half_bw) ? 12 : 11;
     if (pl.profile)
         return 3 + (pl.profile == 8 ? 3 : pl.profile == 4 ? 2 : pl.profile == 2 ? 1 : 0) +
                (std::isfinite(pl.job.half_bw) ? 4 : 0);
@@ -459,7 +460,7 @@ void tdc_server::launch_batch()
     const bool general = kind >= 16;
     const int profile = members[0]->plan.profile;
     const int variant = general ? members[0]->plan.variant : 0;
-    const int bps = profile    ? focus_profile_blocks_per_sm(profile, skip_zero, false, false)
+    const int bps = profile    ? focus_profile_blocks_per_sm(profile, skip_zero, false, 0, members[0]->plan.line)
                     : general  ? focus_general_blocks_per_sm(variant, stage_bytes)
                     : seg      ? focus_fp32_seg_blocks_per_sm(stage_bytes)
                     : anchored ? focus_fp32_anchor_blocks_per_sm(stage_bytes)
@@ -470,7 +471,7 @@ void tdc_server::launch_batch()
     const FocusUnit *units_d = reinterpret_cast<const FocusUnit *>(d + off_units);
     int *counter_d = reinterpret_cast<int *>(d);
     if (profile)
-        err |= launch_focus_profile(profile, skip_zero, false, jobs_d, units_d, (int)n_units, counter_d, grid, st) != cudaSuccess;
+        err |= launch_focus_profile(profile, skip_zero, 0, members[0]->plan.line, jobs_d, units_d, (int)n_units, counter_d, grid, st) != cudaSuccess;
     else if (general)
         err |= launch_focus_general(variant, jobs_d, units_d, (int)n_units, counter_d, counter_d + 1, stage_bytes, grid,
                                     st) != cudaSuccess;
