@@ -17,7 +17,7 @@
 // fits the array. The host knows neither the grid's extent nor the trajectory, so a kernel
 // decides from the inputs on the device (noalloc_decide_kernel): both forms are enqueued, and
 // the one not taken finds its work counter already past its last unit. 200 x 150 pixels x 300
-// chirps x 256 samples: 395 -> 174 us.
+// chirps x 256 samples: 395 -> 138 us.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -93,39 +93,44 @@ struct ProfilePlan {
 // Whether range profiles apply, from the grid's bounding box (words, from grid_bbox_kernel) and
 // the chirp records, as the processor decides it from its host copies: finite inputs, a grid
 // within the unambiguous range, ranges the cell index resolves, a table that fits. Fills in the
-// build inputs and leaves one of the two work counters spent. One block.
+// build inputs and leaves one of the two work counters spent: the first block, with the farthest range in
+// FP32 (FP64 runs at 1/64 of its rate); the others write the unit table.
 __global__ void noalloc_decide_kernel(ProfilePlan plan, int *__restrict__ words, bool band)
 {
-    __shared__ double far2[256];
+    __shared__ float far2[8];
     __shared__ float box[6];
     const int tid = threadIdx.x;
+    if (blockIdx.x > 0) {
+        const int n = plan.n_tiles * plan.n_groups;
+        for (int u = (blockIdx.x - 1) * blockDim.x + tid; u < n; u += (gridDim.x - 1) * blockDim.x)
+            plan.units[u] = FocusUnit{0, u % plan.n_tiles, u / plan.n_tiles, 0};
+        return;
+    }
     if (tid < 6) {
         const int key = words[kWordBox + tid];
         box[tid] = __int_as_float(key >= 0 ? key : key ^ 0x7fffffff);
     }
     __syncthreads();
-    double most = 0.0;
+    float most = 0.f;
     bool finite = true;
     const ChirpRec *recs = reinterpret_cast<const ChirpRec *>(plan.build.chirps);
     for (int c = tid; c < plan.build.C; c += blockDim.x) {
         const ChirpRec r = recs[c];
-        double f = 0.0;
-        const double p[3] = {(double)r.p_hi.x + r.p_lo.x, (double)r.p_hi.y + r.p_lo.y, (double)r.p_hi.z + r.p_lo.z};
+        float f = 0.f;
+        const float p[3] = {r.p_hi.x, r.p_hi.y, r.p_hi.z};
         for (int k = 0; k < 3; ++k) {
-            const double d = fmax(fabs(box[k] - p[k]), fabs(p[k] - box[3 + k]));
+            const float d = fmaxf(fabsf(box[k] - p[k]), fabsf(p[k] - box[3 + k]));
             f += d * d;
         }
-        finite = finite && f < 1e30 &&
+        finite = finite && f < 1e30f && isfinite(r.p_lo.x + r.p_lo.y + r.p_lo.z) &&
                  (band || (isfinite(r.vel.x) && isfinite(r.vel.y) && isfinite(r.vel.z) && isfinite(r.p_hi.w)));
-        most = fmax(most, f);
+        most = fmaxf(most, f);
     }
-    far2[tid] = most;
+    most = __int_as_float(__reduce_max_sync(0xffffffffu, __float_as_int(most)));
+    if ((tid & 31) == 0) far2[tid >> 5] = most;
     finite = __syncthreads_and(finite);
-    for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-        if (tid < s) far2[tid] = fmax(far2[tid], far2[tid + s]);
-        __syncthreads();
-    }
     if (tid) return;
+    for (int w = 1; w < 8; ++w) far2[0] = fmaxf(far2[0], far2[w]);
     ProfileBuild &b = plan.build;
     double diag2 = 0.0;
     for (int k = 0; k < 3; ++k) {
@@ -134,7 +139,7 @@ __global__ void noalloc_decide_kernel(ProfilePlan plan, int *__restrict__ words,
         diag2 += (b.box_max[k] - b.box_min[k]) * (b.box_max[k] - b.box_min[k]);
     }
     const double span = fabs(b.cells_per_m) * sqrt(diag2);
-    const bool take = finite && diag2 < 1e30 && fabs(b.cells_per_m) * sqrt(far2[0]) < 2097152.0 &&
+    const bool take = finite && diag2 < 1e30 && fabs(b.cells_per_m) * (1.0f + 1e-6f) * sqrtf(far2[0]) < 2097152.0 &&
                       span + 7.0 <= (double)plan.max_cells && span + 7.0 <= 4.0 * b.S;
     if (take) {
         b.n_cells = ((int)ceil(span) + 7) / 2 * 2;
@@ -145,13 +150,6 @@ __global__ void noalloc_decide_kernel(ProfilePlan plan, int *__restrict__ words,
     words[kWordProfile] = take;
     words[kWordCounter] = take ? kSpent : 0;
     words[kWordProfileCounter] = take ? 0 : kSpent;
-}
-
-__global__ void noalloc_units_kernel(FocusUnit *units, int n_tiles, int n_groups)
-{
-    const int n = n_tiles * n_groups;
-    for (int u = blockIdx.x * blockDim.x + threadIdx.x; u < n; u += gridDim.x * blockDim.x)
-        units[u] = FocusUnit{0, u % n_tiles, u / n_tiles, 0};
 }
 
 int fail(int code, const std::string &msg) { return set_last_error(code, msg); }
@@ -362,8 +360,7 @@ int enqueue(const tdc_noalloc_focus_args *a, float *image_dev, cudaStream_t st, 
     if (profile) {
         e = launch_grid_bbox(job.grid_hi, P, words + kWordBox, st);
         if (e == cudaSuccess) {
-            noalloc_decide_kernel<<<1, 256, 0, st>>>(pp, words, band);
-            noalloc_units_kernel<<<8, 256, 0, st>>>(pp.units, pp.n_tiles, pp.n_groups);
+            noalloc_decide_kernel<<<9, 256, 0, st>>>(pp, words, band);
             e = cudaGetLastError();
         }
         if (e == cudaSuccess)
