@@ -660,6 +660,9 @@ void set_group_reach(tdc_processor *p, const int *bits)
         std::memcpy(&f, &bits[k], 4);
         p->group_reach[k] = f;
     }
+    float f16;
+    std::memcpy(&f16, &bits[7], 4);
+    p->reach16 = f16;
     // runs parallel to an axis: no offset along the other two in any group (a NaN is one)
     p->run_axis = -1;
     for (int k = 0; k < 3; ++k)
@@ -670,7 +673,7 @@ void set_group_reach(tdc_processor *p, const int *bits)
 // Reach of the anchored pixel groups of the resident grid (range profiles), measured now.
 int measure_group_reach(tdc_processor *p)
 {
-    int bits[7], *reach = p->flag.as<int>() + 10;
+    int bits[8], *reach = p->flag.as<int>() + 10;
     TDC_CK(cudaMemsetAsync(reach, 0, sizeof(bits), p->stream), "reset reach");
     TDC_CK(launch_group_reach(p->grid_hi.as<float4>(), p->grid_lo_valid ? p->grid_lo.as<float4>() : nullptr, p->P, p->grid_run, reach, p->stream), "reach kernel");
     TDC_CK(cudaMemcpyAsync(bits, reach, sizeof(bits), cudaMemcpyDeviceToHost, p->stream), "read reach");
@@ -794,9 +797,9 @@ int upload_grid(tdc_processor *p, int &launches)
     if (P > 0) {
         // bounding box, reach and anchor span of the grid, measured on the device (the box as
         // order-preserving integer keys of the floats)
-        const int init[13] = {0x7fffffff, 0x7fffffff, 0x7fffffff, (int)0x80000000, (int)0x80000000,
-                              (int)0x80000000, 0, 0, 0, 0, 0, 0, 0};
-        int keys[13];
+        const int init[14] = {0x7fffffff, 0x7fffffff, 0x7fffffff, (int)0x80000000, (int)0x80000000,
+                              (int)0x80000000};
+        int keys[14];
         int *box = p->flag.as<int>() + 4;
         TDC_CK(cudaMemcpyAsync(box, init, sizeof(init), cudaMemcpyHostToDevice, st), "init bbox");
         if (p->reach_known)
@@ -1261,6 +1264,9 @@ constexpr double kVibMaxPhase = 0.1, kVibMaxSide = 5e-4, kVibMaxBow = 3e-5, kVib
 
 // Smooth motion through range profiles: largest bend of the phase at a row's ends [rad].
 constexpr double kMoveMaxBend = 0.1;
+// Groups of 16: ranges of at least this many reaches take the short series of the range difference; focuses
+// of at least this many pixels x chirps.
+constexpr double kWideRange = 21.0, kWideMinPairs = 6e7;
 // ... of the phase's third order there (left out, weighted by s~^3) [rad],
 constexpr double kMoveMaxThird = 8e-6;
 // ... and of the bend's difference within a group [rad] (the neglected second order is half its square).
@@ -1353,6 +1359,13 @@ int profile_group(tdc_processor *p, int path, ProfileBuild &b)
     if (!p->reach_known && measure_group_reach(p)) return 0;
     if (!std::isfinite(p->group_reach[0])) return 0;
     if (!p->anchor_enabled) return 1;
+    // 16 pixels a thread and anchor on runs parallel to an axis, once half as many threads are enough: whole
+    // focus at 16 / 8, 1 mm grids x 256 samples: 17 M pairs (256^2 x 256) 84 / 76 us, 67 M (256^2 x 1024) 145 /
+    // 158, 67 M (512^2 x 256) 152 / 156, 300 M (600 x 500 x 1000) 441 / 533, 1074 M (512^2 x 4096) 1397 /
+    // 1579. Under a finite band 16 leave 8 warps an SM: 1024^2 x 4096 x 1024, 3.01 / 2.57 ms.
+    if (path == TDC_PATH_FP32_BULK && !band && p->table_ratio <= 0.0 && p->run_axis >= 0 && (double)P * p->C >= kWideMinPairs &&
+        std::fabs(b.cells_per_m) * p->reach16 <= kProfileReach - 0.52 && std::fabs(gc) * p->reach16 <= kLineMaxCycles)
+        return 16;
     // |t| <= 1/2 (the anchor's place in its cell) + the group's reach
     for (int k = 0; k < 3; ++k)
     {
@@ -1371,8 +1384,8 @@ int profile_group(tdc_processor *p, int path, ProfileBuild &b)
 bool profile_line(const tdc_processor *p, int group, int path)
 {
     const double gc = 2.0 * p->F0 / kC0 + 2.0 * p->F1 / kC0 * (p->S / 2);
-    return path == TDC_PATH_FP32_BULK && group == 8 && p->run_axis >= 0 &&
-           std::fabs(gc) * p->group_reach[0] <= kLineMaxCycles;
+    return group == 16 || (path == TDC_PATH_FP32_BULK && group == 8 && p->run_axis >= 0 &&
+                           std::fabs(gc) * p->group_reach[0] <= kLineMaxCycles);
 }
 
 int profile_build(tdc_processor *p, const FocusPlan &plan, cudaStream_t st, int &launches)
@@ -1451,13 +1464,14 @@ int focus_plan(tdc_processor *p, FocusPlan &plan, double max_unit_work)
 
     const int tile_cols = profile ? 0 : choose_tile_cols(p);
     const int run = profile ? p->grid_run : 0;
-    const long long n_tiles = profile ? profile_tiles(P, run) : tile_count(P, tile_cols, p->cols);
+    const int each = profile == 16 ? 16 : kProfilePixels;
+    const long long n_tiles = profile ? profile_tiles(P, run, each) : tile_count(P, tile_cols, p->cols);
     // (block tiles also depend on the grid's shape, not only on its pixel count)
     const int plan_cols = tile_cols ? p->cols : 0;
     // The chirp groups (each pixel's summation order) follow the grid the job is planned for:
     // its own, or a larger one whose row block this grid is (pixel sharding across GPUs).
     const long long plan_tiles = p->plan_pixels <= P ? n_tiles
-                                 : profile           ? profile_tiles(p->plan_pixels, run)
+                                 : profile           ? profile_tiles(p->plan_pixels, run, each)
                                                      : tile_count(p->plan_pixels, tile_cols, p->cols);
     if (path != p->plan_path || P != p->plan_P || C != p->plan_C || slots != p->plan_slots ||
         max_unit_work != p->plan_unit_cap || tile_cols != p->plan_tile_cols || plan_cols != p->plan_cols ||
@@ -1569,7 +1583,8 @@ int focus_plan(tdc_processor *p, FocusPlan &plan, double max_unit_work)
         split_dd(build.cells_per_m, job.cells_hi, job.cells_lo);
         job.cells_per_cycle = (float)(build.cells_per_m / gc);
         job.inv_gc2x4 = (float)(4.0 / (gc * gc));
-        const double reach = profile == 8   ? p->group_reach[0]
+        const double reach = profile == 16  ? p->reach16
+                             : profile == 8 ? p->group_reach[0]
                              : profile == 4 ? p->group_reach[1]
                              : profile == 2 ? p->group_reach[2]
                                             : 0.0;
@@ -1581,7 +1596,7 @@ int focus_plan(tdc_processor *p, FocusPlan &plan, double max_unit_work)
         job.bend3 = (float)(2.0 * M_PI * h * h * h * g1);
         job.reach = (float)reach;
         job.axis = std::max(0, p->run_axis);
-        job.r_safe = (float)(reach / 0.03);
+        job.r_safe = (float)(profile == 16 ? kWideRange * reach : reach / 0.03);
         plan.build = build;
     }
     // narrow variants take the phase correction in radians

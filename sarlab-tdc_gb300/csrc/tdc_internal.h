@@ -248,9 +248,9 @@ struct ProfileBuild {
 // Tiles of a P-pixel grid whose runs are `run` pixels long: groups of kProfilePixels
 // consecutive pixels of a run, kProfileThreads groups a tile (in bands of kProfileBand runs).
 constexpr int kProfileBand = 8;
-inline long long profile_tiles(long long P, int run)
+inline long long profile_tiles(long long P, int run, int pixels = kProfilePixels)
 {
-    const long long per = (run + kProfilePixels - 1) / kProfilePixels;
+    const long long per = (run + pixels - 1) / pixels;
     const long long groups = (P + run - 1) / run * per;
     return (groups + kProfileThreads - 1) / kProfileThreads;
 }

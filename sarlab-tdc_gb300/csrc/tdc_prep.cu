@@ -225,12 +225,12 @@ __global__ void tile_radius_kernel(const float4 *__restrict__ hi, long long P, i
 
 // Reach of the anchored pixel groups of the range-profile focus: the largest distance from a
 // group's anchor (its middle pixel) to its other pixels, for groups of 8, 4 and 2 consecutive
-// pixels of a run (out[0..2]), and the largest offset along each axis in the groups of 8 (out[4..6]);
-// one thread per 8 pixels of a run.
+// pixels of a run (out[0..2]) and of 16 (out[7]), and the largest offset along each axis in the groups of
+// 16 (out[4..6]); one thread per 8 pixels of a run.
 __global__ void group_reach_kernel(const float4 *__restrict__ hi, const float4 *__restrict__ lo, long long P, int run,
                                    int *__restrict__ out)
 {
-    float spread[3] = {0.f, 0.f, 0.f};
+    float spread[4] = {0.f, 0.f, 0.f, 0.f};
     const int per = (run + 7) / 8;
     const long long n = (P / run) * per + (P % run + 7) / 8;
     float reach[3] = {0.f, 0.f, 0.f};
@@ -244,25 +244,33 @@ __global__ void group_reach_kernel(const float4 *__restrict__ hi, const float4 *
             for (int s = 0; s < valid; s += g) {
                 const int m = min(g, valid - s);
                 const float4 a = hi[p0 + s + m / 2];
-                const float4 b = lo ? lo[p0 + s + m / 2] : make_float4(0.f, 0.f, 0.f, 0.f);
                 for (int i = 0; i < m; ++i) {
                     const float4 v = hi[p0 + s + i];
                     const float dx = v.x - a.x, dy = v.y - a.y, dz = v.z - a.z;
                     const float d = sqrtf(dx * dx + dy * dy + dz * dz);
                     reach[k] = d > reach[k] || d != d ? d : reach[k];
-                    if (k) continue;
-                    const float4 l = lo ? lo[p0 + s + i] : b;
-                    const float o[3] = {fabsf(dx + (l.x - b.x)), fabsf(dy + (l.y - b.y)), fabsf(dz + (l.z - b.z))};
-                    for (int x = 0; x < 3; ++x) spread[x] = o[x] > spread[x] || o[x] != o[x] ? o[x] : spread[x];
                 }
             }
         }
+        if (col & 15) continue;
+        const int valid16 = (int)min((long long)min(16, run - col), P - p0);
+        const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f), a = hi[p0 + valid16 / 2],
+                     b = lo ? lo[p0 + valid16 / 2] : zero;
+        for (int i = 0; i < valid16; ++i) {
+            const float4 v = hi[p0 + i], l = lo ? lo[p0 + i] : zero;
+            const float x = fabsf((v.x - a.x) + (l.x - b.x)), y = fabsf((v.y - a.y) + (l.y - b.y)),
+                        z = fabsf((v.z - a.z) + (l.z - b.z));
+            const float o[4] = {x, y, z, sqrtf(x * x + y * y + z * z)};
+            for (int d = 0; d < 4; ++d) spread[d] = o[d] > spread[d] || o[d] != o[d] ? o[d] : spread[d];
+        }
+    }
+    for (int d = 0; d < 4; ++d) {
+        const int v = __reduce_max_sync(0xffffffffu, __float_as_int(fabsf(spread[d])));
+        if ((threadIdx.x & 31) == 0 && v > 0) atomicMax(&out[4 + d], v);
     }
     for (int k = 0; k < 3; ++k) {
         const int v = __reduce_max_sync(0xffffffffu, __float_as_int(fabsf(reach[k])));
         if ((threadIdx.x & 31) == 0 && v > 0) atomicMax(&out[k], v);
-        const int w = __reduce_max_sync(0xffffffffu, __float_as_int(fabsf(spread[k])));
-        if ((threadIdx.x & 31) == 0 && w > 0) atomicMax(&out[4 + k], w);
     }
 }
 

@@ -197,7 +197,7 @@ struct tdc_processor {
     // Range profiles (tdc_profile.cu): consecutive pixels without a jump (a grid row), the reach of
     // the groups of 8 / 4 / 2 pixels sharing an anchor, the table and the per-length constants.
     int grid_run = 1;
-    double group_reach[3] = {0, 0, 0};
+    double group_reach[3] = {0, 0, 0}, reach16 = 0;
     int run_axis = -1;         // axis the runs are parallel to, or -1
     bool reach_known = false;  // group_reach and run_axis are the resident grid's
     tdc::impl::DevBuf cells, cell_base, twiddle;

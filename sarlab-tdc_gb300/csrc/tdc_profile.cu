@@ -116,11 +116,15 @@ __global__ void profile_twiddle_kernel(float2 *__restrict__ tw, float *__restric
     if (i >= (long long)S * kNodes) return;
     const int s = (int)(i / kNodes), n = (int)(i - (long long)s * kNodes);
     const long long nn = 2LL * S, d = s - S / 2;
-    long long r = (n * d) % nn;
-    if (r < 0) r += nn;
-    double sn, cs;
-    sincospi(2.0 * (double)r / (double)nn, &sn, &cs);
-    tw[i] = make_float2((float)cs, (float)sn);
+    int r = n * (int)d % (int)nn;  // (rows of up to 2^24 samples)
+    if (r < 0) r += (int)nn;
+    if (r > S) r -= (int)nn;
+    // r / nn as a double-float pair, so that the sincos's rounding is all that is left (FP64: 142 us
+    // for 12345 samples)
+    const float fn = (float)nn, ratio = (float)r / fn, rest = fmaf(-ratio, fn, (float)r) / fn;
+    float sn, cs;
+    sincospif(2.0f * ratio, &sn, &cs);
+    tw[i] = make_float2(fmaf(-kTwoPiF * rest, sn, cs), fmaf(kTwoPiF * rest, cs, sn));
     if (n == 0) {
         const double q2 = 0.5 * kKbWidth * 2.0 * 3.14159265358979323846 * (double)d / (double)nn;
         const double q = sqrt(kKbBeta * kKbBeta - q2 * q2);
@@ -490,12 +494,17 @@ constexpr int kFlush = kProfileBlock;                         // chirps summed i
 // terms 1/8 and -5/64, with 7/128 y^4 replaced by its best multiple of y^2 there, 0.828 Y^2 y^2
 // (error below 1.3e-7 at the end of the range, 4e-8 at 0.045, vanishing with y).
 constexpr float kRootRange = 0.061f;
+// The same to y^4 for groups of 16, |y| <= 0.1 (reach / R <= 1 / 21; 6e-8 left), the y^5 term
+// economised: y^5 = 5/4 Y^2 y^3 - 5/16 Y^4 y within Y^5 / 16.
+constexpr float kWide1 = -0.25f + 21.0f / 512.0f * 0.3125f * 1e-4f, kWide2 = 0.125f,
+                kWide3 = -5.0f / 64.0f - 21.0f / 512.0f * 1.25f * 1e-2f, kWide4 = 7.0f / 128.0f;
 constexpr float kRoot2 = 0.125f + 7.0f / 128.0f * 0.828f * kRootRange * kRootRange, kRoot3 = -5.0f / 64.0f;
 
+template <int PT>
 struct SharedSums {
-    float4 s[kPT][kThreads];       // (sum.re, sum.im, comp.re, comp.im)
-    float2 dz[kPT / 2][kThreads];  // z offsets and |d|^2 of the thread's pixel pairs
-    float2 dd[kPT / 2][kThreads];
+    float4 s[PT][kThreads];       // (sum.re, sum.im, comp.re, comp.im)
+    float2 dz[PT / 2][kThreads];  // z offsets and |d|^2 of the thread's pixel pairs
+    float2 dd[PT / 2][kThreads];
 };
 
 // Chirp records of kFlush chirps at a time (position high and low; the velocity with a finite
@@ -507,7 +516,8 @@ struct SharedChirps {
 };
 
 // Kahan step of pixel i's sums: + sum over chirps of (cos + j sin) h, given as sum h cos, sum h sin.
-__device__ __forceinline__ void stash(SharedSums &sums, int i, int tid, float2 hc, float2 hs)
+template <int PT>
+__device__ __forceinline__ void stash(SharedSums<PT> &sums, int i, int tid, float2 hc, float2 hs)
 {
     float4 s = sums.s[i][tid];
     const float yr = (hc.x - hs.y) - s.z, yi = (hc.y + hs.x) - s.w;
@@ -525,9 +535,10 @@ __device__ __forceinline__ void stash(SharedSums &sums, int i, int tid, float2 h
 // down the runs of a band of 8 runs, then along it: a warp covers a block of 8 runs x 32
 // pixels, whose ranges, and so the cells it reads, lie closer together than 256 pixels of one
 // run's do.
+template <int PT>
 __device__ __forceinline__ long long run_pixels(long long P, int run, int t, int tid, int &count)
 {
-    const int per_run = (run + kPT - 1) / kPT;
+    const int per_run = (run + PT - 1) / PT;
     const long long runs = (P + run - 1) / run;
     const long long q = (long long)t * kThreads + tid;
     const long long band = q / ((long long)kProfileBand * per_run);
@@ -535,9 +546,9 @@ __device__ __forceinline__ long long run_pixels(long long P, int run, int t, int
     const int height = (int)min((long long)kProfileBand, runs - band * kProfileBand);
     count = 0;
     if (height <= 0) return 0;
-    const int col = rem / height * kPT;
+    const int col = rem / height * PT;
     const long long p = (band * kProfileBand + rem % height) * run + col;
-    if (col < run && p < P) count = (int)min((long long)min(kPT, run - col), P - p);
+    if (col < run && p < P) count = (int)min((long long)min(PT, run - col), P - p);
     return p;
 }
 
@@ -900,14 +911,16 @@ __device__ __forceinline__ void adjoint_pair(float2 psi, float turn, float t0, f
 // the phase needs no reduction: 5 operations of 45 a pixel and chirp less (1024^2 x 4096 x 1024: 6.52 ->
 // 6.06 ms; adjoint and finite band likewise 7-10%).
 template <int G, bool BAND, bool ADJ, int MOVE, bool LINE>
-__global__ void __launch_bounds__(kThreads, MOVE == 2 ? 4 : G == 1 ? (BAND || ADJ ? 4 : 6) : BAND || MOVE || (ADJ && G == 2) ? 6 : TDC_PROFILE_MINB)
+__global__ void __launch_bounds__(kThreads, G == 16 ? (ADJ ? 4 : 6) : MOVE == 2 ? 4 : G == 1 ? (BAND || ADJ ? 4 : 6) : BAND || MOVE || (ADJ && G == 2) ? 6 : TDC_PROFILE_MINB)
     profile_focus_kernel(const FocusJob *__restrict__ jobs, const FocusUnit *__restrict__ units, int n_units,
                          int *__restrict__ counter, const float2 *__restrict__ gimg, float4 *__restrict__ gpart)
 {
-    constexpr int kSub = kPT / G;  // anchors per thread
-    __shared__ SharedSums sums;
+    constexpr int PT = G == 16 ? 16 : kPT;  // pixels per thread
+    constexpr int kSub = PT / G;            // anchors per thread
+    __shared__ SharedSums<PT> sums;
     static_assert(!MOVE || (!BAND && !ADJ), "smooth motion: unbounded band, forward only");
     static_assert(!LINE || (G > 1 && !MOVE), "runs along an axis: still antennas, shared anchors");
+    static_assert(G < 16 || (LINE && !BAND), "groups of 16: runs along an axis, unbounded band");
     constexpr int kWords = MOVE == 2 ? 6 : MOVE ? 4 : BAND ? 3 : 2;  // float4 staged per record
     constexpr int kStride = MOVE ? kWords : 3;                      // float4 per record in memory
     __shared__ __align__(16) SharedChirps<kWords> recs[2];
@@ -939,9 +952,9 @@ __global__ void __launch_bounds__(kThreads, MOVE == 2 ? 4 : G == 1 ? (BAND || AD
 
         // anchors (the middle pixel of each group) and the pixels' offsets from them, in pairs
         float ax[kSub][6];
-        float2 dx[kPT / 2], dy[kPT / 2];
+        float2 dx[PT / 2], dy[PT / 2];
         int count;
-        long long p0 = run_pixels(sJ.P, sJ.grid_cols, un.tile, tid, count);
+        long long p0 = run_pixels<PT>(sJ.P, sJ.grid_cols, un.tile, tid, count);
 #pragma unroll
         for (int g = 0; g < kSub; ++g) {
             const int valid = min(max(count - g * G, 0), G);
@@ -986,17 +999,17 @@ __global__ void __launch_bounds__(kThreads, MOVE == 2 ? 4 : G == 1 ? (BAND || AD
                 }
             }
         }
-        float2 hc[kPT], hs[kPT];  // (hs stays zero where a pixel is its own anchor)
+        float2 hc[PT], hs[PT];  // (hs stays zero where a pixel is its own anchor)
 #pragma unroll
-        for (int i = 0; i < kPT; ++i) {
+        for (int i = 0; i < PT; ++i) {
             hc[i] = hs[i] = make_float2(0.f, 0.f);
             sums.s[i][tid] = make_float4(0.f, 0.f, 0.f, 0.f);
         }
 
-        float2 gi[kPT];  // (ADJ) image gradient of the pixels
+        float2 gi[PT];  // (ADJ) image gradient of the pixels
         auto load_gradient = [&](unsigned int without) {
 #pragma unroll
-            for (int i = 0; i < kPT; ++i)
+            for (int i = 0; i < PT; ++i)
                 gi[i] = i < count && !(without >> i & 1u) ? __ldg(&gimg[p0 + i]) : make_float2(0.f, 0.f);
         };
         if (ADJ) load_gradient(0);
@@ -1074,7 +1087,7 @@ __global__ void __launch_bounds__(kThreads, MOVE == 2 ? 4 : G == 1 ? (BAND || AD
                 const int k = b0 / sJ.chunk;
                 chunk_end = (k + 1) * sJ.chunk;
                 dropped = 0;
-                p0 = run_pixels(sJ.P, sJ.grid_cols, un.tile, tid, count);  // (cheaper than two registers)
+                p0 = run_pixels<PT>(sJ.P, sJ.grid_cols, un.tile, tid, count);  // (cheaper than two registers)
                 const float4 pf = __ldg(&sJ.skip[(size_t)k * 9].pos_fdc);
                 const float4 v = __ldg(&sJ.skip[(size_t)k * 9].vel);
 #pragma unroll 1
@@ -1172,6 +1185,66 @@ __global__ void __launch_bounds__(kThreads, MOVE == 2 ? 4 : G == 1 ? (BAND || AD
                         for (int m = kProfileCoefs - 2; m >= 0; --m) h = __ffma2_rn(h, both(cur.t0), a[m]);
                         hc[g].x = fmaf(cs, h.x, fmaf(-sn, h.y, hc[g].x));
                         hc[g].y = fmaf(cs, h.y, fmaf(sn, h.x, hc[g].y));
+                    } else if constexpr (G == 16 && !ADJ) {
+                        // (as below, each pair's phase difference formed where it is used: 16 at once do not
+                        // fit the registers)
+                        const float4 jc = fresh(&sP.inv_gc2x4);
+                        const float ea = along(cur.ex, cur.ey, cur.ez);
+                        if (cur.rh >= jc.z) {
+                            const float h = cur.h, e2 = -2.0f * h * ea, k2 = h * jc.x;
+                            const float b1 = kWide1 * k2, b2 = kWide2 * k2 * k2, b3 = kWide3 * k2 * k2 * k2,
+                                        b4 = kWide4 * (k2 * k2) * (k2 * k2);
+#pragma unroll
+                            for (int i = 0; i < G; i += 2) {
+                                const float2 q = __fmul2_rn(dx[i / 2], __ffma2_rn(dx[i / 2], both(h), both(e2)));
+                                float2 f = __ffma2_rn(q, both(b4), both(b3));
+                                f = __ffma2_rn(q, f, both(b2));
+                                f = __ffma2_rn(q, f, both(b1));
+                                add_pair<false, true>(__ffma2_rn(__fmul2_rn(q, q), f, q), cur.turn, cur.t0, jc.y, cur.a,
+                                                      1.f, 1.f, hc[i], hs[i], hc[i + 1], hs[i + 1]);
+                            }
+                        } else if (cur.rh >= jc.z * (10.0f / 21.0f)) {
+                            // |y| <= 0.2: the Taylor series to y^7, 6e-8 left
+                            const float h = cur.h, e2 = -2.0f * h * ea, k2 = h * jc.x;
+#pragma unroll
+                            for (int i = 0; i < G; i += 2) {
+                                const float2 q = __fmul2_rn(dx[i / 2], __ffma2_rn(dx[i / 2], both(h), both(e2)));
+                                const float2 y = __fmul2_rn(q, both(k2));
+                                float2 f = __ffma2_rn(y, both(-429.0f / 16384.0f), both(33.0f / 1024.0f));
+                                f = __ffma2_rn(y, f, both(-21.0f / 512.0f));
+                                f = __ffma2_rn(y, f, both(7.0f / 128.0f));
+                                f = __ffma2_rn(y, f, both(-5.0f / 64.0f));
+                                f = __ffma2_rn(y, f, both(0.125f));
+                                f = __ffma2_rn(y, f, both(-0.25f));
+                                add_pair<false, true>(__ffma2_rn(__fmul2_rn(q, y), f, q), cur.turn, cur.t0, jc.y, cur.a, 1.f,
+                                                      1.f, hc[i], hs[i], hc[i + 1], hs[i + 1]);
+                            }
+                        } else {
+                            // e's part off the axis, squared
+                            const float sx = axis == 0 ? 0.f : cur.ex, sy = axis == 1 ? 0.f : cur.ey,
+                                        sz = axis == 2 ? 0.f : cur.ez;
+                            const float off2 = fmaf(sx, sx, fmaf(sy, sy, sz * sz));
+#pragma unroll
+                            for (int i = 0; i < G; i += 2) {
+                                float2 psi;
+                                bool on[2];
+#pragma unroll
+                                for (int j = 0; j < 2; ++j) {
+                                    const float x = j ? dx[i / 2].y : dx[i / 2].x, v = ea - x;
+                                    const float r2 = fmaf(v, v, off2), den = cur.rh + sqrtf(r2);
+                                    const float d = den > 0.0f ? sP.gc_hi * (x * fmaf(-2.0f, ea, x) / den) : 0.0f;
+                                    if (j) psi.y = d;
+                                    else psi.x = d;
+                                    on[j] = !(r2 > 0.0f);  // (the antenna on the pixel: NaN Doppler, zero window)
+                                    if (on[j] && !(dropped >> (i + j) & 1u)) stash(sums, i + j, tid, hc[i + j], hs[i + j]);
+                                }
+                                add_pair<false, true>(psi, cur.turn, cur.t0, jc.y, cur.a, 1.f, 1.f, hc[i], hs[i], hc[i + 1],
+                                                      hs[i + 1]);
+#pragma unroll
+                                for (int j = 0; j < 2; ++j)
+                                    if (on[j]) hc[i + j] = hs[i + j] = make_float2(0.f, 0.f);
+                            }
+                        }
                     } else {
                         float2 psi[G / 2];
                         unsigned int zero = 0;  // pixels the antenna stands on
@@ -1180,8 +1253,10 @@ __global__ void __launch_bounds__(kThreads, MOVE == 2 ? 4 : G == 1 ? (BAND || AD
                             const float h = cur.h, h2 = -2.0f * h;
                             const float e2x = h2 * cur.ex, e2y = h2 * cur.ey, e2z = h2 * cur.ez;
                             const float k2 = h * jc.x;
-                            const float b1 = -0.25f * k2, b2 = kRoot2 * k2 * k2;
-                            const float b3 = kRoot3 * k2 * k2 * k2;
+                            constexpr bool kWide = G == 16;
+                            const float b1 = (kWide ? kWide1 : -0.25f) * k2, b2 = (kWide ? kWide2 : kRoot2) * k2 * k2;
+                            const float b3 = (kWide ? kWide3 : kRoot3) * k2 * k2 * k2;
+                            const float b4 = kWide4 * (k2 * k2) * (k2 * k2);
 #pragma unroll
                             for (int i = 0; i < G / 2; ++i) {
                                 const int s = g * (G / 2) + i;
@@ -1191,7 +1266,8 @@ __global__ void __launch_bounds__(kThreads, MOVE == 2 ? 4 : G == 1 ? (BAND || AD
                                                       __ffma2_rn(dy[s], both(e2y),
                                                                  __ffma2_rn(fresh2(&sums.dz[s][tid]), both(e2z),
                                                                             __fmul2_rn(fresh2(&sums.dd[s][tid]), both(h)))));
-                                float2 f = __ffma2_rn(q, both(b3), both(b2));
+                                float2 f = kWide ? __ffma2_rn(q, both(b4), both(b3)) : both(b3);
+                                f = __ffma2_rn(q, f, both(b2));
                                 f = __ffma2_rn(q, f, both(b1));
                                 psi[i] = __ffma2_rn(__fmul2_rn(q, q), f, q);
                             }
@@ -1262,7 +1338,7 @@ __global__ void __launch_bounds__(kThreads, MOVE == 2 ? 4 : G == 1 ? (BAND || AD
                                 const int i = __ffs(edge) - 1;
                                 edge &= edge - 1;
                                 int m;
-                                const long long p = run_pixels(sJ.P, sJ.grid_cols, un.tile, tid, m) + g * G + i;
+                                const long long p = run_pixels<PT>(sJ.P, sJ.grid_cols, un.tile, tid, m) + g * G + i;
                                 const float4 ph = recs[buf].p[k][0], pl = recs[buf].p[k][1];
                                 const float4 hi = g * G + i < m ? __ldg(&sJ.grid_hi[p]) : ph;
                                 const float4 lo = g * G + i < m && sJ.grid_lo ? __ldg(&sJ.grid_lo[p])
@@ -1410,7 +1486,7 @@ __global__ void __launch_bounds__(kThreads, MOVE == 2 ? 4 : G == 1 ? (BAND || AD
             }
             // the plain sums of these chirps (of one skip-test chunk) into the Kahan sums
 #pragma unroll
-            for (int i = 0; i < (ADJ ? 0 : kPT); ++i) {
+            for (int i = 0; i < (ADJ ? 0 : PT); ++i) {
                 if (!(dropped >> i & 1u)) stash(sums, i, tid, hc[i], hs[i]);
                 hc[i] = hs[i] = make_float2(0.f, 0.f);
             }
@@ -1419,10 +1495,10 @@ __global__ void __launch_bounds__(kThreads, MOVE == 2 ? 4 : G == 1 ? (BAND || AD
         }
 
         if (ADJ) continue;
-        p0 = run_pixels(sJ.P, sJ.grid_cols, un.tile, tid, count);
+        p0 = run_pixels<PT>(sJ.P, sJ.grid_cols, un.tile, tid, count);
         float4 *__restrict__ part = sJ.partial + (size_t)un.group * sJ.P;
 #pragma unroll
-        for (int i = 0; i < kPT; ++i)
+        for (int i = 0; i < PT; ++i)
             if (i < count) part[p0 + i] = sums.s[i][tid];
     }
 }
@@ -1494,6 +1570,10 @@ static ProfileFn profile_fn(int group)
 
 static ProfileFn profile_fn(int group, bool band, bool adjoint, int motion, bool line)
 {
+    if (line && group == 16) {
+        if (adjoint) return profile_focus_kernel<16, false, true, 0, true>;
+        return profile_focus_kernel<16, false, false, 0, true>;
+    }
     if (line && adjoint) return band ? profile_focus_kernel<8, true, true, 0, true> : profile_focus_kernel<8, false, true, 0, true>;
     if (line) return band ? profile_focus_kernel<8, true, false, 0, true> : profile_focus_kernel<8, false, false, 0, true>;
     if (motion == 2) return profile_fn<false, false, 2>(group);

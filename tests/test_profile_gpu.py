@@ -291,3 +291,77 @@ def test_profile_focus_of_vibration(cuda_device, nx, ny, n_pri, n_samples, spaci
     ref = oracle.focus(prob, oracle.Opts(applyRangeWin=False, dopplerBandwidth=INF), pixels=pix)
     err = rel_l2(img[pix], ref)
     assert err <= 5e-6, err
+
+
+def _axis_grid(sc, axis):
+    """The scene's ground plane with its runs along x, or its rows and columns exchanged (along y)."""
+    return sc.grid if axis == 0 else np.ascontiguousarray(sc.grid.transpose(1, 0, 2))
+
+
+@pytest.mark.parametrize("nx,ny,n_pri,spacing,height,axis,group", [
+    (333, 200, 1000, 1e-3, 0.3, 0, 16),   # ragged groups, a last band of runs, 1.3 groups a tile
+    (200, 333, 1000, 1e-3, 0.3, 1, 16),   # runs along y
+    (320, 256, 800, 0.7e-3, 0.12, 0, 16),  # ranges from 0.12 m: the long series
+    (256, 320, 800, 1e-3, 0.03, 1, 16),   # ranges too short for any series
+    (256, 320, 800, 1.5e-3, 0.3, 0, 8),   # 16 span too many cycles
+    (75, 130, 200, 1e-3, 0.3, 1, 8),      # too few pairs
+    (75, 130, 200, 1e-3, 0.02, 1, 8),
+])
+def test_profile_focus_of_runs_along_an_axis(cuda_device, nx, ny, n_pri, spacing, height, axis, group):
+    """Tolerance 4e-6: the 3e-6 above, and 1.5e-6 of phases at up to 4.5 cycles unreduced."""
+    import _sarlabtdc
+
+    sc = scenes.small_scene(seed=nx + n_pri, n_pri=n_pri, n_samples=160, nx=nx, ny=ny, spacing=spacing, height=height,
+                            y0=0.02 if height < 0.2 else 0.2, device="cuda")
+    api = sc.api_arrays()
+    grid = _axis_grid(sc, axis).astype(np.float32)
+    p = _sarlabtdc.TdcProcessor(0)
+    p.setRawData(*api.values())
+    p.setFocusGrid(grid)
+    p.start(0.0, INF, False, False, True)
+    img, st = p.getFocusedImage().ravel(), p.lastStats()
+    assert st["stage_samples"] == 0 and st["anchor_pixels"] == group
+    cols = grid.shape[1]
+    pix = np.unique(np.concatenate([[0, 15, 16, cols - 1, cols, img.size - 1],
+                                    np.random.default_rng(5).choice(img.size, 60, replace=False)]))
+    prob = oracle.Problem(raw=api["rawData"], sampleTimes=api["sampleTimes"], position=api["position"],
+                          velocity=api["velocity"], attitude=api["attitude"], modRate=api["modRate"],
+                          startFreq=api["startFreq"], grid=grid)
+    ref = oracle.focus(prob, oracle.Opts(applyRangeWin=False, dopplerBandwidth=INF), pixels=pix)
+    assert np.all(np.isfinite(img))
+    err = rel_l2(img[pix], ref)
+    assert err <= 4e-6, err
+
+
+@pytest.mark.parametrize("axis,band,n_pri", [(0, INF, 1000), (1, INF, 1000), (1, INF, 300), (0, 14.0, 300), (1, 14.0, 300)])
+def test_profile_adjoint_of_runs_along_an_axis(cuda_device, axis, band, n_pri):
+    """Groups of 16 and 8 against every pixel's range in double-float (checked against the oracle
+    above): 4e-6 and 3e-6 of either, relative L2 7e-6."""
+    import torch
+
+    import _sarlabtdc
+
+    sc = scenes.small_scene(seed=31, n_pri=n_pri, n_samples=160, nx=301, ny=210, spacing=1e-3, rail_len=0.5,
+                            jitter=0.2e-3, device="cuda")
+    api = sc.api_arrays()
+    vel = np.zeros_like(api["velocity"])
+    vel[..., 0] = 0.08
+    api["velocity"] = vel
+    grid = _axis_grid(sc, axis)
+    n = grid.shape[0] * grid.shape[1]
+    rng = np.random.default_rng(12)
+    g_d = torch.from_numpy((rng.normal(size=n) + 1j * rng.normal(size=n)).astype(np.complex64)).cuda()
+    grads = []
+    for anchored in (True, False):
+        p = _sarlabtdc.TdcProcessor(0)
+        p.setRawData(*api.values())
+        p.setChirpPositionsF64(sc.positions)
+        p.setFocusGridF64(grid)
+        p.setAnchoredRanges(anchored)
+        p.prepare(0.0, band, False, False, True)
+        p.uploadGrid()
+        grad = torch.empty((sc.n_pri, 3), dtype=torch.float64, device="cuda")
+        p.adjointDevice(g_d, grad)
+        grads.append(grad.cpu().numpy())
+    assert np.all(np.isfinite(grads[0])) and np.any(grads[0])
+    assert rel_l2(grads[0], grads[1]) <= (7e-6 if np.isinf(band) else 4e-4)
