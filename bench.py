@@ -10,8 +10,8 @@ One JSON line on stdout:
   value     device-resident throughput of the FP32-bulk focus (inputs in HBM)
   e2e       the same metric through the processor C ABI with host buffers
             (setRawData / setFocusGrid / start: H2D, focus, D2H every step)
-  roofline  focus kernel vs the measured FP32 FFMA peak (8 FLOP = one complex
-            multiply-accumulate per correlation)
+  roofline  focus kernels vs the measured FP32 FFMA peak: the FP32-pipe operations that
+            the kernel which ran spends per (pixel, chirp), 2 FLOP each (see focus_ops)
   cpu_baseline  the FP64 OpenMP oracle loop on the host cores, bounded sample
   plain     the all-FP64-phase comparator kernel and the speed-up over it
   general   the FP32 general kernel (per-sample trajectory) on a row band vs the FP64 one
@@ -42,6 +42,18 @@ import numpy as np  # noqa: E402
 METRIC = "Gcorr/s (pixel*chirp*sample) & p50/p99 focus latency vs plain @<=1e-4 L2"
 UNIT = "Gcorr/s"
 FLOP_PER_CORR = 8.0  # complex multiply-accumulate: 4 FFMA
+
+
+def focus_ops(stats, n_samples):
+    """(FP32-pipe operations per (pixel, chirp), kernel) of the focus that `stats` describes. A direct
+    focus adds up the row: 4 FFMA a sample. A focus through range profiles reads the sum from the
+    chirp's table: 28 operations a pixel with 16 pixels an anchor (phase difference, degree-7
+    complex polynomial, product with the phasor), 32 otherwise, and 100 an anchor; building the table
+    is left out (its time is not)."""
+    if stats["path_name"] == "fp32_bulk" and stats["stage_samples"] == 0:
+        anchor = max(1, stats["anchor_pixels"])
+        return (28.0 if anchor == 16 else 32.0) + 100.0 / anchor, "profile_focus_kernel"
+    return FLOP_PER_CORR / 2 * n_samples, "focus_fp32_kernel"
 
 
 def parse():
@@ -332,14 +344,15 @@ def run_ours(args):
     image = img.cpu().numpy()
 
     peak_tf, fp64_tf, n_sm = fp32_peak_tflops(lib, torch)
-    achieved_tf = kernel_gcorr * FLOP_PER_CORR / 1e3
+    ops, kernel = focus_ops(p.lastStats(), sc.n_samples)
+    achieved_tf = P * sc.n_pri * ops * 2.0 / (step_ms.mean() / 1e3) / 1e12
     traffic = load_traffic()
     roofline = {"bound": "fp32", "achieved": round(achieved_tf, 2), "peak": round(peak_tf, 2), "unit": "TFLOP/s",
                 "frac": round(achieved_tf / peak_tf, 4),
                 "traffic": traffic.get("bytes_per_launch") if traffic else None,
                 "peak_source": "measured FFMA probe (tdc_probe_fma) on this GPU, this run",
-                "flop_per_corr": FLOP_PER_CORR, "fp64_tflops_measured": round(fp64_tf, 3),
-                "kernel": "focus_fp32_kernel"}
+                "flop_per_pixel_chirp": round(2.0 * ops, 1), "fp64_tflops_measured": round(fp64_tf, 3),
+                "kernel": kernel}
 
     out = {"metric": METRIC, "value": round(value, 2), "unit": UNIT, "n_gpus": 1, "steps": args.steps,
            "warmup": args.warmup, "ms_per_step": round(total_ms / args.steps, 3), "higher_is_better": True,
@@ -349,7 +362,8 @@ def run_ours(args):
            "run": {"correlations_per_step": corr, "path": path, "anchor_pixels": p.lastStats()["anchor_pixels"]},
            "latency_ms": {"p50": round(float(np.percentile(step_ms, 50)), 3),
                           "p99": round(float(np.percentile(step_ms, 99)), 3)},
-           "gpu_launches": 2 * args.steps, "clocks": clk, "roofline": roofline}
+           "gpu_launches": (3 if kernel == "profile_focus_kernel" else 2) * args.steps, "clocks": clk,
+           "roofline": roofline}
 
     if args.no_accuracy:
         print(json.dumps(out), flush=True)
@@ -495,7 +509,7 @@ def run_windowed(sc, api, f64, stream, unbounded_ms, speed=0.05, band_hz=10.0, n
             "band_hz": band_hz, "speed_m_s": speed, "tile_cols": stats["tile_cols"],
             "span_permille": stats["span_permille"],
             "rel_l2": float(np.linalg.norm(got[pix] - ref) / np.linalg.norm(ref)), "pixels_checked": int(pix.size),
-            "kernel": "focus_fp32_kernel<SKIP_ZERO>"}
+            "kernel": "focus_fp32_kernel<SKIP_ZERO>" if stats["stage_samples"] else "profile_focus_kernel<BAND>"}
 
 
 def run_general(sc, api, band, rows, pix, stream, bulk_gcorr):
@@ -546,9 +560,11 @@ def run_general(sc, api, band, rows, pix, stream, bulk_gcorr):
             r = oracle.focus(prob, oracle_opts(), pixels=sel)
             acc = float(np.linalg.norm(gim[sel] - r) / np.linalg.norm(r))
         res[name] = {"value": round(gcorr, 2), "rows": n_rows, "path": q.path(), "rel_l2": acc,
+                     "profiles": q.path() == "fp32_motion" and q.lastStats()["stage_samples"] == 0,
                      "motion_segment": q.lastStats()["motion_segment"]}
         del q
-    kernels = {"fp32_motion": "focus_motion_kernel", "general": "focus_general_kernel"}
+    kernels = {"fp32_motion": "profile_focus_kernel<MOVE>" if res["fp32"]["profiles"] else "focus_motion_kernel",
+               "general": "focus_general_kernel"}
     return {"value": res["fp32"]["value"], "unit": UNIT, "kernel": kernels.get(res["fp32"]["path"], res["fp32"]["path"]),
             "workload": "per-sample FP32 positions drifting ~0.3 mm within each chirp, same band",
             "fp32": res["fp32"], "fp32_general": res["fp32_general"], "fp64": res["fp64"],
@@ -985,7 +1001,8 @@ def run_sharded(args):
     stats = sp.proc.lastStats()
     if rank == 0:
         peak_tf, fp64_tf, _ = fp32_peak_tflops(_tdc_lib(), torch)
-        achieved = corr / (float(kernel_ms.item()) / 1e3) / 1e9 * FLOP_PER_CORR / 1e3
+        ops, kernel = focus_ops(p.lastStats(), sc.n_samples)
+        achieved = corr / sc.n_samples * ops * 2.0 / (float(kernel_ms.item()) / 1e3) / 1e12
         out = {"metric": METRIC, "value": round(value, 2), "unit": UNIT, "n_gpus": world, "steps": args.steps,
                "warmup": args.warmup, "ms_per_step": round(1e3 * total_s / args.steps, 3), "higher_is_better": True,
                "scaling": "weak", "vs_baseline": None, "dtype": "f32",
@@ -994,11 +1011,11 @@ def run_sharded(args):
                "run": {"correlations_per_step": world * corr, "sharding": f"{world} row blocks of {rows} x {cols} "
                        "pixels, one per GPU, the whole acquisition on every GPU, no collective while focusing",
                        "path": p.path()},
-               "gpu_launches": 2 * args.steps, "clocks": clk,
+               "gpu_launches": (3 if kernel == "profile_focus_kernel" else 2) * args.steps, "clocks": clk,
                "roofline": {"bound": "fp32", "achieved": round(achieved, 2), "peak": round(peak_tf, 2),
                             "unit": "TFLOP/s", "frac": round(achieved / peak_tf, 4), "traffic": None,
                             "peak_source": "measured FFMA probe (tdc_probe_fma) on rank 0's GPU, this run",
-                            "kernel": "focus_fp32_kernel (slowest rank)"},
+                            "kernel": f"{kernel} (slowest rank)"},
                "e2e": {"value": round(world * corr / float(np.mean(times)) / 1e9, 2), "unit": UNIT,
                        "h2d_bytes_per_step": int(stats["h2d_bytes"]) * world,
                        "d2h_bytes_per_step": int(stats["d2h_bytes"]) * world, "steps": len(times),

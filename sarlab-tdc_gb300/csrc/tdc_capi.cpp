@@ -352,14 +352,6 @@ int prepare(tdc_processor *p, const StartOpts &o, int &launches)
         gres[2 * (size_t)s_pad + s] = (float)(2.0 * M_PI * gsv);
     }
     std::vector<float4> traj, wins;
-    // two samples side by side (FocusJob::traj)
-    auto put_sample = [s_pad](std::vector<float4> &t, int c, int s, float x, float y, float z, float w) {
-        float *f = &t[(size_t)c * s_pad + (s & ~1)].x + (s & 1);
-        f[0] = x;
-        f[2] = y;
-        f[4] = z;
-        f[6] = w;
-    };
     std::vector<float> wdot;
     p->traj_varies = pos_differ;
     p->delta_max = 0.0;
@@ -382,7 +374,8 @@ int prepare(tdc_processor *p, const StartOpts &o, int &launches)
                     const float *ps = p->pos + 3 * ti(c, s);
                     const double dx = (double)ps[0] - p0[0], dy = (double)ps[1] - p0[1], dz = (double)ps[2] - p0[2];
                     m = std::max(m, dx * dx + dy * dy + dz * dz);
-                    put_sample(traj, c, s, (float)dx, (float)dy, (float)dz, (float)(dx * dx + dy * dy + dz * dz));
+                    traj[(size_t)c * s_pad + s] =
+                        make_float4((float)dx, (float)dy, (float)dz, (float)(dx * dx + dy * dy + dz * dz));
                 }
             }
             d2[t] = m;
@@ -395,20 +388,24 @@ int prepare(tdc_processor *p, const StartOpts &o, int &launches)
         // pi rounded to FP32, exactly as the kernel compares). With positions moving within
         // chirps the pixel-independent part u . D_s comes from its own table.
         const bool with_traj = p->traj_varies;
-        wins.assign((size_t)C * s_pad + 2 * (size_t)C, make_float4(0.f, 0.f, 0.f, 0.f));
+        wins.assign((size_t)C * s_pad, make_float4(0.f, 0.f, 0.f, 0.f));
         if (with_traj) wdot.assign((size_t)C * s_pad, 0.f);
         const double cs = 2.0 * (double)3.14159265358979323846f / (double)o.bw, vs = -2.0 / (double)p->lambda * cs;
         parallel_chirps(C, S, [&](int, int cb, int ce) {
             for (int c = cb; c < ce; ++c)
                 for (int s = 0; s < S; ++s) {
                     const size_t i = (size_t)c * s_pad + s;
-                    const ChirpRec r = make_record(p, c, s, o.centroid != 0, o.center);
-                    const double ux = r.vel.x * vs, uy = r.vel.y * vs, uz = r.vel.z * vs;
-                    put_sample(wins, c, s, (float)ux, (float)uy, (float)uz, (float)(r.p_hi.w * cs));
-                    if (with_traj) {
-                        const float *d = &traj[i - (s & 1)].x + (s & 1);
-                        wdot[i] = (float)(ux * d[0] + uy * d[2] + uz * d[4]);
-                    }
+                    const size_t te = ti(c, s);
+                    const float *vl = p->vel ? p->vel + 3 * te : kZero3;
+                    const float centre = window_centre(vl, p->att ? p->att + 4 * te : kQId, p->bore, p->lambda,
+                                                       o.centroid != 0, o.center);
+                    const double ux = vl[0] * vs, uy = vl[1] * vs, uz = vl[2] * vs;
+                    float4 &w = wins[i];
+                    w.x = (float)ux;
+                    w.y = (float)uy;
+                    w.z = (float)uz;
+                    w.w = (float)(centre * cs);
+                    if (with_traj) wdot[i] = (float)(ux * traj[i].x + uy * traj[i].y + uz * traj[i].z);
                 }
         });
     }
@@ -601,7 +598,7 @@ int prepare(tdc_processor *p, const StartOpts &o, int &launches)
                "copy per-sample offsets");
     }
     if (!wins.empty()) {
-        TDC_CK(p->wins.ensure(wins.size() * sizeof(float4)), "alloc per-sample windows");
+        TDC_CK(p->wins.ensure((wins.size() + 2 * (size_t)C) * sizeof(float4)), "alloc per-sample windows");
         TDC_CK(cudaMemcpyAsync(p->wins.p, wins.data(), wins.size() * sizeof(float4), cudaMemcpyHostToDevice, st),
                "copy per-sample windows");
     }
@@ -632,7 +629,14 @@ int prepare(tdc_processor *p, const StartOpts &o, int &launches)
         TDC_CK(launch_prewindow(p->xw.as<float2>(), p->wr.as<float>(), C, S, s_pad, st), "prewindow kernel");
         launches += 2;
     }
+    // the kernels read the tables with two samples side by side
+    if (!traj.empty()) {
+        TDC_CK(launch_pair_samples(p->traj.as<float4>(), (long long)C * s_pad, st), "pair offsets kernel");
+        ++launches;
+    }
     if (!wins.empty()) {
+        TDC_CK(launch_pair_samples(p->wins.as<float4>(), (long long)C * s_pad, st), "pair windows kernel");
+        ++launches;
         TDC_CK(launch_window_bounds(p->wins.as<float4>(), traj.empty() ? nullptr : p->traj.as<const float4>(),
                                     p->xw.as<const float2>(), C, S, s_pad, st),
                "window bounds kernel");

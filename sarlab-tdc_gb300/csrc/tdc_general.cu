@@ -44,6 +44,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <algorithm>
+
 #include "tdc_device.cuh"
 #include "tdc_internal.h"
 
@@ -518,6 +520,18 @@ __global__ void __launch_bounds__(kT, (!TRAJ && WIN && WIDE) ? 1 : TDC_GENERAL_M
     }
 }
 
+// Entries (x, y, z, w) of samples 2 i and 2 i + 1 to (x0, x1, y0, y1)(z0, z1, w0, w1), in place (the host's
+// loops that fill the tables are faster with whole entries).
+__global__ void __launch_bounds__(256) pair_samples_kernel(float4 *__restrict__ t, long long pairs)
+{
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < pairs;
+         i += (long long)gridDim.x * blockDim.x) {
+        const float4 a = t[2 * i], b = t[2 * i + 1];
+        t[2 * i] = make_float4(a.x, b.x, a.y, b.y);
+        t[2 * i + 1] = make_float4(a.z, b.z, a.w, b.w);
+    }
+}
+
 // Per chirp, how far the per-sample windows stray from one: with u_s the scaled velocity, c_s the
 // scaled window centre, and n_s the unit vector from the pixel, q_s = u_s.n_s - c_s. About the
 // mean (u, c) and the direction n_0 from sample 0, |q_s - (u.n_0 - c)| <= max|u_s - u| + max|c_s - c|
@@ -589,6 +603,12 @@ KernelFn select_kernel(int variant)
 }
 
 }  // namespace
+
+cudaError_t launch_pair_samples(float4 *table, long long n, cudaStream_t st)
+{
+    pair_samples_kernel<<<(unsigned)std::min<long long>((n / 2 + 255) / 256, 152 * 16), 256, 0, st>>>(table, n / 2);
+    return cudaGetLastError();
+}
 
 cudaError_t launch_window_bounds(float4 *wins, const float4 *traj, const float2 *xw, int C, int S, int s_pad,
                                  cudaStream_t st)

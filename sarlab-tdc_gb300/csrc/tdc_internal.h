@@ -328,6 +328,8 @@ cudaError_t launch_focus_reduce(const float4 *partial, int n_groups, long long P
 // samples at a time: whole rows (seg_len = s_pad, job.stage_chirps chirps a stage) or
 // segments of one chirp; stage_bytes = chirps x (seg_len x row bytes per sample + one
 // record) + seg_len x table bytes per sample (see general_stage_bytes_for).
+// n (even) entries of a per-sample table to two samples side by side (FocusJob::traj).
+cudaError_t launch_pair_samples(float4 *table, long long n, cudaStream_t st);
 // Bounds on each chirp's windows over its samples, behind the table wins [C][s_pad].
 cudaError_t launch_window_bounds(float4 *wins, const float4 *traj, const float2 *xw, int C, int S, int s_pad,
                                  cudaStream_t st);

@@ -19,8 +19,8 @@
 // polynomial together: <= 2e-7 rms of a row's norm at |t| = 1.5, 1e-8 within the cell.
 //
 // Whole focus, direct kernels -> profiles (GB300, resident acquisition): 1024^2 pixels x 4096
-// chirps x 1024 samples 532 -> 7.4 ms; 1.05 M voxels x 16,384 x 256 587 -> 27.7 ms; 256^2 x 1024 x
-// 512 4.5 -> 0.24 ms; 256^2 x 64 x 12,345 6.5 -> 1.0 ms.
+// chirps x 1024 samples 532 -> 5.27 ms; 1.05 M voxels x 16,384 x 256 587 -> 19.8 ms; 256^2 x 1024 x
+// 512 4.5 -> 0.164 ms; 256^2 x 64 x 12,345 6.5 -> 0.100 ms.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
