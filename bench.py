@@ -268,8 +268,9 @@ def fp32_peak_tflops(lib, torch):
     return best, fp64, n_sm
 
 
-def load_traffic():
-    f = ROOT / "profiles" / "focus_fp32_traffic.json"
+def load_traffic(kernel):
+    name = "focus_profile_traffic.json" if kernel == "profile_focus_kernel" else "focus_fp32_traffic.json"
+    f = ROOT / "profiles" / name
     if f.exists():
         try:
             return json.loads(f.read_text())
@@ -346,7 +347,7 @@ def run_ours(args):
     peak_tf, fp64_tf, n_sm = fp32_peak_tflops(lib, torch)
     ops, kernel = focus_ops(p.lastStats(), sc.n_samples)
     achieved_tf = P * sc.n_pri * ops * 2.0 / (step_ms.mean() / 1e3) / 1e12
-    traffic = load_traffic()
+    traffic = load_traffic(kernel)
     roofline = {"bound": "fp32", "achieved": round(achieved_tf, 2), "peak": round(peak_tf, 2), "unit": "TFLOP/s",
                 "frac": round(achieved_tf / peak_tf, 4),
                 "traffic": traffic.get("bytes_per_launch") if traffic else None,

@@ -679,7 +679,9 @@ int measure_group_reach(tdc_processor *p)
 {
     int bits[8], *reach = p->flag.as<int>() + 10;
     TDC_CK(cudaMemsetAsync(reach, 0, sizeof(bits), p->stream), "reset reach");
-    TDC_CK(launch_group_reach(p->grid_hi.as<float4>(), p->grid_lo_valid ? p->grid_lo.as<float4>() : nullptr, p->P, p->grid_run, reach, p->stream), "reach kernel");
+    TDC_CK(launch_group_reach(p->grid_hi.as<float4>(), p->grid_lo_valid ? p->grid_lo.as<float4>() : nullptr, p->P,
+                              p->grid_run, reach, p->stream),
+           "reach kernel");
     TDC_CK(cudaMemcpyAsync(bits, reach, sizeof(bits), cudaMemcpyDeviceToHost, p->stream), "read reach");
     TDC_CK(cudaStreamSynchronize(p->stream), "reach sync");
     set_group_reach(p, bits);

@@ -17,7 +17,8 @@
 // complex multiply-add (4 FFMA) and no separate phasor advance. Block phasors
 // never accumulate more than S/L rotations of an accurately computed QL.
 // Chirp sums are accumulated per pixel with Kahan compensation; partial sums
-// per chirp group are combined in FP64 by focus_reduce_kernel in a fixed order,
+// per chirp group are combined in a fixed order, in FP64 by focus_reduce_kernel or in double-float by
+// focus_reduce_sliced_kernel (many groups),
 // so results do not depend on scheduling.
 //
 // Chirp sample rows and trajectory records are staged global->shared with

@@ -856,6 +856,15 @@ __device__ __forceinline__ void adjoint_pair(float2 psi, float turn, float t0, f
     sz = __ffma2_rn(dl, dz, sz);
 }
 
+// CTAs per SM the registers of an instance are limited to.
+constexpr int focus_ctas(int group, bool band, bool adjoint, int motion)
+{
+    if (group == 16) return adjoint ? 4 : 6;
+    if (motion == 2) return 4;
+    if (group == 1) return band || adjoint ? 4 : 6;
+    return band || motion || (adjoint && group == 2) ? 6 : TDC_PROFILE_MINB;
+}
+
 // Persistent CTAs of 64 threads over units (tile x chirp group) from an atomic counter, 8
 // pixels a thread. Per chirp, each G consecutive pixels share an anchor pixel: its range R0,
 // the carrier phase frac(gc R0) and the cell it reads (64 bytes, from L1 / L2: neighbouring
@@ -874,6 +883,10 @@ __device__ __forceinline__ void adjoint_pair(float2 psi, float turn, float t0, f
 // 7.2-7.4 (the cells' wait for memory: 1.5 -> 0.4 cycles an instruction). 64-thread CTAs at 128
 // registers: 16 warps an SM; 12 or 18 warps are 2-6% slower. With the cells in L1, forming the next
 // anchor ahead costs more registers than it hides (7.05 -> 6.72 ms without).
+//
+// G = 16: 16 pixels a thread and one anchor for them (LINE only: the offsets of 16 vectors do not fit the
+// registers), 162 registers, 12 warps an SM: 6.06 -> 5.27 ms (5 CTAs an SM 5.42). FMA pipe 66%, issue
+// 53%; half the cells' sectors come from L2.
 //
 // BAND: a finite Doppler band. Chirps out of band for all of a warp's pixels are found first, 32
 // at a time, from the anchors' Doppler and a bound on its change over a group (about 20
@@ -911,7 +924,7 @@ __device__ __forceinline__ void adjoint_pair(float2 psi, float turn, float t0, f
 // the phase needs no reduction: 5 operations of 45 a pixel and chirp less (1024^2 x 4096 x 1024: 6.52 ->
 // 6.06 ms; adjoint and finite band likewise 7-10%).
 template <int G, bool BAND, bool ADJ, int MOVE, bool LINE>
-__global__ void __launch_bounds__(kThreads, G == 16 ? (ADJ ? 4 : 6) : MOVE == 2 ? 4 : G == 1 ? (BAND || ADJ ? 4 : 6) : BAND || MOVE || (ADJ && G == 2) ? 6 : TDC_PROFILE_MINB)
+__global__ void __launch_bounds__(kThreads, focus_ctas(G, BAND, ADJ, MOVE))
     profile_focus_kernel(const FocusJob *__restrict__ jobs, const FocusUnit *__restrict__ units, int n_units,
                          int *__restrict__ counter, const float2 *__restrict__ gimg, float4 *__restrict__ gpart)
 {
@@ -1574,8 +1587,10 @@ static ProfileFn profile_fn(int group, bool band, bool adjoint, int motion, bool
         if (adjoint) return profile_focus_kernel<16, false, true, 0, true>;
         return profile_focus_kernel<16, false, false, 0, true>;
     }
-    if (line && adjoint) return band ? profile_focus_kernel<8, true, true, 0, true> : profile_focus_kernel<8, false, true, 0, true>;
-    if (line) return band ? profile_focus_kernel<8, true, false, 0, true> : profile_focus_kernel<8, false, false, 0, true>;
+    if (line && adjoint)
+        return band ? profile_focus_kernel<8, true, true, 0, true> : profile_focus_kernel<8, false, true, 0, true>;
+    if (line)
+        return band ? profile_focus_kernel<8, true, false, 0, true> : profile_focus_kernel<8, false, false, 0, true>;
     if (motion == 2) return profile_fn<false, false, 2>(group);
     if (motion) return profile_fn<false, false, 1>(group);
     if (adjoint) return band ? profile_fn<true, true, 0>(group) : profile_fn<false, true, 0>(group);
