@@ -1450,7 +1450,9 @@ int focus_plan(tdc_processor *p, FocusPlan &plan, double max_unit_work)
                             ? profile_group(p, path, build)
                             : 0;
     if (profile) {
-        slots = p->n_sm * kProfileCtasPerSm;
+        // (vibration's kernel has registers for half as many CTAs, and units to match: 151 x 97 pixels x 333 x
+        // 500, 96 -> 92 us a pass; the others' launch bounds of 6 gain nothing, a finite band loses 5%)
+        slots = p->n_sm * (build.traj ? kProfileCtasPerSm / 2 : kProfileCtasPerSm);
     } else if (path == TDC_PATH_FP32_MOTION) {
         const int bps = focus_motion_blocks_per_sm(stage_bytes);
         if (bps <= 0) return fail(TDC_ERR_CUDA, "smooth-motion focus kernel does not fit on the device");

@@ -916,7 +916,7 @@ constexpr int focus_ctas(int group, bool band, bool adjoint, int motion)
 // polynomial; the direction turning along the chirp (W1 / R) enters through the derivative of
 // the phi tables, a pixel's own direction as the polynomial's gradient in u, to first order.
 // 151 x 97 pixels x 333 chirps x 500 samples: 1930 us in the general kernel of tdc_general.cu, which
-// corrects every sample, 120 us here (57 the six tables, 57 this kernel).
+// corrects every sample, 92 us here (40 the six tables, 50 this kernel).
 //
 // LINE: every group's pixels lie on a line parallel to one axis (sP.axis; checked when the grid is
 // measured: the offsets along the others are exactly zero) and span at most kLineMaxCycles carrier
