@@ -586,6 +586,18 @@ __device__ __forceinline__ float2 fresh2(const float2 *p)
     return v;
 }
 
+// dd_sub with its high part rounded from the whole difference. The high parts of antenna and pixel
+// alone are an ulp of their coordinates off, and h stands for the direction of the group's range
+// differences here: at coordinates of 1 km and ranges of 0.3 m, 5e-4 of the image without the
+// low parts and 3e-7 with them.
+__device__ __forceinline__ void difference(float ah, float al, float bh, float bl, float &h, float &l)
+{
+    float s, e;
+    dd_sub(ah, al, bh, bl, s, e);
+    h = s + e;
+    l = e - (h - s);
+}
+
 // One (chirp, anchor pixel): e = antenna - anchor, R0, gc / (2 R0), the carrier phase 2 pi frac(gc R0),
 // and the anchor's cell and place in it.
 struct Anchor {
@@ -992,9 +1004,10 @@ __global__ void __launch_bounds__(kThreads, focus_ctas(G, BAND, ADJ, MOVE))
                     if (s < count) {
                         const float4 h = __ldg(&sJ.grid_hi[p0 + s]);
                         const float4 l = sJ.grid_lo ? __ldg(&sJ.grid_lo[p0 + s]) : make_float4(0.f, 0.f, 0.f, 0.f);
-                        ox[i] = (h.x - hi.x) + (l.x - lo.x);
-                        oy[i] = (h.y - hi.y) + (l.y - lo.y);
-                        oz[i] = (h.z - hi.z) + (l.z - lo.z);
+                        float rest;  // (rounded as e is: they are equal where the antenna is on the pixel)
+                        difference(h.x, l.x, hi.x, lo.x, ox[i], rest);
+                        difference(h.y, l.y, hi.y, lo.y, oy[i], rest);
+                        difference(h.z, l.z, hi.z, lo.z, oz[i], rest);
                     }
                 }
 #pragma unroll
@@ -1042,9 +1055,9 @@ __global__ void __launch_bounds__(kThreads, focus_ctas(G, BAND, ADJ, MOVE))
             const float4 g = fresh(&sP.gc_hi);  // gc and cells per metre, high and low parts
             const int n_cells = __float_as_int(fresh(&sP.inv_gc2x4).w);
             float exl, eyl, ezl, rl, rs, dh;
-            dd_sub(ph.x, pl.x, p[0], p[3], n.ex, exl);
-            dd_sub(ph.y, pl.y, p[1], p[4], n.ey, eyl);
-            dd_sub(ph.z, pl.z, p[2], p[5], n.ez, ezl);
+            difference(ph.x, pl.x, p[0], p[3], n.ex, exl);
+            difference(ph.y, pl.y, p[1], p[4], n.ey, eyl);
+            difference(ph.z, pl.z, p[2], p[5], n.ez, ezl);
             dd_range(n.ex, exl, n.ey, eyl, n.ez, ezl, n.rh, rl, rs, dh);
             // gc / (2 R0), 1 / R0 to FP32 rounding (rsqrt is not)
             const float rinv = fmaf(rs, fmaf(-rl, rs, fmaf(-n.rh, rs, 1.0f)), rs);

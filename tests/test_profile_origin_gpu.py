@@ -1,0 +1,107 @@
+"""GPU parity of the focus through range profiles with FP64 positions and grids far from the
+origin, where the high floats of the double-float pairs alone are off by as much as the ranges
+can be resolved: the same scenes as at the origin, all of it moved.
+
+Tolerances: the 3e-6 of the focus through range profiles (4e-6 on runs along an axis, phases
+unreduced), relative L2 against the FP64 oracle, and what a pair of floats holds of the moved
+coordinates, 2^-49 of them rms on each axis of antenna and pixel: 2 x 2 pi 525 cycles / m x that x
+sqrt(3), below 1e-8 at 1 km."""
+import numpy as np
+import pytest
+
+import oracle
+from sarlabtdc import scenes
+from tdc_testutil import rel_l2
+
+pytestmark = pytest.mark.gpu
+
+INF = float("inf")
+KM = np.array([1234.56789, -987.654321, 111.1111])
+
+
+def _moved(shift, **kw):
+    sc = scenes.small_scene(device="cuda", jitter=0.3e-3, **kw)
+    sc.positions = sc.positions + shift
+    sc.grid = sc.grid + shift
+    return sc
+
+
+def _processor(sc, api=None, anchored=True, band=INF):
+    import _sarlabtdc
+
+    p = _sarlabtdc.TdcProcessor(0)
+    p.setRawData(*(sc.api_arrays() if api is None else api).values())
+    p.setChirpPositionsF64(sc.positions)
+    p.setFocusGridF64(sc.grid)
+    p.setAnchoredRanges(anchored)
+    p.prepare(0.0, band, False, False, True)
+    p.uploadGrid()
+    return p
+
+
+def _problem(sc, api):
+    return oracle.Problem(raw=api["rawData"], sampleTimes=api["sampleTimes"], position=sc.positions,
+                          velocity=api["velocity"][:, 0, :], modRate=api["modRate"], startFreq=api["startFreq"],
+                          grid=sc.grid)
+
+
+def _focus(p):
+    import torch
+
+    img = torch.empty(p.numPixels(), dtype=torch.complex64, device="cuda")
+    p.focusDevice(img)
+    p.check()
+    st = p.lastStats()
+    assert st["path_name"] == "fp32_bulk" and st["stage_samples"] == 0
+    return img.cpu().numpy(), st["anchor_pixels"]
+
+
+@pytest.mark.parametrize("nx,ny,n_pri,n_samples,spacing,height,group", [
+    (133, 202, 300, 160, 1e-3, 0.1, 8),
+    (256, 320, 800, 160, 1e-3, 0.3, 16),
+    (77, 154, 169, 300, 8e-3, 0.05, 2),
+    (57, 131, 300, 256, 1e-3, 0.02, 8),   # ranges too short for the series
+])
+def test_far_grid_focus(cuda_device, nx, ny, n_pri, n_samples, spacing, height, group):
+    sc = _moved(KM, seed=nx, n_pri=n_pri, n_samples=n_samples, nx=nx, ny=ny, spacing=spacing, height=height)
+    img, anchor = _focus(_processor(sc))
+    assert anchor == group
+    pix = np.unique(np.concatenate([[0, nx - 1, nx, img.size - 1],
+                                    np.random.default_rng(5).choice(img.size, 60, replace=False)]))
+    ref = oracle.focus(_problem(sc, sc.api_arrays()), oracle.Opts(applyRangeWin=False, dopplerBandwidth=INF), pixels=pix)
+    assert np.all(np.isfinite(img))
+    err = rel_l2(img[pix], ref)
+    assert err <= 4e-6, err
+
+
+@pytest.mark.parametrize("anchored", [True, False])
+def test_far_grid_adjoint(cuda_device, anchored):
+    """An image gradient on a few pixels only, so that the oracle need not take the others."""
+    import torch
+
+    sc = _moved(KM, seed=63, n_pri=300, n_samples=192, nx=83, ny=119, spacing=2e-3)
+    p = _processor(sc, anchored=anchored)
+    n = p.numPixels()
+    rng = np.random.default_rng(4)
+    pix = np.sort(rng.choice(n, 400, replace=False))
+    g = np.zeros(n, np.complex64)
+    g[pix] = (rng.normal(size=pix.size) + 1j * rng.normal(size=pix.size)).astype(np.complex64)
+    grad = torch.empty((sc.n_pri, 3), dtype=torch.float64, device="cuda")
+    p.adjointDevice(torch.from_numpy(g).cuda(), grad)
+    ref = oracle.adjoint_offsets(_problem(sc, sc.api_arrays()), oracle.Opts(applyRangeWin=False), None,
+                                 g[pix].astype(np.complex128), pixels=pix)
+    err = rel_l2(grad.cpu().numpy(), ref)
+    assert err <= 4e-6, err
+
+
+def test_antenna_on_a_far_pixel(cuda_device):
+    """For one chirp the antenna is on a pixel that is not its group's anchor: the pixel's window is
+    zero there (a Doppler frequency that is not a number), the others' is not."""
+    sc = _moved(KM, seed=8, n_pri=300, n_samples=256, nx=72, ny=110, height=0.02, y0=0.01)
+    sc.positions[150] = sc.grid[40, 21]
+    img, anchor = _focus(_processor(sc))
+    assert anchor == 8
+    pix = np.arange(40 * 72 + 16, 40 * 72 + 32)
+    ref = oracle.focus(_problem(sc, sc.api_arrays()), oracle.Opts(applyRangeWin=False, dopplerBandwidth=INF), pixels=pix)
+    err = rel_l2(img[pix], ref)
+    assert err <= 4e-6, err
