@@ -674,10 +674,13 @@ void set_group_reach(tdc_processor *p, const int *bits)
     p->reach_known = true;
 }
 
+// Where the measurements of the resident grid are made: behind the trajectory scan's flags.
+GridBounds *grid_bounds_dev(tdc_processor *p) { return reinterpret_cast<GridBounds *>(p->flag.as<int>() + 4); }
+
 // Reach of the anchored pixel groups of the resident grid (range profiles), measured now.
 int measure_group_reach(tdc_processor *p)
 {
-    int bits[8], *reach = p->flag.as<int>() + 10;
+    int bits[8], *reach = grid_bounds_dev(p)->words;
     TDC_CK(cudaMemsetAsync(reach, 0, sizeof(bits), p->stream), "reset reach");
     TDC_CK(launch_group_reach(p->grid_hi.as<float4>(), p->grid_lo_valid ? p->grid_lo.as<float4>() : nullptr, p->P,
                               p->grid_run, reach, p->stream),
@@ -721,10 +724,11 @@ int measure_tile_radii(tdc_processor *p)
     std::vector<float> r((size_t)n_flat + n_block);
     TDC_CK(p->tile_radius.ensure(r.size() * 4), "alloc tile radii");
     float *dev = p->tile_radius.as<float>();
-    TDC_CK(launch_tile_radius(p->grid_hi.as<float4>(), p->P, p->rows, p->cols, 0, n_flat, dev, p->stream),
+    const float4 *lo = p->grid_lo_valid ? p->grid_lo.as<float4>() : nullptr;
+    TDC_CK(launch_tile_radius(p->grid_hi.as<float4>(), lo, p->P, p->rows, p->cols, 0, n_flat, dev, p->stream),
            "tile radius kernel");
-    TDC_CK(launch_tile_radius(p->grid_hi.as<float4>(), p->P, p->rows, p->cols, kBlockTileCols, n_block, dev + n_flat,
-                              p->stream),
+    TDC_CK(launch_tile_radius(p->grid_hi.as<float4>(), lo, p->P, p->rows, p->cols, kBlockTileCols, n_block,
+                              dev + n_flat, p->stream),
            "tile radius kernel");
     TDC_CK(cudaMemcpyAsync(r.data(), dev, r.size() * 4, cudaMemcpyDeviceToHost, p->stream), "read tile radii");
     TDC_CK(cudaStreamSynchronize(p->stream), "tile radius sync");
@@ -801,30 +805,25 @@ int upload_grid(tdc_processor *p, int &launches)
     // (small focuses do not ask for the reach: measured when a plan first does)
     p->reach_known = p->has_raw && profile_pays((double)std::max(P, p->plan_pixels), p->C, p->S, false);
     if (P > 0) {
-        // bounding box, reach and anchor span of the grid, measured on the device (the box as
-        // order-preserving integer keys of the floats)
-        const int init[14] = {0x7fffffff, 0x7fffffff, 0x7fffffff, (int)0x80000000, (int)0x80000000,
-                              (int)0x80000000};
-        int keys[14];
-        int *box = p->flag.as<int>() + 4;
-        TDC_CK(cudaMemcpyAsync(box, init, sizeof(init), cudaMemcpyHostToDevice, st), "init bbox");
+        // bounding box, reach and anchor span of the grid, measured on the device
+        GridBounds b;
+        grid_bounds_init(b);
+        GridBounds *dev = grid_bounds_dev(p);
+        const float4 *lo = p->grid_lo_valid ? p->grid_lo.as<float4>() : nullptr;
+        TDC_CK(cudaMemcpyAsync(dev, &b, sizeof(b), cudaMemcpyHostToDevice, st), "init bbox");
         if (p->reach_known)
-            TDC_CK(launch_group_reach(p->grid_hi.as<float4>(), p->grid_lo_valid ? p->grid_lo.as<float4>() : nullptr, P,
-                                      p->grid_run, box + 6, st),
-                   "reach kernel");
-        TDC_CK(launch_grid_bbox(p->grid_hi.as<float4>(), P, box, st), "bbox kernel");
-        TDC_CK(cudaMemcpyAsync(keys, box, sizeof(keys), cudaMemcpyDeviceToHost, st), "read bbox");
+            TDC_CK(launch_group_reach(p->grid_hi.as<float4>(), lo, P, p->grid_run, dev->words, st), "reach kernel");
+        TDC_CK(launch_grid_bbox(p->grid_hi.as<float4>(), lo, P, dev, st), "bbox kernel");
+        TDC_CK(cudaMemcpyAsync(&b, dev, sizeof(b), cudaMemcpyDeviceToHost, st), "read bbox");
         TDC_CK(cudaStreamSynchronize(st), "grid sync");
         launches += p->reach_known ? 2 : 1;
-        if (p->reach_known) set_group_reach(p, keys + 6);
+        if (p->reach_known) set_group_reach(p, b.words);
         float span;
-        std::memcpy(&span, &keys[9], 4);
+        std::memcpy(&span, &b.words[3], 4);
         p->anchor_span = span;
-        for (int k = 0; k < 6; ++k) {
-            const int bits = keys[k] >= 0 ? keys[k] : keys[k] ^ 0x7fffffff;
-            float f;
-            std::memcpy(&f, &bits, 4);
-            (k < 3 ? p->grid_min[k] : p->grid_max[k - 3]) = f;
+        for (int k = 0; k < 3; ++k) {
+            p->grid_min[k] = pair_value(b.box[k]);
+            p->grid_max[k] = pair_value(b.box[3 + k]);
         }
     }
     return TDC_OK;

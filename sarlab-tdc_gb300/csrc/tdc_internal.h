@@ -288,9 +288,44 @@ struct RowScan {
     int k, flag;
 };
 cudaError_t launch_rows_differ(const RowScan *scans, int n, int C, int S, int *flags, cudaStream_t st);
-cudaError_t launch_tile_radius(const float4 *hi, long long P, int rows, int cols, int tile_cols, int n_tiles,
-                               float *radius, cudaStream_t st);
-cudaError_t launch_grid_bbox(const float4 *hi, long long P, int *out, cudaStream_t st);
+cudaError_t launch_tile_radius(const float4 *hi, const float4 *lo, long long P, int rows, int cols, int tile_cols,
+                               int n_tiles, float *radius, cudaStream_t st);
+
+// What is measured of a grid on the device. box: minima and maxima of x, y, z as order-preserving keys of
+// the double-float values (pair_key; pair_value on the host and device). words (float bits, starting
+// at 0; a NaN compares above any distance): 0..2 and 7 reach of the groups of 8, 4, 2 and 16 pixels, 3
+// the anchor span, 4..6 largest offset along each axis in the groups of 16.
+struct GridBounds {
+    long long box[6];
+    int words[8];
+};
+
+inline void grid_bounds_init(GridBounds &b)
+{
+    for (int k = 0; k < 3; ++k) {
+        b.box[k] = 0x7fffffffffffffffLL;
+        b.box[3 + k] = -0x7fffffffffffffffLL - 1;
+    }
+    for (int &w : b.words) w = 0;
+}
+
+// The value of a key: the upper word is the high float, the lower one the low float.
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+inline double pair_value(long long key)
+{
+    const int k[2] = {(int)(key >> 32), (int)((unsigned int)key ^ 0x80000000u)};
+    union {
+        int i;
+        float f;
+    } v[2];
+    for (int j = 0; j < 2; ++j) v[j].i = k[j] >= 0 ? k[j] : k[j] ^ 0x7fffffff;
+    // (no low part beside an infinity or NaN)
+    return v[0].f - v[0].f == 0.0f ? (double)v[0].f + (double)v[1].f : (double)v[0].f;
+}
+
+cudaError_t launch_grid_bbox(const float4 *hi, const float4 *lo, long long P, GridBounds *out, cudaStream_t st);
 cudaError_t launch_grid_from_f32(const float *grid, long long P, float4 *hi, cudaStream_t st);
 cudaError_t launch_grid_from_f64(const double *grid, long long P, float4 *hi, float4 *lo, cudaStream_t st);
 
@@ -361,9 +396,8 @@ int focus_profile_blocks_per_sm(int group, bool band, bool adjoint, int motion, 
 // deviation off that direction, |W1|) as float bits (starting at 0; NaN above all).
 cudaError_t launch_vib_fit(const float4 *traj, const ChirpRec *chirps, int C, int S, int s_pad, float phase_per_m,
                            VibRec *recs, int *maxima, cudaStream_t st);
-// out[0..2] = max(out, largest distance of a pixel from the anchor of its group of 8 / 4 / 2
-// consecutive pixels of a run) as float bits (out starts at 0; a NaN compares above any distance).
-cudaError_t launch_group_reach(const float4 *hi, const float4 *lo, long long P, int run, int *out, cudaStream_t st);
+// GridBounds::words but the anchor span, for groups of consecutive pixels of a run.
+cudaError_t launch_group_reach(const float4 *hi, const float4 *lo, long long P, int run, int *words, cudaStream_t st);
 
 // Adjoint of the FP32-bulk focus w.r.t. per-chirp position offsets: per-(tile, chirp)
 // float4 partials, then an FP64 sum over tiles into grad[C][3]. stored: job.xw holds the

@@ -49,7 +49,8 @@ constexpr size_t kOffStatus = 0;    // int counter, int status
 constexpr size_t kOffJob = 256;     // FocusJob
 constexpr size_t kOffUnits = 512;   // FocusUnit[n_units]
 // Words at kOffStatus.
-constexpr int kWordCounter = 0, kWordStatus = 1, kWordProfile = 2, kWordProfileCounter = 3, kWordBox = 8;
+constexpr int kWordCounter = 0, kWordStatus = 1, kWordProfile = 2, kWordProfileCounter = 3;
+constexpr size_t kOffBounds = 32;  // GridBounds
 constexpr int kSpent = 1 << 30;  // a work counter past every unit
 
 size_t layout_bytes(long long P, long long n_units, int n_groups, size_t &off_partial)
@@ -60,7 +61,7 @@ size_t layout_bytes(long long P, long long n_units, int n_groups, size_t &off_pa
 
 // Job record, unit table (tile-major, one unit per tile x chirp group) and zeroed
 // counter / status written into the scratch array by the device itself.
-__global__ void noalloc_setup_kernel(FocusJob job, int n_tiles, int n_groups, unsigned char *base)
+__global__ void noalloc_setup_kernel(FocusJob job, GridBounds bounds, int n_tiles, int n_groups, unsigned char *base)
 {
     const long long n_units = (long long)n_tiles * n_groups;
     const long long i0 = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -69,7 +70,7 @@ __global__ void noalloc_setup_kernel(FocusJob job, int n_tiles, int n_groups, un
         words[kWordCounter] = 0;
         words[kWordStatus] = 0;
         words[kWordProfile] = 0;
-        for (int k = 0; k < 10; ++k) words[kWordBox + k] = k < 3 ? 0x7fffffff : k < 6 ? (int)0x80000000 : 0;
+        *reinterpret_cast<GridBounds *>(base + kOffBounds) = bounds;
         *reinterpret_cast<FocusJob *>(base + kOffJob) = job;
     }
     FocusUnit *units = reinterpret_cast<FocusUnit *>(base + kOffUnits);
@@ -90,15 +91,16 @@ struct ProfilePlan {
     double g1, gc;
 };
 
-// Whether range profiles apply, from the grid's bounding box (words, from grid_bbox_kernel) and
+// Whether range profiles apply, from the grid's bounding box (bounds, from grid_bbox_kernel) and
 // the chirp records, as the processor decides it from its host copies: finite inputs, a grid
 // within the unambiguous range, ranges the cell index resolves, a table that fits. Fills in the
 // build inputs and leaves one of the two work counters spent: the first block, with the farthest range in
 // FP32 (FP64 runs at 1/64 of its rate); the others write the unit table.
-__global__ void noalloc_decide_kernel(ProfilePlan plan, int *__restrict__ words, bool band)
+__global__ void noalloc_decide_kernel(ProfilePlan plan, const GridBounds *__restrict__ bounds, int *__restrict__ words,
+                                      bool band)
 {
     __shared__ float far2[8];
-    __shared__ float box[6];
+    __shared__ double box[6];
     const int tid = threadIdx.x;
     if (blockIdx.x > 0) {
         const int n = plan.n_tiles * plan.n_groups;
@@ -106,10 +108,7 @@ __global__ void noalloc_decide_kernel(ProfilePlan plan, int *__restrict__ words,
             plan.units[u] = FocusUnit{0, u % plan.n_tiles, u / plan.n_tiles, 0};
         return;
     }
-    if (tid < 6) {
-        const int key = words[kWordBox + tid];
-        box[tid] = __int_as_float(key >= 0 ? key : key ^ 0x7fffffff);
-    }
+    if (tid < 6) box[tid] = pair_value(bounds->box[tid]);
     __syncthreads();
     float most = 0.f;
     bool finite = true;
@@ -119,7 +118,7 @@ __global__ void noalloc_decide_kernel(ProfilePlan plan, int *__restrict__ words,
         float f = 0.f;
         const float p[3] = {r.p_hi.x, r.p_hi.y, r.p_hi.z};
         for (int k = 0; k < 3; ++k) {
-            const float d = fmaxf(fabsf(box[k] - p[k]), fabsf(p[k] - box[3 + k]));
+            const float d = fmaxf(fabsf((float)box[k] - p[k]), fabsf(p[k] - (float)box[3 + k]));
             f += d * d;
         }
         finite = finite && f < 1e30f && isfinite(r.p_lo.x + r.p_lo.y + r.p_lo.z) &&
@@ -292,7 +291,9 @@ int enqueue(const tdc_noalloc_focus_args *a, float *image_dev, cudaStream_t st, 
 
     const long long n_units = n_tiles * n_groups;
     const int setup_blocks = (int)std::min<long long>((n_units + 255) / 256, 1024);
-    noalloc_setup_kernel<<<setup_blocks, 256, 0, st>>>(job, (int)n_tiles, n_groups, base);
+    GridBounds bounds;
+    grid_bounds_init(bounds);
+    noalloc_setup_kernel<<<setup_blocks, 256, 0, st>>>(job, bounds, (int)n_tiles, n_groups, base);
     e = cudaGetLastError();
     if (e != cudaSuccess) return fail(TDC_ERR_CUDA, std::string("setup kernel: ") + cudaGetErrorString(e));
     int *words = reinterpret_cast<int *>(base + kOffStatus);
@@ -358,9 +359,10 @@ int enqueue(const tdc_noalloc_focus_args *a, float *image_dev, cudaStream_t st, 
         b.job.inv_gc = (float)(1.0 / gc);
     }
     if (profile) {
-        e = launch_grid_bbox(job.grid_hi, P, words + kWordBox, st);
+        GridBounds *bounds_dev = reinterpret_cast<GridBounds *>(base + kOffBounds);
+        e = launch_grid_bbox(job.grid_hi, job.grid_lo, P, bounds_dev, st);
         if (e == cudaSuccess) {
-            noalloc_decide_kernel<<<9, 256, 0, st>>>(pp, words, band);
+            noalloc_decide_kernel<<<9, 256, 0, st>>>(pp, bounds_dev, words, band);
             e = cudaGetLastError();
         }
         if (e == cudaSuccess)

@@ -142,37 +142,69 @@ __global__ void scale_rows_kernel(const float2 *__restrict__ rows, long long tot
     }
 }
 
-// Bounding box of the grid's high floats: out = (min x, min y, min z, max x, max y, max z),
-// each as an order-preserving int (see float_key); out must start at (INT_MAX x3, INT_MIN x3).
-// out[9] = largest distance of a pixel from the anchor of its 32 consecutive pixels (the 17th, or
-// the last), as float bits (starts at 0; a NaN compares above any distance).
+// Bounding box of the grid and the anchor span (GridBounds, which starts as grid_bounds_init sets it): the
+// largest distance of a pixel from the anchor of its 32 consecutive pixels, the 17th or the last.
+// Low parts count: half an ulp of a high float is 0.25 m at 4.5e6 m, many cells of a range profile.
 __device__ __forceinline__ int float_key(float f)
 {
     const int i = __float_as_int(f);
     return i >= 0 ? i : i ^ 0x7fffffff;
 }
 
-__global__ void grid_bbox_kernel(const float4 *__restrict__ hi, long long P, int *__restrict__ out)
+// (h, l) as one integer that orders as h + l does: the pair is normalised first.
+__device__ __forceinline__ long long pair_key(float h, float l)
 {
-    int mn[3] = {0x7fffffff, 0x7fffffff, 0x7fffffff}, mx[3] = {(int)0x80000000, (int)0x80000000, (int)0x80000000};
+    float s = h, e = l;
+    if (l != 0.f) two_sum(h, l, s, e);
+    return (long long)float_key(s) << 32 | ((unsigned int)float_key(e) ^ 0x80000000u);
+}
+
+// Least (SIGN 1) or greatest (-1) key of the warp.
+template <int SIGN>
+__device__ __forceinline__ long long warp_extreme(long long key)
+{
+    const int h = (int)(key >> 32);
+    const unsigned int l = (unsigned int)key;
+    if (SIGN > 0) {
+        const int m = __reduce_min_sync(0xffffffffu, h);
+        return (long long)m << 32 | __reduce_min_sync(0xffffffffu, h == m ? l : 0xffffffffu);
+    }
+    const int m = __reduce_max_sync(0xffffffffu, h);
+    return (long long)m << 32 | __reduce_max_sync(0xffffffffu, h == m ? l : 0u);
+}
+
+// Pixel p of a grid less a point (a, b) of it.
+__device__ __forceinline__ float3 grid_offset(const float4 *hi, const float4 *lo, long long p, float4 a, float4 b)
+{
+    const float4 v = hi[p], l = lo ? lo[p] : make_float4(0.f, 0.f, 0.f, 0.f);
+    return make_float3((v.x - a.x) + (l.x - b.x), (v.y - a.y) + (l.y - b.y), (v.z - a.z) + (l.z - b.z));
+}
+
+__device__ __forceinline__ float length2(float3 d) { return d.x * d.x + d.y * d.y + d.z * d.z; }
+
+__global__ void __launch_bounds__(256) grid_bbox_kernel(const float4 *__restrict__ hi, const float4 *__restrict__ lo,
+                                                        long long P, GridBounds *__restrict__ out)
+{
+    const long long top = 0x7fffffffffffffffLL;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    long long mn[3] = {top, top, top}, mx[3] = {-top - 1, -top - 1, -top - 1};
     float span2 = 0.f;
     for (long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x; p < P; p += (long long)gridDim.x * blockDim.x) {
-        const float4 v = hi[p];
-        const int k[3] = {float_key(v.x), float_key(v.y), float_key(v.z)};
+        const float4 v = hi[p], l = lo ? lo[p] : zero;
+        const long long k[3] = {pair_key(v.x, l.x), pair_key(v.y, l.y), pair_key(v.z, l.z)};
         for (int d = 0; d < 3; ++d) {
             mn[d] = min(mn[d], k[d]);
             mx[d] = max(mx[d], k[d]);
         }
-        const float4 a = hi[min(P - 1, (p & ~31LL) + 16)];
-        const float dx = v.x - a.x, dy = v.y - a.y, dz = v.z - a.z;
-        const float d2 = dx * dx + dy * dy + dz * dz;
+        const long long a = min(P - 1, (p & ~31LL) + 16);
+        const float d2 = length2(grid_offset(hi, lo, p, hi[a], lo ? lo[a] : zero));
         span2 = d2 > span2 || d2 != d2 ? d2 : span2;
     }
     const int span = __reduce_max_sync(0xffffffffu, __float_as_int(fabsf(sqrtf(span2))));
-    __shared__ int part[8][7];  // one row a warp: the block's atomics are 7, not 7 a warp
+    __shared__ long long part[8][7];  // one row a warp: the block's atomics are 7, not 7 a warp
     for (int d = 0; d < 3; ++d) {
-        mn[d] = __reduce_min_sync(0xffffffffu, mn[d]);
-        mx[d] = __reduce_max_sync(0xffffffffu, mx[d]);
+        mn[d] = warp_extreme<1>(mn[d]);
+        mx[d] = warp_extreme<-1>(mx[d]);
     }
     const int warp = threadIdx.x >> 5;
     if ((threadIdx.x & 31) == 0) {
@@ -185,18 +217,18 @@ __global__ void grid_bbox_kernel(const float4 *__restrict__ hi, long long P, int
     __syncthreads();
     if (threadIdx.x < 7) {
         const int d = threadIdx.x, n_warps = blockDim.x >> 5;
-        int v = part[0][d];
+        long long v = part[0][d];
         for (int w = 1; w < n_warps; ++w) v = d < 3 ? min(v, part[w][d]) : max(v, part[w][d]);
-        if (d < 3) atomicMin(&out[d], v);
-        else if (d < 6) atomicMax(&out[d], v);
-        else if (v > 0) atomicMax(&out[9], v);
+        if (d < 3) atomicMin(&out->box[d], v);
+        else if (d < 6) atomicMax(&out->box[d], v);
+        else if (v > 0) atomicMax(&out->words[3], (int)v);
     }
 }
 
 // Largest distance from each work tile's centre pixel to its other pixels (see FocusJob::tile_cols);
 // one warp a tile.
-__global__ void tile_radius_kernel(const float4 *__restrict__ hi, long long P, int rows, int cols, int tile_cols,
-                                   int n_tiles, float *__restrict__ radius)
+__global__ void tile_radius_kernel(const float4 *__restrict__ hi, const float4 *__restrict__ lo, long long P, int rows,
+                                   int cols, int tile_cols, int n_tiles, float *__restrict__ radius)
 {
     const int t = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
     if (t >= n_tiles) return;
@@ -209,14 +241,12 @@ __global__ void tile_radius_kernel(const float4 *__restrict__ hi, long long P, i
     } else {
         centre = min(P - 1, (long long)t * kFocusTile + kFocusTile / 2);
     }
-    const float4 a = hi[centre];
+    const float4 a = hi[centre], b = lo ? lo[centre] : make_float4(0.f, 0.f, 0.f, 0.f);
     float r2 = 0.f;
     for (int s = lane; s < kFocusTile; s += 32) {
         const long long p = tile_pixel(tile_cols, cols, P, t, s);
         if (p < 0) continue;
-        const float4 v = hi[p];
-        const float dx = v.x - a.x, dy = v.y - a.y, dz = v.z - a.z;
-        const float d2 = dx * dx + dy * dy + dz * dz;
+        const float d2 = length2(grid_offset(hi, lo, p, a, b));
         r2 = d2 > r2 || d2 != d2 ? d2 : r2;
     }
     const int m = __reduce_max_sync(0xffffffffu, __float_as_int(fabsf(r2)));
@@ -225,15 +255,16 @@ __global__ void tile_radius_kernel(const float4 *__restrict__ hi, long long P, i
 
 // Reach of the anchored pixel groups of the range-profile focus: the largest distance from a
 // group's anchor (its middle pixel) to its other pixels, for groups of 8, 4 and 2 consecutive
-// pixels of a run (out[0..2]) and of 16 (out[7]), and the largest offset along each axis in the groups of
-// 16 (out[4..6]); one thread per 8 pixels of a run.
+// pixels of a run and of 16, and the largest offset along each axis in the groups of 16
+// (GridBounds::words); one thread per 8 pixels of a run.
 __global__ void group_reach_kernel(const float4 *__restrict__ hi, const float4 *__restrict__ lo, long long P, int run,
-                                   int *__restrict__ out)
+                                   int *__restrict__ words)
 {
     float spread[4] = {0.f, 0.f, 0.f, 0.f};
     const int per = (run + 7) / 8;
     const long long n = (P / run) * per + (P % run + 7) / 8;
     float reach[3] = {0.f, 0.f, 0.f};
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
     for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x) {
         const long long r = q / per;
         const int col = (int)(q - r * per) * 8;
@@ -243,34 +274,29 @@ __global__ void group_reach_kernel(const float4 *__restrict__ hi, const float4 *
             const int g = 8 >> k;
             for (int s = 0; s < valid; s += g) {
                 const int m = min(g, valid - s);
-                const float4 a = hi[p0 + s + m / 2];
+                const float4 a = hi[p0 + s + m / 2], b = lo ? lo[p0 + s + m / 2] : zero;
                 for (int i = 0; i < m; ++i) {
-                    const float4 v = hi[p0 + s + i];
-                    const float dx = v.x - a.x, dy = v.y - a.y, dz = v.z - a.z;
-                    const float d = sqrtf(dx * dx + dy * dy + dz * dz);
+                    const float d = sqrtf(length2(grid_offset(hi, lo, p0 + s + i, a, b)));
                     reach[k] = d > reach[k] || d != d ? d : reach[k];
                 }
             }
         }
         if (col & 15) continue;
         const int valid16 = (int)min((long long)min(16, run - col), P - p0);
-        const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f), a = hi[p0 + valid16 / 2],
-                     b = lo ? lo[p0 + valid16 / 2] : zero;
+        const float4 a = hi[p0 + valid16 / 2], b = lo ? lo[p0 + valid16 / 2] : zero;
         for (int i = 0; i < valid16; ++i) {
-            const float4 v = hi[p0 + i], l = lo ? lo[p0 + i] : zero;
-            const float x = fabsf((v.x - a.x) + (l.x - b.x)), y = fabsf((v.y - a.y) + (l.y - b.y)),
-                        z = fabsf((v.z - a.z) + (l.z - b.z));
-            const float o[4] = {x, y, z, sqrtf(x * x + y * y + z * z)};
+            const float3 v = grid_offset(hi, lo, p0 + i, a, b);
+            const float o[4] = {fabsf(v.x), fabsf(v.y), fabsf(v.z), sqrtf(length2(v))};
             for (int d = 0; d < 4; ++d) spread[d] = o[d] > spread[d] || o[d] != o[d] ? o[d] : spread[d];
         }
     }
     for (int d = 0; d < 4; ++d) {
         const int v = __reduce_max_sync(0xffffffffu, __float_as_int(fabsf(spread[d])));
-        if ((threadIdx.x & 31) == 0 && v > 0) atomicMax(&out[4 + d], v);
+        if ((threadIdx.x & 31) == 0 && v > 0) atomicMax(&words[4 + d], v);
     }
     for (int k = 0; k < 3; ++k) {
         const int v = __reduce_max_sync(0xffffffffu, __float_as_int(fabsf(reach[k])));
-        if ((threadIdx.x & 31) == 0 && v > 0) atomicMax(&out[k], v);
+        if ((threadIdx.x & 31) == 0 && v > 0) atomicMax(&words[k], v);
     }
 }
 
@@ -384,31 +410,31 @@ cudaError_t launch_scale_rows(const float2 *rows, int C, int s_pad, float2 *rows
     return cudaGetLastError();
 }
 
-cudaError_t launch_grid_bbox(const float4 *hi, long long P, int *out, cudaStream_t st)
+cudaError_t launch_grid_bbox(const float4 *hi, const float4 *lo, long long P, GridBounds *out, cudaStream_t st)
 {
     if (P <= 0) return cudaSuccess;
     long long blocks = (P + 255) / 256;
     if (blocks > 152 * 8) blocks = 152 * 8;
-    grid_bbox_kernel<<<(unsigned)blocks, 256, 0, st>>>(hi, P, out);
+    grid_bbox_kernel<<<(unsigned)blocks, 256, 0, st>>>(hi, lo, P, out);
     return cudaGetLastError();
 }
 
-cudaError_t launch_tile_radius(const float4 *hi, long long P, int rows, int cols, int tile_cols, int n_tiles,
-                               float *radius, cudaStream_t st)
+cudaError_t launch_tile_radius(const float4 *hi, const float4 *lo, long long P, int rows, int cols, int tile_cols,
+                               int n_tiles, float *radius, cudaStream_t st)
 {
     if (n_tiles <= 0) return cudaSuccess;
-    tile_radius_kernel<<<(unsigned)((n_tiles * 32LL + 255) / 256), 256, 0, st>>>(hi, P, rows, cols, tile_cols, n_tiles,
-                                                                                radius);
+    tile_radius_kernel<<<(unsigned)((n_tiles * 32LL + 255) / 256), 256, 0, st>>>(hi, lo, P, rows, cols, tile_cols,
+                                                                                n_tiles, radius);
     return cudaGetLastError();
 }
 
-cudaError_t launch_group_reach(const float4 *hi, const float4 *lo, long long P, int run, int *out, cudaStream_t st)
+cudaError_t launch_group_reach(const float4 *hi, const float4 *lo, long long P, int run, int *words, cudaStream_t st)
 {
     if (P <= 0 || run <= 0) return cudaSuccess;
     long long blocks = (P / 8 + 255) / 256;
     if (blocks > 152 * 8) blocks = 152 * 8;
     if (blocks < 1) blocks = 1;
-    group_reach_kernel<<<(unsigned)blocks, 256, 0, st>>>(hi, lo, P, run, out);
+    group_reach_kernel<<<(unsigned)blocks, 256, 0, st>>>(hi, lo, P, run, words);
     return cudaGetLastError();
 }
 

@@ -105,3 +105,74 @@ def test_antenna_on_a_far_pixel(cuda_device):
     ref = oracle.focus(_problem(sc, sc.api_arrays()), oracle.Opts(applyRangeWin=False, dopplerBandwidth=INF), pixels=pix)
     err = rel_l2(img[pix], ref)
     assert err <= 4e-6, err
+
+
+# Map coordinates. A pair of floats holds them to 2^-29 m at 1e6 m and 2^-26 m at 4.5e6 m (ulp of the low
+# float), and differences of low floats are rounded to the same, once for antenna - anchor and once for
+# pixel - anchor: 3400 rad / m x ulp x (sqrt(2 / 12) + 2 x 2 / sqrt(12)) = 1.0e-5 and 8e-5 rad rms,
+# relative L2 beside the 4e-6.
+FAR = [(np.array([1.0e6, -0.7e6, 0.1e6]) + 0.123, 1.4e-5), (np.array([4.5e6, 3.3e6, -1.0e6]) + 0.456, 8.4e-5)]
+
+
+@pytest.mark.parametrize("shift,tol", FAR)
+@pytest.mark.parametrize("nx,ny,n_pri,n_samples,spacing,height,anchored", [
+    (133, 202, 300, 160, 1e-3, 0.3, True),
+    (256, 320, 800, 160, 1e-3, 0.3, True),
+    (256, 64, 400, 256, 0.3e-3, 0.3, True),   # a grid narrower than half an ulp of its coordinates
+    (77, 154, 169, 300, 8e-3, 0.3, True),
+    (100, 120, 300, 160, 1e-3, 0.3, False),
+])
+def test_map_coordinates_focus(cuda_device, nx, ny, n_pri, n_samples, spacing, height, anchored, shift, tol):
+    """The table's place and extent, and the groups' reach, follow the low parts of the grid too."""
+    sc = _moved(shift, seed=nx, n_pri=n_pri, n_samples=n_samples, nx=nx, ny=ny, spacing=spacing, height=height)
+    img, anchor = _focus(_processor(sc, anchored=anchored))
+    at_origin = _moved(0.0, seed=nx, n_pri=n_pri, n_samples=n_samples, nx=nx, ny=ny, spacing=spacing, height=height)
+    assert anchor == _focus(_processor(at_origin, anchored=anchored))[1]
+    pix = np.unique(np.concatenate([[0, nx - 1, nx, img.size - 1],
+                                    np.random.default_rng(5).choice(img.size, 60, replace=False)]))
+    ref = oracle.focus(_problem(sc, sc.api_arrays()), oracle.Opts(applyRangeWin=False, dopplerBandwidth=INF), pixels=pix)
+    assert np.all(np.isfinite(img))
+    err = rel_l2(img[pix], ref)
+    assert err <= tol, err
+
+
+@pytest.mark.parametrize("shift,tol", FAR)
+def test_map_coordinates_noalloc(cuda_device, shift, tol):
+    import torch
+
+    from test_zz_no_alloc import _noalloc_args, _noalloc_twice
+
+    sc = _moved(shift, seed=9, n_pri=300, n_samples=256, nx=97, ny=83, spacing=1e-3)
+    api = sc.api_arrays()
+    a, keep = _noalloc_args(api, sc.grid, torch, pos64=sc.positions, grid64=sc.grid)
+    got = _noalloc_twice(a)
+    pix = np.unique(np.random.default_rng(5).choice(got.size, 60, replace=False))
+    ref = oracle.focus(_problem(sc, api), oracle.Opts(applyRangeWin=False, dopplerBandwidth=INF), pixels=pix)
+    err = rel_l2(got[pix], ref)
+    assert np.all(np.isfinite(got)) and err <= tol, err
+
+
+def test_measured_geometry_does_not_depend_on_the_origin(cuda_device):
+    """The direct kernels' plans: unit spans under a finite band (radii of the tiles) and anchored
+    ranges (distance of pixels from their anchors) of a grid moved to map coordinates."""
+    shift = FAR[0][0]
+    kw = dict(seed=303, n_pri=600, n_samples=128, nx=64, ny=96, rail_len=0.6)
+    spans = []
+    for s in (0.0, shift):
+        sc = _moved(s, **kw)
+        api = sc.api_arrays()
+        api["velocity"][..., 0] = 0.08
+        p = _processor(sc, api, band=14.0)
+        import torch
+
+        p.focusDevice(torch.empty(p.numPixels(), dtype=torch.complex64, device="cuda"))
+        p.check()
+        st = p.lastStats()
+        assert st["stage_samples"] > 0 and st["tile_cols"] == 16
+        spans.append(st["span_permille"])
+    assert spans[0] < 1000 and abs(spans[0] - spans[1]) <= 1
+    sc = _moved(shift, seed=5, n_pri=256, n_samples=256, nx=64, ny=32, spacing=2e-3)
+    p = _processor(sc)
+    p.focusDevice(torch.empty(p.numPixels(), dtype=torch.complex64, device="cuda"))
+    p.check()
+    assert p.lastStats()["anchor_pixels"] == 32
