@@ -1087,7 +1087,14 @@ __global__ void __launch_bounds__(kThreads, focus_ctas(G, BAND, ADJ, MOVE))
             if (MOVE) n.w = shift;
             if (BAND && G == 1) {
                 const float4 v = recs[buf].p[k][2];
-                const float fd = doppler_freq(sJ.two_over_lambda, v.x, v.y, v.z, n.ex, n.ey, n.ez, rs);
+                // (from the high parts, as the direct kernels, unless the low parts move the direction)
+                float dx = ph.x - p[0], dy = ph.y - p[1], dz = ph.z - p[2];
+                if (fabsf(n.ex - dx) + fabsf(n.ey - dy) + fabsf(n.ez - dz) > 2e-6f * n.rh) {
+                    dx = n.ex;
+                    dy = n.ey;
+                    dz = n.ez;
+                }
+                const float fd = doppler_freq(sJ.two_over_lambda, v.x, v.y, v.z, dx, dy, dz, rs);
                 n.w = doppler_window(fd, ph.w, sJ.half_bw, sJ.inv_bw, (sJ.flags & kFlagTaper) != 0, sJ.az_a);
             }
             return n;
@@ -1145,11 +1152,14 @@ __global__ void __launch_bounds__(kThreads, focus_ctas(G, BAND, ADJ, MOVE))
                 unsigned int live = 0;
                 if (dropped != (1u << count) - 1u)  // (some pixel's chunk is seen)
                     for (int k = 0; k < n; ++k) {
-                        const float4 p = recs[buf].p[k][0], v = recs[buf].p[k][2];
+                        const float4 p = recs[buf].p[k][0], pl = recs[buf].p[k][1], v = recs[buf].p[k][2];
                         bool any = false;
 #pragma unroll
                         for (int g = 0; g < kSub; ++g) {
-                            const float ex = p.x - ax[g][0], ey = p.y - ax[g][1], ez = p.z - ax[g][2];
+                            // (the low parts are a direction of their own: 1e-3 at 1 km and ranges of 6 cm)
+                            const float ex = (p.x - ax[g][0]) + (pl.x - ax[g][3]),
+                                        ey = (p.y - ax[g][1]) + (pl.y - ax[g][4]),
+                                        ez = (p.z - ax[g][2]) + (pl.z - ax[g][5]);
                             const float rs = rsqrtf(fmaf(ex, ex, fmaf(ey, ey, ez * ez)));
                             const float tol = sJ.two_over_lambda;
                             const float fd = doppler_freq(tol, v.x, v.y, v.z, ex, ey, ez, rs);
@@ -1360,7 +1370,8 @@ __global__ void __launch_bounds__(kThreads, focus_ctas(G, BAND, ADJ, MOVE))
                                 }
                             }
                             while (edge) {
-                                // the side of the edge is decided as the direct kernels decide it
+                                // the side of the edge is decided as the direct kernels decide it, from the high
+                                // parts of the direction; low parts that move it further than the doubt count
                                 const int i = __ffs(edge) - 1;
                                 edge &= edge - 1;
                                 int m;
@@ -1373,6 +1384,11 @@ __global__ void __launch_bounds__(kThreads, focus_ctas(G, BAND, ADJ, MOVE))
                                 dd_sub(ph.x, pl.x, hi.x, lo.x, ex, exl);
                                 dd_sub(ph.y, pl.y, hi.y, lo.y, ey, eyl);
                                 dd_sub(ph.z, pl.z, hi.z, lo.z, ez, ezl);
+                                if (fabsf(exl) + fabsf(eyl) + fabsf(ezl) > 2e-6f * cur.rh) {
+                                    difference(ph.x, pl.x, hi.x, lo.x, ex, exl);
+                                    difference(ph.y, pl.y, hi.y, lo.y, ey, eyl);
+                                    difference(ph.z, pl.z, hi.z, lo.z, ez, ezl);
+                                }
                                 dd_range(ex, exl, ey, eyl, ez, ezl, rh, rl, rs, dh);
                                 const float fd = doppler_freq(tol, v.x, v.y, v.z, ex, ey, ez, rs);
                                 const float we = doppler_window(fd, fdc, half, inv_bw, taper, az);

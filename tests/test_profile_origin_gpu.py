@@ -176,3 +176,58 @@ def test_measured_geometry_does_not_depend_on_the_origin(cuda_device):
     p.focusDevice(torch.empty(p.numPixels(), dtype=torch.complex64, device="cuda"))
     p.check()
     assert p.lastStats()["anchor_pixels"] == 32
+
+
+def _banded(shift, **kw):
+    sc = _moved(shift, **kw)
+    api = sc.api_arrays()
+    api["velocity"][..., 0] = 0.08
+    return sc, api
+
+
+@pytest.mark.parametrize("nx,ny,spacing,height,shift,anchored,group", [
+    (57, 131, 1e-3, 0.1, KM, True, 8),
+    (57, 131, 1e-3, 0.03, KM, False, 0),
+    (64, 80, 8e-3, 0.05, KM, True, 2),
+    (57, 131, 1e-3, 0.3, FAR[0][0], True, 8),
+    (57, 131, 1e-3, 0.3, FAR[0][0], False, 0),
+])
+def test_far_grid_under_a_finite_band(cuda_device, nx, ny, spacing, height, shift, anchored, group):
+    """Chirps are left out for a warp from its anchors' Doppler. Tolerance 2e-4, as for every finite band:
+    a chirp at the inclusive edge may fall on either side in FP32 and FP64."""
+    sc, api = _banded(shift, seed=nx + ny, n_pri=750, n_samples=192, nx=nx, ny=ny, spacing=spacing, height=height,
+                      rail_len=0.75, y0=0.05)
+    import _sarlabtdc
+
+    p = _sarlabtdc.TdcProcessor(0)
+    p.setSkipTest(False)  # (its points are FP32 by definition)
+    p.setRawData(*api.values())
+    p.setChirpPositionsF64(sc.positions)
+    p.setFocusGridF64(sc.grid)
+    p.setAnchoredRanges(anchored)
+    p.prepare(0.0, 9.0, False, False, True)
+    p.uploadGrid()
+    img, anchor = _focus(p)
+    assert anchor == group
+    pix = np.unique(np.random.default_rng(5).choice(img.size, 150, replace=False))
+    ref = oracle.focus(_problem(sc, api), oracle.Opts(applyRangeWin=False, dopplerBandwidth=9.0, skip_test=False),
+                       pixels=pix)
+    err = rel_l2(img[pix], ref)
+    assert np.any(ref) and err <= 2e-4, err
+
+
+@pytest.mark.parametrize("height,shift", [(0.03, KM), (0.3, FAR[0][0])])
+def test_far_noalloc_under_a_finite_band(cuda_device, height, shift):
+    import torch
+
+    from test_zz_no_alloc import _noalloc_args, _noalloc_twice
+
+    sc, api = _banded(shift, seed=12, n_pri=750, n_samples=192, nx=57, ny=131, spacing=1e-3, height=height, rail_len=0.75,
+                      y0=0.05)
+    a, keep = _noalloc_args(api, sc.grid, torch, pos64=sc.positions, grid64=sc.grid, band=9.0)
+    got = _noalloc_twice(a)
+    pix = np.unique(np.random.default_rng(5).choice(got.size, 150, replace=False))
+    ref = oracle.focus(_problem(sc, api), oracle.Opts(applyRangeWin=False, dopplerBandwidth=9.0, skip_test=False),
+                       pixels=pix)
+    err = rel_l2(got[pix], ref)
+    assert np.any(ref) and err <= 2e-4, err
