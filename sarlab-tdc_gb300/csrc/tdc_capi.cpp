@@ -1603,7 +1603,9 @@ int focus_plan(tdc_processor *p, FocusPlan &plan, double max_unit_work)
         job.bend3 = (float)(2.0 * M_PI * h * h * h * g1);
         job.reach = (float)reach;
         job.axis = std::max(0, p->run_axis);
-        job.r_safe = (float)(profile == 16 ? kWideRange * reach : reach / 0.03);
+        // (above zero: an antenna on its anchor is none of the series')
+        job.r_safe = std::max((float)(profile == 16 ? kWideRange * reach : reach / 0.03),
+                              std::numeric_limits<float>::min());
         plan.build = build;
     }
     // narrow variants take the phase correction in radians
