@@ -1405,6 +1405,8 @@ int profile_build(tdc_processor *p, const FocusPlan &plan, cudaStream_t st, int 
     }
     TDC_CK(launch_profile_build(plan.build, st), "profile table kernel");
     ++launches;
+    p->table_epoch = p->state_epoch;
+    p->table_job = plan.build.job;
     return TDC_OK;
 }
 
@@ -1688,7 +1690,6 @@ int focus_resident(tdc_processor *p, float2 *image_dev, cudaStream_t st, int &la
     int *status = counter + 1;
     if (plan.profile) {
         if (int rc = profile_build(p, plan, st, launches)) return rc;
-        p->table_epoch = p->state_epoch;
         const bool band = std::isfinite(job.half_bw);
         const int motion = plan.build.traj ? 2 : path == TDC_PATH_FP32_MOTION ? 1 : 0;
         const int grid = std::min(n_units, p->n_sm * focus_profile_blocks_per_sm(plan.profile, band, false, motion, plan.line));
@@ -1741,16 +1742,14 @@ int focus_resident(tdc_processor *p, float2 *image_dev, cudaStream_t st, int &la
 }
 
 // Adjoint through range profiles. The table is the forward's where it was built for the current
-// acquisition, trajectory and grid (stream-ordered before this call, as kept sums are), else
-// built here.
+// acquisition, trajectory and grid (stream-ordered before this call, as kept sums are) and its
+// record for this plan (anchored ranges may have been switched since), else built here.
 int adjoint_profile(tdc_processor *p, const FocusPlan &plan, const float2 *gimg, double *grad, cudaStream_t st)
 {
     const int C = p->C, n_units = (int)p->units_host.size(), n_tiles = plan.job.n_tiles;
     int launches = 0;
-    if (p->table_epoch != p->state_epoch) {
+    if (p->table_epoch != p->state_epoch || std::memcmp(&p->table_job, &plan.build.job, sizeof(ProfileJob)))
         if (int rc = profile_build(p, plan, st, launches)) return rc;
-        p->table_epoch = p->state_epoch;
-    }
     const size_t off_job = 256;
     const size_t off_units = round_up(off_job + sizeof(FocusJob), 256);
     const size_t off_gpart = round_up(off_units + (size_t)n_units * sizeof(FocusUnit), 256);

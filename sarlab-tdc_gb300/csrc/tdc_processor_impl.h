@@ -202,7 +202,8 @@ struct tdc_processor {
     bool reach_known = false;  // group_reach and run_axis are the resident grid's
     tdc::impl::DevBuf cells, cell_base, twiddle;
     double table_ratio = 0.0;  // largest table taken, in bytes per byte of samples (0: no limit)
-    uint64_t table_epoch = 0;  // state_epoch the table was built at by a focus (0: none)
+    uint64_t table_epoch = 0;  // state_epoch the table was built at (0: none)
+    tdc::ProfileJob table_job{};  // ... and the record in cell_base, which follows the plan's group size too
     int twiddle_S = 0;  // samples the constants in `twiddle` are for (0: none)
     bool rec_finite = false;  // every chirp record's velocity and window centre is finite
     double vel_dir[3] = {0, 0, 0};                         // mean antenna velocity direction (0: at rest)
