@@ -1695,6 +1695,7 @@ int focus_resident(tdc_processor *p, float2 *image_dev, cudaStream_t st, int &la
         const int grid = std::min(n_units, p->n_sm * focus_profile_blocks_per_sm(plan.profile, band, false, motion, plan.line));
         TDC_CK(launch_focus_profile(plan.profile, band, motion, plan.line, jobs_dev, units_dev, n_units, counter, grid, st),
                "focus kernel (range profiles)");
+        TDC_CK(cudaEventRecord(p->table_ev, st), "table event");
     } else if (path == TDC_PATH_FP32_BULK) {
         const int grid = std::min(n_units, slots);
         // the zero-window-skipping instances also map block tiles (which come with a finite band)
@@ -1742,12 +1743,14 @@ int focus_resident(tdc_processor *p, float2 *image_dev, cudaStream_t st, int &la
 }
 
 // Adjoint through range profiles. The table is the forward's where it was built for the current
-// acquisition, trajectory and grid (stream-ordered before this call, as kept sums are) and its
-// record for this plan (anchored ranges may have been switched since), else built here.
+// acquisition, trajectory and grid, and its record for this plan (anchored ranges may have been
+// switched since), else built here. A focus may be in flight on another stream, building or reading
+// the table: the adjoint's stream waits for it.
 int adjoint_profile(tdc_processor *p, const FocusPlan &plan, const float2 *gimg, double *grad, cudaStream_t st)
 {
     const int C = p->C, n_units = (int)p->units_host.size(), n_tiles = plan.job.n_tiles;
     int launches = 0;
+    TDC_CK(cudaStreamWaitEvent(st, p->table_ev, 0), "table wait");
     if (p->table_epoch != p->state_epoch || std::memcmp(&p->table_job, &plan.build.job, sizeof(ProfileJob)))
         if (int rc = profile_build(p, plan, st, launches)) return rc;
     const size_t off_job = 256;
@@ -1824,6 +1827,7 @@ int tdc_processor_create(int gpu_num, tdc_processor **out)
     }
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&p->stream, cudaStreamNonBlocking);
     for (int i = 0; i < 6 && e == cudaSuccess; ++i) e = cudaEventCreate(&p->ev[i]);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&p->table_ev, cudaEventDisableTiming);
     if (e != cudaSuccess) {
         tdc_processor_destroy(p);
         return cuda_fail(e, "processor init");
@@ -1841,6 +1845,7 @@ int tdc_processor_destroy(tdc_processor *p)
     if (p->stream) cudaStreamSynchronize(p->stream);
     for (auto &ev : p->ev)
         if (ev) cudaEventDestroy(ev);
+    if (p->table_ev) cudaEventDestroy(p->table_ev);
     if (p->stream) cudaStreamDestroy(p->stream);
     delete p;
     return TDC_OK;

@@ -124,6 +124,7 @@ struct tdc_processor {
     bool host_reads = false;  // the device reads pageable host memory coherently (Grace-Blackwell C2C)
     cudaStream_t stream = nullptr;
     cudaEvent_t ev[6] = {};
+    cudaEvent_t table_ev = nullptr;  // after the last focus that built and read the range-profile table
     // Borrowed inputs (setRawData / setFocusGrid).
     const float *raw = nullptr;
     const float *pri_times = nullptr;

@@ -57,3 +57,36 @@ def test_adjoint_after_anchored_ranges_were_switched(cuda_device, band):
         p.adjointDevice(g, grad)
         assert np.any(ref)
         np.testing.assert_array_equal(grad.cpu().numpy(), ref)
+
+
+def test_adjoint_beside_a_focus_on_another_stream(cuda_device):
+    """A focus in flight on one stream, the adjoint enqueued on another with no order between them:
+    both give what they give alone, bit for bit; with the table of the focus, and with another
+    (anchored ranges switched in between)."""
+    import torch
+
+    kw = dict(height=0.3, n_pri=1500, nx=800, ny=600, n_samples=256)
+    p = _processor(INF, **kw)
+    g, grad = _gradient(p, 1500)
+    img, ref_img = (torch.empty(p.numPixels(), dtype=torch.complex64, device="cuda") for _ in range(2))
+    refs = {}
+    for anchored in (True, False):
+        alone = _processor(INF, **kw)
+        alone.setAnchoredRanges(anchored)
+        alone.adjointDevice(g, grad)
+        refs[anchored] = grad.cpu().numpy()
+        if anchored:
+            alone.focusDevice(ref_img)
+            alone.check()
+    one, two = torch.cuda.Stream(), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    for anchored in (True, False):
+        p.setAnchoredRanges(True)
+        with torch.cuda.stream(one):
+            p.focusDevice(img)
+        p.setAnchoredRanges(anchored)
+        with torch.cuda.stream(two):
+            p.adjointDevice(g, grad)
+        torch.cuda.synchronize()
+        np.testing.assert_array_equal(grad.cpu().numpy(), refs[anchored])
+        np.testing.assert_array_equal(img.cpu().numpy(), ref_img.cpu().numpy())
