@@ -653,8 +653,16 @@ int prepare(tdc_processor *p, const StartOpts &o, int &launches)
     p->plan_path = -1;  // job parameters changed
     if (p->P > 0 && p->traj_varies && !p->win_varies && !std::isfinite(o.bw) &&
         profile_pays((double)std::max(p->P, p->plan_pixels), C, S, false) && choose_path(p) == TDC_PATH_GENERAL)
-        return measure_vibration(p);
+        (void)measured(measure_vibration(p));  // (a plan asks again)
     return TDC_OK;
+}
+
+// What a plan can do without: a failure (memory) is no error of the call, and is not left behind for the next
+// launch's check.
+bool measured(int rc)
+{
+    if (rc) (void)cudaGetLastError();
+    return rc == TDC_OK;
 }
 
 void set_group_reach(tdc_processor *p, const int *bits)
@@ -964,7 +972,7 @@ int choose_tile_cols(const tdc_processor *p)
 void plan_unit_order_and_spans(tdc_processor *p, int tile_cols, bool narrow)
 {
     if (!std::isfinite(p->opts.bw) || p->rec_host.size() != (size_t)p->C || p->units_host.size() < 2) return;
-    if (narrow && !p->tile_radius_known && measure_tile_radii(p)) narrow = false;
+    if (narrow && !p->tile_radius_known && !measured(measure_tile_radii(p))) narrow = false;
     const std::vector<double> &centres = tile_cols ? p->tile_centre_block : p->tile_centre_flat;
     const std::vector<double> &radii = tile_cols ? p->tile_radius_block : p->tile_radius_flat;
     const long long n_tiles = (long long)centres.size() / 3;
@@ -1324,7 +1332,7 @@ int profile_group(tdc_processor *p, int path, ProfileBuild &b)
         // per-sample positions only, uniform sampling, an antenna clear of the grid
         const double rmax_phase = 2.0 * M_PI * 2.0 * p->resid_hz * rmax / kC0;
         if (!p->traj_varies || p->win_varies || !p->motion_enabled || band || !(rmin > 0.0) ||
-            rmax_phase > kUniformPhaseTolRad || (!p->vib_known && measure_vibration(p)))
+            rmax_phase > kUniformPhaseTolRad || (!p->vib_known && !measured(measure_vibration(p))))
             return 0;
         w1 = p->vib_max[2];
         v2 = 0.0;
@@ -1361,7 +1369,7 @@ int profile_group(tdc_processor *p, int path, ProfileBuild &b)
         size_t free_b = 0, total_b = 0;
         if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || bytes > free_b / 2) return 0;
     }
-    if (!p->reach_known && measure_group_reach(p)) return 0;
+    if (!p->reach_known && !measured(measure_group_reach(p))) return 0;
     if (!std::isfinite(p->group_reach[0])) return 0;
     if (!p->anchor_enabled) return 1;
     // 16 pixels a thread and anchor on runs parallel to an axis, once half as many threads are enough: whole
@@ -1410,13 +1418,30 @@ int profile_build(tdc_processor *p, const FocusPlan &plan, cudaStream_t st, int 
     return TDC_OK;
 }
 
-int focus_plan(tdc_processor *p, FocusPlan &plan, double max_unit_work)
+// Gives the table's memory back, its allocation or one beside it having failed.
+void drop_table(tdc_processor *p)
 {
+    (void)cudaGetLastError();
+    p->cells.release();
+    p->table_epoch = 0;
+}
+
+// A plan of one form: range profiles, planned where they pay and what they need can be allocated, or the
+// direct kernels.
+int plan_form(tdc_processor *p, FocusPlan &plan, double max_unit_work, bool profiles, bool &planned)
+{
+    planned = false;
     if (!p->prepared) return fail(TDC_ERR_STATE, "acquisition not prepared");
     if (p->P <= 0) return fail(TDC_ERR_STATE, "no focus grid");
     const int path = choose_path(p);
     const long long P = p->P;
     const int C = p->C;
+    ProfileBuild build{};
+    const int profile =
+        profiles && (path == TDC_PATH_FP32_BULK || path == TDC_PATH_FP32_MOTION || path == TDC_PATH_GENERAL)
+            ? profile_group(p, path, build)
+            : 0;
+    if (profiles && !profile) return TDC_OK;
     if (path == TDC_PATH_GENERAL_FP64)
         if (int rc = sample_records(p)) return rc;
 
@@ -1446,10 +1471,6 @@ int focus_plan(tdc_processor *p, FocusPlan &plan, double max_unit_work)
     const bool motion_exact_ql = path == TDC_PATH_FP32_MOTION && !(2.0 * M_PI * 8.0 * motion_slope_bound(p) <= 0.8);
     int slots;
     bool anchored = false;
-    ProfileBuild build{};
-    const int profile = path == TDC_PATH_FP32_BULK || path == TDC_PATH_FP32_MOTION || path == TDC_PATH_GENERAL
-                            ? profile_group(p, path, build)
-                            : 0;
     if (profile) {
         // (vibration's kernel has registers for half as many CTAs, and units to match: 151 x 97 pixels x 333 x
         // 500, 96 -> 92 us a pass; the others' launch bounds of 6 gain nothing, a finite band loses 5%)
@@ -1537,16 +1558,21 @@ int focus_plan(tdc_processor *p, FocusPlan &plan, double max_unit_work)
         p->plan_run = run;
         p->plan_uploaded = false;
     }
-    if (profile) {
-        TDC_CK(p->cells.ensure((size_t)p->C * build.n_cells * kProfileCoefs * 8 * (build.traj ? kVibTables : 1)),
-               "alloc range profiles");
-        TDC_CK(p->cell_base.ensure(sizeof(ProfileJob) + (size_t)p->C * 4), "alloc range profile bases");
-        const size_t tw_bytes = (size_t)p->S * (kProfileNodes * 8 + 4);
-        if (tw_bytes > p->twiddle.cap) p->twiddle_S = 0;
-        TDC_CK(p->twiddle.ensure(tw_bytes), "alloc profile constants");
-    }
     const int n_units = (int)p->units_host.size();
     const ScratchLayout L = scratch_layout(P, n_units, p->plan_groups);
+    if (profile) {
+        // (the memory was free when the table was planned; others may have taken it since)
+        const size_t tw_bytes = (size_t)p->S * (kProfileNodes * 8 + 4);
+        if (tw_bytes > p->twiddle.cap) p->twiddle_S = 0;
+        if (L.total > p->scratch.cap) p->plan_uploaded = false;
+        if (p->cells.ensure((size_t)p->C * build.n_cells * kProfileCoefs * 8 * (build.traj ? kVibTables : 1)) !=
+                cudaSuccess ||
+            p->cell_base.ensure(sizeof(ProfileJob) + (size_t)p->C * 4) != cudaSuccess ||
+            p->twiddle.ensure(tw_bytes) != cudaSuccess || p->scratch.ensure(L.total) != cudaSuccess) {
+            drop_table(p);
+            return TDC_OK;
+        }
+    }
     if (L.total > p->scratch.cap) {
         TDC_CK(p->scratch.ensure(L.total), "alloc focus scratch");
         p->plan_uploaded = false;
@@ -1612,7 +1638,15 @@ int focus_plan(tdc_processor *p, FocusPlan &plan, double max_unit_work)
     }
     // narrow variants take the phase correction in radians
     if (path == TDC_PATH_GENERAL && !(variant & 4)) plan.job.gsam = p->gres.as<const float>() + 2 * (size_t)p->s_pad;
+    planned = true;
     return TDC_OK;
+}
+
+int focus_plan(tdc_processor *p, FocusPlan &plan, double max_unit_work)
+{
+    bool planned = false;
+    const int rc = plan_form(p, plan, max_unit_work, true, planned);
+    return rc || planned ? rc : plan_form(p, plan, max_unit_work, false, planned);
 }
 
 // Focus the resident acquisition onto the resident grid: image_dev (complex float [P]).
@@ -1746,17 +1780,27 @@ int focus_resident(tdc_processor *p, float2 *image_dev, cudaStream_t st, int &la
 // acquisition, trajectory and grid, and its record for this plan (anchored ranges may have been
 // switched since), else built here. A focus may be in flight on another stream, building or reading
 // the table: the adjoint's stream waits for it.
-int adjoint_profile(tdc_processor *p, const FocusPlan &plan, const float2 *gimg, double *grad, cudaStream_t st)
+// done is false, and nothing launched, where the focus is none of range profiles or memory is short.
+int adjoint_profile(tdc_processor *p, const float2 *gimg, double *grad, cudaStream_t st, bool &done)
 {
+    done = false;
+    FocusPlan plan;
+    bool planned = false;
+    const int rc = plan_form(p, plan, 0.0, true, planned);
+    if (rc || !planned) return rc;
     const int C = p->C, n_units = (int)p->units_host.size(), n_tiles = plan.job.n_tiles;
+    const size_t off_job = 256;
+    const size_t off_units = round_up(off_job + sizeof(FocusJob), 256);
+    const size_t off_gpart = round_up(off_units + (size_t)n_units * sizeof(FocusUnit), 256);
+    if (p->adj_scratch.ensure(off_gpart + (size_t)n_tiles * C * 16) != cudaSuccess) {
+        drop_table(p);
+        return TDC_OK;
+    }
+    done = true;
     int launches = 0;
     TDC_CK(cudaStreamWaitEvent(st, p->table_ev, 0), "table wait");
     if (p->table_epoch != p->state_epoch || std::memcmp(&p->table_job, &plan.build.job, sizeof(ProfileJob)))
         if (int rc = profile_build(p, plan, st, launches)) return rc;
-    const size_t off_job = 256;
-    const size_t off_units = round_up(off_job + sizeof(FocusJob), 256);
-    const size_t off_gpart = round_up(off_units + (size_t)n_units * sizeof(FocusUnit), 256);
-    TDC_CK(p->adj_scratch.ensure(off_gpart + (size_t)n_tiles * C * 16), "alloc adjoint scratch");
     unsigned char *scr = p->adj_scratch.as<unsigned char>();
     TDC_CK(cudaMemcpyAsync(scr + off_job, &plan.job, sizeof(FocusJob), cudaMemcpyHostToDevice, st), "copy job");
     TDC_CK(cudaMemcpyAsync(scr + off_units, p->units_host.data(), (size_t)n_units * sizeof(FocusUnit),
@@ -2184,10 +2228,9 @@ int tdc_processor_adjoint_device(tdc_processor *p, const float *grad_image_dev, 
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (needs_segments(p->s_pad))
         return fail(TDC_ERR_UNSUPPORTED, "the adjoint stages whole chirps: these chirps are too long");
-    FocusPlan plan;
-    if (int rc = focus_plan(p, plan)) return rc;
-    if (plan.profile)
-        return adjoint_profile(p, plan, reinterpret_cast<const float2 *>(grad_image_dev), grad_offsets_dev, st);
+    bool done = false;
+    const int rc = adjoint_profile(p, reinterpret_cast<const float2 *>(grad_image_dev), grad_offsets_dev, st, done);
+    if (done || rc) return rc;
     const long long P = p->P;
     const int C = p->C;
     int cb = 1;

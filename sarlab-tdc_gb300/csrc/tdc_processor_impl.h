@@ -300,10 +300,13 @@ int general_variant(const tdc_processor *p);
 // acquisition and grid, or 0 when that kernel does not take them.
 int motion_segment(const tdc_processor *p);
 int measure_vibration(tdc_processor *p);
+bool measured(int rc);
 int motion_stage_bytes_for(int s_pad, int &cb);
 FocusJob make_job(const tdc_processor *p, float4 *partial, int cb, int path);
 // Plan units (p->units_host) and make sure the processor's scratch holds them and the partials.
 // max_unit_work > 0 bounds the correlations of one unit (the request loop's granularity).
+// Range profiles where they pay and their table, and the scratch beside it, can be allocated; else the
+// direct kernels.
 int focus_plan(tdc_processor *p, FocusPlan &plan, double max_unit_work = 0.0);
 // A (pixel, chirp) pair of a range-profile focus in correlations of the direct FP32-bulk kernel's
 // time (work budgets of the request loop).
