@@ -536,8 +536,9 @@ __global__ void __launch_bounds__(256) pair_samples_kernel(float4 *__restrict__ 
 // scaled window centre, and n_s the unit vector from the pixel, q_s = u_s.n_s - c_s. About the
 // mean (u, c) and the direction n_0 from sample 0, |q_s - (u.n_0 - c)| <= max|u_s - u| + max|c_s - c|
 // + max|u_s| |n_s - n_0|, and |n_s - n_0| <= max|D_s| / (R0 - max|D_s|). Writes (u, c) and (the first two
-// terms plus FP32 rounding, max|u_s|, max|D_s|) behind the windows. A row with a sample that
-// is not finite is never skipped (its product with a zero window is NaN). One warp a chirp.
+// terms plus FP32 rounding, max|u_s|, max|D_s|) behind the windows. A row with a sample, or a position
+// of one, that is not finite is never skipped (its product with a zero window is NaN). One warp a
+// chirp.
 __global__ void __launch_bounds__(128)
     window_bounds_kernel(float4 *__restrict__ wins, const float4 *__restrict__ traj, const float2 *__restrict__ xw,
                          int C, int S, int s_pad)
@@ -563,9 +564,10 @@ __global__ void __launch_bounds__(128)
         const float x = w.x - m.x, y = w.y - m.y, z = w.z - m.z;
         du = fmaxf(du, sqrtf(x * x + y * y + z * z));
         dc = fmaxf(dc, fabsf(w.w - m.w));
-        if (traj) dd = fmaxf(dd, sqrtf(sample_table(traj + row, s).w));
+        const float d = traj ? sqrtf(sample_table(traj + row, s).w) : 0.f;
+        dd = fmaxf(dd, d);  // (drops a NaN)
         const float2 v = xw[row + s];
-        bad |= !isfinite(v.x) || !isfinite(v.y) || !isfinite(x + y + z + w.w + dd);
+        bad |= !isfinite(v.x) || !isfinite(v.y) || !isfinite(x + y + z + w.w + d);
     }
     for (int off = 16; off > 0; off >>= 1) {
         du = fmaxf(du, __shfl_xor_sync(0xffffffffu, du, off));
