@@ -1755,7 +1755,7 @@ int focus_resident(tdc_processor *p, float2 *image_dev, cudaStream_t st, int &la
     } else {
         TDC_CK(launch_focus_fp64(jobs_dev, units_dev, n_units, status, job.per_sample, st), "focus kernel (fp64)");
     }
-    TDC_CK(launch_focus_reduce(job.partial, p->plan_groups, P, image_dev, st), "reduce kernel");
+    TDC_CK(launch_focus_reduce(job.partial, p->plan_groups, P, std::max(P, p->plan_pixels), image_dev, st), "reduce kernel");
     launches += 2;
     p->sums_epoch = store ? p->state_epoch : 0;
     p->stats.path = path;

@@ -17,9 +17,8 @@
 // complex multiply-add (4 FFMA) and no separate phasor advance. Block phasors
 // never accumulate more than S/L rotations of an accurately computed QL.
 // Chirp sums are accumulated per pixel with Kahan compensation; partial sums
-// per chirp group are combined in a fixed order, in FP64 by focus_reduce_kernel or in double-float by
-// focus_reduce_sliced_kernel (many groups),
-// so results do not depend on scheduling.
+// per chirp group are combined in a fixed order, as sums of three floats, by focus_reduce_kernel or
+// focus_reduce_sliced_kernel (many groups), so results do not depend on scheduling.
 //
 // Chirp sample rows and trajectory records are staged global->shared with
 // cp.async.bulk on an mbarrier pipeline (kFocusStages deep) and read back as
@@ -876,71 +875,92 @@ __global__ void __launch_bounds__(kFocusThreads, TDC_FOCUS_MINB)
     }
 }
 
-// image[p] = sum over groups of (sum - comp) in double-float, in a fixed order that depends on
-// n_groups alone (relative error below 2^-44 before the rounding to FP32; adding in FP64 gave the
-// same images, but its conversions and adds run at 1/64 rate here: 43 us instead of 10 for 256^2
-// pixels x 29 groups). Eight slices of a block's threads each add a run of groups, 4 loads in flight
-// at a time, and the slices are added in order: small focuses are planned with up to a group per
-// chirp, and one thread adding them one after another waited for a load at a time (whole start()
-// of 480 pixels x 256 chirps x 128 samples 354 -> 229 us with the slices).
-struct DoubleFloat {
-    float h, l;
-    // += x + y
-    __device__ __forceinline__ void add(float x, float y)
+// image[p] = sum over groups of (sum - comp), in an order fixed by the plan (n_groups and the pixels it
+// was made for, so that a row block of a grid adds as the whole grid does), as the sum of three floats: what two_sum leaves of h goes to m, what it leaves of m to l, so that n terms are
+// added to within n^2 2^-74 of the largest partial sum (FP64: n 2^-53; a pair of floats not
+// renormalised: n^2 2^-50, 1e-3 of a result 1e-9 of what cancels in it). FP64 conversions and adds run
+// at 1/64 rate here: 43 us instead of 10 for 256^2 pixels x 29 groups. Sixteen slices of a block's
+// threads each add a run of groups, 4 loads in flight at a time, and the slices are added in order:
+// small focuses are planned with up to a group per chirp, and one thread adding them one after
+// another waited for a load at a time (480 pixels x 256 groups: 12 us with 8 slices, 8 with 16).
+struct TripleFloat {
+    float h = 0.f, m = 0.f, l = 0.f;
+    __device__ __forceinline__ void add(float x)
     {
         float s, e;
         two_sum(h, x, s, e);
-        l += e + y;
         h = s;
+        two_sum(m, e, s, e);
+        m = s;
+        l += e;
     }
-    __device__ __forceinline__ float value() const { return h + l; }
+    __device__ __forceinline__ void add(float oh, float om, float ol)
+    {
+        float s, e;
+        add(oh);
+        two_sum(m, om, s, e);
+        m = s;
+        l += e + ol;
+    }
+    __device__ __forceinline__ float value() const
+    {
+        float s, e;
+        two_sum(h, m, s, e);  // (they may cancel)
+        return s + (e + l);
+    }
 };
 
-constexpr int kReducePixels = 32, kReduceSlices = 8;
+// Slices up to this many pixels: more are threads enough for a pixel each. Whole focuses of 512 groups
+// sliced / not: 64^2 pixels 61 / 108 us, 256 x 64 110 / 118; of 256 groups: 256^2 175 / 168,
+// 512 x 256 306 / 294.
+constexpr long long kReduceSlicedPixels = 40000;
+constexpr int kReducePixels = 32, kReduceSlices = 16;
 __global__ void __launch_bounds__(kReducePixels *kReduceSlices)
     focus_reduce_sliced_kernel(const float4 *__restrict__ partial, int n_groups, long long P,
                                float2 *__restrict__ image, const int *__restrict__ enabled, int want)
 {
     if (enabled && *enabled != want) return;
-    __shared__ float4 part[kReduceSlices][kReducePixels];
+    __shared__ float part[kReduceSlices][6][kReducePixels];
     const long long p = (long long)blockIdx.x * kReducePixels + threadIdx.x;
     const int per = (n_groups + kReduceSlices - 1) / kReduceSlices;
     const int g0 = threadIdx.y * per, g1 = min(n_groups, g0 + per);
-    DoubleFloat re{0.f, 0.f}, im{0.f, 0.f};
+    TripleFloat re, im;
     if (p < P) {
 #pragma unroll 4
         for (int g = g0; g < g1; ++g) {
             const float4 v = __ldg(&partial[(size_t)g * P + p]);
-            re.add(v.x, -v.z);
-            im.add(v.y, -v.w);
+            re.add(v.x, -v.z, 0.f);
+            im.add(v.y, -v.w, 0.f);
         }
     }
-    part[threadIdx.y][threadIdx.x] = make_float4(re.h, im.h, re.l, im.l);
+    const float mine[6] = {re.h, re.m, re.l, im.h, im.m, im.l};
+#pragma unroll
+    for (int v = 0; v < 6; ++v) part[threadIdx.y][v][threadIdx.x] = mine[v];
     __syncthreads();
     if (threadIdx.y == 0 && p < P) {
-#pragma unroll
+        const int x = threadIdx.x;
+#pragma unroll 1
         for (int k = 1; k < kReduceSlices; ++k) {
-            const float4 v = part[k][threadIdx.x];
-            re.add(v.x, v.z);
-            im.add(v.y, v.w);
+            re.add(part[k][0][x], part[k][1][x], part[k][2][x]);
+            im.add(part[k][3][x], part[k][4][x], part[k][5][x]);
         }
         image[p] = make_float2(re.value(), im.value());
     }
 }
 
-// The same for a few groups: one thread a pixel, the groups in order.
+// The same for a few groups or many pixels: one thread a pixel, the groups in order.
 __global__ void focus_reduce_kernel(const float4 *__restrict__ partial, int n_groups, long long P,
                                     float2 *__restrict__ image, const int *__restrict__ enabled, int want)
 {
     if (enabled && *enabled != want) return;
     const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= P) return;
-    DoubleFloat re{0.f, 0.f}, im{0.f, 0.f};
+    TripleFloat re, im;
 #pragma unroll 4
     for (int g = 0; g < n_groups; ++g) {
         const float4 v = __ldg(&partial[(size_t)g * P + p]);
-        re.add(v.x, -v.z);
-        im.add(v.y, -v.w);
+        re.add(v.x, -v.z, 0.f);
+        im.add(v.y, -v.w, 0.f);
     }
     image[p] = make_float2(re.value(), im.value());
 }
@@ -1026,11 +1046,11 @@ cudaError_t launch_focus_fp32_seg(const FocusJob *jobs_dev, const FocusUnit *uni
     return cudaGetLastError();
 }
 
-cudaError_t launch_focus_reduce(const float4 *partial, int n_groups, long long P, float2 *image, cudaStream_t st,
-                                const int *enabled, int want)
+cudaError_t launch_focus_reduce(const float4 *partial, int n_groups, long long P, long long plan_pixels, float2 *image,
+                                cudaStream_t st, const int *enabled, int want)
 {
     if (P <= 0) return cudaSuccess;
-    if (n_groups >= 2 * kReduceSlices) {
+    if (n_groups >= kReduceSlices && plan_pixels <= kReduceSlicedPixels) {
         const long long blocks = (P + kReducePixels - 1) / kReducePixels;
         focus_reduce_sliced_kernel<<<(unsigned)blocks, dim3(kReducePixels, kReduceSlices), 0, st>>>(
             partial, n_groups, P, image, enabled, want);

@@ -354,8 +354,9 @@ int focus_motion_smem_bytes(int stage_bytes);
 // Plain FP64-phase focus (comparator and general fallback), one CTA per unit.
 cudaError_t launch_focus_fp64(const FocusJob *jobs_dev, const FocusUnit *units_dev, int n_units,
                               int *status_dev, int per_sample, cudaStream_t st);
-// (enabled, when given: the launch does nothing unless *enabled == want.)
-cudaError_t launch_focus_reduce(const float4 *partial, int n_groups, long long P, float2 *image,
+// (plan_pixels: pixels of the grid that the groups were planned for; enabled, when given: the launch does
+// nothing unless *enabled == want.)
+cudaError_t launch_focus_reduce(const float4 *partial, int n_groups, long long P, long long plan_pixels, float2 *image,
                                 cudaStream_t st, const int *enabled = nullptr, int want = 0);
 // FP32 general focus (tdc_general.cu). variant bits: 1 per-sample positions, 2 per-sample
 // windows, 4 wide (non-uniform sampling residual, large intra-chirp motion: reduced phase

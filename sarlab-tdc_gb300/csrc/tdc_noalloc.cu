@@ -374,7 +374,7 @@ int enqueue(const tdc_noalloc_focus_args *a, float *image_dev, cudaStream_t st, 
         if (e == cudaSuccess)
             e = launch_focus_profile(1, band, 0, false, pp.job_out, pp.units, n, words + kWordProfileCounter, ctas, st);
         if (e == cudaSuccess)
-            e = launch_focus_reduce(pp.job.partial, pp.n_groups, P, reinterpret_cast<float2 *>(image_dev), st,
+            e = launch_focus_reduce(pp.job.partial, pp.n_groups, P, P, reinterpret_cast<float2 *>(image_dev), st,
                                     words + kWordProfile, 1);
         if (e != cudaSuccess)
             return fail(TDC_ERR_CUDA, std::string("range profile kernels: ") + cudaGetErrorString(e));
@@ -385,7 +385,7 @@ int enqueue(const tdc_noalloc_focus_args *a, float *image_dev, cudaStream_t st, 
                           reinterpret_cast<int *>(base + kOffStatus), reinterpret_cast<int *>(base + kOffStatus) + 1,
                           stage_bytes, grid, std::isfinite(job.half_bw), false, false, st);
     if (e != cudaSuccess) return fail(TDC_ERR_CUDA, std::string("focus kernel: ") + cudaGetErrorString(e));
-    e = launch_focus_reduce(job.partial, n_groups, P, reinterpret_cast<float2 *>(image_dev), st,
+    e = launch_focus_reduce(job.partial, n_groups, P, P, reinterpret_cast<float2 *>(image_dev), st,
                             words + kWordProfile, 0);
     if (e != cudaSuccess) return fail(TDC_ERR_CUDA, std::string("reduce kernel: ") + cudaGetErrorString(e));
     *status_word = reinterpret_cast<int *>(base + kOffStatus) + 1;

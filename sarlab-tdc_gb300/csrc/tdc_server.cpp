@@ -490,7 +490,7 @@ void tdc_server::launch_batch()
     for (Job *j : b.finishing) {
         tdc_processor *p = j->slot;
         const long long P = p->P;
-        err |= launch_focus_reduce(j->plan.job.partial, j->plan.job.n_groups, P, p->image_dev.as<float2>(), st) !=
+        err |= launch_focus_reduce(j->plan.job.partial, j->plan.job.n_groups, P, P, p->image_dev.as<float2>(), st) !=
                cudaSuccess;
         err |= cudaMemcpyAsync(p->image_host.p, p->image_dev.p, (size_t)P * 8, cudaMemcpyDeviceToHost, st) !=
                cudaSuccess;

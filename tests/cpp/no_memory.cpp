@@ -113,7 +113,7 @@ cudaError_t launch_rows_differ(const RowScan *, int, int, int, int *, cudaStream
 cudaError_t launch_tile_radius(const float4 *, const float4 *, long long, int, int, int, int, float *, cudaStream_t) { return launch(); }
 cudaError_t launch_adjoint_fp32(const FocusJob *, const FocusUnit *, int, int *, int *, int, int, int, const float2 *, float4 *, bool, cudaStream_t) { return launch(g_direct); }
 cudaError_t launch_focus_motion(const FocusJob *, const FocusUnit *, int, int *, int *, int, int, bool, cudaStream_t) { return launch(); }
-cudaError_t launch_focus_reduce(const float4 *, int, long long, float2 *, cudaStream_t, const int *, int) { return launch(); }
+cudaError_t launch_focus_reduce(const float4 *, int, long long, long long, float2 *, cudaStream_t, const int *, int) { return launch(); }
 cudaError_t launch_pair_samples(float4 *, long long, cudaStream_t) { return launch(); }
 cudaError_t launch_range_window(float *, int, int, cudaStream_t) { return launch(); }
 cudaError_t launch_focus_general(int, const FocusJob *, const FocusUnit *, int, int *, int *, int, int, cudaStream_t) { return launch(g_direct); }
