@@ -178,12 +178,21 @@ int tdc_range_window(float *w_dev, int n_samples, int apply_range_win, void *str
 int tdc_processor_set_skip_test(tdc_processor *proc, int enable);
 
 /* Plan the chirp groups of the next focuses as for a grid of n_pix pixels (0, default: the
- * resident grid's own count). A pixel's summation order depends only on the chirp groups, so
- * a processor focusing a block of rows of a larger grid gives, with the larger grid's pixel
- * count set here, bit for bit the values a focus of the whole grid gives on the same kind of
- * GPU (pixel sharding across GPUs, sarlabtdc.sharding). Extension without a reference
- * counterpart (the reference binds one GPU, tdcprocessor.cpp:39-55). */
+ * resident grid's own count): a pixel's summation order depends only on them. The kernel, the pixels
+ * that share an anchor and the constants of their series follow the resident grid's geometry
+ * all the same (tdc_processor_set_plan_grid). Extension without a reference counterpart (the
+ * reference binds one GPU, tdcprocessor.cpp:39-55). */
 int tdc_processor_set_plan_pixels(tdc_processor *proc, int64_t n_pix);
+
+/* Plan the next focuses as for a larger grid, of which the grid set by setFocusGrid is a block of
+ * whole rows starting on a multiple of 32 pixels: n_rows x n_cols points, FP32 (grid) or FP64
+ * (grid_f64), the other null; both null: the resident grid's own geometry again. Sets the plan
+ * pixels to n_rows x n_cols, and every choice that depends on a grid's geometry (path, range profiles,
+ * pixels per anchor, series limits) is made for the larger grid, so that the block's values are
+ * bit for bit those of a focus of the whole grid on the same kind of GPU (pixel sharding across
+ * GPUs, sarlabtdc.sharding) where both have the device memory for the same form. The array is
+ * borrowed: start() and tdc_processor_upload_grid read it. Extension without a reference counterpart. */
+int tdc_processor_set_plan_grid(tdc_processor *proc, const float *grid, const double *grid_f64, int n_rows, int n_cols);
 
 /* Smooth-motion path (TDC_PATH_FP32_MOTION) on (1, default) or off (0: such inputs take
  * the FP32 general kernel). Extension without a reference counterpart; takes effect at the

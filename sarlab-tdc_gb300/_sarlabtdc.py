@@ -207,9 +207,24 @@ class TdcProcessor:
         _lib.check(_lib.lib().tdc_processor_set_precision(self._h, code))
 
     def setPlanPixels(self, n_pix: int):
-        """Extension: plan the chirp groups as for a grid of n_pix pixels (0: the grid's own), so
-        a row block of a larger grid focuses bit for bit like that grid (pixel sharding)."""
+        """Extension: plan the chirp groups as for a grid of n_pix pixels (0: the grid's own)."""
         _lib.check(_lib.lib().tdc_processor_set_plan_pixels(self._h, int(n_pix)))
+
+    def setPlanGrid(self, grid):
+        """Extension: plan as for a larger grid [rows, cols, 3] (float64, else taken as float32) of which
+        the focus grid is a block of whole rows starting on a multiple of 32 pixels, so that the block
+        focuses bit for bit like that grid (pixel sharding); None: the grid's own geometry."""
+        g = None
+        if grid is not None:
+            g = np.asarray(grid)
+            g = np.ascontiguousarray(g, dtype=np.float64 if g.dtype == np.float64 else np.float32)
+            if g.ndim != 3 or g.shape[2] != 3:
+                raise RuntimeError("plan grid shape is incorrect")
+        f64 = g is not None and g.dtype == np.float64
+        _lib.check(_lib.lib().tdc_processor_set_plan_grid(
+            self._h, None if g is None or f64 else _lib.ptr(g), _lib.ptr(g) if f64 else None,
+            0 if g is None else int(g.shape[0]), 0 if g is None else int(g.shape[1])))
+        self._plan_grid_ref = g
 
     def setMotionPath(self, enable: bool):
         """Extension: per-sample positions that move smoothly within each chirp take the

@@ -162,6 +162,7 @@ SIGNATURES = [
     ("tdc_processor_set_motion_path", C.c_int, [_vp, C.c_int]),
     ("tdc_processor_set_anchored_ranges", C.c_int, [_vp, C.c_int]),
     ("tdc_processor_set_plan_pixels", C.c_int, [_vp, C.c_int64]),
+    ("tdc_processor_set_plan_grid", C.c_int, [_vp, _vp, _vp, C.c_int, C.c_int]),
     ("tdc_processor_prepare", C.c_int, [_vp, C.c_float, C.c_float, C.c_int, C.c_int, C.c_int]),
     ("tdc_processor_upload_grid", C.c_int, [_vp]),
     ("tdc_processor_focus_device", C.c_int, [_vp, _vp, _vp]),

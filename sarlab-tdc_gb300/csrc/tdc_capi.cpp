@@ -746,6 +746,44 @@ int measure_tile_radii(tdc_processor *p)
     return TDC_OK;
 }
 
+// Device layout of a host grid (FP32 or FP64), on the processor's stream; lo for FP64 only. `stage` holds the
+// host's values where the device does not read them in place.
+int load_grid(tdc_processor *p, const float *grid, const double *grid64, long long P, DevBuf &stage, DevBuf &hi, DevBuf &lo)
+{
+    const size_t elt = grid64 ? 8 : 4;
+    const void *src = grid64 ? (const void *)grid64 : (const void *)grid;
+    TDC_CK(hi.ensure((size_t)P * 16), "alloc grid");
+    if (!p->host_reads) {
+        TDC_CK(stage.ensure((size_t)P * 3 * elt), "alloc grid staging");
+        TDC_CK(cudaMemcpyAsync(stage.p, src, (size_t)P * 3 * elt, cudaMemcpyHostToDevice, p->stream), "copy grid");
+        src = stage.p;
+    }
+    p->stats.h2d_bytes += (int64_t)P * 3 * elt;
+    if (grid64) {
+        TDC_CK(lo.ensure((size_t)P * 16), "alloc grid");
+        TDC_CK(launch_grid_from_f64(static_cast<const double *>(src), P, hi.as<float4>(), lo.as<float4>(), p->stream),
+               "grid kernel");
+    } else {
+        TDC_CK(launch_grid_from_f32(static_cast<const float *>(src), P, hi.as<float4>(), p->stream), "grid kernel");
+    }
+    return TDC_OK;
+}
+
+// Bounding box and anchor span, and the groups' reach, of a device grid in runs of p->grid_run pixels.
+// Waits for the stream.
+int measure_grid(tdc_processor *p, const DevBuf &hi, const DevBuf *lo, long long P, bool reach, GridBounds &b)
+{
+    GridBounds *dev = grid_bounds_dev(p);
+    const float4 *h = hi.as<const float4>(), *l = lo ? lo->as<const float4>() : nullptr;
+    grid_bounds_init(b);
+    TDC_CK(cudaMemcpyAsync(dev, &b, sizeof(b), cudaMemcpyHostToDevice, p->stream), "init bbox");
+    if (reach) TDC_CK(launch_group_reach(h, l, P, p->grid_run, dev->words, p->stream), "reach kernel");
+    TDC_CK(launch_grid_bbox(h, l, P, dev, p->stream), "bbox kernel");
+    TDC_CK(cudaMemcpyAsync(&b, dev, sizeof(b), cudaMemcpyDeviceToHost, p->stream), "read bbox");
+    TDC_CK(cudaStreamSynchronize(p->stream), "grid sync");
+    return TDC_OK;
+}
+
 // Device grid from a host (FP32 or FP64) grid.
 int upload_grid(tdc_processor *p, int &launches)
 {
@@ -755,10 +793,6 @@ int upload_grid(tdc_processor *p, int &launches)
     p->P = P;
     ++p->state_epoch;
     p->plan_path = -1;  // unit spans and costs follow the grid's coordinates
-    cudaStream_t st = p->stream;
-    const size_t elt = p->grid64 ? 8 : 4;
-    TDC_CK(p->grid_hi.ensure((size_t)P * 16), "alloc grid");
-    const void *src = p->grid64 ? (const void *)p->grid64 : (const void *)p->grid;
     {
         auto g = [&](long long i, int k) { return p->grid64 ? p->grid64[3 * i + k] : (double)p->grid[3 * i + k]; };
         for (int k = 0; k < 3; ++k) {
@@ -790,41 +824,34 @@ int upload_grid(tdc_processor *p, int &launches)
                 }
         }
     }
-    if (!p->host_reads) {
-        TDC_CK(p->grid_stage.ensure((size_t)P * 3 * elt), "alloc grid staging");
-        TDC_CK(cudaMemcpyAsync(p->grid_stage.p, src, (size_t)P * 3 * elt, cudaMemcpyHostToDevice, st), "copy grid");
-        src = p->grid_stage.p;
-    }
-    p->stats.h2d_bytes += (int64_t)P * 3 * elt;
-    if (p->grid64) {
-        TDC_CK(p->grid_lo.ensure((size_t)P * 16), "alloc grid");
-        TDC_CK(launch_grid_from_f64(static_cast<const double *>(src), P, p->grid_hi.as<float4>(),
-                                    p->grid_lo.as<float4>(), st),
-               "grid kernel");
-        p->grid_lo_valid = true;
-    } else {
-        TDC_CK(launch_grid_from_f32(static_cast<const float *>(src), P, p->grid_hi.as<float4>(), st), "grid kernel");
-        p->grid_lo_valid = false;
-    }
+    if (int rc = load_grid(p, p->grid, p->grid64, P, p->grid_stage, p->grid_hi, p->grid_lo)) return rc;
+    p->grid_lo_valid = p->grid64 != nullptr;
     launches += 1;
     TDC_CK(p->flag.ensure(128), "alloc flag");
-    p->grid_run = detect_run(
-        P, [&](long long i, int k) { return p->grid64 ? p->grid64[3 * i + k] : (double)p->grid[3 * i + k]; });
+    // What plans follow is measured of the grid they are made for: the resident one, or the larger grid
+    // that it is a block of (row blocks of one grid then take the same forms with the same constants).
+    const bool whole = p->plan_grid || p->plan_grid64;
+    const long long plan_P = whole ? p->plan_grid_pixels : P;
+    const float *pg = whole ? p->plan_grid : p->grid;
+    const double *pg64 = whole ? p->plan_grid64 : p->grid64;
+    p->grid_run = detect_run(plan_P, [&](long long i, int k) { return pg64 ? pg64[3 * i + k] : (double)pg[3 * i + k]; });
     // (small focuses do not ask for the reach: measured when a plan first does)
-    p->reach_known = p->has_raw && profile_pays((double)std::max(P, p->plan_pixels), p->C, p->S, false);
+    p->reach_known = whole || (p->has_raw && profile_pays((double)std::max(P, p->plan_pixels), p->C, p->S, false));
     if (P > 0) {
-        // bounding box, reach and anchor span of the grid, measured on the device
         GridBounds b;
-        grid_bounds_init(b);
-        GridBounds *dev = grid_bounds_dev(p);
-        const float4 *lo = p->grid_lo_valid ? p->grid_lo.as<float4>() : nullptr;
-        TDC_CK(cudaMemcpyAsync(dev, &b, sizeof(b), cudaMemcpyHostToDevice, st), "init bbox");
-        if (p->reach_known)
-            TDC_CK(launch_group_reach(p->grid_hi.as<float4>(), lo, P, p->grid_run, dev->words, st), "reach kernel");
-        TDC_CK(launch_grid_bbox(p->grid_hi.as<float4>(), lo, P, dev, st), "bbox kernel");
-        TDC_CK(cudaMemcpyAsync(&b, dev, sizeof(b), cudaMemcpyDeviceToHost, st), "read bbox");
-        TDC_CK(cudaStreamSynchronize(st), "grid sync");
-        launches += p->reach_known ? 2 : 1;
+        if (int rc = measure_grid(p, p->grid_hi, p->grid_lo_valid ? &p->grid_lo : nullptr, P, p->reach_known && !whole, b))
+            return rc;
+        launches += p->reach_known && !whole ? 2 : 1;
+        for (int k = 0; k < 3; ++k) {
+            p->own_min[k] = pair_value(b.box[k]);
+            p->own_max[k] = pair_value(b.box[3 + k]);
+        }
+        if (whole) {
+            DevBuf stage, hi, lo;  // (given back when the measuring is done)
+            if (int rc = load_grid(p, pg, pg64, plan_P, stage, hi, lo)) return rc;
+            if (int rc = measure_grid(p, hi, pg64 ? &lo : nullptr, plan_P, true, b)) return rc;
+            launches += 3;
+        }
         if (p->reach_known) set_group_reach(p, b.words);
         float span;
         std::memcpy(&span, &b.words[3], 4);
@@ -1310,15 +1337,18 @@ int profile_group(tdc_processor *p, int path, ProfileBuild &b)
     if (!profile_pays((double)P, p->C, p->S, band)) return 0;
     const double g1 = 2.0 * p->F1 / kC0, gc = 2.0 * p->F0 / kC0 + g1 * (p->S / 2);
     b.cells_per_m = 4.0 * p->S * g1;
-    double diag2 = 0.0;
+    // (the table spans the resident grid; whether it fits is decided for the grid planned for)
+    double diag2 = 0.0, own2 = 0.0;
     for (int k = 0; k < 3; ++k) {
-        b.box_min[k] = p->grid_min[k];
-        b.box_max[k] = p->grid_max[k];
+        b.box_min[k] = p->own_min[k];
+        b.box_max[k] = p->own_max[k];
         diag2 += (p->grid_max[k] - p->grid_min[k]) * (p->grid_max[k] - p->grid_min[k]);
+        own2 += (p->own_max[k] - p->own_min[k]) * (p->own_max[k] - p->own_min[k]);
     }
     const double rmax = max_range(p->ant_min, p->ant_max, p->grid_min, p->grid_max);
     if (!(std::fabs(b.cells_per_m) * rmax < 2097152.0) || !(diag2 >= 0.0) || !(std::fabs(gc) > 0.0)) return 0;
-    b.n_cells = profile_cells(b.cells_per_m, std::sqrt(diag2));
+    int plan_cells = profile_cells(b.cells_per_m, std::sqrt(diag2));
+    b.n_cells = std::min(plan_cells, profile_cells(b.cells_per_m, std::sqrt(own2)));
     b.margin = 0;
     b.chirp_words = 3;
     const bool vibration = path == TDC_PATH_GENERAL;
@@ -1351,6 +1381,7 @@ int profile_group(tdc_processor *p, int path, ProfileBuild &b)
         if (band || !(bend <= kMoveMaxBend) || !(shift <= 64.0) || !(third <= kMoveMaxThird)) return 0;
         b.margin = 2 * (int)std::ceil(0.5 * shift) + 2;
         b.n_cells += 2 * b.margin;
+        plan_cells += 2 * b.margin;
         b.chirp_words = vibration ? 6 : 4;
         if (vibration) {
             b.traj = p->traj.as<const float4>();
@@ -1360,7 +1391,7 @@ int profile_group(tdc_processor *p, int path, ProfileBuild &b)
         slack = shift;
         max_bend = bend;
     }
-    if (b.n_cells > 4LL * p->S || !profile_table_fits(b.n_cells, p->S, p->table_ratio)) return 0;
+    if (plan_cells > 4LL * p->S || !profile_table_fits(plan_cells, p->S, p->table_ratio)) return 0;
     b.C = p->C;
     b.S = p->S;
     b.s_pad = p->s_pad;
@@ -2002,6 +2033,19 @@ int tdc_processor_set_plan_pixels(tdc_processor *p, int64_t n_pix)
     if (int rc = check_proc(p)) return rc;
     if (n_pix < 0) return fail(TDC_ERR_INVALID_ARGUMENT, "n_pix must not be negative");
     p->plan_pixels = n_pix;
+    return TDC_OK;
+}
+
+int tdc_processor_set_plan_grid(tdc_processor *p, const float *grid, const double *grid_f64, int n_rows, int n_cols)
+{
+    if (int rc = check_proc(p)) return rc;
+    if (n_rows < 0 || n_cols < 0) return fail(TDC_ERR_INVALID_ARGUMENT, "negative grid shape");
+    if (grid && grid_f64) return fail(TDC_ERR_INVALID_ARGUMENT, "two plan grids");
+    const bool any = (grid || grid_f64) && (long long)n_rows * n_cols > 0;
+    p->plan_grid = any ? grid : nullptr;
+    p->plan_grid64 = any ? grid_f64 : nullptr;
+    p->plan_grid_pixels = any ? (long long)n_rows * n_cols : 0;
+    p->plan_pixels = p->plan_grid_pixels;
     return TDC_OK;
 }
 

@@ -188,7 +188,10 @@ struct tdc_processor {
     // Device grid.
     long long P = 0;
     bool grid_lo_valid = false;
+    // Boxes: of the grid that focuses are planned for (plan_grid, else the resident one), which paths and
+    // forms are chosen by, and of the resident grid.
     double grid_min[3] = {0, 0, 0}, grid_max[3] = {0, 0, 0};
+    double own_min[3] = {0, 0, 0}, own_max[3] = {0, 0, 0};
     double axis_c[3] = {0, 0, 0}, axis_r[3] = {0, 0, 0};  // grid column / row steps (first pixel's)
     // Anchored ranges of the FP32-bulk kernel: the largest distance of a pixel from the anchor
     // of its group of 32 consecutive pixels (the group's 17th pixel, or its last); the kernel
@@ -232,6 +235,10 @@ struct tdc_processor {
     double plan_unit_cap = 0.0;
     long long plan_tiles = -1;   // tiles the chirp groups were planned for
     long long plan_pixels = 0;   // plan the chirp groups for a grid of this many pixels (0: the grid's own)
+    // Borrowed: the grid whose geometry plans follow (the resident grid is a block of its rows); null: own.
+    const float *plan_grid = nullptr;
+    const double *plan_grid64 = nullptr;
+    long long plan_grid_pixels = 0;
     bool plan_uploaded = false;
 
     // Adjoint (autofocus) scratch.

@@ -8,12 +8,13 @@ moving between ranks, and the blocks are gathered once at the end. The work is s
 with no collective on the data path: the gather moves only the finished image (8 bytes a
 pixel).
 
-Each rank plans its chirp groups for the whole grid's pixel count
-(``TdcProcessor.setPlanPixels``), and every block starts on a multiple of 32 pixels (the
-engine's anchored ranges share an anchor among up to 32 consecutive pixels of a grid). A
-pixel's arithmetic then depends only on the chirp groups and its own group of 32 pixels, so
-on GPUs of one kind the gathered image equals a single-GPU focus of the whole grid bit for
-bit.
+Each rank plans for the whole grid: its chirp groups for the whole grid's pixel count
+(``TdcProcessor.setPlanPixels``), and what depends on a grid's geometry, which kernel runs and
+which pixels share an anchor, from the whole grid (``setPlanGrid``). Every block starts on a
+multiple of 32 pixels (anchors are shared among up to 32 consecutive pixels of a grid). A
+pixel's arithmetic then depends only on the chirp groups and its own group of 32 pixels, so on
+GPUs of one kind, with the memory for the same plan, the gathered image equals a single-GPU
+focus of the whole grid bit for bit.
 """
 from __future__ import annotations
 
@@ -122,12 +123,14 @@ class ShardedProcessor:
         self.shape = (n_rows, n_cols)
         setter(np.ascontiguousarray(g[r0:r1]))
         self.proc.setPlanPixels(n_rows * n_cols)
+        if hasattr(self.proc, "setPlanGrid"):  # (the engine)
+            self.proc.setPlanGrid(g)
 
     def setFocusGrid(self, focusGrid):
-        self._set_grid(focusGrid, self.proc.setFocusGrid)
+        self._set_grid(np.asarray(focusGrid, np.float32), self.proc.setFocusGrid)
 
     def setFocusGridF64(self, focusGrid):
-        self._set_grid(focusGrid, self.proc.setFocusGridF64)
+        self._set_grid(np.asarray(focusGrid, np.float64), self.proc.setFocusGridF64)
 
     def start(self, dopplerWinCenter, dopplerBandwidth, dopCentroidWin, applyRangeWin, dopplerWinTaper=True):
         self.proc.start(dopplerWinCenter, dopplerBandwidth, dopCentroidWin, applyRangeWin, dopplerWinTaper)
