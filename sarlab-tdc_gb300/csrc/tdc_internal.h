@@ -377,7 +377,8 @@ int focus_general_smem_bytes(int stage_bytes);
 // Range profiles: the per-length constants (twiddle [S][kProfileNodes], factor [S]), the table
 // of the resident acquisition over the grid's ranges, and the focus that reads it, with
 // `group` (8, 4, 2 or 1) consecutive pixels sharing an anchor (band: a finite Doppler band).
-cudaError_t launch_profile_twiddle(float2 *twiddle, float *factor, int S, cudaStream_t st);
+// (enabled, when given: nothing where *enabled is 0)
+cudaError_t launch_profile_twiddle(float2 *twiddle, float *factor, int S, cudaStream_t st, const int *enabled = nullptr);
 cudaError_t launch_profile_build(const ProfileBuild &b, cudaStream_t st);
 // The same with its inputs in device memory, of at most max_cells cells; nothing where *enabled is 0.
 cudaError_t launch_profile_build_indirect(const ProfileBuild *dev, const int *enabled, int C, int S, int max_cells,

@@ -366,7 +366,8 @@ int enqueue(const tdc_noalloc_focus_args *a, float *image_dev, cudaStream_t st, 
             e = cudaGetLastError();
         }
         if (e == cudaSuccess)
-            e = launch_profile_twiddle(const_cast<float2 *>(pp.build.twiddle), const_cast<float *>(pp.build.factor), S, st);
+            e = launch_profile_twiddle(const_cast<float2 *>(pp.build.twiddle), const_cast<float *>(pp.build.factor), S, st,
+                                       words + kWordProfile);
         if (e == cudaSuccess)
             e = launch_profile_build_indirect(pp.build_out, words + kWordProfile, C, S, pp.max_cells, st);
         const int n = pp.n_tiles * pp.n_groups;

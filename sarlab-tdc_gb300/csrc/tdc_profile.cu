@@ -110,8 +110,10 @@ ProfileStencil make_stencil()
 // Per-length constants: phasors e^{j 2 pi n (s - sc) / (2 S)} for the nodes of one CTA
 // ([S][kNodes]) and the samples' factors 1 / phi^ (the Kaiser-Bessel kernel's transform at the
 // sample's frequency in node units).
-__global__ void profile_twiddle_kernel(float2 *__restrict__ tw, float *__restrict__ factor, int S)
+__global__ void profile_twiddle_kernel(float2 *__restrict__ tw, float *__restrict__ factor, int S,
+                                       const int *__restrict__ enabled)
 {
+    if (enabled && *enabled == 0) return;
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= (long long)S * kNodes) return;
     const int s = (int)(i / kNodes), n = (int)(i - (long long)s * kNodes);
@@ -1547,10 +1549,10 @@ __global__ void __launch_bounds__(kThreads, focus_ctas(G, BAND, ADJ, MOVE))
 
 }  // namespace
 
-cudaError_t launch_profile_twiddle(float2 *twiddle, float *factor, int S, cudaStream_t st)
+cudaError_t launch_profile_twiddle(float2 *twiddle, float *factor, int S, cudaStream_t st, const int *enabled)
 {
     const long long n = (long long)S * kNodes;
-    profile_twiddle_kernel<<<(unsigned)((n + 127) / 128), 128, 0, st>>>(twiddle, factor, S);
+    profile_twiddle_kernel<<<(unsigned)((n + 127) / 128), 128, 0, st>>>(twiddle, factor, S, enabled);
     return cudaGetLastError();
 }
 

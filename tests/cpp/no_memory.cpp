@@ -127,7 +127,7 @@ cudaError_t launch_focus_fp32_seg(const FocusJob *, const FocusUnit *, int, int 
 cudaError_t launch_prewindow_from(const float2 *, const float *, int, int, int, float2 *, cudaStream_t) { return launch(); }
 cudaError_t launch_adjoint_profile(int, bool, bool, const FocusJob *, const FocusUnit *, int, int *, int, const float2 *, float4 *, cudaStream_t) { return launch(g_profile); }
 cudaError_t launch_chirp_positions(ChirpRec *, const double *, const double *, int, cudaStream_t) { return launch(); }
-cudaError_t launch_profile_twiddle(float2 *, float *, int, cudaStream_t) { return launch(); }
+cudaError_t launch_profile_twiddle(float2 *, float *, int, cudaStream_t, const int *) { return launch(); }
 int focus_fp32_blocks_per_sm(int) { return 3; }
 int adjoint_fp32_blocks_per_sm(int, int, bool) { return 3; }
 int focus_motion_blocks_per_sm(int) { return 3; }
