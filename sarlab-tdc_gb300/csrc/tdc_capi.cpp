@@ -1296,6 +1296,11 @@ bool profile_pays(double n_pix, double n_pri, double n_samples, bool band)
     return n_pix >= 4.0 * n_samples && n_pix * n_pri * n_samples >= (band ? 5e8 : TDC_PROFILE_MIN_WORK);
 }
 
+// Every pixel its own range: about 9 ps a pair, more than the direct sum of a few samples. 1024^2 shuffled
+// pixels x 1024 chirps, direct / profiles: 16 samples 8.4 / 9.1 ms, 32 10.5 / 9.1; under 8 Hz 16 3.8 /
+// 4.7, 32 4.5 / 4.7, 64 (512 x 1024 pixels) 7.3 / 6.8.
+bool profile_own_pays(int n_samples, bool band) { return n_samples > (band ? 32 : 16); }
+
 // Vibration through range profiles [rad]: largest carrier phase of the deviations from constant
 // velocity (their series leaves 5e-7 at 0.1), of their part off the chirp's principal direction
 // (kept to first order), of the range's second order (kept at the middle carrier), and of the
@@ -1402,7 +1407,8 @@ int profile_group(tdc_processor *p, int path, ProfileBuild &b)
     }
     if (!p->reach_known && !measured(measure_group_reach(p))) return 0;
     if (!std::isfinite(p->group_reach[0])) return 0;
-    if (!p->anchor_enabled) return 1;
+    const int own = path != TDC_PATH_FP32_BULK || profile_own_pays(p->S, band) ? 1 : 0;
+    if (!p->anchor_enabled) return own;
     // 16 pixels a thread and anchor on runs parallel to an axis, once half as many threads are enough: whole
     // focus at 16 / 8, 1 mm grids x 256 samples: 17 M pairs (256^2 x 256) 84 / 76 us, 67 M (256^2 x 1024) 145 /
     // 158, 67 M (512^2 x 256) 152 / 156, 300 M (600 x 500 x 1000) 441 / 533, 1074 M (512^2 x 4096) 1397 /
@@ -1421,7 +1427,7 @@ int profile_group(tdc_processor *p, int path, ProfileBuild &b)
             continue;
         if (std::fabs(b.cells_per_m) * reach + slack * turn <= kProfileReach - 0.52) return 8 >> k;
     }
-    return 1;
+    return own;
 }
 
 // Runs parallel to an axis whose groups span few carrier cycles (kernels with LINE).

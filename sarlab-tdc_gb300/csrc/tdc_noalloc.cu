@@ -301,7 +301,8 @@ int enqueue(const tdc_noalloc_focus_args *a, float *image_dev, cudaStream_t st, 
     // ---- range profiles, where the call is large enough and a table may fit ----
     const bool band = std::isfinite(job.half_bw);
     ProfilePlan pp{};
-    bool profile = impl::profile_pays((double)P, C, S, band) && (band || job.half_bw > 0.0f);
+    bool profile = impl::profile_pays((double)P, C, S, band) && impl::profile_own_pays(S, band) &&
+                   (band || job.half_bw > 0.0f);
     if (profile) {
         const double gc = a->g0 + a->g1 * (S / 2), cells_per_m = 4.0 * S * a->g1;
         const int tiles = (int)profile_tiles(P, (int)std::min<long long>(P, 1 << 30));

@@ -324,6 +324,8 @@ constexpr double kProfilePairCost = 14.0;
 // (table_ratio: the largest table taken, in bytes per byte of samples; 0: no limit.)
 bool profile_table_fits(int n_cells, int n_samples, double table_ratio);
 bool profile_pays(double n_pix, double n_pri, double n_samples, bool band);
+// The same where every pixel is its own anchor (direct kernels, FP32-bulk path).
+bool profile_own_pays(int n_samples, bool band);
 int profile_cells(double cells_per_m, double diagonal);
 template <class Get>
 int detect_run(long long P, const Get &g)
