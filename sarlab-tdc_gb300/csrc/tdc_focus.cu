@@ -879,8 +879,8 @@ __global__ void __launch_bounds__(kFocusThreads, TDC_FOCUS_MINB)
 // was made for, so that a row block of a grid adds as the whole grid does), as the sum of three floats: what two_sum leaves of h goes to m, what it leaves of m to l, so that n terms are
 // added to within n^2 2^-74 of the largest partial sum (FP64: n 2^-53; a pair of floats not
 // renormalised: n^2 2^-50, 1e-3 of a result 1e-9 of what cancels in it). FP64 conversions and adds run
-// at 1/64 rate here: 43 us instead of 10 for 256^2 pixels x 29 groups. Sixteen slices of a block's
-// threads each add a run of groups, 4 loads in flight at a time, and the slices are added in order:
+// at 1/64 rate here: 43 us instead of 10 for 256^2 pixels x 29 groups. Sixteen or eight slices of a
+// block's threads each add a run of groups, 4 loads in flight at a time, and the slices are added in order:
 // small focuses are planned with up to a group per chirp, and one thread adding them one after
 // another waited for a load at a time (480 pixels x 256 groups: 12 us with 8 slices, 8 with 16).
 struct TripleFloat {
@@ -910,19 +910,21 @@ struct TripleFloat {
     }
 };
 
-// Slices up to this many pixels: more are threads enough for a pixel each. Whole focuses of 512 groups
+// Slices up to kReduceSlicedPixels: more are threads enough for a pixel each. Whole focuses of 512 groups
 // sliced / not: 64^2 pixels 61 / 108 us, 256 x 64 110 / 118; of 256 groups: 256^2 175 / 168,
-// 512 x 256 306 / 294.
-constexpr long long kReduceSlicedPixels = 40000;
+// 512 x 256 306 / 294. Eight slices from kReduceFewPixels on: 16 / 8, 480 pixels x 256 groups 21.4 / 23.4 us,
+// 14,616 x 142 46.8 / 44.8, 29,970 x 124 48.1 / 45.6.
+constexpr long long kReduceSlicedPixels = 40000, kReduceFewPixels = 8192;
 constexpr int kReducePixels = 32, kReduceSlices = 16;
-__global__ void __launch_bounds__(kReducePixels *kReduceSlices)
+template <int SLICES>
+__global__ void __launch_bounds__(kReducePixels *SLICES)
     focus_reduce_sliced_kernel(const float4 *__restrict__ partial, int n_groups, long long P,
                                float2 *__restrict__ image, const int *__restrict__ enabled, int want)
 {
     if (enabled && *enabled != want) return;
-    __shared__ float part[kReduceSlices][6][kReducePixels];
+    __shared__ float part[SLICES][6][kReducePixels];
     const long long p = (long long)blockIdx.x * kReducePixels + threadIdx.x;
-    const int per = (n_groups + kReduceSlices - 1) / kReduceSlices;
+    const int per = (n_groups + SLICES - 1) / SLICES;
     const int g0 = threadIdx.y * per, g1 = min(n_groups, g0 + per);
     TripleFloat re, im;
     if (p < P) {
@@ -940,7 +942,7 @@ __global__ void __launch_bounds__(kReducePixels *kReduceSlices)
     if (threadIdx.y == 0 && p < P) {
         const int x = threadIdx.x;
 #pragma unroll 1
-        for (int k = 1; k < kReduceSlices; ++k) {
+        for (int k = 1; k < SLICES; ++k) {
             re.add(part[k][0][x], part[k][1][x], part[k][2][x]);
             im.add(part[k][3][x], part[k][4][x], part[k][5][x]);
         }
@@ -1052,8 +1054,13 @@ cudaError_t launch_focus_reduce(const float4 *partial, int n_groups, long long P
     if (P <= 0) return cudaSuccess;
     if (n_groups >= kReduceSlices && plan_pixels <= kReduceSlicedPixels) {
         const long long blocks = (P + kReducePixels - 1) / kReducePixels;
-        focus_reduce_sliced_kernel<<<(unsigned)blocks, dim3(kReducePixels, kReduceSlices), 0, st>>>(
-            partial, n_groups, P, image, enabled, want);
+        if (plan_pixels < kReduceFewPixels)
+            focus_reduce_sliced_kernel<kReduceSlices><<<(unsigned)blocks, dim3(kReducePixels, kReduceSlices), 0, st>>>(
+                partial, n_groups, P, image, enabled, want);
+        else
+            focus_reduce_sliced_kernel<kReduceSlices / 2>
+                <<<(unsigned)blocks, dim3(kReducePixels, kReduceSlices / 2), 0, st>>>(partial, n_groups, P, image, enabled,
+                                                                                       want);
         return cudaGetLastError();
     }
     const int threads = 256;

@@ -16,7 +16,9 @@ pytestmark = pytest.mark.gpu
 INF = float("inf")
 
 
-@pytest.mark.parametrize("nx,ny,half", [(8, 8, 200), (33, 1, 100), (40, 12, 6), (31, 1, 7)])
+@pytest.mark.parametrize("nx,ny,half", [(8, 8, 200), (33, 1, 100), (40, 12, 6), (31, 1, 7),
+                                        (128, 66, 150),    # eight slices
+                                        (210, 195, 30)])   # many pixels: a thread each
 def test_opposite_chirps_cancel(cuda_device, nx, ny, half):
     n_pri = 2 * half + 1
     sc = scenes.small_scene(seed=nx + half, n_pri=n_pri, n_samples=64, nx=nx, ny=ny, device="cuda")
