@@ -145,7 +145,7 @@ typedef struct tdc_start_stats {
     int adjoint_stored;   /* the last adjoint read the kept per-chirp sums (1) or recomputed them (0) */
     int motion_segment;   /* smooth-motion path: samples per linearised segment; 0 on the other paths */
     int anchor_pixels;    /* FP32-bulk path with anchored ranges: consecutive pixels sharing one anchor
-                             (32; 8, 4 or 2 through range profiles); 0 when every pixel's range is formed
+                             (32; 16, 8, 4 or 2 through range profiles); 0 when every pixel's range is formed
                              in double-float */
     int span_permille;    /* chirps the work units visit, per mille of tiles x chirps: below 1000 when a
                              finite Doppler band lets units skip chirps out of band for their whole tile */
@@ -215,8 +215,9 @@ int tdc_processor_set_motion_path(tdc_processor *proc, int enable);
  * multiple of 32 pixels, or narrower than 5 cm, at up to 3 mm spacing), which keeps each
  * (pixel, chirp) phase within about 3e-5 rad of the per-pixel double-float range's at 77 GHz
  * (1e-5 rad on 1 mm grids). Through range profiles groups of 8, 4 or 2 consecutive pixels of a
- * row share an anchor, the largest that stays within one range cell of it. Off: every (pixel, chirp) range in double-float. Extension without
- * a reference counterpart; takes effect at the next focus. */
+ * row share an anchor, the largest that stays within one range cell of it, or 16 in large focuses of
+ * rows parallel to an axis under an unbounded band. Off: every (pixel, chirp) range in double-float.
+ * Extension without a reference counterpart; takes effect at the next focus. */
 int tdc_processor_set_anchored_ranges(tdc_processor *proc, int enable);
 
 /*

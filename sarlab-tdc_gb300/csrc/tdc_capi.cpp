@@ -1284,10 +1284,11 @@ bool anchor_eligible(const tdc_processor *p, int cb)
 // and a launch large enough for one more kernel. Whole focus, direct / profiles, 2 mm grids: at
 // 0.54 Gcorr 140 / 66 us (128^2 pixels x 128 chirps x 256 samples), 173 / 71 (256^2 x 128 x 64),
 // 144 / 69 (64^2 x 512 x 256); at 0.27 Gcorr 106 / 63 (128^2 x 128 x 128), 74 / 67 (64^2 x 256 x
-// 256); at 0.03 Gcorr 40 / 50. Below the line the gain is at most 50 us, and callers that choose
-// between anchored and double-float ranges keep the direct kernels. 64^2 pixels = 4 x 1024
-// samples, 1024 chirps: 601 / 102. Under a finite band the line is at 0.5 Gcorr: callers that read
-// the direct kernel's block tiles and unit spans do so at 0.47 (there 490-530 / 66-78 us).
+// 256); at 0.03 Gcorr 40 / 50; under a finite band at 0.47 Gcorr 490-530 / 66-78. The lines at 0.3 and
+// 0.5 Gcorr are not the break-even, which lies near 0.13 (50 / 59), nor is 4 pixels a sample (64^2 pixels
+// = 4 x 1024 samples, 1024 chirps: 601 / 102): below them a focus keeps the direct kernels and what it
+// reports of their plans (anchors of 32 pixels, block tiles, unit spans), which callers and tests rely on
+// at up to 0.30 Gcorr, 0.47 under a band.
 #ifndef TDC_PROFILE_MIN_WORK
 #define TDC_PROFILE_MIN_WORK 3e8
 #endif
@@ -1309,13 +1310,13 @@ constexpr double kVibMaxPhase = 0.1, kVibMaxSide = 5e-4, kVibMaxBow = 3e-5, kVib
 
 // Smooth motion through range profiles: largest bend of the phase at a row's ends [rad].
 constexpr double kMoveMaxBend = 0.1;
-// Groups of 16: ranges of at least this many reaches take the short series of the range difference; focuses
-// of at least this many pixels x chirps.
-constexpr double kWideRange = 21.0, kWideMinPairs = 6e7;
 // ... of the phase's third order there (left out, weighted by s~^3) [rad],
 constexpr double kMoveMaxThird = 8e-6;
 // ... and of the bend's difference within a group [rad] (the neglected second order is half its square).
 constexpr double kMoveMaxTurn = 2e-3;
+// Groups of 16: ranges of at least this many reaches take the short series of the range difference; focuses
+// of at least this many pixels x chirps.
+constexpr double kWideRange = 21.0, kWideMinPairs = 6e7;
 
 bool profile_table_fits(int n_cells, int n_samples, double table_ratio)
 {

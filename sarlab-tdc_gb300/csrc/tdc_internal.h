@@ -376,7 +376,8 @@ int focus_general_smem_bytes(int stage_bytes);
 
 // Range profiles: the per-length constants (twiddle [S][kProfileNodes], factor [S]), the table
 // of the resident acquisition over the grid's ranges, and the focus that reads it, with
-// `group` (8, 4, 2 or 1) consecutive pixels sharing an anchor (band: a finite Doppler band).
+// `group` (16, 8, 4, 2 or 1) consecutive pixels sharing an anchor (band: a finite Doppler band; line: runs
+// parallel to an axis, the only form with 16).
 // (enabled, when given: nothing where *enabled is 0)
 cudaError_t launch_profile_twiddle(float2 *twiddle, float *factor, int S, cudaStream_t st, const int *enabled = nullptr);
 cudaError_t launch_profile_build(const ProfileBuild &b, cudaStream_t st);

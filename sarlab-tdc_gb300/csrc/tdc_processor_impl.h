@@ -199,7 +199,7 @@ struct tdc_processor {
     double anchor_span = 0.0;
     bool anchor_enabled = true;
     // Range profiles (tdc_profile.cu): consecutive pixels without a jump (a grid row), the reach of
-    // the groups of 8 / 4 / 2 pixels sharing an anchor, the table and the per-length constants.
+    // the groups of 16 / 8 / 4 / 2 pixels sharing an anchor, the table and the per-length constants.
     int grid_run = 1;
     double group_reach[3] = {0, 0, 0}, reach16 = 0;
     int run_axis = -1;         // axis the runs are parallel to, or -1
@@ -275,7 +275,7 @@ struct FocusPlan {
     int stage_bytes = 0;  // bytes per pipeline stage
     int slots = 0;        // resident CTAs of the kernel on the device
     bool anchored = false;  // FP32-bulk kernel with anchored ranges
-    int profile = 0;      // FP32-bulk focus through range profiles: pixels sharing an anchor (8, 4, 2, 1); else 0
+    int profile = 0;      // focus through range profiles: pixels sharing an anchor (16, 8, 4, 2, 1); else 0
     ProfileBuild build{};  // its table (profile > 0)
     bool line = false;     // ... through the kernels for runs parallel to an axis
     size_t off_job = 0;   // job record and unit table offsets in the processor's scratch

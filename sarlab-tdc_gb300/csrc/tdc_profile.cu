@@ -19,7 +19,7 @@
 // polynomial together: <= 2e-7 rms of a row's norm at |t| = 1.5, 1e-8 within the cell.
 //
 // Whole focus, direct kernels -> profiles (GB300, resident acquisition): 1024^2 pixels x 4096
-// chirps x 1024 samples 532 -> 5.27 ms; 1.05 M voxels x 16,384 x 256 587 -> 19.8 ms; 256^2 x 1024 x
+// chirps x 1024 samples 532 -> 5.32 ms; 1.05 M voxels x 16,384 x 256 587 -> 20.1 ms; 256^2 x 1024 x
 // 512 4.5 -> 0.164 ms; 256^2 x 64 x 12,345 6.5 -> 0.100 ms.
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -887,8 +887,9 @@ constexpr int focus_ctas(int group, bool band, bool adjoint, int motion)
 //   Q = gc (R^2 - R0^2) / (2 R0) = d.e' + |d|^2 h     (d = pixel - anchor, 4 operations),
 //   psi = Q (1 + b1 Q + b2 Q^2 + b3 Q^3)              (sqrt(1 + y) - 1, y = Q k2 small),
 // where y is small (|y| <= 0.061, reach / R0 <= 0.03), or from the exact
-// quotient otherwise, and the cell's polynomial at t0 + psi x cells per cycle. About 36
-// operations a pixel and chirp plus 100 per anchor, whatever the row's length.
+// quotient otherwise, and the cell's polynomial at t0 + psi x cells per cycle. About 28
+// operations a pixel and chirp on runs along an axis, 33 off it, plus 110 per anchor, whatever the
+// row's length.
 //
 // Bound: the FMA pipe (72% busy, 61% of the issue slots, on 512^2 x 2048 x 1024). What brought it
 // there, 1024^2 x 4096 x 1024 each: scalar FMAs 9.6 ms; pairs of pixels in FFMA2 (half the issue
@@ -919,7 +920,7 @@ constexpr int focus_ctas(int group, bool band, bool adjoint, int motion)
 // B = s~^2 A (in units of the half row) and so on, e^{j eps s~^2} A = A + j eps B - eps^2 / 2 C
 // - j eps^3 / 6 E, all polynomials of the cell formed once an anchor; the pixel's difference in
 // eps from its anchor, at most a few per cent of it, enters to first order. 64 x 512 pixels x 512
-// chirps x 1024 samples: 2.64 ms in the per-segment kernel of tdc_motion.cu, 0.21 ms here.
+// chirps x 1024 samples: 2.64 ms in the per-segment kernel of tdc_motion.cu, 0.092 ms here.
 //
 // MOVE = 2: vibration about a constant velocity, rho_s = P[c, s] minus the chirp's line. Its phase is
 // psi_s = u.phi_s (u = e / R the direction of the antenna, phi = 2 pi g_s rho, at most 0.1 rad), so
@@ -930,7 +931,7 @@ constexpr int focus_ctas(int group, bool band, bool adjoint, int motion)
 // polynomial; the direction turning along the chirp (W1 / R) enters through the derivative of
 // the phi tables, a pixel's own direction as the polynomial's gradient in u, to first order.
 // 151 x 97 pixels x 333 chirps x 500 samples: 1930 us in the general kernel of tdc_general.cu, which
-// corrects every sample, 92 us here (40 the six tables, 50 this kernel).
+// corrects every sample, 94 us here (40 the six tables, 52 this kernel).
 //
 // LINE: every group's pixels lie on a line parallel to one axis (sP.axis; checked when the grid is
 // measured: the offsets along the others are exactly zero) and span at most kLineMaxCycles carrier
